@@ -181,6 +181,82 @@ def run(s):
     return s["op"](s["q"], s["k"], s["v"])
 
 
+def _attend(q, k, v, scale, visible=None, bias=None):
+    """softmax(scale Q K^T + bias) V in 64 bits, one (image, KV head) and a run of query rows at a time."""
+    B, Sq, Hq, D = q.shape
+    Sk, Hkv = k.shape[1], k.shape[2]
+    out = torch.empty(B, Sq, Hq, D, dtype=torch.float64, device=q.device)
+    rows = max(1, min(Sq, (1 << 27) // (Sk * (Hq // Hkv))))
+    for b in range(B):
+        for h in range(Hkv):
+            heads = slice(h * (Hq // Hkv), (h + 1) * (Hq // Hkv))
+            kt, vv = k[b, :, h].double().t().contiguous(), v[b, :, h].double()
+            for r in range(0, Sq, rows):
+                s = torch.matmul(q[b, r:r + rows, heads].double().transpose(0, 1), kt).mul_(scale)  # [heads, rows, Sk]
+                if bias is not None:
+                    s += bias[r:r + rows].double()
+                if visible is not None:
+                    i = torch.arange(r, r + s.shape[1], device=q.device)[:, None]
+                    s.masked_fill_(~visible(i, torch.arange(Sk, device=q.device)), -math.inf)
+                out[b, r:r + rows, heads] = torch.matmul(torch.softmax(s, dim=-1), vv).transpose(0, 1)
+    return out
+
+
+def _rotate(x, table):
+    """Pairs of dimensions as complex numbers times cos + i sin."""
+    x, t = x.unflatten(-1, (-1, 2)), table.double().unflatten(-1, (-1, 2))
+    re = x[..., 0] * t[..., 0] - x[..., 1] * t[..., 1]
+    im = x[..., 0] * t[..., 1] + x[..., 1] * t[..., 0]
+    return torch.stack([re, im], dim=-1).flatten(-2)
+
+
+def _rms(x, weight, dims):
+    return x if weight is None else x * torch.rsqrt((x * x).mean(dim=dims, keepdim=True) + 1e-6) * weight.double()
+
+
+def exact(case, seed):
+    """What `run` returns, in 64 bits from the same inputs."""
+    if work(case)["flops"] > 3e13:  # the 720p clip: minutes of 64-bit arithmetic
+        return None
+    s, kind, D = prepare(case, seed), case["kind"], case["D"]
+    if kind in ("self", "cross"):
+        return _attend(s["q"], s["k"], s["v"], D ** -0.5)
+    if kind in ("prefill", "decode"):
+        past = s["k"].shape[1] - s["q"].shape[1]
+        return _attend(s["q"], s["k"], s["v"], D ** -0.5, lambda i, j: j <= i + past)
+    if kind == "masked":
+        return _attend(s["q"], s["k"], s["v"], D ** -0.5, (lambda i, j: j <= i) if case["causal"] else None, s["mask"][0, 0])
+    if kind == "projected":
+        op = s["op"]
+        return _attend(s["q"], s["k"], s["v"], D ** -0.5).flatten(2) @ op.weight.double().t() + op.bias.double()
+    if kind == "step":
+        table = s["rotary"].view(1, 1, 1, D)
+        q = _rotate(_rms(s["q"].double(), s["q_norm_weight"], -1), table)
+        k, v = s["k_cache"].double(), s["v_cache"].double()
+        k[:, s["cached"]:] = _rotate(_rms(s["k_new"].double(), s["k_norm_weight"], -1), table)
+        v[:, s["cached"]:] = s["v_new"].double()
+        return {"out": _attend(q, k, v, D ** -0.5), "k_cache": k, "v_cache": v}
+    if kind == "prologue":
+        outs = []
+        for x, w in ((s["q"], s["q_weight"]), (s["k"], s["k_weight"])):
+            n = _rms(x.double().flatten(2), w, -1).view(x.shape) if s["per_token"] else _rms(x.double(), w, -1)
+            outs.append(_rotate(n, s["rotary"]) * s["post_scale"])
+        return tuple(outs)
+    q, raw, comp, selected = s["q"][0].double(), s["raw"][0, :, 0].double(), s["comp"][0, :, 0].double(), s["selected"].long()
+    Sq, Sr, W = case["Sq"], case["Sr"], case["W"]
+    out, sinks = torch.empty_like(q), s["sinks"].double().reshape(-1, 1)
+    for r in range(0, Sq, 128):
+        own = torch.arange(Sr - Sq + r, Sr - Sq + min(Sq, r + 128), device=q.device)[:, None]
+        near = own - torch.arange(min(W, Sr), device=q.device)
+        picked = selected[r:r + 128]
+        keys = torch.cat([raw[near.clamp(min=0)], comp[picked.clamp(min=0)]], dim=1)  # [tokens, keys, D]
+        score = torch.matmul(q[r:r + 128], keys.transpose(1, 2)).mul_(D ** -0.5)  # [tokens, heads, keys]
+        score.masked_fill_(torch.cat([near, picked], dim=1)[:, None] < 0, -math.inf)
+        p = torch.softmax(torch.cat([score, sinks.expand(score.shape[0], -1, 1)], dim=-1), dim=-1)[..., :-1]
+        out[r:r + 128] = torch.matmul(p, keys)
+    return out[None]
+
+
 def work(case):
     """Visible (query, key) pairs count, four FLOPs per pair and dimension; every tensor moves once."""
     kind, D, es = case["kind"], case["D"], 4 if case["dtype"] == "f32" else 2
