@@ -178,6 +178,9 @@ static Kernel choose(const dt_sdpa_params& p) {
   return kGeneric;
 }
 
+// The scratch with which a call that choose() leaves to the CUDA cores runs on the tensor cores (0: it stays there).
+static size_t optional_scratch(const dt_sdpa_params& p) { return f32_mma_supported(p) ? f32_mma_workspace_bytes(p) : 0; }
+
 }  // namespace dt
 
 using namespace dt;
@@ -217,7 +220,7 @@ int dt_sdpa_workspace_size(const dt_sdpa_params* p, size_t* bytes) {
   if (st != DT_OK) return st;
   if (!bytes) return DT_BAD_ARG;
   const Kernel k = choose(*p);
-  *bytes = k == kDecode ? decode_workspace_bytes(*p) : k == kPrefill ? prefill_workspace_bytes(*p) : 0;
+  *bytes = k == kDecode ? decode_workspace_bytes(*p) : k == kPrefill ? prefill_workspace_bytes(*p) : k == kGeneric ? optional_scratch(*p) : 0;
   return DT_OK;
 }
 
@@ -235,7 +238,12 @@ int dt_sdpa_forward(const dt_sdpa_params* p, void* workspace, size_t workspace_b
     case kDecode: return launch_decode(*p, workspace, workspace_bytes, stream);
     case kPrefill: return launch_prefill(*p, stream, nullptr, 0, workspace, workspace_bytes);
     case kShortKV: return launch_short_kv(*p, stream);
-    default: return launch_generic(*p, stream);
+    default: {
+      const size_t scratch = optional_scratch(*p);
+      if (scratch == 0 || !workspace || reinterpret_cast<uintptr_t>(workspace) % 16 || workspace_bytes < scratch)
+        return launch_generic(*p, stream);
+      return launch_f32_mma(*p, workspace, stream);
+    }
   }
 }
 
@@ -393,9 +401,16 @@ int dt_sdpa_forward_host(const dt_sdpa_params* ph) {
     if (g_hs.ws) cudaFree(g_hs.ws);
     g_hs.ws = nullptr;
     g_hs.ws_bytes = 0;
-    DT_CUDA_TRY(cudaMalloc(&g_hs.ws, wsb));
-    g_hs.ws_bytes = wsb;
-    DT_CUDA_TRY(cudaMemsetAsync(g_hs.ws, 0, wsb, g_hs.stream));
+    const cudaError_t e = cudaMalloc(&g_hs.ws, wsb);
+    if (e == cudaSuccess) {
+      g_hs.ws_bytes = wsb;
+      DT_CUDA_TRY(cudaMemsetAsync(g_hs.ws, 0, wsb, g_hs.stream));
+    } else if (choose(p) == kGeneric) {  // fp32: the CUDA-core kernel needs no scratch
+      cudaGetLastError();
+      g_hs.ws = nullptr;
+    } else {
+      return record_cuda_error(e);
+    }
   }
   cudaStream_t s = g_hs.stream;
   if (nsink) DT_CUDA_TRY(cudaMemcpyAsync(const_cast<void*>(p.sinks), ph->sinks, nsink, cudaMemcpyHostToDevice, s));

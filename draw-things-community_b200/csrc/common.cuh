@@ -32,7 +32,14 @@ inline size_t dtype_size(int dtype) { return dtype == DT_F32 ? 4 : 2; }
 // ---- kernel entry points (each in its own .cu) --------------------------------------------------
 
 // CUDA-core flash kernel: any D <= 256, any dtype, mask, causal, GQA.  Fallback and second opinion.
-int launch_generic(const dt_sdpa_params& p, cudaStream_t stream);
+// only_if (device memory, may be null): the kernel returns at once when it reads zero there.
+int launch_generic(const dt_sdpa_params& p, cudaStream_t stream, const uint32_t* only_if = nullptr);
+
+// fp32 tensors on the tensor cores: the plain operator, D <= 128 (a multiple of 8), with a workspace of
+// f32_mma_workspace_bytes (any contents).
+bool f32_mma_supported(const dt_sdpa_params& p);
+size_t f32_mma_workspace_bytes(const dt_sdpa_params& p);
+int launch_f32_mma(const dt_sdpa_params& p, void* workspace, cudaStream_t stream);
 
 // Argument rules every attention entry point shares (null or misaligned pointers, extents, NaN scale, negative
 // window, variable-length bookkeeping): DT_OK, DT_BAD_ARG or DT_UNSUPPORTED.  Nothing is launched.

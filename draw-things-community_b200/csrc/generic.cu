@@ -25,7 +25,8 @@ generic_sdpa_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* _
                     int64_t m_sb, int64_t m_sh, int64_t m_sq,
                     int Sq, int Sk, int Hq, int Hkv, int D, float scale_log2, int is_causal,
                     const T* __restrict__ sinks, int window, const int32_t* __restrict__ off_q,
-                    const int32_t* __restrict__ off_k) {
+                    const int32_t* __restrict__ off_k, const uint32_t* __restrict__ only_if) {
+  if (only_if && *only_if == 0u) return;  // another kernel has computed this call
   extern __shared__ float smem[];
   const int Dp = D | 1;
   float* Qs = smem;                    // [kRows][D]
@@ -182,7 +183,8 @@ generic_tiled_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
                      int64_t m_sb, int64_t m_sh, int64_t m_sq,
                      int Sq, int Sk, int Hq, int Hkv, int D, float scale_log2, int is_causal,
                      const T* __restrict__ sinks, int window, const int32_t* __restrict__ off_q,
-                     const int32_t* __restrict__ off_k) {
+                     const int32_t* __restrict__ off_k, const uint32_t* __restrict__ only_if) {
+  if (only_if && *only_if == 0u) return;  // another kernel has computed this call
   extern __shared__ __align__(16) float smem[];
   const int P1 = tiled_pitch(D);
   float* Qs = smem;              // [64][P1]
@@ -379,7 +381,7 @@ generic_tiled_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
 }
 
 template <typename T, int R>
-int launch_tiled(const dt_sdpa_params& p, cudaStream_t stream) {
+int launch_tiled(const dt_sdpa_params& p, cudaStream_t stream, const uint32_t* only_if) {
   const int D = p.D;
   const size_t smem = sizeof(float) * ((size_t)(kTM + kTN) * tiled_pitch(D) + (size_t)kTN * D + (size_t)kTM * kPPitch);
   auto kern = generic_tiled_kernel<T, R>;
@@ -391,20 +393,20 @@ int launch_tiled(const dt_sdpa_params& p, cudaStream_t stream) {
       p.q.stride_b, p.q.stride_s, p.q.stride_h, p.k.stride_b, p.k.stride_s, p.k.stride_h,
       p.v.stride_b, p.v.stride_s, p.v.stride_h, p.o.stride_b, p.o.stride_s, p.o.stride_h,
       p.mask_stride_b, p.mask_stride_h, p.mask_stride_q, p.Sq, p.Sk, p.Hq, p.Hkv, D, p.scale * kLog2e,
-      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k);
+      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if);
   DT_CUDA_TRY(cudaGetLastError());
   return DT_OK;
 }
 
 template <typename T>
-int launch_t(const dt_sdpa_params& p, cudaStream_t stream) {
+int launch_t(const dt_sdpa_params& p, cudaStream_t stream, const uint32_t* only_if) {
   const int D = p.D;
   // enough query rows to fill 64-row tiles (a variable-length batch: by its longest sequence) and 16-byte rows of fp32
   const int rows = p.seq_offsets_q ? p.max_seq_q : p.Sq;
   if (D % 4 == 0 && rows >= 32) {
-    if (D <= 64) return launch_tiled<T, 1>(p, stream);
-    if (D <= 128) return launch_tiled<T, 2>(p, stream);
-    return launch_tiled<T, 4>(p, stream);
+    if (D <= 64) return launch_tiled<T, 1>(p, stream, only_if);
+    if (D <= 128) return launch_tiled<T, 2>(p, stream, only_if);
+    return launch_tiled<T, 4>(p, stream, only_if);
   }
   const size_t smem = sizeof(float) * ((size_t)kRows * D + (size_t)kKeys * (D | 1) + (size_t)kKeys * D);
   auto kern = generic_sdpa_kernel<T>;
@@ -416,20 +418,20 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream) {
       p.q.stride_b, p.q.stride_s, p.q.stride_h, p.k.stride_b, p.k.stride_s, p.k.stride_h,
       p.v.stride_b, p.v.stride_s, p.v.stride_h, p.o.stride_b, p.o.stride_s, p.o.stride_h,
       p.mask_stride_b, p.mask_stride_h, p.mask_stride_q, p.Sq, p.Sk, p.Hq, p.Hkv, D, p.scale * kLog2e,
-      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k);
+      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if);
   DT_CUDA_TRY(cudaGetLastError());
   return DT_OK;
 }
 
 }  // namespace
 
-int launch_generic(const dt_sdpa_params& p, cudaStream_t stream) {
+int launch_generic(const dt_sdpa_params& p, cudaStream_t stream, const uint32_t* only_if) {
   if (p.D > 256) return DT_UNSUPPORTED;
   if (p.Hq > 65535 || p.B > 65535 || p.n_seq > 65535) return DT_UNSUPPORTED;
   switch (p.dtype) {
-    case DT_F32: return launch_t<float>(p, stream);
-    case DT_F16: return launch_t<__half>(p, stream);
-    case DT_BF16: return launch_t<__nv_bfloat16>(p, stream);
+    case DT_F32: return launch_t<float>(p, stream, only_if);
+    case DT_F16: return launch_t<__half>(p, stream, only_if);
+    case DT_BF16: return launch_t<__nv_bfloat16>(p, stream, only_if);
   }
   return DT_BAD_ARG;
 }

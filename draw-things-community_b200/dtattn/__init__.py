@@ -248,8 +248,12 @@ def sdpa_forward(q, k, v, scale, is_causal=False, mask=None, out=None, lse=None,
                     seq_offsets_k, max_seq_q, max_seq_k)
     if q.is_cuda:
         s = stream if stream is not None else torch.cuda.current_stream(q.device).cuda_stream
-        ws = workspace if workspace is not None else _default_workspace(q.device)
-        ptr, nbytes = ws.ensure(workspace_size(p), s)
+        if workspace is None and q.dtype == torch.float32 and kernel_name(p) == "generic":
+            scratch = _call_scratch(workspace_size(p), q.device, s)
+            ptr, nbytes = (None, 0) if scratch is None else (scratch.data_ptr(), scratch.numel())
+        else:
+            ws = workspace if workspace is not None else _default_workspace(q.device)
+            ptr, nbytes = ws.ensure(workspace_size(p), s)
         _check(lib().dt_sdpa_forward(ctypes.byref(p), ctypes.c_void_p(ptr) if ptr else None, nbytes,
                                      ctypes.c_void_p(s)), "dt_sdpa_forward")
     else:
@@ -430,6 +434,20 @@ class SparseIndexedAttention:
         return sparse_indexed_attention(queries, raw_keys, raw_values, compressed_keys, compressed_values, selected_rows,
                                         self.scale, None if sinks is None else sinks.reshape(-1).contiguous(),
                                         self.sliding_window, self.is_causal, out=out)
+
+
+def _call_scratch(nbytes, device, stream):
+    """Optional scratch of one call (any contents), its own so that calls on several streams stay independent; None when
+    there is no room for it, which the library answers with the kernel that needs none."""
+    if nbytes == 0:
+        return None
+    try:
+        buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return None
+    if stream != torch.cuda.current_stream(device).cuda_stream:
+        buf.record_stream(torch.cuda.ExternalStream(stream, device=device))
+    return buf
 
 
 _workspaces = {}
