@@ -963,6 +963,9 @@ int g_options = 0;
 float* g_dbg = nullptr;
 #endif
 
+// The first 4 KB of a workspace hold the split-KV ticket counters, which every call leaves zero: the flags start behind.
+constexpr size_t kTicketBytes = 4096;
+
 template <typename T, int D, bool kMask>
 int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, int n_extra, void* workspace,
              size_t workspace_bytes) {
@@ -992,12 +995,12 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
     const int Bm = p.mask_stride_b ? p.B : 1, Hm = p.mask_stride_h ? p.Hq : 1;
     a.n_rg = (p.Sq + 31) / 32;
     a.n_kh = ((p.Sk + 63) / 64 + 1) & ~1;
-    a.mask_flags = static_cast<const unsigned char*>(workspace);
+    unsigned char* flags = static_cast<unsigned char*>(workspace) + kTicketBytes;
+    a.mask_flags = flags;
     dim3 fgrid((a.n_kh + 7) / 8, a.n_rg, Bm * Hm);
     if (fgrid.y > 65535 || fgrid.z > 65535) return DT_UNSUPPORTED;
     mask_flags_kernel<<<fgrid, 256, 0, stream>>>(static_cast<const unsigned short*>(p.mask), p.mask_stride_b, p.mask_stride_h,
-                                                p.mask_stride_q, Hm, p.Sq, p.Sk, a.n_rg, a.n_kh, p.is_causal,
-                                                static_cast<unsigned char*>(workspace));
+                                                p.mask_stride_q, Hm, p.Sq, p.Sk, a.n_rg, a.n_kh, p.is_causal, flags);
     DT_CUDA_TRY(cudaGetLastError());
   }
   a.is_causal = p.is_causal;
@@ -1049,7 +1052,7 @@ size_t prefill_workspace_bytes(const dt_sdpa_params& p) {
   if (!p.mask) return 0;
   const size_t Bm = p.mask_stride_b ? p.B : 1, Hm = p.mask_stride_h ? p.Hq : 1;
   const size_t n_rg = (p.Sq + 31) / 32, n_kh = ((p.Sk + 63) / 64 + 1) & ~(size_t)1;
-  return (Bm * Hm * n_rg * n_kh + 255) / 256 * 256;
+  return kTicketBytes + (Bm * Hm * n_rg * n_kh + 255) / 256 * 256;
 }
 
 int launch_prefill(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra_outputs, int n_extra, void* workspace,
