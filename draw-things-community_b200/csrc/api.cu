@@ -179,7 +179,11 @@ static Kernel choose(const dt_sdpa_params& p) {
 }
 
 // The scratch with which a call that choose() leaves to the CUDA cores runs on the tensor cores (0: it stays there).
-static size_t optional_scratch(const dt_sdpa_params& p) { return f32_mma_supported(p) ? f32_mma_workspace_bytes(p) : 0; }
+static size_t optional_scratch(const dt_sdpa_params& p) {
+  if (f32_mma_supported(p)) return f32_mma_workspace_bytes(p);
+  if (prefill_repack_supported(p)) return prefill_repack_workspace_bytes(p);
+  return 0;
+}
 
 }  // namespace dt
 
@@ -242,7 +246,7 @@ int dt_sdpa_forward(const dt_sdpa_params* p, void* workspace, size_t workspace_b
       const size_t scratch = optional_scratch(*p);
       if (scratch == 0 || !workspace || reinterpret_cast<uintptr_t>(workspace) % 16 || workspace_bytes < scratch)
         return launch_generic(*p, stream);
-      return launch_f32_mma(*p, workspace, stream);
+      return p->dtype == DT_F32 ? launch_f32_mma(*p, workspace, stream) : launch_prefill_repack(*p, stream, workspace, workspace_bytes);
     }
   }
 }

@@ -59,6 +59,12 @@ int launch_prefill(const dt_sdpa_params& p, cudaStream_t stream, void* const* ex
 // Scratch of the masked variant: one byte per (32 query rows x 64 keys) patch of the mask, "has a non-zero entry".
 size_t prefill_workspace_bytes(const dt_sdpa_params& p);
 
+// The masked operator with mask rows that are not 16-byte aligned: the same kernel behind a pass that copies the mask to
+// aligned rows.  Scratch of prefill_repack_workspace_bytes (its first 4 KB are left alone).
+bool prefill_repack_supported(const dt_sdpa_params& p);
+size_t prefill_repack_workspace_bytes(const dt_sdpa_params& p);
+int launch_prefill_repack(const dt_sdpa_params& p, cudaStream_t stream, void* workspace, size_t workspace_bytes);
+
 // Cross-attention over a short key/value sequence (Sk <= 96, head dim <= 64, the plain operator): three independent
 // warpgroup pipelines per CTA, TMA + tcgen05.
 bool short_kv_supported(const dt_sdpa_params& p);

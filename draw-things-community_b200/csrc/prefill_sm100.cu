@@ -160,6 +160,18 @@ __device__ __forceinline__ void issue_pv(uint32_t o_tmem, uint32_t p_tmem, uint6
   }
 }
 
+// The same for the weights of the kSplit variant: their high parts and, 64 columns further, what those leave over.
+template <bool kSplit>
+__device__ __forceinline__ void issue_pv_parts(uint32_t o_tmem, uint32_t p_tmem, uint64_t v_desc, uint32_t idesc,
+                                               uint32_t accumulate, int k_begin, int k_end) {
+  issue_pv(o_tmem, p_tmem, v_desc, idesc, accumulate, k_begin, k_end);
+  if constexpr (kSplit) {
+#pragma unroll 1
+    for (int kk = k_begin; kk < k_end; ++kk)
+      ptx::mma_ts(o_tmem, p_tmem + 64 + kk * 8, v_desc + (uint64_t)(kk * (2048 >> 4)), idesc, 1u);
+  }
+}
+
 // Experiment builds (-DDT_PREFILL_OPTIONS=bits, never the product): bit 3 = the softmax warps skip the exponentials;
 // bit 4 = nobody waits for S or P (free-running softmax and MMA: garbage results, the pure throughput of each
 // side); bit 5 = the softmax warps skip the row maximum; bit 6 (with bit 4) = the softmax warps do nothing per block.  Bring-up builds: a.options bit 1 = timeline probe of CTA 0.
@@ -207,6 +219,45 @@ __global__ void __launch_bounds__(256) mask_flags_kernel(const unsigned short* _
   if (lane == 0) flags[((int64_t)bh * n_rg + rg) * n_kh + kh] = nz ? 1 : 0;
 }
 
+// Pre-pass for masks whose rows do not start on 16 bytes (a dense [S, S] mask of an odd S): the same flags, and the
+// flagged patches copied to rows of `ld` entries, a multiple of 8 (patches of zeros are never read, so they are not
+// written either).  One warp per patch, two entries of a row per lane, the whole patch in 32 registers.
+__global__ void __launch_bounds__(256) mask_repack_kernel(const unsigned short* __restrict__ mask, int64_t m_sb, int64_t m_sh,
+                                                          int64_t m_sq, int Hm, int Sq, int Sk, int n_rg, int n_kh,
+                                                          int is_causal, unsigned char* __restrict__ flags,
+                                                          unsigned short* __restrict__ copy, int ld) {
+  const int lane = threadIdx.x & 31;
+  const int kh = blockIdx.x * 8 + (threadIdx.x >> 5), rg = blockIdx.y, bh = blockIdx.z;
+  if (kh >= n_kh) return;
+  const int mb = bh / Hm, mh = bh - mb * Hm;
+  const unsigned short* base = mask + mb * m_sb + mh * m_sh;
+  const int k0 = kh * 64 + lane, k1 = k0 + 32;
+  uint32_t v[32], any = 0u;
+  const bool visited = !is_causal || (long long)kh * 64 <= (long long)rg * 32 + 31 + (Sk - Sq);
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    const int row = rg * 32 + i;
+    const unsigned short* src = base + (int64_t)row * m_sq;
+    v[i] = 0u;
+    if (visited && row < Sq) {
+      if (k0 < Sk) v[i] = __ldg(src + k0);
+      if (k1 < Sk) v[i] |= (uint32_t)__ldg(src + k1) << 16;
+    }
+    any |= v[i];
+  }
+  const bool nz = __any_sync(0xffffffffu, any != 0u);
+  if (lane == 0) flags[((int64_t)bh * n_rg + rg) * n_kh + kh] = nz ? 1 : 0;
+  if (!nz) return;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    const int row = rg * 32 + i;
+    if (row >= Sq) break;
+    unsigned short* dst = copy + ((int64_t)bh * Sq + row) * ld;
+    if (k0 < Sk) dst[k0] = (unsigned short)v[i];
+    if (k1 < Sk) dst[k1] = (unsigned short)(v[i] >> 16);
+  }
+}
+
 // 16-bit pair -> two floats (the mask is stored in the tensors' type)
 template <typename T>
 __device__ __forceinline__ float2 unpack_pair(uint32_t x) {
@@ -214,7 +265,7 @@ __device__ __forceinline__ float2 unpack_pair(uint32_t x) {
   else return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x));
 }
 
-template <typename T, int D, bool kMask>
+template <typename T, int D, bool kMask, bool kSplit>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
@@ -472,11 +523,11 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
               advance();
               if (!ptx::mbar_wait(&bars->p_half[b][0], pph, abort_flag)) { fail(4u); break; }
               ptx::tc_fence_after();
-              issue_pv(o0, sb, vd, idesc_pv, j > 0 ? 1u : 0u, 0, k_mid);
+              issue_pv_parts<kSplit>(o0, sb, vd, idesc_pv, j > 0 ? 1u : 0u, 0, k_mid);
               if (!ptx::mbar_wait(&bars->p_half[b][1], pph, abort_flag)) { fail(4u); break; }
               pph ^= 1;
               ptx::tc_fence_after();
-              issue_pv(o0, sb, vd, idesc_pv, 1u, k_mid, ksteps);
+              issue_pv_parts<kSplit>(o0, sb, vd, idesc_pv, 1u, k_mid, ksteps);
               ptx::tc_commit(&bars->kv_empty[slot_v]);
               ptx::tc_commit(&bars->pv_done);
               if (j + 2 < w.nkv && !qk(j + 2)) break;  // overwrites the S / P columns the P V above has just read
@@ -530,11 +581,11 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             if (!DT_OPT(16) && !ptx::mbar_wait(&bars->p_half[0][0], pph0, abort_flag)) { fail(4u); break; }
             if (j == 0) stamp(a, 16 * n_item + 2);
             ptx::tc_fence_after();
-            issue_pv(o0, s0, vd, idesc_pv, j > 0 ? 1u : 0u, 0, k_mid);
+            issue_pv_parts<kSplit>(o0, s0, vd, idesc_pv, j > 0 ? 1u : 0u, 0, k_mid);
             if (!DT_OPT(16) && !ptx::mbar_wait(&bars->p_half[0][1], pph0, abort_flag)) { fail(4u); break; }
             pph0 ^= 1;
             ptx::tc_fence_after();
-            issue_pv(o0, s0, vd, idesc_pv, 1u, k_mid, ksteps);
+            issue_pv_parts<kSplit>(o0, s0, vd, idesc_pv, 1u, k_mid, ksteps);
             if (ntile == 1) ptx::tc_commit(&bars->kv_empty[slot_v]);
             if (more) issue_qk<D>(s0, qd0, kd, idesc_qk);
             ptx::tc_commit(more ? &bars->s_full[0] : &bars->o_full[0]);  // next S ready, or (last block) O complete
@@ -547,11 +598,11 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             if (ntile == 2) {
               if (!DT_OPT(16) && !ptx::mbar_wait(&bars->p_half[1][0], pph1, abort_flag)) { fail(4u); break; }
               ptx::tc_fence_after();
-              issue_pv(o1, s1, vd, idesc_pv, j > 0 ? 1u : 0u, 0, k_mid);
+              issue_pv_parts<kSplit>(o1, s1, vd, idesc_pv, j > 0 ? 1u : 0u, 0, k_mid);
               if (!DT_OPT(16) && !ptx::mbar_wait(&bars->p_half[1][1], pph1, abort_flag)) { fail(4u); break; }
               pph1 ^= 1;
               ptx::tc_fence_after();
-              issue_pv(o1, s1, vd, idesc_pv, 1u, k_mid, ksteps);
+              issue_pv_parts<kSplit>(o1, s1, vd, idesc_pv, 1u, k_mid, ksteps);
               ptx::tc_commit(&bars->kv_empty[slot_v]);
               if (more) issue_qk<D>(s1, qd1, kd, idesc_qk);
               ptx::tc_commit(more ? &bars->s_full[1] : &bars->o_full[1]);
@@ -815,6 +866,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         for (int c = 0; c < 4; ++c) {
           lsum[c] = 0ull;
           if (c < nch) {
+          uint32_t rest[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             const uint64_t x2 = ptx::fma_f32x2(ptx::pack_f32x2(__uint_as_float(s[c][2 * i]), __uint_as_float(s[c][2 * i + 1])),
@@ -832,10 +884,16 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             }
             lsum[c] = ptx::add_f32x2(lsum[c], ptx::pack_f32x2(p0, p1));
             // the packed pair goes into the register score i of this chunk came in (scores 2i and 2i+1 are used up)
-            if constexpr (kBf16 != 0) ptx::cvt_pack_bf16_into(s[c][i], p0, p1);
+            if constexpr (kSplit) {  // weights of 16 bits and more: the rounded one and the rest of it
+              const uint32_t hi = pack_pair<T>(p0, p1);
+              const float2 f = unpack_pair<T>(hi);
+              s[c][i] = hi;
+              rest[i] = pack_pair<T>(p0 - f.x, p1 - f.y);
+            } else if constexpr (kBf16 != 0) ptx::cvt_pack_bf16_into(s[c][i], p0, p1);
             else ptx::cvt_pack_f16_into(s[c][i], p0, p1);
           }
           ptx::tmem_st16(t_s + c * 16, s[c]);
+          if constexpr (kSplit) ptx::tmem_st16(t_s + 64 + c * 16, rest);
           }
           if (c == 1 || c == 3) {  // 64 keys of P are in TMEM: let the MMA warp start on them
             ptx::tc_wait_st();
@@ -963,10 +1021,19 @@ int g_options = 0;
 float* g_dbg = nullptr;
 #endif
 
+bool mask_rows_aligned(const dt_sdpa_params& p) {
+  return !(reinterpret_cast<uintptr_t>(p.mask) % 16 || p.mask_stride_b % 8 || p.mask_stride_h % 8 || p.mask_stride_q % 8);
+}
 // The first 4 KB of a workspace hold the split-KV ticket counters, which every call leaves zero: the flags start behind.
 constexpr size_t kTicketBytes = 4096;
+size_t mask_flag_bytes(const dt_sdpa_params& p) {
+  const size_t Bm = p.mask_stride_b ? p.B : 1, Hm = p.mask_stride_h ? p.Hq : 1;
+  const size_t n_rg = (p.Sq + 31) / 32, n_kh = ((p.Sk + 63) / 64 + 1) & ~(size_t)1;
+  return kTicketBytes + (Bm * Hm * n_rg * n_kh + 255) / 256 * 256;
+}
+int repacked_row(const dt_sdpa_params& p) { return (p.Sk + 7) / 8 * 8; }
 
-template <typename T, int D, bool kMask>
+template <typename T, int D, bool kMask, bool kSplit = false>
 int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, int n_extra, void* workspace,
              size_t workspace_bytes) {
   using C = Cfg<D, kMask>;
@@ -991,7 +1058,7 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
   a.mask = p.mask;
   a.m_sb = p.mask_stride_b; a.m_sh = p.mask_stride_h; a.m_sq = p.mask_stride_q;
   if (kMask) {
-    if (!workspace || workspace_bytes < prefill_workspace_bytes(p)) return DT_WORKSPACE;
+    if (!workspace || workspace_bytes < (kSplit ? prefill_repack_workspace_bytes(p) : prefill_workspace_bytes(p))) return DT_WORKSPACE;
     const int Bm = p.mask_stride_b ? p.B : 1, Hm = p.mask_stride_h ? p.Hq : 1;
     a.n_rg = (p.Sq + 31) / 32;
     a.n_kh = ((p.Sk + 63) / 64 + 1) & ~1;
@@ -999,6 +1066,17 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
     a.mask_flags = flags;
     dim3 fgrid((a.n_kh + 7) / 8, a.n_rg, Bm * Hm);
     if (fgrid.y > 65535 || fgrid.z > 65535) return DT_UNSUPPORTED;
+    if (kSplit) {
+      const int ld = repacked_row(p);
+      unsigned short* copy = reinterpret_cast<unsigned short*>(static_cast<uint8_t*>(workspace) + mask_flag_bytes(p));
+      mask_repack_kernel<<<fgrid, 256, 0, stream>>>(static_cast<const unsigned short*>(p.mask), p.mask_stride_b, p.mask_stride_h,
+                                                   p.mask_stride_q, Hm, p.Sq, p.Sk, a.n_rg, a.n_kh, p.is_causal,
+                                                   flags, copy, ld);
+      a.mask = copy;
+      a.m_sq = ld;
+      a.m_sh = Hm > 1 ? (int64_t)p.Sq * ld : 0;
+      a.m_sb = Bm > 1 ? (int64_t)Hm * p.Sq * ld : 0;
+    } else
     mask_flags_kernel<<<fgrid, 256, 0, stream>>>(static_cast<const unsigned short*>(p.mask), p.mask_stride_b, p.mask_stride_h,
                                                 p.mask_stride_q, Hm, p.Sq, p.Sk, a.n_rg, a.n_kh, p.is_causal, flags);
     DT_CUDA_TRY(cudaGetLastError());
@@ -1015,7 +1093,7 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
   a.off_k = p.seq_offsets_k;
   a.n_qpairs = ((varlen ? p.max_seq_q : p.Sq) + C::kTiles * kBM - 1) / (C::kTiles * kBM);
   a.n_items = a.n_qpairs * p.Hq * (varlen ? p.n_seq : p.B);
-  auto kern = prefill_tcgen05_kernel<T, D, kMask>;
+  auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit>;
   DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
   const int n_sm = device_sm_count();
   dim3 grid(a.n_items < n_sm ? a.n_items : n_sm);  // one persistent CTA per SM
@@ -1034,9 +1112,7 @@ bool prefill_supported(const dt_sdpa_params& p) {
   if (p.sliding_window > 0 && p.Sq > p.Sk) return false;  // rows that may see no key: generic kernel
   if (p.dtype != DT_F16 && p.dtype != DT_BF16) return false;
   if (p.D < 8 || p.D > 256 || p.D % 8) return false;  // head dims below 64 / 128 / 256 run zero-padded (SD1.5: 40, 80, 160)
-  // additive mask: each row's entries are read with 16-byte loads
-  if (p.mask && (reinterpret_cast<uintptr_t>(p.mask) % 16 || p.mask_stride_b % 8 || p.mask_stride_h % 8 || p.mask_stride_q % 8))
-    return false;
+  if (p.mask && !mask_rows_aligned(p)) return false;  // each row's entries are read with 16-byte loads
   if (!(p.scale > 0.f)) return false;
   if (p.Hq % p.Hkv) return false;
   if (p.Hq > 65535 || p.B > 65535) return false;
@@ -1048,11 +1124,32 @@ bool prefill_supported(const dt_sdpa_params& p) {
   return ok(p.q) && ok(p.k) && ok(p.v) && ok(p.o);
 }
 
-size_t prefill_workspace_bytes(const dt_sdpa_params& p) {
-  if (!p.mask) return 0;
+size_t prefill_workspace_bytes(const dt_sdpa_params& p) { return p.mask ? mask_flag_bytes(p) : 0; }
+
+// Masks whose rows are not 16-byte aligned: copied to aligned rows first.  The calls come from the CUDA-core kernel, whose
+// weights are fp32, so this variant multiplies V with two 16-bit parts of every weight: 333 tokens, 32 / 8 heads of 128,
+// causal and padding mask, bf16: 117 us there, 30 us here, error against 64 bits 1.6e-3 (the rounding of the result) in both.  A mask per head of a long
+// sequence would need a copy as large as itself: up to 256 MB.
+bool prefill_repack_supported(const dt_sdpa_params& p) {
+  if (!p.mask || mask_rows_aligned(p) || (p.flags & DT_FLAG_FORCE_GENERIC)) return false;
+  dt_sdpa_params plain = p;
+  plain.mask = nullptr;
+  if (!prefill_supported(plain) || (p.Sq + 31) / 32 > 65535) return false;
   const size_t Bm = p.mask_stride_b ? p.B : 1, Hm = p.mask_stride_h ? p.Hq : 1;
-  const size_t n_rg = (p.Sq + 31) / 32, n_kh = ((p.Sk + 63) / 64 + 1) & ~(size_t)1;
-  return kTicketBytes + (Bm * Hm * n_rg * n_kh + 255) / 256 * 256;
+  return Bm * Hm <= 65535 && Bm * Hm * p.Sq * (size_t)repacked_row(p) * 2 <= ((size_t)256 << 20);
+}
+
+size_t prefill_repack_workspace_bytes(const dt_sdpa_params& p) {
+  const size_t Bm = p.mask_stride_b ? p.B : 1, Hm = p.mask_stride_h ? p.Hq : 1;
+  return mask_flag_bytes(p) + Bm * Hm * p.Sq * (size_t)repacked_row(p) * 2;
+}
+
+int launch_prefill_repack(const dt_sdpa_params& p, cudaStream_t stream, void* workspace, size_t workspace_bytes) {
+#define DT_REPACK_GO(T, DD) launch_t<T, DD, true, true>(p, stream, nullptr, 0, workspace, workspace_bytes)
+#define DT_REPACK_BY_D(T) (p.D > 128 ? DT_REPACK_GO(T, 256) : p.D > 64 ? DT_REPACK_GO(T, 128) : DT_REPACK_GO(T, 64))
+  return p.dtype == DT_F16 ? DT_REPACK_BY_D(__half) : DT_REPACK_BY_D(__nv_bfloat16);
+#undef DT_REPACK_BY_D
+#undef DT_REPACK_GO
 }
 
 int launch_prefill(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra_outputs, int n_extra, void* workspace,

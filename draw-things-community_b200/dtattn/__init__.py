@@ -248,7 +248,7 @@ def sdpa_forward(q, k, v, scale, is_causal=False, mask=None, out=None, lse=None,
                     seq_offsets_k, max_seq_q, max_seq_k)
     if q.is_cuda:
         s = stream if stream is not None else torch.cuda.current_stream(q.device).cuda_stream
-        if workspace is None and q.dtype == torch.float32 and kernel_name(p) == "generic":
+        if workspace is None and (mask is not None or q.dtype == torch.float32) and kernel_name(p) == "generic":
             scratch = _call_scratch(workspace_size(p), q.device, s)
             ptr, nbytes = (None, 0) if scratch is None else (scratch.data_ptr(), scratch.numel())
         else:

@@ -121,8 +121,8 @@ int dt_abi_version(void);
  */
 
 /* Bytes of scratch dt_sdpa_forward needs for these params (0 is a valid answer).  Where dt_sdpa_kernel_name says
-   "generic" the scratch is optional (any contents): with it the plain fp32 operator runs on the tensor cores, without it,
-   or with less, on the CUDA cores. */
+   "generic" the scratch is optional (any contents): with it the plain fp32 operator and masks of
+   unaligned rows run on the tensor cores, without it, or with less, on the CUDA cores. */
 int dt_sdpa_workspace_size(const dt_sdpa_params* p, size_t* bytes);
 /* Zero the workspace's ticket counters.  Call once after allocating a workspace (and again after any
    call that returned an error); dt_sdpa_forward leaves them zero on success. */

@@ -1,0 +1,66 @@
+"""Masks whose rows do not start on 16 bytes (dense [S, S] masks of odd lengths, odd offsets): copied to aligned rows and
+served by the tensor-core kernel with two 16-bit parts per weight, against the oracle and the CUDA-core kernel, whose
+weights are fp32."""
+import pytest
+import torch
+
+from oracle import sdpa_oracle as so
+from test_gpu_masked_prefill import make_mask
+from test_gpu_parity import DEV, check, inputs
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("case", [
+    # B, mask batch, mask heads, Sq, Sk, Hq, Hkv, D, causal, dtype: lengths around the 32 x 64 patches and 128-key blocks,
+    # every width of the kernel, broadcast and full masks, a mask one element off a 16-byte boundary
+    (1, 1, 1, 33, 33, 4, 2, 128, True, torch.bfloat16), (2, 1, 1, 77, 77, 4, 4, 64, False, torch.float16),
+    (1, 1, 1, 333, 333, 8, 2, 128, True, torch.bfloat16), (2, 2, 1, 129, 191, 4, 4, 64, False, torch.bfloat16),
+    (1, 1, 6, 65, 127, 6, 3, 40, False, torch.float16), (2, 2, 4, 257, 259, 4, 1, 80, True, torch.float16),
+    (1, 1, 1, 300, 301, 4, 2, 256, True, torch.bfloat16), (1, 1, 1, 131, 515, 2, 2, 160, False, torch.float16),
+    (1, 1, 1, 64, 1, 2, 2, 64, False, torch.bfloat16)])
+def test_against_oracle_and_cuda_cores(dtattn, case):
+    B, bm, hm, Sq, Sk, Hq, Hkv, D, causal, dtype = case
+    q, k, v = inputs(B, Sq, Sk, Hq, Hkv, D, dtype, 1401)
+    mask = make_mask(bm, hm, Sq, Sk, dtype, 1402)
+    mask[..., 3 * Sk // 4:] = mask[..., 3 * Sk // 4:].clamp(max=0) * 0  # a share of the patches holds zeros only
+    ref, ref_lse = so.sdpa_explicit(q, k, v, D ** -0.5, causal, mask, compute_dtype=torch.float64, return_lse=True)
+    store = torch.zeros(mask.numel() + 1, dtype=dtype, device=DEV)
+    shifted = store[1:].view(mask.shape).copy_(mask)  # rows at odd element offsets whatever Sk is
+    err = []
+    for flags in (0, dtattn.DT_FLAG_FORCE_GENERIC):
+        lse = torch.full((B, Hq, Sq), float("nan"), device=DEV)
+        out = dtattn.sdpa_forward(q.to(DEV), k.to(DEV), v.to(DEV), D ** -0.5, causal, shifted, lse=lse, flags=flags)
+        torch.cuda.synchronize()
+        assert dtattn.device_status() == 0
+        check(out, ref.float(), dtype, f"{case} flags={flags}")
+        assert torch.allclose(lse.cpu(), ref_lse.float(), atol=2e-3, rtol=1e-4)
+        err.append(float((out.cpu().double() - ref).pow(2).mean().sqrt()))
+    # both errors are the rounding of the 16-bit result: no precision is given up for the tensor cores
+    assert err[0] <= 1.02 * err[1] + 1e-9, err
+
+
+def test_scratch_limits(dtattn):
+    """Without scratch, or with less, the call stays on the CUDA cores; a mask per head whose copy would be larger than
+    256 MB asks for none."""
+    import ctypes
+    B, S, H, D, dtype = 1, 99, 2, 64, torch.float16
+    q, k, v = (x.to(DEV) for x in inputs(B, S, S, H, H, D, dtype, 1411))
+    mask = make_mask(1, 1, S, S, dtype, 1412).to(DEV)
+    want = dtattn.sdpa_forward(q, k, v, D ** -0.5, mask=mask, flags=dtattn.DT_FLAG_FORCE_GENERIC)
+    out = torch.zeros_like(q)
+    p = dtattn.make_params(q, k, v, out, D ** -0.5, mask=mask)
+    need = dtattn.workspace_size(p)
+    scratch = torch.full((need,), 0xff, dtype=torch.uint8, device=DEV)
+    s = torch.cuda.current_stream().cuda_stream
+    for ptr, nbytes in ((None, 0), (scratch.data_ptr(), need - 1), (scratch.data_ptr(), need)):
+        out.zero_()
+        assert dtattn.lib().dt_sdpa_forward(ctypes.byref(p), ctypes.c_void_p(ptr), nbytes, ctypes.c_void_p(s)) == dtattn.DT_OK
+        torch.cuda.synchronize()
+        if nbytes < need:
+            assert torch.equal(out, want)
+        assert float((out.float() - want.float()).abs().max()) < 2e-3
+    assert bool((scratch[:4096] == 0xff).all())
+    p.Sq = p.Sk = 8201
+    p.mask_stride_q, p.mask_stride_h = 8201, 8201 * 8201
+    assert dtattn.workspace_size(p) == 0
