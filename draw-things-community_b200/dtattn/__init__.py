@@ -17,6 +17,7 @@ from __future__ import annotations
 import ctypes
 import enum
 import os
+import struct
 
 import torch
 
@@ -81,6 +82,36 @@ class SparseIndexedParams(ctypes.Structure):
                 ("q", Tensor4), ("o", Tensor4), ("k_raw", Tensor4), ("v_raw", Tensor4), ("k_comp", Tensor4), ("v_comp", Tensor4),
                 ("selected", ctypes.c_void_p), ("selected_stride_b", ctypes.c_int64), ("selected_stride_q", ctypes.c_int64),
                 ("sinks", ctypes.c_void_p), ("lse", ctypes.c_void_p), ("flags", ctypes.c_uint32)]
+
+
+# The structures above as struct formats (native alignment; "0P" pads the end).  A call fills one in a single pack
+# instead of a ctypes assignment per field: 20 us of host time became 6 for a decode step, whose kernel takes about 10.
+_PACK_T4 = "Pqqq"
+_PACK_SDPA = struct.Struct("@7ifiI" + 4 * _PACK_T4 + "PqqqPP4iPP")
+_PACK_STEP = struct.Struct(f"@{_PACK_SDPA.size}s" + 2 * _PACK_T4 + "iPqqPPf0P")
+_PACK_PROLOGUE = struct.Struct("@5i" + 2 * _PACK_T4 + "PifPqqqf0P")
+_PACK_SPARSE = struct.Struct("@9if2i" + 6 * _PACK_T4 + "PqqPPI0P")
+for _pack, _cls in ((_PACK_SDPA, SdpaParams), (_PACK_STEP, DecodeStepParams), (_PACK_PROLOGUE, QkPrologueParams),
+                    (_PACK_SPARSE, SparseIndexedParams)):
+    assert _pack.size == ctypes.sizeof(_cls), _cls
+_NO_TENSOR = (0, 0, 0, 0)
+
+
+def _f32(x):
+    """x as the nearest fp32 value (an overflow is an infinity, as in a C assignment)."""
+    return ctypes.c_float(x).value
+
+
+def _quad(t):
+    """(pointer, batch, token and head stride) of a [B,S,H,D] view."""
+    st = t.stride()
+    assert len(st) == 4 and (st[3] == 1 or t.shape[3] == 1), "expect a [B,S,H,D] view with contiguous D"
+    return t.data_ptr(), st[0], st[1], st[2]
+
+
+def _stream_of(device, stream):
+    return stream if stream is not None else torch._C._cuda_getCurrentRawStream(
+        device.index if device.index is not None else torch.cuda.current_device())
 
 
 class DtError(RuntimeError):
@@ -159,39 +190,44 @@ def _view4(t: torch.Tensor) -> Tensor4:
     return Tensor4(t.data_ptr(), t.stride(0), t.stride(1), t.stride(2))
 
 
-def make_params(q, k, v, o, scale, is_causal=False, mask=None, lse=None, flags=0, sinks=None, sliding_window=0,
-                seq_offsets_q=None, seq_offsets_k=None, max_seq_q=0, max_seq_k=0) -> SdpaParams:
+def _pack_params(q, k, v, o, scale, is_causal, mask, lse, flags, sinks, sliding_window, seq_offsets_q, seq_offsets_k,
+                 max_seq_q, max_seq_k, Sk=None):
+    """The bytes of an SdpaParams; Sk: the leading rows of k and v that take part (default: all)."""
     B, Sq, Hq, D = q.shape
-    _, Sk, Hkv, _ = k.shape
-    p = SdpaParams()
-    p.B, p.Sq, p.Sk, p.Hq, p.Hkv, p.D = B, Sq, Sk, Hq, Hkv, D
-    p.dtype = _DTYPES[q.dtype]
-    p.scale = float(scale)
-    p.is_causal = int(bool(is_causal))
-    p.flags = int(flags)
-    p.q, p.k, p.v, p.o = _view4(q), _view4(k), _view4(v), _view4(o)
+    _, k_rows, Hkv, _ = k.shape
+    if Sk is None:
+        Sk = k_rows
+    mask_fields = _NO_TENSOR
     if mask is not None:
         assert mask.dtype == q.dtype and mask.dim() == 4 and mask.shape[2] == Sq and mask.shape[3] == Sk
         assert mask.stride(3) == 1 or Sk == 1
-        p.mask = mask.data_ptr()
-        p.mask_stride_b = mask.stride(0) if mask.shape[0] > 1 else 0
-        p.mask_stride_h = mask.stride(1) if mask.shape[1] > 1 else 0
-        p.mask_stride_q = mask.stride(2)
+        mask_fields = (mask.data_ptr(), mask.stride(0) if mask.shape[0] > 1 else 0, mask.stride(1) if mask.shape[1] > 1 else 0,
+                       mask.stride(2))
+    lse_ptr = sinks_ptr = offs_q = offs_k = n_seq = 0
     if lse is not None:
         assert lse.dtype == torch.float32 and lse.is_contiguous() and tuple(lse.shape) == (B, Hq, Sq)
-        p.lse = lse.data_ptr()
+        lse_ptr = lse.data_ptr()
     if sinks is not None:
         assert sinks.dtype == q.dtype and sinks.is_contiguous() and sinks.numel() == Hq
-        p.sinks = sinks.data_ptr()
-    p.sliding_window = int(sliding_window)
+        sinks_ptr = sinks.data_ptr()
     if seq_offsets_q is not None:
         for t in (seq_offsets_q, seq_offsets_k):
             assert t.dtype == torch.int32 and t.is_contiguous() and t.device == q.device
         assert seq_offsets_q.numel() == seq_offsets_k.numel() >= 2
-        p.n_seq = seq_offsets_q.numel() - 1
-        p.seq_offsets_q, p.seq_offsets_k = seq_offsets_q.data_ptr(), seq_offsets_k.data_ptr()
-        p.max_seq_q, p.max_seq_k = int(max_seq_q or Sq), int(max_seq_k or Sk)
-    return p
+        n_seq = seq_offsets_q.numel() - 1
+        offs_q, offs_k = seq_offsets_q.data_ptr(), seq_offsets_k.data_ptr()
+        max_seq_q, max_seq_k = int(max_seq_q or Sq), int(max_seq_k or Sk)
+    else:
+        max_seq_q = max_seq_k = 0
+    return _PACK_SDPA.pack(B, Sq, Sk, Hq, Hkv, D, _DTYPES[q.dtype], _f32(scale), 1 if is_causal else 0, int(flags) & 0xffffffff,
+                           *_quad(q), *_quad(k), *_quad(v), *_quad(o), *mask_fields, lse_ptr, sinks_ptr, int(sliding_window),
+                           n_seq, max_seq_q, max_seq_k, offs_q, offs_k)
+
+
+def make_params(q, k, v, o, scale, is_causal=False, mask=None, lse=None, flags=0, sinks=None, sliding_window=0,
+                seq_offsets_q=None, seq_offsets_k=None, max_seq_q=0, max_seq_k=0) -> SdpaParams:
+    return SdpaParams.from_buffer_copy(_pack_params(q, k, v, o, scale, is_causal, mask, lse, flags, sinks, sliding_window,
+                                                    seq_offsets_q, seq_offsets_k, max_seq_q, max_seq_k))
 
 
 def kernel_name(p: SdpaParams) -> str:
@@ -233,6 +269,10 @@ class Workspace:
         return self.buf.data_ptr(), self.buf.numel()
 
 
+def _new_output(q):
+    return torch.empty_like(q) if q.is_contiguous() else torch.empty(q.shape, dtype=q.dtype, device=q.device)
+
+
 def sdpa_forward(q, k, v, scale, is_causal=False, mask=None, out=None, lse=None, flags=0, workspace=None,
                  stream=None, sinks=None, sliding_window=0, seq_offsets_q=None, seq_offsets_k=None, max_seq_q=0,
                  max_seq_k=0):
@@ -241,13 +281,12 @@ def sdpa_forward(q, k, v, scale, is_causal=False, mask=None, out=None, lse=None,
     CUDA tensors -> dt_sdpa_forward on the current (or given) stream; CPU tensors -> dt_sdpa_forward_host,
     which stages through device memory (the end-to-end path).
     """
-    B, Sq, Hq, D = q.shape
     if out is None:
-        out = torch.empty((B, Sq, Hq, D), dtype=q.dtype, device=q.device)
+        out = _new_output(q)
     p = make_params(q, k, v, out, scale, is_causal, mask, lse, flags, sinks, sliding_window, seq_offsets_q,
                     seq_offsets_k, max_seq_q, max_seq_k)
     if q.is_cuda:
-        s = stream if stream is not None else torch.cuda.current_stream(q.device).cuda_stream
+        s = _stream_of(q.device, stream)
         if workspace is None and (mask is not None or q.dtype == torch.float32) and kernel_name(p) == "generic":
             scratch = _call_scratch(workspace_size(p), q.device, s)
             ptr, nbytes = (None, 0) if scratch is None else (scratch.data_ptr(), scratch.numel())
@@ -266,23 +305,25 @@ def make_step_params(q, k_cache, v_cache, k_new, v_new, rotary, o, scale, total_
                      sliding_window=0) -> DecodeStepParams:
     """k_cache / v_cache: [B, capacity, Hkv, D]; the step attends over their first `total_len` rows, of which
     the last k_new.shape[1] are written by the call."""
-    sp = DecodeStepParams()
-    sp.attn = make_params(q, k_cache[:, :total_len], v_cache[:, :total_len], o, scale, is_causal, None, lse, flags, sinks,
-                          sliding_window)
-    sp.k_new, sp.v_new = _view4(k_new), _view4(v_new)
-    sp.T_new = k_new.shape[1]
+    total_len = int(total_len)
+    if not 0 < total_len <= min(k_cache.shape[1], v_cache.shape[1]):  # the slices' own rules for anything else
+        k_cache, v_cache = k_cache[:, :total_len], v_cache[:, :total_len]
+        total_len = None
+    attn = _pack_params(q, k_cache, v_cache, o, scale, is_causal, None, lse, flags, sinks, sliding_window, None, None, 0, 0, total_len)
+    T_new = k_new.shape[1]
+    rot = (0, 0, 0)
     if rotary is not None:
-        assert rotary.dim() == 3 and rotary.dtype == q.dtype and rotary.shape[1] == k_new.shape[1]
-        assert rotary.stride(2) == 1
-        sp.rotary = rotary.data_ptr()
-        sp.rotary_stride_b = rotary.stride(0) if rotary.shape[0] > 1 else 0
-        sp.rotary_stride_s = rotary.stride(1)
-    for name, wt in (("q_norm_weight", q_norm_weight), ("k_norm_weight", k_norm_weight)):
+        assert rotary.dim() == 3 and rotary.dtype == q.dtype and rotary.shape[1] == T_new
+        st = rotary.stride()
+        assert st[2] == 1
+        rot = (rotary.data_ptr(), st[0] if rotary.shape[0] > 1 else 0, st[1])
+    weights = [0, 0]
+    for i, wt in enumerate((q_norm_weight, k_norm_weight)):
         if wt is not None:
             assert wt.dtype == q.dtype and wt.is_contiguous() and wt.numel() == q.shape[3]
-            setattr(sp, name, wt.data_ptr())
-    sp.norm_eps = float(norm_eps)
-    return sp
+            weights[i] = wt.data_ptr()
+    return DecodeStepParams.from_buffer_copy(_PACK_STEP.pack(attn, *_quad(k_new), *_quad(v_new), T_new, *rot, *weights,
+                                                             _f32(norm_eps)))
 
 
 def decode_step(q, k_cache, v_cache, k_new, v_new, rotary, scale, cached_len, out=None, lse=None, workspace=None,
@@ -292,15 +333,14 @@ def decode_step(q, k_cache, v_cache, k_new, v_new, rotary, scale, cached_len, ou
     [cached_len, cached_len + T_new) and return causal attention of the rotated queries over rows
     [0, cached_len + T_new).  q holds the last Sq <= T_new tokens' queries."""
     assert q.is_cuda, "the fused decode step takes device tensors"
-    B, Sq, Hq, D = q.shape
     if out is None:
-        out = torch.empty((B, Sq, Hq, D), dtype=q.dtype, device=q.device)
+        out = _new_output(q)
     sp = make_step_params(q, k_cache, v_cache, k_new, v_new, rotary, out, scale, cached_len + k_new.shape[1], True, lse,
                           flags, q_norm_weight, k_norm_weight, norm_eps, sinks, sliding_window)
     need = ctypes.c_size_t(0)
     _check(lib().dt_sdpa_decode_step_workspace_size(ctypes.byref(sp), ctypes.byref(need)),
            "dt_sdpa_decode_step_workspace_size")
-    s = stream if stream is not None else torch.cuda.current_stream(q.device).cuda_stream
+    s = _stream_of(q.device, stream)
     ws = workspace if workspace is not None else _default_workspace(q.device)
     ptr, nbytes = ws.ensure(need.value, s)
     _check(lib().dt_sdpa_decode_step(ctypes.byref(sp), ctypes.c_void_p(ptr) if ptr else None, nbytes,
@@ -310,25 +350,20 @@ def decode_step(q, k_cache, v_cache, k_new, v_new, rotary, scale, cached_len, ou
 
 def make_prologue_params(x, y, norm_weight=None, rotary=None, eps=1e-6, norm_per_token=False,
                          post_scale=1.0) -> QkPrologueParams:
-    p = QkPrologueParams()
-    p.B, p.S, p.H, p.D = x.shape
-    p.dtype = _DTYPES[x.dtype]
-    p.x, p.y = _view4(x), _view4(y)
+    B, S, H, D = x.shape
+    weight = 0
     if norm_weight is not None:
         assert norm_weight.dtype == x.dtype and norm_weight.is_contiguous()
-        assert norm_weight.numel() == (p.H * p.D if norm_per_token else p.D)
-        p.norm_weight = norm_weight.data_ptr()
-    p.norm_per_token = int(bool(norm_per_token))
-    p.eps = float(eps)
+        assert norm_weight.numel() == (H * D if norm_per_token else D)
+        weight = norm_weight.data_ptr()
+    rot = _NO_TENSOR
     if rotary is not None:
         assert rotary.dim() == 4 and rotary.dtype == x.dtype and rotary.stride(3) == 1
-        assert rotary.shape[1] == p.S and rotary.shape[3] == p.D
-        p.rotary = rotary.data_ptr()
-        p.rotary_stride_b = rotary.stride(0) if rotary.shape[0] > 1 else 0
-        p.rotary_stride_s = rotary.stride(1)
-        p.rotary_stride_h = rotary.stride(2) if rotary.shape[2] > 1 else 0
-    p.post_scale = float(post_scale)
-    return p
+        assert rotary.shape[1] == S and rotary.shape[3] == D
+        rot = (rotary.data_ptr(), rotary.stride(0) if rotary.shape[0] > 1 else 0, rotary.stride(1),
+               rotary.stride(2) if rotary.shape[2] > 1 else 0)
+    return QkPrologueParams.from_buffer_copy(_PACK_PROLOGUE.pack(
+        B, S, H, D, _DTYPES[x.dtype], *_quad(x), *_quad(y), weight, 1 if norm_per_token else 0, _f32(eps), *rot, _f32(post_scale)))
 
 
 def qk_prologue(q, k=None, *, q_out=None, k_out=None, q_weight=None, k_weight=None, rotary=None, rotary_k=None,
@@ -344,7 +379,7 @@ def qk_prologue(q, k=None, *, q_out=None, k_out=None, q_weight=None, k_weight=No
         k_out = torch.empty_like(k) if k_out is None else k_out
         pk = make_prologue_params(k, k_out, k_weight, rotary if rotary_k is None else rotary_k, eps, norm_per_token,
                                   post_scale)
-    s = stream if stream is not None else torch.cuda.current_stream(q.device).cuda_stream
+    s = _stream_of(q.device, stream)
     _check(lib().dt_qk_prologue(ctypes.byref(pq), ctypes.byref(pk) if pk is not None else None, ctypes.c_void_p(s)),
            "dt_qk_prologue")
     return q_out, k_out
@@ -371,7 +406,7 @@ def sdpa_forward_projected(q, k, v, scale, weight, bias=None, is_causal=False, o
     need = ctypes.c_size_t(0)
     _check(lib().dt_sdpa_projected_workspace_size(ctypes.byref(p), ctypes.byref(pr), ctypes.byref(need)),
            "dt_sdpa_projected_workspace_size")
-    s = stream if stream is not None else torch.cuda.current_stream(q.device).cuda_stream
+    s = _stream_of(q.device, stream)
     ws = workspace if workspace is not None else _default_workspace(q.device)
     ptr, nbytes = ws.ensure(need.value, s)
     _check(lib().dt_sdpa_forward_projected(ctypes.byref(p), ctypes.byref(pr), ctypes.c_void_p(ptr), nbytes,
@@ -389,31 +424,25 @@ def sparse_indexed_attention(q, k_raw, v_raw, k_comp, v_comp, selected, scale, s
     B, Sq, Hq, D = q.shape
     if out is None:
         out = torch.empty_like(q)
-    p = SparseIndexedParams()
-    p.B, p.Sq, p.Hq, p.Hkv, p.D = B, Sq, Hq, k_raw.shape[2], D
-    p.Sr = k_raw.shape[1]
-    p.Sc = 0 if k_comp is None else k_comp.shape[1]
-    p.dtype = _DTYPES[q.dtype]
-    p.scale = float(scale)
-    p.is_causal = int(bool(is_causal))
-    p.sliding_window = int(sliding_window)
-    p.flags = int(flags)
-    p.q, p.o, p.k_raw, p.v_raw = _view4(q), _view4(out), _view4(k_raw), _view4(v_raw)
-    if k_comp is not None and p.Sc > 0:
-        p.k_comp, p.v_comp = _view4(k_comp), _view4(v_comp)
+    Sc = 0 if k_comp is None else k_comp.shape[1]
+    comp = (_quad(k_comp), _quad(v_comp)) if Sc > 0 else (_NO_TENSOR, _NO_TENSOR)
+    n_selected, sel = 0, (0, 0, 0)
     if selected is not None:
         assert selected.dtype == torch.int32 and selected.dim() == 3 and selected.shape[1] == Sq and selected.stride(2) == 1
-        p.n_selected = selected.shape[2]
-        p.selected = selected.data_ptr()
-        p.selected_stride_b = selected.stride(0) if selected.shape[0] > 1 else 0
-        p.selected_stride_q = selected.stride(1)
+        n_selected = selected.shape[2]
+        sel = (selected.data_ptr(), selected.stride(0) if selected.shape[0] > 1 else 0, selected.stride(1))
+    sinks_ptr = lse_ptr = 0
     if sinks is not None:
         assert sinks.dtype == q.dtype and sinks.is_contiguous() and sinks.numel() == Hq
-        p.sinks = sinks.data_ptr()
+        sinks_ptr = sinks.data_ptr()
     if lse is not None:
         assert lse.dtype == torch.float32 and lse.is_contiguous() and tuple(lse.shape) == (B, Hq, Sq)
-        p.lse = lse.data_ptr()
-    s = stream if stream is not None else torch.cuda.current_stream(q.device).cuda_stream
+        lse_ptr = lse.data_ptr()
+    p = SparseIndexedParams.from_buffer_copy(_PACK_SPARSE.pack(
+        B, Sq, Hq, k_raw.shape[2], D, k_raw.shape[1], Sc, n_selected, _DTYPES[q.dtype], _f32(scale), 1 if is_causal else 0,
+        int(sliding_window), *_quad(q), *_quad(out), *_quad(k_raw), *_quad(v_raw), *comp[0], *comp[1], *sel, sinks_ptr, lse_ptr,
+        int(flags) & 0xffffffff))
+    s = _stream_of(q.device, stream)
     _check(lib().dt_sparse_indexed_attention(ctypes.byref(p), ctypes.c_void_p(s)), "dt_sparse_indexed_attention")
     return out
 
@@ -514,6 +543,15 @@ class ScaledDotProductAttention:
         if GEMMFlag.Int8 in f:
             raise NotImplementedError("quantised attention ([.Int8, .Float16]) is never selected off Metal")
 
+    @property
+    def flags(self):
+        return self._flags
+
+    @flags.setter
+    def flags(self, f):
+        self._flags = f
+        self._abi_flags = DT_FLAG_FP16_ACCUM_HINT if GEMMFlag.Float16 in f else 0
+
     def set_output_projection(self, weight, bias=None):
         self.weight, self.bias = weight, bias
 
@@ -537,7 +575,6 @@ class ScaledDotProductAttention:
             raise ValueError("more inputs than the operator was built for")
         if self.has_attention_mask != (mask is not None):
             raise ValueError("hasAttentionMask and the number of inputs disagree")
-        abi_flags = DT_FLAG_FP16_ACCUM_HINT if GEMMFlag.Float16 in self.flags else 0
         if self.multi_head_output_projection_fused:
             if self.weight is None:
                 raise ValueError("multiHeadOutputProjectionFused: set_output_projection(weight, bias) first")
@@ -545,7 +582,7 @@ class ScaledDotProductAttention:
                 raise NotImplementedError("the fused output projection takes the plain operator only")
             return sdpa_forward_projected(queries, keys, values, self.scale, self.weight, self.bias, self.is_causal, out=out)
         mq, mk = self.max_sequence_length if self.max_sequence_length else (0, 0)
-        return sdpa_forward(queries, keys, values, self.scale, self.is_causal, mask, out=out, lse=lse, flags=abi_flags,
+        return sdpa_forward(queries, keys, values, self.scale, self.is_causal, mask, out=out, lse=lse, flags=self._abi_flags,
                             sinks=sinks, sliding_window=self.sliding_window, seq_offsets_q=offs_q, seq_offsets_k=offs_k,
                             max_seq_q=mq, max_seq_k=mk)
 
