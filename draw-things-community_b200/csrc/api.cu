@@ -138,6 +138,18 @@ bool make_bshd_tensor_map(CUtensorMap* map, const dt_tensor4& t, int B, int S, i
   return true;
 }
 
+bool make_rows_tensor_map(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols, int64_t row_stride, int dtype) {
+  EncodeTiledFn enc = get_encode_tiled();
+  if (!enc || (dtype != DT_F16 && dtype != DT_BF16) || reinterpret_cast<uintptr_t>(ptr) % 16) return false;
+  if (rows <= 0 || cols <= 0 || rows > 0x7fffffff || cols > 0x7fffffff) return false;
+  if (row_stride <= 0 || row_stride % 8 || row_stride >= ((int64_t)1 << 39)) return false;
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)row_stride * 2};
+  cuuint32_t box[2] = {64, 1}, estr[2] = {1, 1};
+  return enc(map, dtype == DT_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr),
+             dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // ---- validation and dispatch -------------------------------------------------------------------------
 
 int validate_params(const dt_sdpa_params* p) {

@@ -70,6 +70,11 @@ int launch_prefill_repack(const dt_sdpa_params& p, cudaStream_t stream, void* wo
 bool short_kv_supported(const dt_sdpa_params& p);
 int launch_short_kv(const dt_sdpa_params& p, cudaStream_t stream);
 
+// Sparse indexed attention of many tokens on tcgen05 (the shapes sparse_tcgen05_supported names; 16-bit tensors with
+// 16-byte aligned rows are the caller's check).
+bool sparse_tcgen05_supported(const dt_sparse_indexed_params& p, bool same_kv);
+int launch_sparse_tcgen05(const dt_sparse_indexed_params& p, cudaStream_t stream);
+
 // C[B,S,N] = A[B,S,K] . W[N,K]^T + bias: the output projection behind the attention kernel (TMA + tcgen05 GEMM).
 int launch_out_proj(const dt_tensor4& a_view, int B, int S, int K, const void* weight, const void* bias, int N,
                     const dt_tensor4& out, int dtype, cudaStream_t stream);

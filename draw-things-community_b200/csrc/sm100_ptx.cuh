@@ -125,6 +125,16 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
+// Four rows of a 2-D map whose box is one row high, named one by one (a row outside the tensor reads as zeros): 4 x box
+// width elements to consecutive rows at smem_dst.
+__device__ __forceinline__ void tma_gather4_2d(uint32_t smem_dst, const CUtensorMap* map, uint64_t* bar, int col, int r0, int r1,
+                                               int r2, int r3) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(col), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
+      : "memory");
+}
+
 // Same tile, but only pulled into L2 (no shared-memory destination, no barrier).
 __device__ __forceinline__ void tma_prefetch_l2_4d(const CUtensorMap* map, int c0, int c1, int c2, int c3) {
   asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(
@@ -243,10 +253,54 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_
       : "memory");
 }
 
+// The same two for a whole warp in converged control flow, of which only the lane that passes on = true issues: the operands
+// stay in uniform registers, where an issue from inside a one-lane branch moves them there one by one and takes longer than
+// a narrow MMA runs.
+__device__ __forceinline__ void mma_ss_on(bool on, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "}\n" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"((uint32_t)on)
+      : "memory");
+}
+__device__ __forceinline__ void mma_ts_on(bool on, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"((uint32_t)on)
+      : "memory");
+}
+// One lane of a converged warp, the same one every time.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t is;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(is));
+  return is != 0;
+}
+
 // The mbarrier observes completion of every tcgen05 op this thread issued before.
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
+}
+
+__device__ __forceinline__ void tc_commit_on(bool on, uint64_t* bar) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+      "}\n" ::"r"(smem_u32(bar)), "r"((uint32_t)on)
+      : "memory");
 }
 
 // 32 lanes x 32-bit, 32 consecutive columns: thread i of the warp reads TMEM lane (base lane + i).
@@ -406,5 +460,9 @@ EncodeTiledFn get_encode_tiled();
 // not meet TMA's rules (16-byte aligned base, strides multiples of 16 bytes).
 bool make_bshd_tensor_map(CUtensorMap* map, const dt_tensor4& t, int B, int S, int H, int D, int dtype,
                           int box_rows);
+
+// 2-D map over `rows` rows of `cols` 16-bit elements, `row_stride` elements apart, box [64, 1] (for tma_gather4_2d),
+// 128-byte swizzle, zero fill out of bounds.
+bool make_rows_tensor_map(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols, int64_t row_stride, int dtype);
 
 }  // namespace dt

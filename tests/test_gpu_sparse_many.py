@@ -1,0 +1,65 @@
+"""Sparse indexed attention of many tokens (the tcgen05 kernel: 64 heads per KV head, values = keys, head dim 256 or 512)
+against the oracle, at the edges of its 48-key tiles, its head groups and its dispatch."""
+import pytest
+import torch
+
+from oracle import sdpa_oracle as so
+from test_gpu_parity import DEV
+from test_gpu_sparse_indexed import ROUND, make_case
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("case", [
+    # B, Sq, Sr, Sc, n_sel, Hq, Hkv, D, dtype, window, sinks, causal
+    (1, 64, 64, 0, 0, 64, 1, 512, torch.bfloat16, 48, True, True),      # one tile at most, the smallest dispatched count
+    (1, 70, 120, 30, 1, 64, 1, 512, torch.float16, 48, True, True),     # one key more than a tile
+    (1, 150, 300, 64, 48, 64, 1, 512, torch.bfloat16, 128, True, True),  # more tokens than SMs: a second token per CTA
+    (1, 320, 500, 90, 200, 64, 1, 512, torch.float16, 128, False, True),  # lists longer than the rows, no sinks, third tokens
+    (2, 70, 100, 40, 33, 128, 1, 512, torch.bfloat16, 0, True, True),   # two head groups, batch, no window
+    (1, 40, 90, 25, 60, 128, 2, 256, torch.float16, 20, True, True),    # two KV heads, head dim 256
+    (1, 80, 100, 16, 16, 64, 1, 256, torch.bfloat16, 0, True, False),   # every token sees every raw row
+])
+def test_against_the_oracle(dtattn, case):
+    B, Sq, Sr, Sc, n_sel, Hq, Hkv, D, dtype, window, with_sinks, causal = case
+    q, kr, _, kc, _, sel, sinks = make_case(B, Sq, Sr, Sc, n_sel, Hq, Hkv, D, dtype, 1501, per_batch_lists=B > 1)
+    if not with_sinks:
+        sinks = None
+    if n_sel:
+        sel[:, 3] = -1  # a token without any selected row
+    ref, ref_lse = so.sparse_indexed_explicit(q, kr, kr, kc if Sc else None, kc if Sc else None, sel if n_sel else None, D ** -0.5,
+                                              sinks, window, compute_dtype=torch.float64, return_lse=True, is_causal=causal)
+    rd, cd = kr.to(DEV), kc.to(DEV) if Sc else None
+    wide = torch.full((B, Sq, Hq, D + 64), 7.0, dtype=dtype, device=DEV)
+    lse = torch.full((B, Hq, Sq), float("nan"), device=DEV)
+    out = dtattn.sparse_indexed_attention(q.to(DEV), rd, rd, cd, cd, sel.to(DEV) if n_sel else None, D ** -0.5,
+                                          None if sinks is None else sinks.to(DEV), window, is_causal=causal, out=wide[..., :D], lse=lse)
+    torch.cuda.synchronize()
+    assert dtattn.device_status() == 0
+    got = out.float().cpu()
+    assert torch.isfinite(got).all() and bool((wide[..., D:] == 7.0).all())
+    mx, mean = so.error_stats(got, ref.float())
+    assert mx <= so.TOL_MAX_ABS + 2 * ROUND[dtype] * float(ref.abs().max()), (case, mx)
+    assert mean <= so.TOL_MEAN_ABS + ROUND[dtype] * float(ref.abs().mean()), (case, mean)
+    assert (lse.cpu().double() - ref_lse).abs().max() < 2e-3
+
+
+def test_growing_scores_and_hidden_tokens(dtattn):
+    """Keys ordered so that every tile raises each head's maximum by more than the rescale threshold, and tokens that see
+    nothing at all (zeros without sinks)."""
+    B, Sq, Sr, Hq, D, dtype = 1, 66, 400, 64, 512, torch.bfloat16
+    q = torch.ones(B, Sq, Hq, D, dtype=dtype) * 0.25
+    kr = (torch.linspace(0.01, 3.0, Sr).view(1, Sr, 1, 1) * torch.ones(D)).to(dtype) + so.seeded_normal((1, Sr, 1, D), 1511).to(dtype) * 0.1
+    ref = so.sparse_indexed_explicit(q, kr, kr, None, None, None, 1.0, None, 350, compute_dtype=torch.float64)
+    out = dtattn.sparse_indexed_attention(q.to(DEV), kr.to(DEV), (d := kr.to(DEV)), None, None, None, 1.0, None, 350)
+    same = dtattn.sparse_indexed_attention(q.to(DEV), d, d, None, None, None, 1.0, None, 350)
+    torch.cuda.synchronize()
+    assert dtattn.device_status() == 0
+    for got in (out, same):
+        assert float((got.float().cpu() - ref.float()).abs().max()) <= 2 * ROUND[dtype] * float(ref.abs().max()) + so.TOL_MAX_ABS
+    sel = torch.full((1, Sq, 5), -1, dtype=torch.int32, device=DEV)
+    comp = torch.full((1, 7, 1, D), float("nan"), dtype=dtype, device=DEV)  # rows nobody names are never used
+    empty = torch.zeros(1, 1, 1, D, dtype=dtype, device=DEV)[:, :0]
+    got = dtattn.sparse_indexed_attention(q.to(DEV), empty, empty, comp, comp, sel, 1.0, None, 128)
+    torch.cuda.synchronize()
+    assert dtattn.device_status() == 0 and bool((got == 0).all())
