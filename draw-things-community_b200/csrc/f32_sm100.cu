@@ -11,30 +11,35 @@
 // take the small partial products first, and O is accumulated over ONE block of keys in TMEM and added to fp32 registers
 // from there, rounded to nearest.
 //
-// f32_tcgen05_kernel: one CTA = one (batch, head, 128 query rows) at a time, persistent over the work items.  8 warps:
+// f32_tcgen05_kernel: one CTA = one (batch, head, 128 query rows) at a time, persistent over the work items.  12 warps:
 //   warp 0      TMA producer: Q planes per item, then K and V planes of kBN keys through a ring in the order
 //               K(0) K(1) V(0) K(2) V(1) ...
 //   warp 1      MMA issuer: S = Q K^T (6 * D/16 products per block, both operands in shared memory), O_blk = P V
 //               (P in TMEM), ordered QK(0) QK(1) | PV(0) QK(2) | PV(1) QK(3) | ... over two S buffers
 //   warp 2      TMEM allocation / release
-//   warps 4-7   softmax, one thread per query row: scores -> weights -> three bf16 planes over the S columns, then the
-//               previous block's O from TMEM into the row's fp32 accumulators
+//   warps 4-7   softmax of the first half of every block's keys, one thread per query row: scores -> weights -> three
+//               bf16 planes over the S columns, then the previous block's O from TMEM into the row's fp32 accumulators
+//   warps 8-11  the same for the second half, with a maximum, a sum and an O of their own; the two are put together when
+//               the item ends
+// The halves need nothing from each other while an item runs, so a scheduler has two warps to choose from, and a thread
+// with 64 scores has registers left to work on several at a time (one warpgroup for all 128 spent 100 cycles on each pair
+// of weights, the latency of the chain, and the call took 700 us).
 // Measured (SD1.5 upcast self-attention: 2 images, 4096 tokens, 8 heads of 40): 3309 us on the CUDA cores (fp32 multiply-
-// adds, 13 TFLOP/s), 700 us here; error against 64 bits 1.2e-6 there, 3.9e-7 here (2-norm, relative).
-// Per 128 x 128 scores at D = 40 it needs 18 N=128 MMAs for Q K^T and 48 N=48 MMAs for P V, 2304
-// cycles, under which the softmax of the other buffer (about seven instructions per score) runs.
+// adds, 13 TFLOP/s), 301 us here; error against 64 bits 1.2e-6 there, 3.9e-7 here (2-norm, relative).
+// Per 128 x 128 scores at D = 40 the tensor pipe has 18 N=128 MMAs for Q K^T and 48 N=48 MMAs for P V.
 // Every mbarrier wait is bounded, as in the half-precision kernel.
 //
 // Inputs that hold an infinity, a NaN or a magnitude of 2^58 and above (a score of 128 such products may leave the fp32
-// range) are not for this kernel: split_planes_kernel reports them, f32_tcgen05_kernel then does nothing and the CUDA-core kernel behind
-// it in the stream, which otherwise returns at once, computes the call.
+// range) are not for this kernel: split_planes_kernel reports them, f32_tcgen05_kernel then does nothing and the CUDA-core
+// kernel behind it in the stream, which otherwise returns at once, computes the call.
 #include "sm100_ptx.cuh"
 
 namespace dt {
 namespace {
 
 constexpr int kBM = 128;
-constexpr int kThreads = 256;
+constexpr int kThreads = 384;
+constexpr int kRegsLow = 80, kRegsHigh = 208;  // 128 * low + 256 * high <= 384 threads * 168 at launch
 constexpr int kSplitThreads = 256;
 constexpr int kSplitCtas = 1184;  // 8 per SM: the flag words in front of the planes are this many
 
@@ -50,18 +55,20 @@ struct F32Cfg {
   static constexpr int kQBytes = 3 * kQPlane;
   static constexpr int kSlotBytes = 3 * kKvPlane;
   static constexpr int kSlots = NPV > 64 ? 2 : 3;
-  static constexpr int kSmemBytes = kQBytes + kSlots * kSlotBytes + 256 + 1024;
-  static constexpr uint32_t kPlaneCols = kBN / 2;       // TMEM columns of one 16-bit plane of P
-  static constexpr uint32_t kBufCols = 3 * kPlaneCols;  // S (kBN columns) and the planes of P over it
-  static constexpr uint32_t kColO = 2 * kBufCols;
-  static_assert(kColO + NPV <= 512, "TMEM columns");
+  static constexpr int kSmemBytes = kQBytes + kSlots * kSlotBytes + 256 + 2 * kBM * 4 + 1024;
+  static constexpr int kHN = kBN / 2;                   // keys of a softmax warpgroup's half
+  // TMEM columns of a buffer: S, whose halves the first two planes of the halves' P overwrite, and behind it the third
+  static constexpr uint32_t kBufCols = kBN + kHN;
+  static constexpr uint32_t kColO = 2 * kBufCols;       // two of NPV columns
+  static_assert(kColO + 2 * NPV <= 512, "TMEM columns");
   static_assert(kSmemBytes <= 227 * 1024, "shared memory");
 };
 
 struct F32Bars {
   uint64_t q_full, q_empty;
-  uint64_t s_full[2], p_full[2];
-  uint64_t o_full;  // completes once per P V
+  uint64_t s_full[2], p_full[2][2];  // [buffer], [half][buffer]
+  uint64_t o_full[2];                // [half] completes once per block's P V
+  uint64_t x_full, x_empty;          // the second half's O, maximum and sum of a finished item: there / read
   uint64_t kv_full[3], kv_empty[3];
   uint32_t tmem_base;
   int abort_flag;
@@ -148,14 +155,19 @@ f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   F32Bars* bars = reinterpret_cast<F32Bars*>(base_ptr + C::kQBytes + C::kSlots * C::kSlotBytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+  float* xch = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);  // [2][kBM]: the second half's maximum, sum
+
   if (threadIdx.x == 0) {
     ptx::mbar_init(&bars->q_full, 1);
     ptx::mbar_init(&bars->q_empty, 1);
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(&bars->s_full[i], 1);
-      ptx::mbar_init(&bars->p_full[i], 4);  // one arrival per softmax warp
+      ptx::mbar_init(&bars->p_full[0][i], 4);  // one arrival per softmax warp
+      ptx::mbar_init(&bars->p_full[1][i], 4);
+      ptx::mbar_init(&bars->o_full[i], 1);
     }
-    ptx::mbar_init(&bars->o_full, 1);
+    ptx::mbar_init(&bars->x_full, 4);
+    ptx::mbar_init(&bars->x_empty, 4);
     for (int i = 0; i < C::kSlots; ++i) {
       ptx::mbar_init(&bars->kv_full[i], 1);
       ptx::mbar_init(&bars->kv_empty[i], 1);
@@ -180,57 +192,60 @@ f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   const int nkv = (a.Sk + kBN - 1) / kBN, G = a.Hq / a.Hkv;
   const int dsteps = (a.D + 15) >> 4;  // k-steps of Q K^T (columns beyond D are zeros in both operands)
 
-  if (warp == 0) {
-    // =========================== TMA producer ===========================
-    if (lane == 0) {
-      ptx::prefetch_tensormap(&map_q);
-      ptx::prefetch_tensormap(&map_k);
-      ptx::prefetch_tensormap(&map_v);
-      const int halves = (a.D + 63) >> 6;  // 64-column halves that exist (the second one of a plane is 16-byte aligned too)
-      int slot = 0, n_item = 0;
-      uint32_t par = 1;  // parity of kv_empty: the first round over the ring passes at once
-      bool ok = true;
-      auto fail = [&]() {
-        atomicCAS(a.status, 0u, 2u);
-        *abort_flag = 1;
-        ok = false;
-        return false;
-      };
-      for (int item = blockIdx.x; item < a.n_items && ok; item += gridDim.x, ++n_item) {
-        const int qt = item % a.n_qt, bh = item / a.n_qt, h = bh % a.Hq, b = bh / a.Hq, kvh = h / G;
-        auto load_kv = [&](const CUtensorMap* map, int j) -> bool {
-          if (!ptx::mbar_wait(&bars->kv_empty[slot], par, abort_flag)) return fail();
-          ptx::mbar_arrive_expect_tx(&bars->kv_full[slot], (uint32_t)(3 * halves * C::kKvHalf));
+  if (warp < 4) {
+    ptx::setmaxnreg_dec<kRegsLow>();
+    if (warp == 0) {
+      // =========================== TMA producer ===========================
+      if (lane == 0) {
+        ptx::prefetch_tensormap(&map_q);
+        ptx::prefetch_tensormap(&map_k);
+        ptx::prefetch_tensormap(&map_v);
+        const int halves = (a.D + 63) >> 6;  // 64-column halves of a plane that exist
+        int slot = 0, n_item = 0;
+        uint32_t par = 1;  // parity of kv_empty: the first round over the ring passes at once
+        bool ok = true;
+        auto fail = [&]() {
+          atomicCAS(a.status, 0u, 2u);
+          *abort_flag = 1;
+          ok = false;
+          return false;
+        };
+        for (int item = blockIdx.x; item < a.n_items && ok; item += gridDim.x, ++n_item) {
+          const int qt = item % a.n_qt, bh = item / a.n_qt, h = bh % a.Hq, b = bh / a.Hq, kvh = h / G;
+          auto load_kv = [&](const CUtensorMap* map, int j) -> bool {
+            if (!ptx::mbar_wait(&bars->kv_empty[slot], par, abort_flag)) return fail();
+            ptx::mbar_arrive_expect_tx(&bars->kv_full[slot], (uint32_t)(3 * halves * C::kKvHalf));
+            for (int p = 0; p < 3; ++p)
+              for (int hf = 0; hf < halves; ++hf)
+                ptx::tma_load_4d(base_ptr + C::kQBytes + slot * C::kSlotBytes + p * C::kKvPlane + hf * C::kKvHalf, map,
+                                 &bars->kv_full[slot], hf * 64, kvh * 3 + p, j * kBN, b);
+            if (++slot == C::kSlots) { slot = 0; par ^= 1; }
+            return true;
+          };
+          if (!load_kv(&map_k, 0)) break;
+          if (n_item > 0 && !ptx::mbar_wait(&bars->q_empty, (n_item - 1) & 1, abort_flag)) { fail(); break; }
+          ptx::mbar_arrive_expect_tx(&bars->q_full, (uint32_t)(3 * halves * kBM * 128));
           for (int p = 0; p < 3; ++p)
             for (int hf = 0; hf < halves; ++hf)
-              ptx::tma_load_4d(base_ptr + C::kQBytes + slot * C::kSlotBytes + p * C::kKvPlane + hf * C::kKvHalf, map,
-                               &bars->kv_full[slot], hf * 64, kvh * 3 + p, j * kBN, b);
-          if (++slot == C::kSlots) { slot = 0; par ^= 1; }
-          return true;
-        };
-        if (!load_kv(&map_k, 0)) break;
-        if (n_item > 0 && !ptx::mbar_wait(&bars->q_empty, (n_item - 1) & 1, abort_flag)) { fail(); break; }
-        ptx::mbar_arrive_expect_tx(&bars->q_full, (uint32_t)(3 * halves * kBM * 128));
-        for (int p = 0; p < 3; ++p)
-          for (int hf = 0; hf < halves; ++hf)
-            ptx::tma_load_4d(base_ptr + p * C::kQPlane + hf * kBM * 128, &map_q, &bars->q_full, hf * 64, h * 3 + p, qt * kBM, b);
-        if (nkv > 1 && !load_kv(&map_k, 1)) break;
-        for (int j = 0; j < nkv && ok; ++j) ok = load_kv(&map_v, j) && (j + 2 >= nkv || load_kv(&map_k, j + 2));
+              ptx::tma_load_4d(base_ptr + p * C::kQPlane + hf * kBM * 128, &map_q, &bars->q_full, hf * 64, h * 3 + p, qt * kBM, b);
+          if (nkv > 1 && !load_kv(&map_k, 1)) break;
+          for (int j = 0; j < nkv && ok; ++j) ok = load_kv(&map_v, j) && (j + 2 >= nkv || load_kv(&map_k, j + 2));
+        }
       }
-    }
-  } else if (warp == 1) {
-    // =========================== MMA issuer ===========================
-    if (lane == 0) {
+    } else if (warp == 1) {
+      // =========================== MMA issuer (the whole warp, one lane issues) ===========================
+      const bool on = ptx::elect_one();
       constexpr uint32_t idesc_qk = ptx::make_idesc_f16(1, kBM, kBN, 0, 0);
       constexpr uint32_t idesc_pv = ptx::make_idesc_f16(1, kBM, NPV, 0, 1);
       const uint64_t q_desc = ptx::make_smem_desc_sw128(base, 16, 1024);
       const uint64_t k_desc = ptx::make_smem_desc_sw128(ring_smem, 16, 1024);
       const uint64_t v_desc = ptx::make_smem_desc_sw128(ring_smem, C::kKvHalf, 1024);
       int slot = 0, n_item = 0;
-      uint32_t par = 0, g = 0;  // g: key blocks handed to the tensor pipe so far; its low bit names the S buffer
+      uint32_t par = 0, g = 0;  // g: key blocks handed to the tensor pipe before this item; block g + j uses S buffer (g + j) & 1
       bool ok = true;
-      auto fail = [&](unsigned code) {
-        atomicCAS(a.status, 0u, code);
+      auto wait = [&](uint64_t* bar, uint32_t parity, unsigned code) -> bool {
+        if (__all_sync(0xffffffffu, ptx::mbar_wait(bar, parity, abort_flag))) return true;
+        if (on) atomicCAS(a.status, 0u, code);
         *abort_flag = 1;
         ok = false;
         return false;
@@ -239,86 +254,91 @@ f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         if (++slot == C::kSlots) { slot = 0; par ^= 1; }
       };
       for (int item = blockIdx.x; item < a.n_items && ok; item += gridDim.x, ++n_item) {
-        if (!ptx::mbar_wait(&bars->q_full, n_item & 1, abort_flag)) { fail(1u); break; }
+        if (!wait(&bars->q_full, n_item & 1, 1u)) break;
         auto qk = [&](int j) -> bool {
-          if (!ptx::mbar_wait(&bars->kv_full[slot], par, abort_flag)) return fail(1u);
+          if (!wait(&bars->kv_full[slot], par, 1u)) return false;
           ptx::tc_fence_after();
           const uint32_t buf = (g + (uint32_t)j) & 1u;
           const uint64_t kd = k_desc + (uint64_t)(slot * (C::kSlotBytes >> 4));
 #pragma unroll
-          for (int i = 0; i < 6; ++i) {
-            const uint64_t qp = q_desc + (uint64_t)(kProdA[i] * (C::kQPlane >> 4)), kp = kd + (uint64_t)(kProdB[i] * (C::kKvPlane >> 4));
-            for (int ks = 0; ks < dsteps; ++ks)
-              ptx::mma_ss(tmem + buf * C::kBufCols, qp + (uint64_t)(((ks >> 2) * (kBM * 128) + (ks & 3) * 32) >> 4),
-                          kp + (uint64_t)(((ks >> 2) * C::kKvHalf + (ks & 3) * 32) >> 4), idesc_qk, (i | ks) ? 1u : 0u);
-          }
-          ptx::tc_commit(&bars->s_full[buf]);
-          ptx::tc_commit(&bars->kv_empty[slot]);
-          if (j == nkv - 1) ptx::tc_commit(&bars->q_empty);
+          for (int i = 0; i < 6; ++i)
+#pragma unroll
+            for (int ks = 0; ks < (NPV + 15) / 16; ++ks)
+              if (ks < dsteps)
+                ptx::mma_ss_on(on, tmem + buf * C::kBufCols,
+                               q_desc + (uint64_t)((kProdA[i] * C::kQPlane + (ks >> 2) * (kBM * 128) + (ks & 3) * 32) >> 4),
+                               kd + (uint64_t)((kProdB[i] * C::kKvPlane + (ks >> 2) * C::kKvHalf + (ks & 3) * 32) >> 4), idesc_qk,
+                               (i | ks) ? 1u : 0u);
+          ptx::tc_commit_on(on, &bars->s_full[buf]);
+          ptx::tc_commit_on(on, &bars->kv_empty[slot]);
+          if (j == nkv - 1) ptx::tc_commit_on(on, &bars->q_empty);
           advance();
           return true;
         };
         if (!qk(0) || (nkv > 1 && !qk(1))) break;
         for (int j = 0; j < nkv && ok; ++j) {
           const uint32_t gj = g + (uint32_t)j, buf = gj & 1u;
-          const int ksteps = (min(kBN, a.Sk - j * kBN) + 15) >> 4;
-          if (!ptx::mbar_wait(&bars->kv_full[slot], par, abort_flag)) { fail(1u); break; }
-          if (!ptx::mbar_wait(&bars->p_full[buf], (gj >> 1) & 1u, abort_flag)) { fail(4u); break; }
+          const int left = a.Sk - j * kBN;
+          if (!wait(&bars->kv_full[slot], par, 1u)) break;
+          // both halves, then their MMAs in turn: neighbours in the pipe do not wait for each other's accumulator
+          if (!wait(&bars->p_full[0][buf], (gj >> 1) & 1u, 4u) || !wait(&bars->p_full[1][buf], (gj >> 1) & 1u, 4u)) break;
           ptx::tc_fence_after();
+          const uint32_t pb = tmem + buf * C::kBufCols;
           const uint64_t vd = v_desc + (uint64_t)(slot * (C::kSlotBytes >> 4));
+          const int steps0 = min(C::kHN, left + 15) >> 4, steps1 = min(C::kHN, max(left - C::kHN, 1) + 15) >> 4;  // (P is zero beyond the keys)
 #pragma unroll
-          for (int i = 0; i < 6; ++i) {
-            const uint32_t pp = tmem + buf * C::kBufCols + kProdA[i] * C::kPlaneCols;
-            const uint64_t vp = vd + (uint64_t)(kProdB[i] * (C::kKvPlane >> 4));
-            if (ksteps == kBN / 16) {  // unrolled: an N=48 MMA lasts 24 cycles, a looped issue longer
+          for (int i = 0; i < 6; ++i)
 #pragma unroll
-              for (int ks = 0; ks < kBN / 16; ++ks)
-                ptx::mma_ts(tmem + C::kColO, pp + ks * 8, vp + (uint64_t)(ks * (2048 >> 4)), idesc_pv, (i | ks) ? 1u : 0u);
-            } else {
-#pragma unroll 1
-              for (int ks = 0; ks < ksteps; ++ks)
-                ptx::mma_ts(tmem + C::kColO, pp + ks * 8, vp + (uint64_t)(ks * (2048 >> 4)), idesc_pv, (i | ks) ? 1u : 0u);
-            }
-          }
-          ptx::tc_commit(&bars->kv_empty[slot]);
-          ptx::tc_commit(&bars->o_full);
+            for (int ks = 0; ks < C::kHN / 16; ++ks)
+#pragma unroll
+              for (int hf = 0; hf < 2; ++hf)
+                if (ks < (hf ? steps1 : steps0))
+                  ptx::mma_ts_on(on, tmem + C::kColO + hf * NPV,
+                                 pb + (kProdA[i] < 2 ? hf * C::kHN + kProdA[i] * (C::kHN / 2) : kBN + hf * (C::kHN / 2)) + ks * 8,
+                                 vd + (uint64_t)((kProdB[i] * C::kKvPlane + (hf * (C::kHN / 16) + ks) * 2048) >> 4), idesc_pv,
+                                 (i | ks) ? 1u : 0u);
+          ptx::tc_commit_on(on, &bars->kv_empty[slot]);
+          ptx::tc_commit_on(on, &bars->o_full[0]);
+          ptx::tc_commit_on(on, &bars->o_full[1]);
           advance();
           if (j + 2 < nkv && !qk(j + 2)) break;  // into the columns the P V above has just read
         }
         g += (uint32_t)nkv;
       }
     }
-  } else if (warp >= 4) {
+  } else {
+    ptx::setmaxnreg_inc<kRegsHigh>();
     // =========================== softmax / accumulation / store ===========================
+    const int hf = (warp - 4) >> 2;  // which half of a block's keys
     const int row_in_tile = ((warp & 3) << 5) + lane;
-    const uint32_t tl = tmem + ((uint32_t)((warp & 3) << 5) << 16);
+    const uint32_t tl = tmem + ((uint32_t)((warp & 3) << 5) << 16), t_o = tl + C::kColO + hf * NPV;
     const float sl2 = a.scale_log2;
     const uint64_t scale2 = ptx::pack_f32x2(sl2, sl2);
     uint32_t g = 0;  // key blocks seen so far
+    int n_item = 0;
     bool ok = true;
-    auto fail = [&](unsigned code) {
+    auto wait = [&](uint64_t* bar, uint32_t parity, unsigned code) -> bool {
+      if (__all_sync(0xffffffffu, ptx::mbar_wait(bar, parity, abort_flag))) return true;
       atomicCAS(a.status, 0u, code);
       *abort_flag = 1;
       ok = false;
+      return false;
     };
-    for (int item = blockIdx.x; item < a.n_items && ok; item += gridDim.x) {
+    for (int item = blockIdx.x; item < a.n_items && ok; item += gridDim.x, ++n_item) {
       const int qt = item % a.n_qt, bh = item / a.n_qt, h = bh % a.Hq, b = bh / a.Hq;
       const int row = qt * kBM + row_in_tile;
       float m = -INFINITY, l = 0.f;
-      uint64_t acc[NPV / 2];  // the row's output, two columns each
+      uint64_t acc[NPV / 2];  // the row's output over this half of the keys, two columns each
 #pragma unroll
       for (int i = 0; i < NPV / 2; ++i) acc[i] = 0ull;
       // a block's O (its P V has run) joins the row's accumulators
       auto add_block = [&](uint32_t block) -> bool {
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&bars->o_full, block & 1u, abort_flag))) {
-          fail(5u);
-          return false;
-        }
+        if (!wait(&bars->o_full[hf], block & 1u, 5u)) return false;
         ptx::tc_fence_after();
 #pragma unroll
         for (int c = 0; c < NPV / 16; ++c) {
           uint32_t ov[16];
-          ptx::tmem_ld16(tl + C::kColO + c * 16, ov);
+          ptx::tmem_ld16(t_o + c * 16, ov);
           ptx::tc_wait_ld();
 #pragma unroll
           for (int i = 0; i < 8; ++i)
@@ -328,40 +348,42 @@ f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       };
       for (int j = 0; j < nkv; ++j, ++g) {
         const uint32_t buf = g & 1u, ts = tl + buf * C::kBufCols;
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&bars->s_full[buf], (g >> 1) & 1u, abort_flag))) {
-          fail(3u);
-          break;
-        }
+        if (!wait(&bars->s_full[buf], (g >> 1) & 1u, 3u)) break;
         ptx::tc_fence_after();
-        uint32_t s[kBN / 32][32];
+        uint32_t s[C::kHN / 32][32];
 #pragma unroll
-        for (int c = 0; c < kBN / 32; ++c) ptx::tmem_ld32(ts + c * 32, s[c]);
+        for (int c = 0; c < C::kHN / 32; ++c) ptx::tmem_ld32(ts + hf * C::kHN + c * 32, s[c]);
         ptx::tc_wait_ld();
-        const int left = a.Sk - j * kBN;  // keys of this block
-        if (left < kBN) {
+        const int left = a.Sk - j * kBN - hf * C::kHN;  // keys of this half of the block (none, or fewer: the last block's)
+        if (left < C::kHN) {
 #pragma unroll
-          for (int c = 0; c < kBN / 32; ++c)
+          for (int c = 0; c < C::kHN / 32; ++c)
 #pragma unroll
             for (int i = 0; i < 32; ++i)
               if (c * 32 + i >= left) s[c][i] = 0xff800000u;  // -inf
         }
-        float mxc[kBN / 32];
+        float mx = -INFINITY;
+        {
+          float mxc[4];
 #pragma unroll
-        for (int c = 0; c < kBN / 32; ++c) {
-          mxc[c] = ptx::max3(__uint_as_float(s[c][0]), __uint_as_float(s[c][1]), __uint_as_float(s[c][2]));
+          for (int e = 0; e < 4; ++e) mxc[e] = __uint_as_float(s[0][e]);
 #pragma unroll
-          for (int i = 3; i < 31; i += 2) mxc[c] = ptx::max3(mxc[c], __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
-          mxc[c] = fmaxf(mxc[c], __uint_as_float(s[c][31]));
+          for (int i = 4; i < C::kHN; i += 8)  // four chains of 3-input maxima
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int x = i + e, y = i + 4 + e;
+              mxc[e] = y < C::kHN ? ptx::max3(mxc[e], __uint_as_float(s[x >> 5][x & 31]), __uint_as_float(s[y >> 5][y & 31]))
+                                  : fmaxf(mxc[e], __uint_as_float(s[x >> 5][x & 31]));
+            }
+          mx = fmaxf(fmaxf(mxc[0], mxc[1]), fmaxf(mxc[2], mxc[3]));
         }
-        float mx = fmaxf(mxc[0], mxc[1]);
-        if constexpr (kBN == 128) mx = fmaxf(mx, fmaxf(mxc[2], mxc[3]));
-        const float m_new = fmaxf(m, mx * sl2);  // finite: every block holds a key, and scale > 0
-        const float alpha = fast_exp2(m - m_new);
-        const uint64_t neg_m2 = ptx::pack_f32x2(-m_new, -m_new);
-        uint64_t lsum[kBN / 32];
+        const float m_new = fmaxf(m, mx * sl2);  // -inf while this half has seen no key at all; scale > 0
+        const float alpha = m_new == -INFINITY ? 1.f : fast_exp2(m - m_new);
+        const float neg_m = m_new == -INFINITY ? 0.f : -m_new;
+        const uint64_t neg_m2 = ptx::pack_f32x2(neg_m, neg_m);
+        uint64_t lsum[2] = {0ull, 0ull};
 #pragma unroll
-        for (int c = 0; c < kBN / 32; ++c) {
-          lsum[c] = 0ull;
+        for (int c = 0; c < C::kHN / 32; ++c) {
           uint32_t w[3][16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
@@ -370,7 +392,7 @@ f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             float x0, x1;
             ptx::unpack_f32x2(x2, x0, x1);
             const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
-            lsum[c] = ptx::add_f32x2(lsum[c], ptx::pack_f32x2(p0, p1));
+            lsum[i & 1] = ptx::add_f32x2(lsum[i & 1], ptx::pack_f32x2(p0, p1));
             // three planes, cut off and not rounded: the same exact split as the inputs'
             const float r0 = p0 - __uint_as_float(__float_as_uint(p0) & 0xffff0000u);
             const float r1 = p1 - __uint_as_float(__float_as_uint(p1) & 0xffff0000u);
@@ -380,11 +402,16 @@ f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             w[1][i] = __byte_perm(__float_as_uint(r0), __float_as_uint(r1), 0x7632);
             w[2][i] = __byte_perm(__float_as_uint(t0), __float_as_uint(t1), 0x7632);
           }
-#pragma unroll
-          for (int p = 0; p < 3; ++p) ptx::tmem_st16(ts + p * C::kPlaneCols + c * 16, w[p]);
+          ptx::tmem_st16(ts + hf * C::kHN + c * 16, w[0]);
+          ptx::tmem_st16(ts + hf * C::kHN + C::kHN / 2 + c * 16, w[1]);
+          ptx::tmem_st16(ts + kBN + hf * (C::kHN / 2) + c * 16, w[2]);
         }
         ptx::tc_wait_st();
-        if (j > 0 && !add_block(g - 1)) break;
+        if (j > 0) {
+          if (!add_block(g - 1)) break;
+        } else if (hf == 1 && n_item > 0 && !wait(&bars->x_empty, (n_item - 1) & 1, 6u)) {
+          break;  // (the other warpgroup still reads the previous item's O of this half)
+        }
         if (__any_sync(0xffffffffu, m_new != m)) {
           const uint64_t alpha2 = ptx::pack_f32x2(alpha, alpha);
 #pragma unroll
@@ -395,31 +422,61 @@ f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         // the weights are in TMEM and the O columns are free: P V of this block may run
         ptx::tc_fence_before();
         __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&bars->p_full[buf]);
-        float s0, s1, s2, s3;
+        if (lane == 0) ptx::mbar_arrive(&bars->p_full[hf][buf]);
+        float s0, s1;
         ptx::unpack_f32x2(ptx::add_f32x2(lsum[0], lsum[1]), s0, s1);
         l += s0 + s1;
-        if constexpr (kBN == 128) {
-          ptx::unpack_f32x2(ptx::add_f32x2(lsum[2], lsum[3]), s2, s3);
-          l += s2 + s3;
-        }
       }
       if (!ok || !add_block(g - 1)) break;
-      ptx::tc_fence_before();
-      if (row < a.Sq) {
-        const float inv = 1.f / l;  // l >= the weight of the row's maximum, 1
-        float4* orow = reinterpret_cast<float4*>(a.o + b * a.o_sb + (int64_t)row * a.o_ss + h * a.o_sh);
+      if (hf == 1) {
+        // this half's result to the other warpgroup: O through this half's TMEM columns, the rest through shared memory
 #pragma unroll
-        for (int c = 0; c < NPV / 4; ++c) {
-          if (c * 4 < a.D) {
-            float x, y, z, w;
-            ptx::unpack_f32x2(acc[2 * c], x, y);
-            ptx::unpack_f32x2(acc[2 * c + 1], z, w);
-            orow[c] = make_float4(x * inv, y * inv, z * inv, w * inv);
+        for (int c = 0; c < NPV / 16; ++c) {
+          uint32_t ov[16];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            float x, y;
+            ptx::unpack_f32x2(acc[c * 8 + i], x, y);
+            ov[2 * i] = __float_as_uint(x);
+            ov[2 * i + 1] = __float_as_uint(y);
           }
+          ptx::tmem_st16(t_o + c * 16, ov);
         }
-        if (a.lse) a.lse[((int64_t)b * a.Hq + h) * a.Sq + row] = m * kLn2 + logf(l);
+        ptx::tc_wait_st();
+        ptx::tc_fence_before();
+        xch[row_in_tile] = m;
+        xch[kBM + row_in_tile] = l;
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&bars->x_full);
+        continue;
       }
+      if (!wait(&bars->x_full, n_item & 1, 6u)) break;
+      ptx::tc_fence_after();
+      const float m1 = xch[row_in_tile], l1 = xch[kBM + row_in_tile];
+      const float m_all = fmaxf(m, m1);  // finite: the first half of the first block holds a key
+      const float f0 = fast_exp2(m - m_all), f1 = m1 == -INFINITY ? 0.f : fast_exp2(m1 - m_all);
+      l = l * f0 + l1 * f1;
+      const float inv = 1.f / l;  // l >= the weight of the row's maximum, 1
+      float* orow = a.o + b * a.o_sb + (int64_t)row * a.o_ss + h * a.o_sh;
+#pragma unroll
+      for (int c = 0; c < NPV / 16; ++c) {
+        uint32_t ov[16];
+        ptx::tmem_ld16(t_o + NPV + c * 16, ov);
+        ptx::tc_wait_ld();
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          float x, y, z, w;
+          ptx::unpack_f32x2(acc[c * 8 + v * 2], x, y);
+          ptx::unpack_f32x2(acc[c * 8 + v * 2 + 1], z, w);
+          const float4 o4 = make_float4((x * f0 + __uint_as_float(ov[4 * v]) * f1) * inv, (y * f0 + __uint_as_float(ov[4 * v + 1]) * f1) * inv,
+                                        (z * f0 + __uint_as_float(ov[4 * v + 2]) * f1) * inv, (w * f0 + __uint_as_float(ov[4 * v + 3]) * f1) * inv);
+          if (row < a.Sq && c * 16 + v * 4 < a.D) *reinterpret_cast<float4*>(orow + c * 16 + v * 4) = o4;
+        }
+      }
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&bars->x_empty);
+      if (a.lse && row < a.Sq) a.lse[((int64_t)b * a.Hq + h) * a.Sq + row] = m_all * kLn2 + logf(l);
     }
   }
 

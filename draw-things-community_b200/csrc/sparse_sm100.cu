@@ -8,7 +8,7 @@
 // bytes as [dims][keys] (M = 128 dims, N = 64 heads, D / 128 of them).  The transposed second product runs the tensor core
 // at full height where [64 heads] x [256 dims] would use half of it, and its accumulator is 256 columns of TMEM, which
 // leaves room for two S buffers of two accumulators each (neighbouring MMAs on one accumulator wait for each other: a chain
-// of M = 64, N = 48 MMAs took 66 cycles each, twice its share of the pipe).  7 warps:
+// of M = 64, N = 48 MMAs took 66 cycles each, twice its share of the pipe).  10 warps:
 //   warps 0-3   softmax, one thread per head (the 64 rows of S are lanes 0-15 of the four TMEM quarters); P goes to shared
 //               memory; O^T is rescaled only when a head's maximum grew by more than 2^8; at the end O^T / l is stored,
 //               two neighbouring dims per 4-byte store
@@ -18,8 +18,8 @@
 //   warp 9      TMEM allocation, TMA of the next token's queries
 // Measured (prompt of 4096 tokens, 64 heads of 512, 128 + up to 512 keys each): 2110 us with warp-level MMAs, 512 us here
 // (538 TFLOP/s of visible work, tensor pipe 58 % active).
-// What set the time on the way: the gather.  With asynchronous 16-byte copies of four warps it moved 11 bytes per cycle (1775 us), with all the TMA
-// loads issued by one warp, 68 cycles each, 7 (1446 us).
+// What set the time on the way: the gather.  With asynchronous 16-byte copies of four warps it moved 11 bytes per cycle
+// (1775 us), with all the TMA loads issued by one warp, 68 cycles each, 7 (1446 us).
 // Every mbarrier wait is bounded.  The softmax warps also meet at a named barrier once per tile; a wait that ran out is part
 // of what they vote on there, so that all four leave together.
 #include <type_traits>
