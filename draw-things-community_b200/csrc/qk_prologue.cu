@@ -477,12 +477,12 @@ PrologueTensor to_arg(const dt_qk_prologue_params* p) {
 }
 
 // Normalised and rotated with nothing behind, a token's heads share their rotary row, and there are enough of them to fill
-// half of the rows a warp takes at a time (the reference's joint and LLM attention); everything else, a table per head or a
-// lone KV head among it, stays with the row kernel.
+// the rows a warp takes at a time (the reference's joint attention: 12 heads, 20000 tokens 64.5 -> 55.3 us; 5 heads, 256
+// tokens 2.6 against 2.9 us); everything else, a table per head or a few KV heads among it, stays with the row kernel.
 bool by_token(const PrologueArgs& a, int rows_per_warp) {
   for (int i = 0; i < a.n; ++i) {
     const PrologueTensor& t = a.t[i];
-    if (!t.weight || !t.rot || t.post_scale != 1.f || (t.r_sh != 0 && t.H > 1) || t.H < rows_per_warp * kHeadRows / 2) return false;
+    if (!t.weight || !t.rot || t.post_scale != 1.f || (t.r_sh != 0 && t.H > 1) || t.H < rows_per_warp * kHeadRows) return false;
   }
   return true;
 }

@@ -509,7 +509,9 @@ bool sparse_tcgen05_supported(const dt_sparse_indexed_params& p, bool same_kv) {
   if (p.D % 256 || p.D > kMaxD || !same_kv || !(p.scale > 0.f) || (p.Hq / p.Hkv) % kHeads) return false;
   const bool raw = p.Sr > 0, comp = p.Sc > 0 && p.n_selected > 0;
   if ((!raw && !comp) || (raw && !key_map_fits(p.k_raw, p.Sr, p)) || (comp && !key_map_fits(p.k_comp, p.Sc, p))) return false;
-  return (long long)p.B * p.Sq * p.Hq / kHeads >= 64 && (long long)p.B * p.Sq * p.Hq / kHeads < (1LL << 30);
+  // below 16 the keys of a token are better spread over a cluster of CTAs (8 tokens of 640 keys: 21 us there, 24 us here;
+  // 16: 30 and 24 us; 64: 76 and 24 us)
+  return (long long)p.B * p.Sq * p.Hq / kHeads >= 16 && (long long)p.B * p.Sq * p.Hq / kHeads < (1LL << 30);
 }
 
 int launch_sparse_tcgen05(const dt_sparse_indexed_params& p, cudaStream_t stream) {

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("case", [
     # B, Sq, Sr, Sc, n_sel, Hq, Hkv, D, dtype, window, sinks, causal
-    (1, 64, 64, 0, 0, 64, 1, 512, torch.bfloat16, 48, True, True),      # one tile at most, the smallest dispatched count
+    (1, 16, 64, 0, 0, 64, 1, 512, torch.bfloat16, 48, True, True),      # one tile at most, the smallest dispatched count
     (1, 70, 120, 30, 1, 64, 1, 512, torch.float16, 48, True, True),     # one key more than a tile
     (1, 150, 300, 64, 48, 64, 1, 512, torch.bfloat16, 128, True, True),  # more tokens than SMs: a second token per CTA
     (1, 320, 500, 90, 200, 64, 1, 512, torch.float16, 128, False, True),  # lists longer than the rows, no sinks, third tokens
