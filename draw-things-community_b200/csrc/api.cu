@@ -421,7 +421,7 @@ int dt_sdpa_forward_host(const dt_sdpa_params* ph) {
     if (e == cudaSuccess) {
       g_hs.ws_bytes = wsb;
       DT_CUDA_TRY(cudaMemsetAsync(g_hs.ws, 0, wsb, g_hs.stream));
-    } else if (choose(p) == kGeneric) {  // fp32: the CUDA-core kernel needs no scratch
+    } else if (choose(p) != kDecode) {  // (no masks here) the other kernels' scratch is optional
       cudaGetLastError();
       g_hs.ws = nullptr;
     } else {
@@ -442,7 +442,8 @@ int dt_sdpa_forward_host(const dt_sdpa_params* ph) {
       return t.stride_h == p.D && t.stride_s >= (int64_t)H * p.D && (p.B == 1 || t.stride_b == (int64_t)S * t.stride_s);
     };
     const bool big = nq + nk + nv >= (size_t)(16u << 20);
-    const bool pipelined = big && !p.lse && choose(p) == kPrefill && regular(p.q, p.Sq, p.Hq) &&
+    // (a call whose work is cut over the SMs has few query rows to send back: it goes in one piece, cut the same way)
+    const bool pipelined = big && !p.lse && choose(p) == kPrefill && wsb == 0 && regular(p.q, p.Sq, p.Hq) &&
                            regular(p.k, p.Sk, p.Hkv) && regular(p.v, p.Sk, p.Hkv) && regular(p.o, p.Sq, p.Hq);
     if (pipelined && !g_hs.s_in) {
       DT_CUDA_TRY(cudaStreamCreateWithFlags(&g_hs.s_in, cudaStreamNonBlocking));
@@ -469,13 +470,12 @@ int dt_sdpa_forward_host(const dt_sdpa_params* ph) {
       while (left > per + per / 2) { runs[n_runs++] = per; left -= per; }
       if (left >= 3) { runs[n_runs++] = (2 * left + 2) / 3; left -= runs[n_runs - 1]; }
       runs[n_runs++] = left;
-      bool same_kernel = true;  // every run must take the tensor-core kernel within the workspace sized for the whole
+      bool same_kernel = true;  // every run must take the tensor-core kernel (whose scratch is optional: no masks here)
       for (int c = 0, r = 0; c < n_runs; ++c) {
         dt_sdpa_params pc = p;
         pc.Sq = c + 1 < n_runs ? runs[c] * kItemRows : p.Sq - r;
         r += pc.Sq;
-        size_t w = 0;
-        same_kernel = same_kernel && choose(pc) == kPrefill && dt_sdpa_workspace_size(&pc, &w) == DT_OK && w <= g_hs.ws_bytes;
+        same_kernel = same_kernel && choose(pc) == kPrefill;
       }
       if (same_kernel) {
       DT_CUDA_TRY(cudaMemcpyAsync(p.k.ptr, ph->k.ptr, nk, cudaMemcpyHostToDevice, g_hs.s_in));
@@ -493,7 +493,7 @@ int dt_sdpa_forward_host(const dt_sdpa_params* ph) {
         pc.Sq = rows;
         pc.q.ptr = static_cast<char*>(p.q.ptr) + r0 * row_bytes;
         pc.o.ptr = static_cast<char*>(p.o.ptr) + r0 * row_bytes;
-        st = dt_sdpa_forward(&pc, g_hs.ws, g_hs.ws_bytes, s);
+        st = dt_sdpa_forward(&pc, nullptr, 0, s);  // no scratch, so no cut: as in the whole call, bit for bit
         if (st != DT_OK) return st;
         DT_CUDA_TRY(cudaEventRecord(g_hs.ev_done[c], s));
         DT_CUDA_TRY(cudaStreamWaitEvent(g_hs.s_out, g_hs.ev_done[c], 0));
@@ -530,7 +530,7 @@ int dt_sdpa_forward_host(const dt_sdpa_params* ph) {
         pg.v.ptr = static_cast<char*>(p.v.ptr) + (size_t)g * hk * p.D * es;
         pg.o.ptr = static_cast<char*>(p.o.ptr) + (size_t)g * hq * p.D * es;
         if (p.sinks) pg.sinks = static_cast<const char*>(p.sinks) + (size_t)g * hq * es;
-        st = dt_sdpa_forward(&pg, g_hs.ws, g_hs.ws_bytes, s);
+        st = dt_sdpa_forward(&pg, nullptr, 0, s);
         if (st != DT_OK) return st;
         DT_CUDA_TRY(cudaEventRecord(g_hs.ev_done[g], s));
         DT_CUDA_TRY(cudaStreamWaitEvent(g_hs.s_out, g_hs.ev_done[g], 0));

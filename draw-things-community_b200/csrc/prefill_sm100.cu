@@ -95,8 +95,17 @@ struct PrefillArgs {
   const unsigned char* mask_flags;
   int n_rg, n_kh;
   float scale;  // the plain scale (scale_log2 = scale * log2(e)); the masked variant adds the mask in this domain
-  int n_qpairs, n_items;  // work items = (batch, head, pair of query tiles)
-  int n_slots;            // n_items rounded up to whole rounds over the grid (the causal order leaves some slots empty)
+  int item_rows;          // query rows of a work item: a pair of tiles, or one tile where pairs would leave SMs idle
+  int n_qpairs, n_items;  // work items = (batch, head, item_rows query rows)
+  // Items in whole rounds over the grid: n_slots of them, of which the causal order may leave some empty.  The items from
+  // n_slots on (fewer than one round) are n_single / 2 pairs of tiles taken tile by tile, or else cut into n_cuts runs of
+  // K/V blocks of equal length, in the same order, of which CTA c < n_cuts takes run c.  A run's share of an item that it does not hold
+  // whole goes to `part`; cut_combine_kernel puts the shares together.
+  int n_slots;
+  int n_single;
+  int n_cuts;
+  int cut_blocks;         // K/V blocks of those items together (times n_cuts below 2^31)
+  float* part;            // [2 n_cuts][warps of an item][D + 2][32]: weights' maximum, their sum, O
   // variable-length batch (both null otherwise): packed rows, sequence s owns query rows [off_q[s], off_q[s+1])
   // and key rows [off_k[s], off_k[s+1]); the item's batch index is then the sequence
   const int32_t* off_q;
@@ -135,40 +144,40 @@ __device__ __forceinline__ uint32_t pack_pair(float lo, float hi) {
 // S = Q K^T for one 128-row tile: both operands K-major with 128-byte swizzle, D/16 steps of k = 16.
 // Descriptor start addresses advance by 32 B per step inside a 64-element half and by 16 KB to the next half.
 template <int D>
-__device__ __forceinline__ void issue_qk(uint32_t s_tmem, uint64_t q_desc, uint64_t k_desc, uint32_t idesc) {
+__device__ __forceinline__ void issue_qk(bool on, uint32_t s_tmem, uint64_t q_desc, uint64_t k_desc, uint32_t idesc) {
 #pragma unroll
   for (int ks = 0; ks < D / 16; ++ks) {
     const uint64_t o = (uint64_t)(((ks >> 2) * kHalfBytes + (ks & 3) * 32) >> 4);
-    ptx::mma_ss(s_tmem, q_desc + o, k_desc + o, idesc, ks > 0 ? 1u : 0u);
+    ptx::mma_ss_on(on, s_tmem, q_desc + o, k_desc + o, idesc, ks > 0 ? 1u : 0u);
   }
 }
 
 // O (+)= P V for one tile: P from TMEM (two 16-bit keys per 32-bit column, 8 columns per step), V is
 // [key][d] = MN-major; one step consumes 16 keys = 2 KB of each 64-wide half.
-__device__ __forceinline__ void issue_pv(uint32_t o_tmem, uint32_t p_tmem, uint64_t v_desc, uint32_t idesc,
+__device__ __forceinline__ void issue_pv(bool on, uint32_t o_tmem, uint32_t p_tmem, uint64_t v_desc, uint32_t idesc,
                                          uint32_t accumulate, int k_begin, int k_end) {
   if (k_end - k_begin == 4) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int kk = k_begin + i;
-      ptx::mma_ts(o_tmem, p_tmem + kk * 8, v_desc + (uint64_t)(kk * (2048 >> 4)), idesc, (kk > 0) ? 1u : accumulate);
+      ptx::mma_ts_on(on, o_tmem, p_tmem + kk * 8, v_desc + (uint64_t)(kk * (2048 >> 4)), idesc, (kk > 0) ? 1u : accumulate);
     }
   } else {
 #pragma unroll 1
     for (int kk = k_begin; kk < k_end; ++kk)
-      ptx::mma_ts(o_tmem, p_tmem + kk * 8, v_desc + (uint64_t)(kk * (2048 >> 4)), idesc, (kk > 0) ? 1u : accumulate);
+      ptx::mma_ts_on(on, o_tmem, p_tmem + kk * 8, v_desc + (uint64_t)(kk * (2048 >> 4)), idesc, (kk > 0) ? 1u : accumulate);
   }
 }
 
 // The same for the weights of the kSplit variant: their high parts and, 64 columns further, what those leave over.
 template <bool kSplit>
-__device__ __forceinline__ void issue_pv_parts(uint32_t o_tmem, uint32_t p_tmem, uint64_t v_desc, uint32_t idesc,
+__device__ __forceinline__ void issue_pv_parts(bool on, uint32_t o_tmem, uint32_t p_tmem, uint64_t v_desc, uint32_t idesc,
                                                uint32_t accumulate, int k_begin, int k_end) {
-  issue_pv(o_tmem, p_tmem, v_desc, idesc, accumulate, k_begin, k_end);
+  issue_pv(on, o_tmem, p_tmem, v_desc, idesc, accumulate, k_begin, k_end);
   if constexpr (kSplit) {
 #pragma unroll 1
     for (int kk = k_begin; kk < k_end; ++kk)
-      ptx::mma_ts(o_tmem, p_tmem + 64 + kk * 8, v_desc + (uint64_t)(kk * (2048 >> 4)), idesc, 1u);
+      ptx::mma_ts_on(on, o_tmem, p_tmem + 64 + kk * 8, v_desc + (uint64_t)(kk * (2048 >> 4)), idesc, 1u);
   }
 }
 
@@ -187,6 +196,149 @@ __device__ __forceinline__ void stamp(const PrefillArgs& a, int slot) {
 #else
 __device__ __forceinline__ void stamp(const PrefillArgs&, int) {}
 #endif
+
+// ---- the cut part of a call's work (see PrefillArgs) ----
+__device__ __forceinline__ int cut_at(const PrefillArgs& a, int c) { return a.cut_blocks * c / a.n_cuts; }  // first block of run c
+
+// K/V blocks from key 0 to the last one that the query rows below `end` may see (not for variable lengths)
+__device__ __forceinline__ int blocks_to(const PrefillArgs& a, int end) {
+  int nkv = (a.Sk + kBN - 1) / kBN;
+  if (a.is_causal) {
+    const long long lim = (long long)min(a.Sq, end) + (a.Sk - a.Sq);
+    nkv = max(1, min(nkv, (int)((max(0LL, min((long long)a.Sk, lim)) + kBN - 1) / kBN)));
+  }
+  return nkv;
+}
+
+// (query tile (pair), batch x head) at a place of the processing order: query rows fastest, so that CTAs running at the
+// same time share one head's K/V in L2; under the causal rule heaviest first (all heads' last rows, then the ones before,
+// ...), because an item's work grows with its query position.
+__device__ __forceinline__ void place_of(const PrefillArgs& a, int order, int& qt, int& bh) {
+  if (a.is_causal) {
+    const int nbh = a.n_items / a.n_qpairs, level = order / nbh;
+    bh = order - level * nbh;
+    qt = a.n_qpairs - 1 - level;
+  } else {
+    bh = order / a.n_qpairs;
+    qt = order - bh * a.n_qpairs;
+  }
+}
+
+// Moves (order, start) on to the cut item that holds block `pos` of the runs' numbering and returns its K/V blocks;
+// under the causal rule a level of equal items at a time.
+__device__ __forceinline__ int find_cut_item(const PrefillArgs& a, int pos, int& order, int& start) {
+  const int nbh = a.n_items / a.n_qpairs;
+  for (;;) {
+    const int level = a.is_causal ? order / nbh : 0;
+    const int same = a.is_causal ? nbh - (order - level * nbh) : a.n_items - order;
+    const int n = blocks_to(a, a.is_causal ? (a.n_qpairs - level) * a.item_rows : 0);
+    const int skip = min((pos - start) / n, same);
+    order += skip;
+    start += skip * n;
+    if (skip < same) return n;
+  }
+}
+
+// Run c's share of 32 rows (one softmax warp's) of the item that starts at block `item_begin`: a run holds at most one
+// share that lies at its start and one that reaches its end.
+template <int D>
+__device__ __forceinline__ float* share_of(const PrefillArgs& a, int units, int c, int item_begin, int unit) {
+  const int slot = 2 * c + (item_begin > cut_at(a, c) ? 1 : 0);
+  return a.part + ((size_t)slot * units + unit) * (size_t)((D + 2) * 32);
+}
+
+// Puts the shares of the cut items together, added in the order of the keys: one block per item, softmax warp's 32 rows
+// and 64 columns.  (As the last step of the attention kernel itself, by the warp that arrives last, it took longer than the
+// cut saved: 256 columns from three shares are a chain of two dozen L2 round trips for one warp.)
+// Bound: the latency of L2; a thread keeps eight shares' loads in flight.
+template <typename T, int D>
+__global__ void __launch_bounds__(256) cut_combine_kernel(const PrefillArgs a, const int units) {
+  __shared__ __align__(16) uint16_t rows[32][64 + 8];
+  const int item = blockIdx.x / units, unit = blockIdx.x - item * units, col0 = blockIdx.y * 64;
+  const int r = threadIdx.x & 31, cg = threadIdx.x >> 5;  // two groups of four columns per thread: cg and cg + 8
+  int order = a.n_slots, begin = 0, n;
+  if (a.is_causal) {  // where the item's blocks start: its level's first item, then equal items
+    const int nbh = a.n_items / a.n_qpairs;
+    const int want = a.n_slots + item;
+    for (;;) {
+      const int level = order / nbh, next = min((level + 1) * nbh, want);
+      n = blocks_to(a, (a.n_qpairs - level) * a.item_rows);
+      begin += (next - order) * n;
+      order = next;
+      if (order == want) break;
+    }
+    n = blocks_to(a, (a.n_qpairs - order / nbh) * a.item_rows);
+  } else {
+    n = blocks_to(a, 0);
+    begin = item * n;
+    order += item;
+  }
+  int c_first = (int)((long long)begin * a.n_cuts / a.cut_blocks);
+  while (cut_at(a, c_first + 1) <= begin) ++c_first;
+  while (cut_at(a, c_first) > begin) --c_first;
+  int c_last = c_first;
+  while (cut_at(a, c_last + 1) < begin + n) ++c_last;
+  if (c_first == c_last) return;  // one run holds the whole item: the attention kernel has stored it
+  int qt, bh;
+  place_of(a, order, qt, bh);
+  const int h = bh % a.Hq, b = bh / a.Hq, row0 = qt * a.item_rows + unit * 32, row = row0 + r;
+  if (unit * 32 >= a.item_rows || row0 >= a.Sq) return;
+
+  // the first run's share lies at its start or reaches its end; all the others start their runs
+  const size_t share = (size_t)((D + 2) * 32), run = 2 * (size_t)units * share;
+  const float* first = share_of<D>(a, units, c_first, begin, unit);
+  const float* rest = a.part + (size_t)unit * share;
+  const int n_shares = c_last - c_first + 1;
+  auto at = [&](int i) { return i == 0 ? first : rest + (size_t)(c_first + i) * run; };
+  float m = -INFINITY;
+#pragma unroll 8
+  for (int i = 0; i < n_shares; ++i) m = fmaxf(m, __ldg(at(i) + r));
+  float l = 0.f;
+  float4 acc[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+#pragma unroll 8
+  for (int i = 0; i < n_shares; ++i) {
+    const float* sh = at(i);
+    const float mc = __ldg(sh + r), lc = __ldg(sh + 32 + r);
+    float4 x[2];
+#pragma unroll
+    for (int g = 0; g < 2; ++g) x[g] = __ldg(reinterpret_cast<const float4*>(sh + 64) + (col0 / 4 + cg + 8 * g) * 32 + r);
+    if (mc != -INFINITY) {  // (a share that saw no key holds no numbers)
+      const float f = fast_exp2(mc - m);
+      l = fmaf(f, lc, l);
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        acc[g].x = fmaf(f, x[g].x, acc[g].x);
+        acc[g].y = fmaf(f, x[g].y, acc[g].y);
+        acc[g].z = fmaf(f, x[g].z, acc[g].z);
+        acc[g].w = fmaf(f, x[g].w, acc[g].w);
+      }
+    }
+  }
+  if (a.sinks) {  // as in the attention kernel's epilogue
+    const float sl = to_float(reinterpret_cast<const T*>(a.sinks)[h]) * kLog2e;
+    if (m == -INFINITY) {
+      m = sl;
+      l = 1.f;
+    } else {
+      l += fast_exp2(sl - m);
+    }
+  }
+  const float inv = (l > 0.f && m != -INFINITY) ? 1.f / l : 0.f;
+  if (a.lse && cg == 0 && col0 == 0 && row < a.Sq)
+    a.lse[((int64_t)b * a.Hq + h) * a.Sq + row] = (l > 0.f && m != -INFINITY) ? m * kLn2 + logf(l) : -INFINITY;
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    uint2 pk;
+    pk.x = pack_pair<T>(acc[g].x * inv, acc[g].y * inv);
+    pk.y = pack_pair<T>(acc[g].z * inv, acc[g].w * inv);
+    *reinterpret_cast<uint2*>(&rows[r][(cg + 8 * g) * 4]) = pk;
+  }
+  __syncthreads();
+  T* obase = reinterpret_cast<T*>(a.o) + (int64_t)b * a.o_sb + (int64_t)h * a.o_sh + col0;
+  const int rr = threadIdx.x >> 3, ch = threadIdx.x & 7;
+  if (row0 + rr < a.Sq && col0 + ch * 8 < a.d_real)
+    *reinterpret_cast<uint4*>(obase + (int64_t)(row0 + rr) * a.o_ss + ch * 8) = *reinterpret_cast<const uint4*>(&rows[rr][ch * 8]);
+}
 
 // Pre-pass of the masked variant: which (32 rows x 64 keys) patches of the additive mask hold anything but zeros.
 // A padding mask is zero almost everywhere, and the attention kernel skips the patches flagged zero altogether.
@@ -286,40 +438,21 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = a.Hq / a.Hkv;
 
-  // Work items (batch, head, pair of query tiles), q-tile pair fastest so that CTAs running at the same
-  // time share one head's K/V in L2.  The CTA is persistent: it takes items blockIdx.x, + gridDim.x, ...
+  // Work items (batch, head, item_rows query rows).  The CTA is persistent: it takes items blockIdx.x, + gridDim.x, ...
   struct Item {
     int b, h, kvh, q0, nkv, j0;  // K/V blocks j0 .. j0 + nkv - 1; nkv == 0: nothing to do (q0 beyond the sequence)
     int sq, sk, off;             // rows of this (batch item | sequence); causal: key j visible to query i iff j <= i + off
     int qrow, krow;              // first packed row of the sequence (0 unless variable-length)
     bool two;
   };
-  auto decode_item = [&](int item) {
+  auto item_at = [&](int order, int tile) {  // tile: one of the pair's tiles, or -1 for the whole item
     Item it;
-    int qt = item % a.n_qpairs;
-    int bh = item / a.n_qpairs;
-    if (a.is_causal) {
-      // Under the causal rule an item's work grows with its query position.  The items are dealt out heaviest
-      // first (all heads' last tile pair, then the one before, ...), forwards in even rounds over the CTAs and
-      // backwards in odd rounds, so that every CTA's items add up to about the same number of K/V blocks.
-      const int round = item / (int)gridDim.x;
-      int pos = item - round * (int)gridDim.x;
-      if (round & 1) pos = (int)gridDim.x - 1 - pos;
-      const int order = round * (int)gridDim.x + pos;
-      const int nbh = a.n_items / a.n_qpairs;
-      const int level = order / nbh;
-      bh = order - level * nbh;
-      qt = a.n_qpairs - 1 - level;
-      if (order >= a.n_items) {  // a slot of the last, incomplete round without an item
-        it = Item{};
-        it.nkv = 0;
-        return it;
-      }
-    }
+    int qt, bh;
+    place_of(a, order, qt, bh);
     it.h = bh % a.Hq;
     it.b = bh / a.Hq;
     it.kvh = it.h / G;
-    it.q0 = qt * (C::kTiles * kBM);
+    it.q0 = qt * a.item_rows + max(tile, 0) * kBM;
     it.sq = a.Sq;
     it.sk = a.Sk;
     it.qrow = it.krow = 0;
@@ -331,25 +464,58 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       it.b = 0;
     }
     it.off = it.sk - it.sq;
-    it.two = C::kTiles == 2 && it.q0 + kBM < it.sq;
+    it.two = C::kTiles == 2 && tile < 0 && a.item_rows > kBM && it.q0 + kBM < it.sq;
     it.j0 = 0;
-    if (it.q0 >= it.sq) {  // only with variable lengths: this sequence is shorter than the longest one
+    if (it.q0 >= it.sq) {  // a pair without a second tile, or a sequence shorter than the longest one
       it.nkv = 0;
       return it;
     }
     int nkv = max(1, (it.sk + kBN - 1) / kBN);  // a sequence without keys still runs one (fully masked) block
-    if (a.is_causal) {
-      const int last_row = min(it.sq, it.q0 + C::kTiles * kBM) - 1;
-      const long long lim = (long long)last_row + it.off + 1;  // keys [0, lim) can be visible
-      const int need = (int)((max(0LL, min((long long)it.sk, lim)) + kBN - 1) / kBN);
-      nkv = max(1, min(nkv, need));
-    }
+    if (a.is_causal) nkv = blocks_to(a, it.q0 + (it.two ? 2 : 1) * kBM);  // (never together with variable lengths)
     if (a.window > 0) {  // blocks entirely below the first row's window are never visited
       const long long lo = (long long)it.q0 + it.off - a.window + 1;
       it.j0 = (int)min((long long)(nkv - 1), max(0LL, lo) / kBN);
     }
     it.nkv = nkv - it.j0;
     return it;
+  };
+  // Whole items: place `item` of the CTAs' turns.  Under the causal rule the turns go forwards over the CTAs in even
+  // rounds and backwards in odd ones, so that every CTA's items add up to about the same number of K/V blocks.
+  auto decode_item = [&](int item) {
+    int order = item;
+    if (a.is_causal) {
+      const int round = item / (int)gridDim.x;
+      int pos = item - round * (int)gridDim.x;
+      if (round & 1) pos = (int)gridDim.x - 1 - pos;
+      order = round * (int)gridDim.x + pos;
+    }
+    if (order >= a.n_items) {  // a slot of the last, incomplete round without an item
+      return Item{};
+    }
+    return item_at(order, -1);
+  };
+  // This CTA's work in turn: its whole items and then a single tile, or (a cut call has neither) its run of blocks, one
+  // item or share of one at a time.  One word of state, because the softmax warps carry it through their loops, where two
+  // more registers cost the 256-wide variant 2 %: the next whole item, n_slots + the next single tile, or the next block.
+  auto first_work = [&]() { return (int)blockIdx.x < a.n_cuts ? cut_at(a, blockIdx.x) : (int)blockIdx.x; };
+  auto next_work = [&](int& next, Item& w) -> bool {
+    if (a.n_cuts == 0) {
+      while (next < a.n_slots + a.n_single) {
+        w = next < a.n_slots ? decode_item(next) : item_at(a.n_slots + ((next - a.n_slots) >> 1), (next - a.n_slots) & 1);
+        next += gridDim.x;
+        if (w.nkv > 0) return true;
+      }
+      return false;
+    }
+    const int end = cut_at(a, blockIdx.x + 1);
+    if (next >= end) return false;
+    int order = 0, start = 0;
+    const int n = find_cut_item(a, next, order, start);
+    w = item_at(order, -1);
+    w.j0 = next - start;
+    w.nkv = min(n, end - start) - w.j0;
+    next += w.nkv;
+    return true;
   };
 
   if (threadIdx.x == 0) {
@@ -410,21 +576,20 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           ++ring_it;
           return true;
         };
-        for (int item = blockIdx.x; item < a.n_slots && ok; item += gridDim.x, ++n_item) {
-          const Item w = decode_item(item);
-          if (w.nkv == 0) {  // empty item: not counted (the loop header increments n_item)
-            --n_item;
-            continue;
-          }
+        int walk = first_work();
+        Item w, nx;
+        bool more_work = next_work(walk, nx);
+        for (; more_work && ok; ++n_item) {
+          w = nx;
+          more_work = next_work(walk, nx);
           // The Q tiles of the NEXT item are pulled into L2 now: their rows are 256-byte pieces a whole
           // token stride apart (slow to gather from HBM), and the real load sits on the critical path
           // between two items.
-          if (item + (int)gridDim.x < a.n_slots) {
-            const Item nx = decode_item(item + gridDim.x);
+          if (more_work) {
             for (int t = 0; t < (nx.two ? 2 : 1); ++t)
 #pragma unroll
               for (int hf = 0; hf < C::kHalves; ++hf)
-                if (nx.nkv > 0) ptx::tma_prefetch_l2_4d(&map_q, hf * 64, nx.h, nx.qrow + nx.q0 + t * kBM, nx.b);
+                ptx::tma_prefetch_l2_4d(&map_q, hf * 64, nx.h, nx.qrow + nx.q0 + t * kBM, nx.b);
           }
           // first K/V block of this item may be fetched while the previous item still owns the Q buffers
           // (one tile per item: the MMA warp consumes K(0), K(1), V(0), K(2), V(1), ..., and the ring follows that order)
@@ -453,7 +618,12 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       }
     } else if (warp == 1) {
       // =========================== MMA issuer ===========================
-      if (lane == 0) {
+      // The whole warp walks the loop and one lane issues, which keeps the operands in uniform registers (Flux joint
+      // attention 227 -> 223 us, 2047 tokens with an unaligned mask 97 -> 88 us); the 64-wide variant, whose MMAs are fewer
+      // than its softmax warps can follow, is 1 % faster with one lane walking it (SD1.5 self-attention 125 against 127 us).
+      constexpr bool kWarpIssue = D >= 128;
+      if (kWarpIssue || lane == 0) {
+        const bool on = kWarpIssue ? ptx::elect_one() : true;
         constexpr uint32_t idesc_qk = ptx::make_idesc_f16(kBf16, kBM, kBN, 0, 0);
         constexpr uint32_t idesc_pv = ptx::make_idesc_f16(kBf16, kBM, D, 0, 1);
         // Descriptors differ only in the 14-bit start-address field, so stepping through a tile is one add.
@@ -468,19 +638,20 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         int n_item = 0;
         bool ok = true;
         auto fail = [&](unsigned code) {
-          atomicCAS(a.status, 0u, code);
+          if (on) atomicCAS(a.status, 0u, code);
           *abort_flag = 1;
           ok = false;
+        };
+        auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+          const bool done = ptx::mbar_wait(bar, parity, abort_flag);
+          return kWarpIssue ? __all_sync(0xffffffffu, done) : done;
         };
         auto advance = [&]() {
           if (++slot == C::kSlots) { slot = 0; par ^= 1; }
         };
-        for (int item = blockIdx.x; item < a.n_slots && ok; item += gridDim.x, ++n_item) {
-          const Item w = decode_item(item);
-          if (w.nkv == 0) {  // empty item: not counted (the loop header increments n_item)
-            --n_item;
-            continue;
-          }
+        int walk = first_work();
+        Item w;
+        for (; ok && next_work(walk, w); ++n_item) {
           const int ntile = w.two ? 2 : 1;
           const int qb = n_item % C::kQBufs;
           const uint64_t qd0 = qd_base + (uint64_t)(qb * C::kTiles * (C::kTileBytes >> 4));
@@ -489,20 +660,20 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             // One tile per item (D = 256): S is double-buffered in TMEM (the columns a second tile would use), so that
             // Q K(j+1)^T and P V(j-1) run while the softmax works on block j.  Order on the tensor pipe:
             // QK(0) QK(1) | PV(0) QK(2) | PV(1) QK(3) | ...
-            if (!ptx::mbar_wait(&bars->q_full[qb], (n_item / C::kQBufs) & 1, abort_flag)) {
+            if (!wait(&bars->q_full[qb], (n_item / C::kQBufs) & 1)) {
               fail(1u);
               break;
             }
             auto qk = [&](int i) -> bool {  // S[i & 1] = Q K(i)^T from the ring's next slot
-              if (!ptx::mbar_wait(&bars->kv_full[slot], par, abort_flag)) {
+              if (!wait(&bars->kv_full[slot], par)) {
                 fail(1u);
                 return false;
               }
               ptx::tc_fence_after();
-              issue_qk<D>((i & 1) ? s1 : s0, qd0, ring_k + (uint64_t)(slot * (C::kTileBytes >> 4)), idesc_qk);
-              ptx::tc_commit(&bars->s_full[i & 1]);
-              ptx::tc_commit(&bars->kv_empty[slot]);
-              if (i == w.nkv - 1) ptx::tc_commit(&bars->q_empty[qb]);  // Q is no longer needed: the next item may load its own
+              issue_qk<D>(on, (i & 1) ? s1 : s0, qd0, ring_k + (uint64_t)(slot * (C::kTileBytes >> 4)), idesc_qk);
+              ptx::tc_commit_on(on, &bars->s_full[i & 1]);
+              ptx::tc_commit_on(on, &bars->kv_empty[slot]);
+              if (i == w.nkv - 1) ptx::tc_commit_on(on, &bars->q_empty[qb]);  // Q is no longer needed: the next item may load its own
               advance();
               return true;
             };
@@ -514,50 +685,50 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
               const int valid = max(16, min(kBN, w.sk - (w.j0 + j) * kBN));
               const int ksteps = (valid + 15) >> 4;
               const int k_mid = min(ksteps, 4);
-              if (!ptx::mbar_wait(&bars->kv_full[slot], par, abort_flag)) {  // V(j)
+              if (!wait(&bars->kv_full[slot], par)) {  // V(j)
                 fail(1u);
                 break;
               }
               const int slot_v = slot;
               const uint64_t vd = ring_v + (uint64_t)(slot_v * (C::kTileBytes >> 4));
               advance();
-              if (!ptx::mbar_wait(&bars->p_half[b][0], pph, abort_flag)) { fail(4u); break; }
+              if (!wait(&bars->p_half[b][0], pph)) { fail(4u); break; }
               ptx::tc_fence_after();
-              issue_pv_parts<kSplit>(o0, sb, vd, idesc_pv, j > 0 ? 1u : 0u, 0, k_mid);
-              if (!ptx::mbar_wait(&bars->p_half[b][1], pph, abort_flag)) { fail(4u); break; }
+              issue_pv_parts<kSplit>(on, o0, sb, vd, idesc_pv, j > 0 ? 1u : 0u, 0, k_mid);
+              if (!wait(&bars->p_half[b][1], pph)) { fail(4u); break; }
               pph ^= 1;
               ptx::tc_fence_after();
-              issue_pv_parts<kSplit>(o0, sb, vd, idesc_pv, 1u, k_mid, ksteps);
-              ptx::tc_commit(&bars->kv_empty[slot_v]);
-              ptx::tc_commit(&bars->pv_done);
+              issue_pv_parts<kSplit>(on, o0, sb, vd, idesc_pv, 1u, k_mid, ksteps);
+              ptx::tc_commit_on(on, &bars->kv_empty[slot_v]);
+              ptx::tc_commit_on(on, &bars->pv_done);
               if (j + 2 < w.nkv && !qk(j + 2)) break;  // overwrites the S / P columns the P V above has just read
-              if (j + 1 == w.nkv) ptx::tc_commit(&bars->o_full[0]);
+              if (j + 1 == w.nkv) ptx::tc_commit_on(on, &bars->o_full[0]);
             }
             continue;
           }
           // ---- S_t(0) = Q_t K(0)^T ----
-          stamp(a, 16 * n_item + 5);
-          if (!ptx::mbar_wait(&bars->q_full[qb], (n_item / C::kQBufs) & 1, abort_flag)) {
+          if (on) stamp(a, 16 * n_item + 5);
+          if (!wait(&bars->q_full[qb], (n_item / C::kQBufs) & 1)) {
             fail(1u);
             break;
           }
-          stamp(a, 16 * n_item + 6);
-          if (!ptx::mbar_wait(&bars->kv_full[slot], par, abort_flag)) {
+          if (on) stamp(a, 16 * n_item + 6);
+          if (!wait(&bars->kv_full[slot], par)) {
             fail(1u);
             break;
           }
-          stamp(a, 16 * n_item + 1);
+          if (on) stamp(a, 16 * n_item + 1);
           ptx::tc_fence_after();
           {
             const uint64_t kd = ring_k + (uint64_t)(slot * (C::kTileBytes >> 4));
-            issue_qk<D>(s0, qd0, kd, idesc_qk);
-            ptx::tc_commit(&bars->s_full[0]);
+            issue_qk<D>(on, s0, qd0, kd, idesc_qk);
+            ptx::tc_commit_on(on, &bars->s_full[0]);
             if (ntile == 2) {
-              issue_qk<D>(s1, qd1, kd, idesc_qk);
-              ptx::tc_commit(&bars->s_full[1]);
+              issue_qk<D>(on, s1, qd1, kd, idesc_qk);
+              ptx::tc_commit_on(on, &bars->s_full[1]);
             }
-            ptx::tc_commit(&bars->kv_empty[slot]);
-            if (w.nkv == 1) ptx::tc_commit(&bars->q_empty[qb]);  // Q is no longer needed: the next item may load its own
+            ptx::tc_commit_on(on, &bars->kv_empty[slot]);
+            if (w.nkv == 1) ptx::tc_commit_on(on, &bars->q_empty[qb]);  // Q is no longer needed: the next item may load its own
             advance();
           }
           for (int j = 0; j < w.nkv && ok; ++j) {
@@ -569,8 +740,8 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             const int valid = max(16, min(kBN, w.sk - (w.j0 + j) * kBN));  // at least one 16-key step (P = 0 there if sk = 0)
             const int ksteps = (valid + 15) >> 4;
             const int k_mid = min(ksteps, 4);
-            if (!ptx::mbar_wait(&bars->kv_full[slot_v], par_v, abort_flag) ||
-                (more && !ptx::mbar_wait(&bars->kv_full[slot_k], par_k, abort_flag))) {
+            if (!wait(&bars->kv_full[slot_v], par_v) ||
+                (more && !wait(&bars->kv_full[slot_k], par_k))) {
               fail(1u);
               break;
             }
@@ -578,37 +749,37 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             const uint64_t kd = ring_k + (uint64_t)(slot_k * (C::kTileBytes >> 4));
             const bool last_qk = more && (j + 2 == w.nkv);  // the QK issued in this iteration is the item's last
             // ---- tile 0 ----  (P arrives in two halves of 64 keys so P*V starts while the softmax still runs)
-            if (!DT_OPT(16) && !ptx::mbar_wait(&bars->p_half[0][0], pph0, abort_flag)) { fail(4u); break; }
-            if (j == 0) stamp(a, 16 * n_item + 2);
+            if (!DT_OPT(16) && !wait(&bars->p_half[0][0], pph0)) { fail(4u); break; }
+            if (j == 0 && on) stamp(a, 16 * n_item + 2);
             ptx::tc_fence_after();
-            issue_pv_parts<kSplit>(o0, s0, vd, idesc_pv, j > 0 ? 1u : 0u, 0, k_mid);
-            if (!DT_OPT(16) && !ptx::mbar_wait(&bars->p_half[0][1], pph0, abort_flag)) { fail(4u); break; }
+            issue_pv_parts<kSplit>(on, o0, s0, vd, idesc_pv, j > 0 ? 1u : 0u, 0, k_mid);
+            if (!DT_OPT(16) && !wait(&bars->p_half[0][1], pph0)) { fail(4u); break; }
             pph0 ^= 1;
             ptx::tc_fence_after();
-            issue_pv_parts<kSplit>(o0, s0, vd, idesc_pv, 1u, k_mid, ksteps);
-            if (ntile == 1) ptx::tc_commit(&bars->kv_empty[slot_v]);
-            if (more) issue_qk<D>(s0, qd0, kd, idesc_qk);
-            ptx::tc_commit(more ? &bars->s_full[0] : &bars->o_full[0]);  // next S ready, or (last block) O complete
-            if (!more) stamp(a, 16 * n_item + 3);
+            issue_pv_parts<kSplit>(on, o0, s0, vd, idesc_pv, 1u, k_mid, ksteps);
+            if (ntile == 1) ptx::tc_commit_on(on, &bars->kv_empty[slot_v]);
+            if (more) issue_qk<D>(on, s0, qd0, kd, idesc_qk);
+            ptx::tc_commit_on(on, more ? &bars->s_full[0] : &bars->o_full[0]);  // next S ready, or (last block) O complete
+            if (!more && on) stamp(a, 16 * n_item + 3);
             if (more && ntile == 1) {
-              ptx::tc_commit(&bars->kv_empty[slot_k]);
-              if (last_qk) ptx::tc_commit(&bars->q_empty[qb]);
+              ptx::tc_commit_on(on, &bars->kv_empty[slot_k]);
+              if (last_qk) ptx::tc_commit_on(on, &bars->q_empty[qb]);
             }
             // ---- tile 1 ----
             if (ntile == 2) {
-              if (!DT_OPT(16) && !ptx::mbar_wait(&bars->p_half[1][0], pph1, abort_flag)) { fail(4u); break; }
+              if (!DT_OPT(16) && !wait(&bars->p_half[1][0], pph1)) { fail(4u); break; }
               ptx::tc_fence_after();
-              issue_pv_parts<kSplit>(o1, s1, vd, idesc_pv, j > 0 ? 1u : 0u, 0, k_mid);
-              if (!DT_OPT(16) && !ptx::mbar_wait(&bars->p_half[1][1], pph1, abort_flag)) { fail(4u); break; }
+              issue_pv_parts<kSplit>(on, o1, s1, vd, idesc_pv, j > 0 ? 1u : 0u, 0, k_mid);
+              if (!DT_OPT(16) && !wait(&bars->p_half[1][1], pph1)) { fail(4u); break; }
               pph1 ^= 1;
               ptx::tc_fence_after();
-              issue_pv_parts<kSplit>(o1, s1, vd, idesc_pv, 1u, k_mid, ksteps);
-              ptx::tc_commit(&bars->kv_empty[slot_v]);
-              if (more) issue_qk<D>(s1, qd1, kd, idesc_qk);
-              ptx::tc_commit(more ? &bars->s_full[1] : &bars->o_full[1]);
+              issue_pv_parts<kSplit>(on, o1, s1, vd, idesc_pv, 1u, k_mid, ksteps);
+              ptx::tc_commit_on(on, &bars->kv_empty[slot_v]);
+              if (more) issue_qk<D>(on, s1, qd1, kd, idesc_qk);
+              ptx::tc_commit_on(on, more ? &bars->s_full[1] : &bars->o_full[1]);
               if (more) {
-                ptx::tc_commit(&bars->kv_empty[slot_k]);
-                if (last_qk) ptx::tc_commit(&bars->q_empty[qb]);
+                ptx::tc_commit_on(on, &bars->kv_empty[slot_k]);
+                if (last_qk) ptx::tc_commit_on(on, &bars->q_empty[qb]);
               }
             }
           }
@@ -632,9 +803,9 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     uint32_t n_blocks = 0;  // K/V blocks this warpgroup has handed over so far, over all items (one tile per item)
     const bool probe = (warp == 4 && lane == 0);
 
-    for (int item = blockIdx.x; item < a.n_slots && ok; item += gridDim.x) {
-      const Item w = decode_item(item);
-      if (w.nkv == 0) continue;
+    int walk = first_work();
+    Item w;
+    while (ok && next_work(walk, w)) {
       if (t == 1 && !w.two) continue;  // this item has no second tile: neither side touches tile 1's barriers
       const int row = w.q0 + t * kBM + row_in_tile;
       const long long vis = a.is_causal ? (long long)row + w.off : (long long)w.sk;  // last visible key
@@ -924,6 +1095,27 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       oph ^= 1;
       if (probe) stamp(a, 16 * n_item + 10);
       ptx::tc_fence_after();
+      // a share of an item: leave (maximum, sum, O) and go on
+      int item_begin = 0, item_order = 0;
+      if (a.n_cuts > 0 && w.nkv < find_cut_item(a, walk - w.nkv, item_order, item_begin)) {
+        float* mine = share_of<D>(a, C::kTiles * 4, blockIdx.x, item_begin, t * 4 + (warp & 3));
+        __stcg(mine + lane, m_used);
+        __stcg(mine + 32 + lane, l);
+#pragma unroll 1
+        for (int c = 0; c < D / 16; ++c) {
+          uint32_t ov[16];
+          ptx::tmem_ld16(t_o + c * 16, ov);
+          ptx::tc_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 4; ++i)  // [D / 4][32 rows][4]: a warp writes 512 consecutive bytes
+            __stcg(reinterpret_cast<float4*>(mine + 64) + (c * 4 + i) * 32 + lane,
+                   make_float4(__uint_as_float(ov[4 * i]), __uint_as_float(ov[4 * i + 1]), __uint_as_float(ov[4 * i + 2]),
+                               __uint_as_float(ov[4 * i + 3])));
+        }
+        ptx::tc_fence_before();
+        ++n_item;
+        continue;
+      }
       if (a.sinks && row < w.sq) {
         // attention sink: one more score without a value row joins the denominator (l and O are relative to m_used)
         const float sl = to_float(reinterpret_cast<const T*>(a.sinks)[w.h]) * kLog2e;
@@ -1021,6 +1213,68 @@ int g_options = 0;
 float* g_dbg = nullptr;
 #endif
 
+size_t align256(size_t x) { return (x + 255) / 256 * 256; }
+
+// How a call's work is laid out over the SMs.
+struct Plan {
+  int item_rows, n_q, n_items;
+  int n_whole;           // items taken whole, in full rounds
+  int n_single, n_cuts;  // the items behind them as single tiles, or cut into this many runs (0, 0: they are whole too)
+  int cut_blocks;
+};
+
+long long blocks_of_item(const dt_sdpa_params& p, int item_rows, int qt) {
+  const long long all = (p.Sk + kBN - 1) / kBN;
+  if (!p.is_causal) return all;
+  const long long end = (long long)(qt + 1) * item_rows < p.Sq ? (long long)(qt + 1) * item_rows : p.Sq;
+  long long lim = end + (p.Sk - p.Sq);
+  if (lim > p.Sk) lim = p.Sk;
+  const long long n = (lim + kBN - 1) / kBN;
+  return n < 1 ? 1 : n;
+}
+
+Plan make_plan(const dt_sdpa_params& p, int tiles) {
+  Plan r{};
+  const int sms = device_sm_count();
+  const bool varlen = p.seq_offsets_q != nullptr;
+  const int rows = varlen ? p.max_seq_q : p.Sq, bh = p.Hq * (varlen ? p.n_seq : p.B);
+  // One tile per item where even that does not fill the SMs once: a pair of tiles on one SM takes about 1.5 times as long
+  // as one tile, and half of the SMs would have nothing to do.
+  const long long singles = (long long)((rows + kBM - 1) / kBM) * bh;
+  r.item_rows = tiles == 2 && singles > sms ? 2 * kBM : kBM;
+  r.n_q = (rows + r.item_rows - 1) / r.item_rows;
+  r.n_items = r.n_whole = r.n_q * bh;
+  if (varlen) return r;
+  const int rest = r.n_items % sms;
+  // For the same reason a last round of pairs that fills less than half of the SMs is taken tile by tile (2 images, 4096
+  // tokens, 20 heads of 64: 4.3 rounds).  The rows' results do not depend on it.
+  if (r.item_rows > kBM && r.n_items > sms && rest > 0 && 2 * rest <= sms) {
+    r.n_whole = r.n_items - rest;
+    r.n_single = 2 * rest;
+    return r;
+  }
+  // A call that leaves half of the SMs without any item (a short chunk of queries behind a long prefix): its K/V blocks cut
+  // into equal runs over all SMs, when that saves at least kCutGain blocks' time on the longest item.  A cut costs
+  // about two: the shares' way through L2 and one more launch.
+  constexpr int kCutGain = 4, kMinRun = 4;
+  if (2 * r.n_items > sms || p.sliding_window > 0) return r;
+  long long blocks = 0, longest = 0;
+  for (int qt = 0; qt < r.n_q; ++qt) {
+    const long long n = blocks_of_item(p, r.item_rows, qt);
+    blocks += n * bh;
+    if (n > longest) longest = n;
+  }
+  const long long runs = blocks / kMinRun < sms ? blocks / kMinRun : sms;
+  if (runs <= r.n_items || blocks * runs >= (1LL << 31) || longest - (blocks + runs - 1) / runs < kCutGain) return r;
+  r.n_whole = 0;
+  r.n_cuts = (int)runs;
+  r.cut_blocks = (int)blocks;
+  return r;
+}
+size_t split_bytes(const Plan& plan, int tiles, int D) {  // two shares per run
+  return (size_t)2 * plan.n_cuts * tiles * 4 * (D + 2) * 32 * sizeof(float);
+}
+
 bool mask_rows_aligned(const dt_sdpa_params& p) {
   return !(reinterpret_cast<uintptr_t>(p.mask) % 16 || p.mask_stride_b % 8 || p.mask_stride_h % 8 || p.mask_stride_q % 8);
 }
@@ -1032,6 +1286,14 @@ size_t mask_flag_bytes(const dt_sdpa_params& p) {
   return kTicketBytes + (Bm * Hm * n_rg * n_kh + 255) / 256 * 256;
 }
 int repacked_row(const dt_sdpa_params& p) { return (p.Sk + 7) / 8 * 8; }
+size_t prefill_repack_bytes_needed(const dt_sdpa_params& p) {  // the flags and the copy
+  const size_t Bm = p.mask_stride_b ? p.B : 1, Hm = p.mask_stride_h ? p.Hq : 1;
+  return mask_flag_bytes(p) + Bm * Hm * p.Sq * (size_t)repacked_row(p) * 2;
+}
+size_t cut_bytes(const dt_sdpa_params& p) {
+  const int D = p.D > 128 ? 256 : p.D > 64 ? 128 : 64, tiles = D == 256 ? 1 : 2;
+  return split_bytes(make_plan(p, tiles), tiles, D);
+}
 
 template <typename T, int D, bool kMask, bool kSplit = false>
 int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, int n_extra, void* workspace,
@@ -1058,7 +1320,7 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
   a.mask = p.mask;
   a.m_sb = p.mask_stride_b; a.m_sh = p.mask_stride_h; a.m_sq = p.mask_stride_q;
   if (kMask) {
-    if (!workspace || workspace_bytes < (kSplit ? prefill_repack_workspace_bytes(p) : prefill_workspace_bytes(p))) return DT_WORKSPACE;
+    if (!workspace || workspace_bytes < (kSplit ? prefill_repack_bytes_needed(p) : mask_flag_bytes(p))) return DT_WORKSPACE;
     const int Bm = p.mask_stride_b ? p.B : 1, Hm = p.mask_stride_h ? p.Hq : 1;
     a.n_rg = (p.Sq + 31) / 32;
     a.n_kh = ((p.Sk + 63) / 64 + 1) & ~1;
@@ -1088,18 +1350,36 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
   a.n_extra = n_extra;
   a.d_real = p.D;
   for (int i = 0; i < n_extra; ++i) a.extra_o[i] = extra[i];
-  const bool varlen = p.seq_offsets_q != nullptr;
   a.off_q = p.seq_offsets_q;
   a.off_k = p.seq_offsets_k;
-  a.n_qpairs = ((varlen ? p.max_seq_q : p.Sq) + C::kTiles * kBM - 1) / (C::kTiles * kBM);
-  a.n_items = a.n_qpairs * p.Hq * (varlen ? p.n_seq : p.B);
+  const Plan plan = make_plan(p, C::kTiles);
+  a.item_rows = plan.item_rows;
+  a.n_qpairs = plan.n_q;
+  a.n_items = plan.n_items;
   auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit>;
   DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
   const int n_sm = device_sm_count();
-  dim3 grid(a.n_items < n_sm ? a.n_items : n_sm);  // one persistent CTA per SM
-  a.n_slots = (a.n_items + (int)grid.x - 1) / (int)grid.x * (int)grid.x;
+  const size_t split_at = kMask ? (kSplit ? prefill_repack_bytes_needed(p) : mask_flag_bytes(p)) : kTicketBytes;
+  const bool cut = plan.n_cuts > 0 && workspace && reinterpret_cast<uintptr_t>(workspace) % 16 == 0 &&
+                   workspace_bytes >= align256(split_at) + split_bytes(plan, C::kTiles, D);
+  dim3 grid(cut ? plan.n_cuts : a.n_items < n_sm ? a.n_items : n_sm);  // one persistent CTA per SM
+  if (plan.n_single > 0) {
+    a.n_slots = plan.n_whole;
+    a.n_single = plan.n_single;
+  } else if (cut) {
+    a.n_slots = 0;
+    a.n_cuts = plan.n_cuts;
+    a.cut_blocks = plan.cut_blocks;
+    a.part = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + align256(split_at));
+  } else {
+    a.n_slots = (a.n_items + (int)grid.x - 1) / (int)grid.x * (int)grid.x;
+  }
   kern<<<grid, kThreads, C::kSmemBytes, stream>>>(mq, mk, mv, mo, a);
   DT_CUDA_TRY(cudaGetLastError());
+  if (cut) {
+    cut_combine_kernel<T, D><<<dim3((a.n_items - a.n_slots) * C::kTiles * 4, (p.D + 63) / 64), 256, 0, stream>>>(a, C::kTiles * 4);
+    DT_CUDA_TRY(cudaGetLastError());
+  }
   return DT_OK;
 }
 
@@ -1124,7 +1404,12 @@ bool prefill_supported(const dt_sdpa_params& p) {
   return ok(p.q) && ok(p.k) && ok(p.v) && ok(p.o);
 }
 
-size_t prefill_workspace_bytes(const dt_sdpa_params& p) { return p.mask ? mask_flag_bytes(p) : 0; }
+// The masked variant needs its flags; the scratch of cut items is optional (without it, or with less, nothing is cut).
+size_t prefill_workspace_bytes(const dt_sdpa_params& p) {
+  const size_t cut = cut_bytes(p);
+  if (cut) return align256(p.mask ? mask_flag_bytes(p) : kTicketBytes) + cut;
+  return p.mask ? mask_flag_bytes(p) : 0;
+}
 
 // Masks whose rows are not 16-byte aligned: copied to aligned rows first.  The calls come from the CUDA-core kernel, whose
 // weights are fp32, so this variant multiplies V with two 16-bit parts of every weight: 333 tokens, 32 / 8 heads of 128,
@@ -1134,14 +1419,16 @@ bool prefill_repack_supported(const dt_sdpa_params& p) {
   if (!p.mask || mask_rows_aligned(p) || (p.flags & DT_FLAG_FORCE_GENERIC)) return false;
   dt_sdpa_params plain = p;
   plain.mask = nullptr;
-  if (!prefill_supported(plain) || (p.Sq + 31) / 32 > 65535) return false;
+  // up to one 64-key tile the CUDA-core kernel takes a single step (41 tokens, 32 heads: 18.2 us there, 19.2 us here; 77
+  // tokens, 12 heads: 23.1 and 17.3 us)
+  if (p.Sk <= 64 || !prefill_supported(plain) || (p.Sq + 31) / 32 > 65535) return false;
   const size_t Bm = p.mask_stride_b ? p.B : 1, Hm = p.mask_stride_h ? p.Hq : 1;
   return Bm * Hm <= 65535 && Bm * Hm * p.Sq * (size_t)repacked_row(p) * 2 <= ((size_t)256 << 20);
 }
 
 size_t prefill_repack_workspace_bytes(const dt_sdpa_params& p) {
-  const size_t Bm = p.mask_stride_b ? p.B : 1, Hm = p.mask_stride_h ? p.Hq : 1;
-  return mask_flag_bytes(p) + Bm * Hm * p.Sq * (size_t)repacked_row(p) * 2;
+  const size_t cut = cut_bytes(p);
+  return cut ? align256(prefill_repack_bytes_needed(p)) + cut : prefill_repack_bytes_needed(p);
 }
 
 int launch_prefill_repack(const dt_sdpa_params& p, cudaStream_t stream, void* workspace, size_t workspace_bytes) {

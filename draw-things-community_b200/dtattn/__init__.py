@@ -287,12 +287,13 @@ def sdpa_forward(q, k, v, scale, is_causal=False, mask=None, out=None, lse=None,
                     seq_offsets_k, max_seq_q, max_seq_k)
     if q.is_cuda:
         s = _stream_of(q.device, stream)
-        if workspace is None and (mask is not None or q.dtype == torch.float32) and kernel_name(p) == "generic":
-            scratch = _call_scratch(workspace_size(p), q.device, s)
+        need = workspace_size(p)
+        if need and workspace is None and kernel_name(p) != "decode_splitkv":
+            scratch = _call_scratch(need, q.device, s)
             ptr, nbytes = (None, 0) if scratch is None else (scratch.data_ptr(), scratch.numel())
         else:
             ws = workspace if workspace is not None else _default_workspace(q.device)
-            ptr, nbytes = ws.ensure(workspace_size(p), s)
+            ptr, nbytes = ws.ensure(need, s)
         _check(lib().dt_sdpa_forward(ctypes.byref(p), ctypes.c_void_p(ptr) if ptr else None, nbytes,
                                      ctypes.c_void_p(s)), "dt_sdpa_forward")
     else:
@@ -466,8 +467,8 @@ class SparseIndexedAttention:
 
 
 def _call_scratch(nbytes, device, stream):
-    """Optional scratch of one call (any contents), its own so that calls on several streams stay independent; None when
-    there is no room for it, which the library answers with the kernel that needs none."""
+    """Scratch of one call (any contents), its own so that calls on several streams stay independent; None when there is
+    no room for it, which the library answers with a way that needs none (a masked call on the tensor cores has none)."""
     if nbytes == 0:
         return None
     try:
