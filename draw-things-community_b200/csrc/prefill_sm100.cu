@@ -581,16 +581,6 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         bool more_work = next_work(walk, nx);
         for (; more_work && ok; ++n_item) {
           w = nx;
-          more_work = next_work(walk, nx);
-          // The Q tiles of the NEXT item are pulled into L2 now: their rows are 256-byte pieces a whole
-          // token stride apart (slow to gather from HBM), and the real load sits on the critical path
-          // between two items.
-          if (more_work) {
-            for (int t = 0; t < (nx.two ? 2 : 1); ++t)
-#pragma unroll
-              for (int hf = 0; hf < C::kHalves; ++hf)
-                ptx::tma_prefetch_l2_4d(&map_q, hf * 64, nx.h, nx.qrow + nx.q0 + t * kBM, nx.b);
-          }
           // first K/V block of this item may be fetched while the previous item still owns the Q buffers
           // (one tile per item: the MMA warp consumes K(0), K(1), V(0), K(2), V(1), ..., and the ring follows that order)
           if constexpr (C::kTiles == 1) ok = load_kv(w, 0, false) && (w.nkv == 1 || load_kv(w, 1, false));
@@ -609,6 +599,16 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             for (int hf = 0; hf < C::kHalves; ++hf)
               ptx::tma_load_4d(base_ptr + (qb * C::kTiles + t) * C::kTileBytes + hf * kHalfBytes, &map_q, &bars->q_full[qb], hf * 64,
                                w.h, w.qrow + w.q0 + t * kBM, w.b);
+          // The Q tiles of the NEXT item are pulled into L2 now: their rows are 256-byte pieces a whole
+          // token stride apart (slow to gather from HBM), and the real load sits on the critical path
+          // between two items.
+          more_work = next_work(walk, nx);  // (behind this item's own first loads: finding it takes a few hundred cycles)
+          if (more_work) {
+            for (int t = 0; t < (nx.two ? 2 : 1); ++t)
+#pragma unroll
+              for (int hf = 0; hf < C::kHalves; ++hf)
+                ptx::tma_prefetch_l2_4d(&map_q, hf * 64, nx.h, nx.qrow + nx.q0 + t * kBM, nx.b);
+          }
           if constexpr (C::kTiles == 1) {
             for (int j = 0; j < w.nkv && ok; ++j) ok = load_kv(w, j, true) && (j + 2 >= w.nkv || load_kv(w, j + 2, false));
           } else {
@@ -619,9 +619,10 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     } else if (warp == 1) {
       // =========================== MMA issuer ===========================
       // The whole warp walks the loop and one lane issues, which keeps the operands in uniform registers (Flux joint
-      // attention 227 -> 223 us, 2047 tokens with an unaligned mask 97 -> 88 us); the 64-wide variant, whose MMAs are fewer
-      // than its softmax warps can follow, is 1 % faster with one lane walking it (SD1.5 self-attention 125 against 127 us).
-      constexpr bool kWarpIssue = D >= 128;
+      // attention 227 -> 216 us, 2047 tokens with an unaligned mask 97 -> 86 us); the 64- and 256-wide variants, whose MMAs
+      // are fewer or longer, are 1 % faster with one lane walking it (SD1.5 self-attention 125 against 126 us, 1777 x 5873
+      // prompt chunk of dim 256 125 against 126 us).
+      constexpr bool kWarpIssue = D == 128;
       if (kWarpIssue || lane == 0) {
         const bool on = kWarpIssue ? ptx::elect_one() : true;
         constexpr uint32_t idesc_qk = ptx::make_idesc_f16(kBf16, kBM, kBN, 0, 0);
