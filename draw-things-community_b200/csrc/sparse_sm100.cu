@@ -10,14 +10,19 @@
 // leaves room for two S buffers of two accumulators each (neighbouring MMAs on one accumulator wait for each other: a chain
 // of M = 64, N = 48 MMAs took 66 cycles each, twice its share of the pipe).  10 warps:
 //   warps 0-3   softmax, one thread per head (the 64 rows of S are lanes 0-15 of the four TMEM quarters); P goes to shared
-//               memory; O^T is rescaled only when a head's maximum grew by more than 2^8; at the end O^T / l is stored,
-//               two neighbouring dims per 4-byte store
+//               memory in two 16-bit parts per weight; O^T is rescaled only when a head's maximum grew by more than 2^8; at
+//               the end O^T / l is stored, two neighbouring dims per 4-byte store
 //   warps 4-7   gather: TMA loads of four named rows x 64 dims; entries that name no row read zeros; entries behind a
 //               token's last valid one are left out (a prompt's first tokens have few)
 //   warp 8      MMA issuer: QK(0) QK(1) | PV(0) QK(2) | PV(1) QK(3) | ...
 //   warp 9      TMEM allocation, TMA of the next token's queries
-// Measured (prompt of 4096 tokens, 64 heads of 512, 128 + up to 512 keys each): 2110 us with warp-level MMAs, 512 us here
-// (538 TFLOP/s of visible work, tensor pipe 58 % active).
+// Why two parts: a weight of 16 bits relative to a maximum that is older than the tile makes the result's error against 64 bits
+// 4 % larger than relative to the running maximum (2.07e-3 -> 2.15e-3 in bf16 for N(0,1) scores; 20 % where few keys carry the
+// weight), and rescaling O^T for every growth costs as much as the second part's products (659 and 660 us where one part and the
+// older maximum take 514).  With two parts the error is the rounding of the result, 1.66e-3.
+// Measured (prompt of 4096 tokens, 64 heads of 512, 128 + up to 512 keys each): 2110 us with warp-level MMAs, 660 us here
+// (415 TFLOP/s of visible work).  Bound: shared-memory reads of the products' operands (a second part's M = 128, N = 64 MMA takes 52
+// cycles where its share of the tensor pipe is 32) and the softmax warps' chain.
 // What set the time on the way: the gather.  With asynchronous 16-byte copies of four warps it moved 11 bytes per cycle
 // (1775 us), with all the TMA loads issued by one warp, 68 cycles each, 7 (1446 us).
 // Every mbarrier wait is bounded.  The softmax warps also meet at a named barrier once per tile; a wait that ran out is part
@@ -38,7 +43,7 @@ constexpr int kSub = kTK * 128;                     // 64 dims of a tile: [kTK k
 constexpr int kTileBytes = (kMaxD / 64) * kSub;
 constexpr int kQSub = kHeads * 128;
 constexpr int kQBytes = (kMaxD / 64) * kQSub;
-constexpr int kPBytes = kHeads * 128;               // [64 heads][up to 64 keys]
+constexpr int kPBytes = kHeads * 128;               // [64 heads][up to 64 keys], one part of the weights
 constexpr int kSmemBytes = kQBytes + kBufs * kTileBytes + 2 * kPBytes + 1024 + 1024;
 constexpr uint32_t kColS = 256;                     // S buffers behind the 256 columns of O^T
 constexpr float kRescaleThreshold = 8.f;
@@ -48,8 +53,10 @@ static_assert(kTK % 16 == 0 && kTK <= 64 && kSub % 1024 == 0, "tile");
 struct Bars {
   uint64_t q_full, q_empty;
   uint64_t kv_full[kBufs], kv_empty[kBufs];
-  uint64_t s_full[2], p_full[2];
-  uint64_t pv_done;  // completes once per tile's P V
+  uint64_t s_full[2];
+  // One phase per tile: its weights are in shared memory; its P V has run.  The softmax warps wait for every tile's P V in
+  // turn: a phase left out would let the next wait's parity be that of an older one.
+  uint64_t p_full, pv_done;
   uint32_t tmem_base;
   int abort_flag;
   uint32_t valid[kBufs][4];  // bit 4 k + i of word w: row 4 (w + 4 k) + i of the tile holds a key
@@ -94,6 +101,23 @@ __device__ __forceinline__ Item decode_item(const Args& a, int item) {
   return w;
 }
 
+// two floats -> 16-bit pair and back
+template <typename T>
+__device__ __forceinline__ uint32_t pack_pair(uint64_t x2) {
+  float lo, hi;
+  ptx::unpack_f32x2(x2, lo, hi);
+  return std::is_same<T, __half>::value ? ptx::cvt_pack_f16(lo, hi) : ptx::cvt_pack_bf16(lo, hi);
+}
+template <typename T>
+__device__ __forceinline__ uint64_t unpack_pair(uint32_t x) {
+  if constexpr (std::is_same<T, __half>::value) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&x));
+    return ptx::pack_f32x2(f.x, f.y);
+  } else {
+    return ptx::pack_f32x2(__uint_as_float(x << 16), __uint_as_float(x & 0xffff0000u));
+  }
+}
+
 // OR of a predicate over the 128 softmax threads, the same answer for all of them.
 __device__ __forceinline__ bool vote_any(bool x) {
   uint32_t r;
@@ -123,10 +147,8 @@ sparse_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       ptx::mbar_init(&bars->kv_full[i], 4);  // one arrival per gather warp (and the bytes)
       ptx::mbar_init(&bars->kv_empty[i], 1);
     }
-    for (int i = 0; i < 2; ++i) {
-      ptx::mbar_init(&bars->s_full[i], 1);
-      ptx::mbar_init(&bars->p_full[i], 4);  // one arrival per softmax warp
-    }
+    for (int i = 0; i < 2; ++i) ptx::mbar_init(&bars->s_full[i], 1);
+    ptx::mbar_init(&bars->p_full, 4);  // one arrival per softmax warp
     ptx::mbar_init(&bars->pv_done, 1);
     bars->abort_flag = 0;
     ptx::fence_mbar_init();
@@ -256,17 +278,18 @@ sparse_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       };
       if (!qk() || (!last_qk && !qk())) break;
       for (uint32_t t = 0; ok; ++t) {
-        const uint32_t pb = gv & 1u;
-        if (!wait(&bars->p_full[pb], (gv >> 1) & 1u, 4u)) break;
+        if (!wait(&bars->p_full, gv & 1u, 4u)) break;
         ptx::tc_fence_after();
-        const uint64_t vd = vt_desc + (uint64_t)(vbuf * (kTileBytes >> 4)), pd = p_desc + (uint64_t)(pb * (kPBytes >> 4));
+        const uint64_t vd = vt_desc + (uint64_t)(vbuf * (kTileBytes >> 4));
 #pragma unroll
-        for (int ks = 0; ks < kTK / 16; ++ks)
+        for (int part = 0; part < 2; ++part)  // the weights' high parts, then what those leave over
 #pragma unroll
-          for (int mt = 0; mt < kMaxD / 128; ++mt)
-            if (2 * mt < subs)
-              ptx::mma_ss_on(on, tmem + mt * kHeads, vd + (uint64_t)((mt * 2 * kSub + ks * 2048) >> 4), pd + (uint64_t)((ks * 32) >> 4),
-                             idesc_pv, (t > 0 || ks > 0) ? 1u : 0u);
+          for (int ks = 0; ks < kTK / 16; ++ks)
+#pragma unroll
+            for (int mt = 0; mt < kMaxD / 128; ++mt)
+              if (2 * mt < subs)
+                ptx::mma_ss_on(on, tmem + mt * kHeads, vd + (uint64_t)((mt * 2 * kSub + ks * 2048) >> 4),
+                               p_desc + (uint64_t)((part * kPBytes + ks * 32) >> 4), idesc_pv, (t > 0 || part > 0 || ks > 0) ? 1u : 0u);
         ptx::tc_commit_on(on, &bars->kv_empty[vbuf]);
         ptx::tc_commit_on(on, &bars->pv_done);
         ++gv;
@@ -299,7 +322,7 @@ sparse_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     uint32_t g = 0;
     int kbuf = 0;
     uint32_t kpar = 0;
-    bool ok = true;
+    bool ok = true, lost = false;  // lost: a wait for P V ran out, part of what the next vote is about
     for (int item = blockIdx.x; item < a.n_items && ok; item += gridDim.x) {
       const Item w = decode_item(a, item);
       float m = -INFINITY, l = 0.f;
@@ -307,7 +330,7 @@ sparse_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       for (int t = 0; !last; ++t, ++g) {
         const uint32_t sb = g & 1u;
         bool failed = !__all_sync(0xffffffffu, ptx::mbar_wait(&bars->s_full[sb], (g >> 1) & 1u, abort_flag) &&
-                                                   ptx::mbar_wait(&bars->kv_full[kbuf], kpar, abort_flag));
+                                                   ptx::mbar_wait(&bars->kv_full[kbuf], kpar, abort_flag)) || lost;
         ptx::tc_fence_after();
         uint32_t s[kTK], s_odd[kTK];
 #pragma unroll
@@ -371,31 +394,39 @@ sparse_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         const float neg_m = m == -INFINITY ? 0.f : -m;
         const uint64_t neg_m2 = ptx::pack_f32x2(neg_m, neg_m), scale2 = ptx::pack_f32x2(sl2, sl2);
         uint64_t lsum = 0ull;
-        uint32_t pw[kTK / 2];
+        uint32_t pw[kTK / 2], rest[kTK / 2];
 #pragma unroll
         for (int i = 0; i < kTK / 2; ++i) {
           const uint64_t x2 = ptx::fma_f32x2(ptx::pack_f32x2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), scale2, neg_m2);
           float x0, x1;
           ptx::unpack_f32x2(x2, x0, x1);
-          const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
-          lsum = ptx::add_f32x2(lsum, ptx::pack_f32x2(p0, p1));
-          pw[i] = kBf16 ? ptx::cvt_pack_bf16(p0, p1) : ptx::cvt_pack_f16(p0, p1);
+          const uint64_t p2 = ptx::pack_f32x2(fast_exp2(x0), fast_exp2(x1));
+          lsum = ptx::add_f32x2(lsum, p2);
+          pw[i] = pack_pair<T>(p2);
+          rest[i] = pack_pair<T>(ptx::fma_f32x2(unpack_pair<T>(pw[i]), ptx::pack_f32x2(-1.f, -1.f), p2));
         }
         float s0, s1;
         ptx::unpack_f32x2(lsum, s0, s1);
         l += s0 + s1;
-        if (mine) {
-          const uint32_t prow = pbuf + sb * kPBytes + (uint32_t)head * 128;
+        // the previous tile's P V has read its weights (it ran behind this tile's Q K^T: usually over by now)
+        if (g > 0) lost = !__all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done, (g - 1) & 1u, abort_flag));
+        if (mine && !lost) {
+          const uint32_t prow = pbuf + (uint32_t)head * 128;
 #pragma unroll
-          for (int q = 0; q < kTK / 8; ++q)
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(prow + (uint32_t)((q ^ (head & 7)) << 4)), "r"(pw[4 * q]),
-                         "r"(pw[4 * q + 1]), "r"(pw[4 * q + 2]), "r"(pw[4 * q + 3])
+          for (int q = 0; q < kTK / 8; ++q) {
+            const uint32_t at = prow + (uint32_t)((q ^ (head & 7)) << 4);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(pw[4 * q]), "r"(pw[4 * q + 1]), "r"(pw[4 * q + 2]),
+                         "r"(pw[4 * q + 3])
                          : "memory");
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + kPBytes), "r"(rest[4 * q]), "r"(rest[4 * q + 1]),
+                         "r"(rest[4 * q + 2]), "r"(rest[4 * q + 3])
+                         : "memory");
+          }
         }
         ptx::fence_proxy_async_smem();
         ptx::tc_fence_before();
         __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&bars->p_full[sb]);
+        if (lane == 0) ptx::mbar_arrive(&bars->p_full);
       }
       if (!ok) break;
 
@@ -410,7 +441,7 @@ sparse_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       }
       if (mine) bars->inv[head] = inv;
       if (a.lse && mine) a.lse[((int64_t)w.b * a.Hq + w.h0 + head) * a.Sq + w.i] = l > 0.f ? m_f * kLn2 + logf(l) : -INFINITY;
-      const bool late = !__all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done, (g - 1) & 1u, abort_flag));
+      const bool late = !__all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done, (g - 1) & 1u, abort_flag)) || lost;
       if (vote_any(late)) {
         if (late) report(5u);
         ok = false;
