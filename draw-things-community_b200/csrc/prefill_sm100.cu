@@ -302,16 +302,16 @@ __global__ void __launch_bounds__(256) cut_combine_kernel(const PrefillArgs a, c
     float4 x[2];
 #pragma unroll
     for (int g = 0; g < 2; ++g) x[g] = __ldg(reinterpret_cast<const float4*>(sh + 64) + (col0 / 4 + cg + 8 * g) * 32 + r);
-    if (mc != -INFINITY) {  // (a share that saw no key holds no numbers)
-      const float f = fast_exp2(mc - m);
-      l = fmaf(f, lc, l);
+    // A share that saw no key counts nothing, but it is not left out: a row whose scores are all NaN has no maximum either
+    // (a maximum ignores NaN), and its NaN sum and O must reach the result as they do in a call that is not cut.
+    const float f = mc == -INFINITY ? 0.f : fast_exp2(mc - m);
+    l = fmaf(f, lc, l);
 #pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        acc[g].x = fmaf(f, x[g].x, acc[g].x);
-        acc[g].y = fmaf(f, x[g].y, acc[g].y);
-        acc[g].z = fmaf(f, x[g].z, acc[g].z);
-        acc[g].w = fmaf(f, x[g].w, acc[g].w);
-      }
+    for (int g = 0; g < 2; ++g) {
+      acc[g].x = fmaf(f, x[g].x, acc[g].x);
+      acc[g].y = fmaf(f, x[g].y, acc[g].y);
+      acc[g].z = fmaf(f, x[g].z, acc[g].z);
+      acc[g].w = fmaf(f, x[g].w, acc[g].w);
     }
   }
   if (a.sinks) {  // as in the attention kernel's epilogue

@@ -61,6 +61,40 @@ def test_against_the_oracle_and_the_uncut_call(dtattn, case):
         check(out, ref.float(), dtype, f"{case} uncut")
 
 
+@pytest.mark.parametrize("where", ["one query row", "a run of keys"])
+@pytest.mark.parametrize("extra", ["", "causal", "sinks", "mask"])
+@pytest.mark.parametrize("D", [64, 256])
+def test_nan_is_kept(dtattn, D, extra, where):
+    """A NaN in a query row makes every score of the row NaN, which no maximum shows; NaN keys do so for a whole share.  The
+    cut call must give NaN where the uncut one does, and every other row as without the NaN."""
+    B, Sq, Sk, Hq, Hkv, dtype = 1, 200, 2304, 4, 2, torch.bfloat16
+    q, k, v = (x.to(DEV) for x in inputs(B, Sq, Sk, Hq, Hkv, D, dtype, 1621))
+    mask = make_mask(1, 1, Sq, Sk, dtype, 1622).to(DEV) if extra == "mask" else None
+    sinks = so.seeded_normal((Hq,), 1623).to(dtype).to(DEV) if extra == "sinks" else None
+
+    def run(scratch_bytes):
+        out, lse = torch.zeros_like(q), torch.zeros(B, Hq, Sq, device=DEV)
+        p = dtattn.make_params(q, k, v, out, D ** -0.5, extra == "causal", mask, lse, sinks=sinks)
+        need = dtattn.workspace_size(p) if scratch_bytes is None else scratch_bytes
+        forward(dtattn, p, torch.zeros(need, dtype=torch.uint8, device=DEV) if need else None)
+        return out, lse, need
+
+    clean, clean_lse, need = run(None)
+    flags_only = 4096 + (((Sq + 31) // 32 * ((Sk + 127) // 128 * 2) + 255) // 256) * 256 if mask is not None else 0
+    assert need > 4096 + flags_only, "this case is meant to be cut"
+    if where == "one query row":
+        q[0, 77, 1, 5] = float("nan")
+    else:
+        k[0, 256:Sk - 100] = float("nan")  # with the causal rule every row sees some of them
+    (cut, cut_lse, _), (whole, whole_lse, _) = run(None), run(flags_only)
+    assert bool(whole.isnan().any())
+    assert torch.equal(cut.isnan(), whole.isnan()) and torch.equal(cut_lse.isnan(), whole_lse.isnan())
+    assert torch.equal(cut_lse == -float("inf"), whole_lse == -float("inf"))
+    rows = ~cut.isnan().any(dim=-1)
+    assert torch.equal(cut[rows], clean[rows])
+    assert torch.equal(cut_lse.transpose(1, 2)[rows], clean_lse.transpose(1, 2)[rows])
+
+
 @pytest.mark.parametrize("case", [
     # B, Sq, Sk, Hq, Hkv, D, causal, dtype: single tiles throughout (up to 148 of them), and a last round of pairs tile by
     # tile (149 to 222 pairs), with and without a second tile in the last pair
