@@ -256,9 +256,11 @@ int dt_sdpa_forward(const dt_sdpa_params* p, void* workspace, size_t workspace_b
     case kShortKV: return launch_short_kv(*p, stream);
     default: {
       const size_t scratch = optional_scratch(*p);
-      if (scratch == 0 || !workspace || reinterpret_cast<uintptr_t>(workspace) % 16 || workspace_bytes < scratch)
-        return launch_generic(*p, stream);
-      return p->dtype == DT_F32 ? launch_f32_mma(*p, workspace, stream) : launch_prefill_repack(*p, stream, workspace, workspace_bytes);
+      if (scratch != 0 && workspace && reinterpret_cast<uintptr_t>(workspace) % 16 == 0 && workspace_bytes >= scratch) {
+        st = p->dtype == DT_F32 ? launch_f32_mma(*p, workspace, stream) : launch_prefill_repack(*p, stream, workspace, workspace_bytes);
+        if (st != DT_UNSUPPORTED) return st;  // (views that no tensor map describes, an expanded axis for one: nothing was launched)
+      }
+      return launch_generic(*p, stream);
     }
   }
 }

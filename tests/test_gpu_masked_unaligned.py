@@ -64,3 +64,33 @@ def test_scratch_limits(dtattn):
     p.Sq = p.Sk = 8201
     p.mask_stride_q, p.mask_stride_h = 8201, 8201 * 8201
     assert dtattn.workspace_size(p) == 0
+
+
+@pytest.mark.parametrize("what", ["k and v over the heads", "k and v over the batch", "v over the tokens", "q over the batch"])
+def test_expanded_views_stay_on_the_cuda_cores(dtattn, what):
+    """A view with a zero stride (torch.expand) is not for tensor maps: served as before, whatever scratch there is."""
+    B, S, H, D, dtype = 2, 101, 4, 64, torch.bfloat16
+    q, k, v = inputs(B, S, S, H, H, D, dtype, 1431)
+    if what == "k and v over the heads":
+        k, v = k[:, :, :1].expand(B, S, H, D), v[:, :, :1].expand(B, S, H, D)
+    elif what == "k and v over the batch":
+        k, v = k[:1].expand(B, S, H, D), v[:1].expand(B, S, H, D)
+    elif what == "v over the tokens":
+        v = v[:, :1].expand(B, S, H, D)
+    else:
+        q = q[:1].expand(B, S, H, D)
+    mask = make_mask(1, 1, S, S, dtype, 1432)
+    ref = so.sdpa_explicit(q, k, v, D ** -0.5, False, mask, compute_dtype=torch.float64)
+
+    def dev(t):  # the same view on the device
+        small = t[tuple(slice(0, 1) if st == 0 else slice(None) for st in t.stride())]
+        return small.to(DEV).expand(t.shape)
+
+    qd, kd, vd = dev(q), dev(k), dev(v)
+    out = torch.zeros(B, S, H, D, dtype=dtype, device=DEV)
+    dtattn.sdpa_forward(qd, kd, vd, D ** -0.5, mask=mask.to(DEV), out=out)
+    want = dtattn.sdpa_forward(qd, kd, vd, D ** -0.5, mask=mask.to(DEV), flags=dtattn.DT_FLAG_FORCE_GENERIC)
+    torch.cuda.synchronize()
+    assert dtattn.device_status() == 0
+    check(out, ref.float(), dtype, what)
+    assert torch.equal(out, want)
