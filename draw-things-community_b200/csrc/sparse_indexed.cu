@@ -610,7 +610,10 @@ int launch_sparse_mma_t(const dt_sparse_indexed_params& p, const SparseArgs& a, 
     return u.ptr == v.ptr && u.stride_b == v.stride_b && u.stride_s == v.stride_s && u.stride_h == v.stride_h;
   };
   const bool same_kv = same(p.k_raw, p.v_raw) && (p.Sc == 0 || p.n_selected == 0 || same(p.k_comp, p.v_comp));
-  if (sparse_tcgen05_supported(p, same_kv)) return launch_sparse_tcgen05(p, stream);
+  if (sparse_tcgen05_supported(p, same_kv)) {
+    const int st = launch_sparse_tcgen05(p, stream);
+    if (st != DT_UNSUPPORTED) return st;  // (views that no tensor map describes, expanded queries for one: nothing was launched)
+  }
   const int keys = (p.sliding_window > 0 ? (p.sliding_window < p.Sr ? p.sliding_window : p.Sr) : p.Sr) + (p.Sc > 0 ? p.n_selected : 0);
   if (same_kv && keys >= 256 && (long long)p.Sq * p.B >= 64) return launch_sparse_mma_tk<T, 64>(p, a, stream);
   return launch_sparse_mma_tk<T, 32>(p, a, stream);

@@ -98,3 +98,33 @@ def test_many_short_tokens_per_cta(dtattn, n_keys):
     assert dtattn.device_status() == 0
     assert float((outs[0].float().cpu() - ref.float()).abs().max()) <= 2 * ROUND[dtype] * float(ref.abs().max()) + so.TOL_MAX_ABS
     assert all(torch.equal(o, outs[0]) for o in outs)
+
+
+@pytest.mark.parametrize("what", ["q over the batch", "q over the tokens", "q over the heads", "keys over the batch", "keys over the KV heads",
+                                  "keys stored by head", "lone key row"])
+def test_views_of_every_stride(dtattn, what):
+    """Views that tensor maps do not describe (an expanded axis has stride 0) and unusual ones that they may: as the oracle."""
+    B, Sq, Sr, Sc, n_sel, Hq, Hkv, D, dtype = 2, 40, 90, 30, 20, 128, 2, 256, torch.bfloat16
+    if what == "lone key row":
+        Sr, Sc = 60, 1
+    q, kr, _, kc, _, sel, sinks = make_case(B, Sq, Sr, Sc, n_sel, Hq, Hkv, D, dtype, 1541, per_batch_lists=True)
+    axis = {"q over the batch": (0, 0), "q over the tokens": (0, 1), "q over the heads": (0, 2), "keys over the batch": (1, 0),
+            "keys over the KV heads": (1, 2)}.get(what)
+    if axis is not None:
+        one = lambda t: t.narrow(axis[1], 0, 1).contiguous().to(DEV).expand(t.shape)  # noqa: E731
+    if axis is not None and axis[0] == 0:
+        qd, rd, cd = one(q), kr.to(DEV), kc.to(DEV)
+    elif axis is not None:
+        qd, rd, cd = q.to(DEV), one(kr), one(kc)
+    elif what == "keys stored by head":
+        qd, rd, cd = q.to(DEV), kr.to(DEV).transpose(1, 2).contiguous().transpose(1, 2), kc.to(DEV).transpose(1, 2).contiguous().transpose(1, 2)
+    else:
+        qd, rd, cd = q.to(DEV), kr.to(DEV), kc.to(DEV)
+    ref = so.sparse_indexed_explicit(qd.cpu(), rd.cpu(), rd.cpu(), cd.cpu(), cd.cpu(), sel, D ** -0.5, sinks, 40, compute_dtype=torch.float64)
+    out = torch.zeros(B, Sq, Hq, D, dtype=dtype, device=DEV)
+    dtattn.sparse_indexed_attention(qd, rd, rd, cd, cd, sel.to(DEV), D ** -0.5, sinks.to(DEV), 40, out=out)
+    torch.cuda.synchronize()
+    assert dtattn.device_status() == 0
+    mx, mean = so.error_stats(out.float().cpu(), ref.float())
+    assert mx <= so.TOL_MAX_ABS + 2 * ROUND[dtype] * float(ref.abs().max()), (what, mx)
+    assert mean <= so.TOL_MEAN_ABS + ROUND[dtype] * float(ref.abs().mean()), (what, mean)
