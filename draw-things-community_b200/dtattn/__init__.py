@@ -252,6 +252,15 @@ def device_status(stream=None) -> int:
     return code.value
 
 
+def _alloc(nbytes, device, stream):
+    """Device memory in the order of `stream` (a raw handle): a block that torch hands out on another stream may still be in
+    use by that stream's queued kernels."""
+    if stream == torch.cuda.current_stream(device).cuda_stream:
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+    with torch.cuda.stream(torch.cuda.ExternalStream(stream, device=device)):
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+
+
 class Workspace:
     """Caller-owned scratch for dt_sdpa_forward, grown on demand and zero-initialised when (re)allocated."""
 
@@ -263,7 +272,7 @@ class Workspace:
         if nbytes == 0:
             return None, 0
         if self.buf is None or self.buf.numel() < nbytes:
-            self.buf = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+            self.buf = _alloc(nbytes, self.device, stream)
             _check(lib().dt_sdpa_workspace_init(ctypes.c_void_p(self.buf.data_ptr()), self.buf.numel(),
                                                 ctypes.c_void_p(stream)), "dt_sdpa_workspace_init")
         return self.buf.data_ptr(), self.buf.numel()
@@ -472,12 +481,9 @@ def _call_scratch(nbytes, device, stream):
     if nbytes == 0:
         return None
     try:
-        buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        return _alloc(nbytes, device, stream)
     except torch.cuda.OutOfMemoryError:
         return None
-    if stream != torch.cuda.current_stream(device).cuda_stream:
-        buf.record_stream(torch.cuda.ExternalStream(stream, device=device))
-    return buf
 
 
 _workspaces = {}

@@ -1,4 +1,5 @@
-"""One workspace serves calls of different kinds one after another: each leaves what the next one relies on."""
+"""Scratch: one workspace serves calls of different kinds one after another, and each leaves what the next one relies on; the
+scratch of a call belongs to the stream that the call runs on."""
 import pytest
 import torch
 
@@ -19,3 +20,32 @@ def test_masked_calls_leave_the_ticket_counters_alone(dtattn):
     got = dtattn.sdpa_forward(dq, dk, dv, 128 ** -0.5, workspace=ws, out=torch.zeros_like(dq))
     torch.cuda.synchronize()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("kind", ["cut", "fp32", "unaligned mask"])
+def test_scratch_is_in_the_order_of_the_calls_stream(dtattn, kind):
+    """A call with stream=, while the current stream still has kernels queued that write to a block torch has already taken
+    back: the call's scratch is not that block."""
+    dtype = torch.float32 if kind == "fp32" else torch.bfloat16
+    Sq, Sk = (200, 4096) if kind == "cut" else (333, 333)
+    q, k, v = (x.to(DEV) for x in inputs(1, Sq, Sk, 4, 4, 64, dtype, 1431))
+    mask = make_mask(1, 1, Sq, Sk, dtype, 1432).to(DEV) if kind == "unaligned mask" else None
+    want = dtattn.sdpa_forward(q, k, v, 0.125, mask=mask)
+    out, side = torch.zeros_like(want), torch.cuda.Stream()
+    need = dtattn.workspace_size(dtattn.make_params(q, k, v, out, 0.125, mask=mask))
+    assert need > 0
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()  # the only free block of this size is the one below
+    for _ in range(3):
+        busy = torch.empty(need, dtype=torch.uint8, device=DEV)
+        torch.cuda._sleep(int(2e6))  # a millisecond or so, while the rest is queued
+        for _ in range(400):
+            busy.fill_(0x7f)
+        del busy
+        for _ in range(60):  # over the sleep and into the fills
+            dtattn.sdpa_forward(q, k, v, 0.125, mask=mask, out=out, stream=side.cuda_stream)
+        torch.cuda.synchronize()
+        assert dtattn.device_status() == 0
+        assert torch.equal(out, want)
+        out.zero_()
+        torch.cuda.synchronize()
