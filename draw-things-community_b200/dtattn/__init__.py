@@ -268,11 +268,17 @@ class Workspace:
         self.device = device
         self.buf = None
 
-    def ensure(self, nbytes, stream):
+    def ensure(self, nbytes, stream, optional=False):
+        """(pointer, bytes) of at least nbytes; optional: of what there is when there is no room for more."""
         if nbytes == 0:
             return None, 0
         if self.buf is None or self.buf.numel() < nbytes:
-            self.buf = _alloc(nbytes, self.device, stream)
+            try:
+                self.buf = _alloc(nbytes, self.device, stream)
+            except torch.cuda.OutOfMemoryError:
+                if not optional:
+                    raise
+                return (None, 0) if self.buf is None else (self.buf.data_ptr(), self.buf.numel())
             _check(lib().dt_sdpa_workspace_init(ctypes.c_void_p(self.buf.data_ptr()), self.buf.numel(),
                                                 ctypes.c_void_p(stream)), "dt_sdpa_workspace_init")
         return self.buf.data_ptr(), self.buf.numel()
@@ -297,12 +303,15 @@ def sdpa_forward(q, k, v, scale, is_causal=False, mask=None, out=None, lse=None,
     if q.is_cuda:
         s = _stream_of(q.device, stream)
         need = workspace_size(p)
-        if need and workspace is None and kernel_name(p) != "decode_splitkv":
-            scratch = _call_scratch(need, q.device, s)
+        name = kernel_name(p) if need else ""
+        # the split-KV partials and the flags of a mask have to be there; anything else is a faster way that may be left out
+        optional = name != "decode_splitkv" and (mask is None or name == "generic")
+        if name and workspace is None and name != "decode_splitkv":
+            scratch = _call_scratch(need, q.device, s, optional)
             ptr, nbytes = (None, 0) if scratch is None else (scratch.data_ptr(), scratch.numel())
         else:
             ws = workspace if workspace is not None else _default_workspace(q.device)
-            ptr, nbytes = ws.ensure(need, s)
+            ptr, nbytes = ws.ensure(need, s, optional)
         _check(lib().dt_sdpa_forward(ctypes.byref(p), ctypes.c_void_p(ptr) if ptr else None, nbytes,
                                      ctypes.c_void_p(s)), "dt_sdpa_forward")
     else:
@@ -475,14 +484,14 @@ class SparseIndexedAttention:
                                         self.sliding_window, self.is_causal, out=out)
 
 
-def _call_scratch(nbytes, device, stream):
-    """Scratch of one call (any contents), its own so that calls on several streams stay independent; None when there is
-    no room for it, which the library answers with a way that needs none (a masked call on the tensor cores has none)."""
-    if nbytes == 0:
-        return None
+def _call_scratch(nbytes, device, stream, optional):
+    """Scratch of one call (any contents), its own so that calls on several streams stay independent; None when it is
+    optional and there is no room for it, which the library answers with a way that needs none."""
     try:
         return _alloc(nbytes, device, stream)
     except torch.cuda.OutOfMemoryError:
+        if not optional:
+            raise
         return None
 
 

@@ -49,3 +49,31 @@ def test_scratch_is_in_the_order_of_the_calls_stream(dtattn, kind):
         assert torch.equal(out, want)
         out.zero_()
         torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("kind", ["cut", "fp32", "unaligned mask", "aligned mask", "decode"])
+@pytest.mark.parametrize("own", [False, True])
+def test_no_room_for_scratch(dtattn, monkeypatch, kind, own):
+    """Scratch that only makes a call faster may be missing, with a caller's workspace as without; what a call cannot do
+    without is torch's out-of-memory error."""
+    dtype = torch.float32 if kind == "fp32" else torch.bfloat16
+    Sq, Sk = {"cut": (200, 4096), "decode": (1, 4096), "aligned mask": (512, 512)}.get(kind, (333, 333))
+    q, k, v = (x.to(DEV) for x in inputs(1, Sq, Sk, 4, 4, 64, dtype, 1441))
+    mask = make_mask(1, 1, Sq, Sk, dtype, 1442).to(DEV) if kind.endswith("mask") else None
+    want = dtattn.sdpa_forward(q, k, v, 0.125, mask=mask)
+    torch.cuda.synchronize()
+
+    def no_room(nbytes, device, stream):
+        raise torch.cuda.OutOfMemoryError("no room")
+
+    monkeypatch.setattr(dtattn, "_alloc", no_room)
+    monkeypatch.setattr(dtattn, "_workspaces", {})
+    kw = dict(workspace=dtattn.Workspace(torch.device(DEV))) if own else {}
+    if kind in ("aligned mask", "decode"):
+        with pytest.raises(torch.cuda.OutOfMemoryError):
+            dtattn.sdpa_forward(q, k, v, 0.125, mask=mask, **kw)
+        return
+    got = dtattn.sdpa_forward(q, k, v, 0.125, mask=mask, **kw)
+    torch.cuda.synchronize()
+    assert dtattn.device_status() == 0
+    assert float((got.float() - want.float()).abs().max()) <= (4e-5 if kind == "fp32" else 2 ** -7)
