@@ -426,8 +426,12 @@ def sdpa_forward_projected(q, k, v, scale, weight, bias=None, is_causal=False, o
     _check(lib().dt_sdpa_projected_workspace_size(ctypes.byref(p), ctypes.byref(pr), ctypes.byref(need)),
            "dt_sdpa_projected_workspace_size")
     s = _stream_of(q.device, stream)
-    ws = workspace if workspace is not None else _default_workspace(q.device)
-    ptr, nbytes = ws.ensure(need.value, s)
+    if workspace is None and kernel_name(p) != "decode_splitkv":  # (whose tickets have to start at zero)
+        scratch = _call_scratch(need.value, q.device, s, False)  # holds the attention output: a call's own
+        ptr, nbytes = scratch.data_ptr(), scratch.numel()
+    else:
+        ws = workspace if workspace is not None else _default_workspace(q.device)
+        ptr, nbytes = ws.ensure(need.value, s)
     _check(lib().dt_sdpa_forward_projected(ctypes.byref(p), ctypes.byref(pr), ctypes.c_void_p(ptr), nbytes,
                                            ctypes.c_void_p(s)), "dt_sdpa_forward_projected")
     return out

@@ -77,3 +77,25 @@ def test_no_room_for_scratch(dtattn, monkeypatch, kind, own):
     torch.cuda.synchronize()
     assert dtattn.device_status() == 0
     assert float((got.float() - want.float()).abs().max()) <= (4e-5 if kind == "fp32" else 2 ** -7)
+
+
+@pytest.mark.parametrize("Sk", [512, 4096])  # not cut; cut
+def test_projected_calls_on_two_streams(dtattn, Sk):
+    """The attention output of a projected call lives in scratch: calls on several streams keep theirs apart."""
+    H, D, dtype = 4, 64, torch.float16
+    cases, streams = [], [torch.cuda.Stream(), torch.cuda.Stream()]
+    for i in range(2):
+        q, k, v = (x.to(DEV) for x in inputs(1, 256, Sk, H, H, D, dtype, 1451 + 10 * i))
+        w = (torch.randn(H * D, H * D, generator=torch.Generator().manual_seed(i)) / 16).to(dtype).to(DEV)
+        cases.append((q, k, v, 0.125, w))
+    wants = [dtattn.sdpa_forward_projected(*c) for c in cases]
+    torch.cuda.synchronize()
+    outs = [[], []]
+    for _ in range(40):
+        for i, c in enumerate(cases):
+            with torch.cuda.stream(streams[i]):
+                outs[i].append(dtattn.sdpa_forward_projected(*c))
+    torch.cuda.synchronize()
+    assert dtattn.device_status() == 0
+    for i in range(2):
+        assert all(torch.equal(o, wants[i]) for o in outs[i])
