@@ -1248,8 +1248,13 @@ Plan make_plan(const dt_sdpa_params& p, int tiles) {
   if (varlen) return r;
   const int rest = r.n_items % sms;
   // For the same reason a last round of pairs that fills less than half of the SMs is taken tile by tile (2 images, 4096
-  // tokens, 20 heads of 64: 4.3 rounds).  The rows' results do not depend on it.
-  if (r.item_rows > kBM && r.n_items > sms && rest > 0 && 2 * rest <= sms) {
+  // tokens, 20 heads of 64: 4.3 rounds, 302 -> 293 us).  The rows' results do not depend on it.  Under the causal rule the last
+  // round holds the lightest pairs, and behind an odd number of rounds its order gives them to the CTAs with the least work:
+  // twice as many tiles reach CTAs that have more (32 / 8 heads of 128, 1280 and 1536 tokens: 29.6 and 33.6 us in pairs, 34.4
+  // and 41.7 us by tiles; of 64, 4096 tokens: 125 and 133 us).  So there only behind an even number, and for enough pairs (32 / 8
+  // heads of 64: 56 pairs at 2816 tokens 72.5 us in pairs, 70.0 by tiles; 24 pairs at 2400 tokens 56.7 and 60.1 us).
+  const bool tiles_pay = !p.is_causal || (r.n_items / sms % 2 == 0 && 3 * rest >= sms);
+  if (r.item_rows > kBM && r.n_items > sms && rest > 0 && 2 * rest <= sms && tiles_pay) {
     r.n_whole = r.n_items - rest;
     r.n_single = 2 * rest;
     return r;

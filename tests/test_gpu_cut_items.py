@@ -100,7 +100,9 @@ def test_nan_is_kept(dtattn, D, extra, where):
     # tile (149 to 222 pairs), with and without a second tile in the last pair
     (1, 300, 200, 40, 8, 64, False, torch.float16), (1, 400, 400, 37, 37, 128, True, torch.bfloat16),
     (1, 1280, 140, 32, 8, 40, False, torch.float16), (1, 1100, 1100, 38, 2, 64, True, torch.bfloat16),
-    (2, 900, 70, 20, 20, 128, False, torch.bfloat16)])
+    (2, 900, 70, 20, 20, 128, False, torch.bfloat16),
+    # causal: pairs in an odd last round, tiles in an even one
+    (1, 600, 600, 55, 5, 40, True, torch.float16), (1, 600, 600, 120, 4, 40, True, torch.float16)])
 def test_single_tiles(dtattn, case):
     B, Sq, Sk, Hq, Hkv, D, causal, dtype = case
     q, k, v = inputs(B, Sq, Sk, Hq, Hkv, D, dtype, 1605)
