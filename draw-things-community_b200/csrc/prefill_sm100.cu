@@ -98,14 +98,13 @@ struct PrefillArgs {
   int item_rows;          // query rows of a work item: a pair of tiles, or one tile where pairs would leave SMs idle
   int n_qpairs, n_items;  // work items = (batch, head, item_rows query rows)
   // Items in whole rounds over the grid: n_slots of them, of which the causal order may leave some empty.  The items from
-  // n_slots on (fewer than one round) are n_single / 2 pairs of tiles taken tile by tile, or else cut into n_cuts runs of
-  // K/V blocks of equal length, in the same order, of which CTA c < n_cuts takes run c.  A run's share of an item that it does not hold
-  // whole goes to `part`; cut_combine_kernel puts the shares together.
+  // n_slots on (fewer than one round) are pairs of tiles taken tile by tile; n_places counts those tiles too.
   int n_slots;
-  int n_single;
-  int n_cuts;
-  int cut_blocks;         // K/V blocks of those items together (times n_cuts below 2^31)
-  float* part;            // [2 n_cuts][warps of an item][D + 2][32]: weights' maximum, their sum, O
+  int n_places;
+  // The cut kernel: an item's K/V blocks are the work of n_splits CTAs in turn, whose shares of the result go to `part`;
+  // cut_combine_kernel puts them together.
+  int n_splits;           // (times an item's K/V blocks below 2^31)
+  float* part;            // [n_items * n_splits][kBM / 32][D + 2][32]: weights' maximum, their sum, O
   // variable-length batch (both null otherwise): packed rows, sequence s owns query rows [off_q[s], off_q[s+1])
   // and key rows [off_k[s], off_k[s+1]); the item's batch index is then the sequence
   const int32_t* off_q;
@@ -197,8 +196,8 @@ __device__ __forceinline__ void stamp(const PrefillArgs& a, int slot) {
 __device__ __forceinline__ void stamp(const PrefillArgs&, int) {}
 #endif
 
-// ---- the cut part of a call's work (see PrefillArgs) ----
-__device__ __forceinline__ int cut_at(const PrefillArgs& a, int c) { return a.cut_blocks * c / a.n_cuts; }  // first block of run c
+// First of an item's n K/V blocks that belongs to its run c
+__device__ __forceinline__ int cut_at(const PrefillArgs& a, int n, int c) { return n * c / a.n_splits; }
 
 // K/V blocks from key 0 to the last one that the query rows below `end` may see (not for variable lengths)
 __device__ __forceinline__ int blocks_to(const PrefillArgs& a, int end) {
@@ -224,72 +223,29 @@ __device__ __forceinline__ void place_of(const PrefillArgs& a, int order, int& q
   }
 }
 
-// Moves (order, start) on to the cut item that holds block `pos` of the runs' numbering and returns its K/V blocks;
-// under the causal rule a level of equal items at a time.
-__device__ __forceinline__ int find_cut_item(const PrefillArgs& a, int pos, int& order, int& start) {
-  const int nbh = a.n_items / a.n_qpairs;
-  for (;;) {
-    const int level = a.is_causal ? order / nbh : 0;
-    const int same = a.is_causal ? nbh - (order - level * nbh) : a.n_items - order;
-    const int n = blocks_to(a, a.is_causal ? (a.n_qpairs - level) * a.item_rows : 0);
-    const int skip = min((pos - start) / n, same);
-    order += skip;
-    start += skip * n;
-    if (skip < same) return n;
-  }
-}
-
-// Run c's share of 32 rows (one softmax warp's) of the item that starts at block `item_begin`: a run holds at most one
-// share that lies at its start and one that reaches its end.
+// Run c's share of 32 rows (one softmax warp's).
 template <int D>
-__device__ __forceinline__ float* share_of(const PrefillArgs& a, int units, int c, int item_begin, int unit) {
-  const int slot = 2 * c + (item_begin > cut_at(a, c) ? 1 : 0);
-  return a.part + ((size_t)slot * units + unit) * (size_t)((D + 2) * 32);
+__device__ __forceinline__ float* share_of(const PrefillArgs& a, int run, int unit) {
+  return a.part + ((size_t)run * (kBM / 32) + unit) * (size_t)((D + 2) * 32);
 }
 
-// Puts the shares of the cut items together, added in the order of the keys: one block per item, softmax warp's 32 rows
-// and 64 columns.  (As the last step of the attention kernel itself, by the warp that arrives last, it took longer than the
-// cut saved: 256 columns from three shares are a chain of two dozen L2 round trips for one warp.)
+// Puts the shares of cut items together, added in the order of the keys: one block per 32 rows of an item and 64 columns.
+// (As the last step of the attention kernel itself, by the warp that arrives last, it took longer than the cut saved: 256
+// columns from three shares are a chain of two dozen L2 round trips for one warp.)
 // Bound: the latency of L2; a thread keeps eight shares' loads in flight.
 template <typename T, int D>
-__global__ void __launch_bounds__(256) cut_combine_kernel(const PrefillArgs a, const int units) {
+__global__ void __launch_bounds__(256) cut_combine_kernel(const PrefillArgs a) {
   __shared__ __align__(16) uint16_t rows[32][64 + 8];
-  const int item = blockIdx.x / units, unit = blockIdx.x - item * units, col0 = blockIdx.y * 64;
+  const int item = blockIdx.x / (kBM / 32), unit = blockIdx.x - item * (kBM / 32), col0 = blockIdx.y * 64;
   const int r = threadIdx.x & 31, cg = threadIdx.x >> 5;  // two groups of four columns per thread: cg and cg + 8
-  int order = a.n_slots, begin = 0, n;
-  if (a.is_causal) {  // where the item's blocks start: its level's first item, then equal items
-    const int nbh = a.n_items / a.n_qpairs;
-    const int want = a.n_slots + item;
-    for (;;) {
-      const int level = order / nbh, next = min((level + 1) * nbh, want);
-      n = blocks_to(a, (a.n_qpairs - level) * a.item_rows);
-      begin += (next - order) * n;
-      order = next;
-      if (order == want) break;
-    }
-    n = blocks_to(a, (a.n_qpairs - order / nbh) * a.item_rows);
-  } else {
-    n = blocks_to(a, 0);
-    begin = item * n;
-    order += item;
-  }
-  int c_first = (int)((long long)begin * a.n_cuts / a.cut_blocks);
-  while (cut_at(a, c_first + 1) <= begin) ++c_first;
-  while (cut_at(a, c_first) > begin) --c_first;
-  int c_last = c_first;
-  while (cut_at(a, c_last + 1) < begin + n) ++c_last;
-  if (c_first == c_last) return;  // one run holds the whole item: the attention kernel has stored it
   int qt, bh;
-  place_of(a, order, qt, bh);
-  const int h = bh % a.Hq, b = bh / a.Hq, row0 = qt * a.item_rows + unit * 32, row = row0 + r;
-  if (unit * 32 >= a.item_rows || row0 >= a.Sq) return;
-
-  // the first run's share lies at its start or reaches its end; all the others start their runs
-  const size_t share = (size_t)((D + 2) * 32), run = 2 * (size_t)units * share;
-  const float* first = share_of<D>(a, units, c_first, begin, unit);
-  const float* rest = a.part + (size_t)unit * share;
-  const int n_shares = c_last - c_first + 1;
-  auto at = [&](int i) { return i == 0 ? first : rest + (size_t)(c_first + i) * run; };
+  place_of(a, item, qt, bh);
+  const int h = bh % a.Hq, b = bh / a.Hq, row0 = qt * kBM + unit * 32, row = row0 + r;
+  if (row0 >= a.Sq) return;
+  const int n = blocks_to(a, (qt + 1) * kBM);
+  // with fewer blocks than runs some of them are empty: run i of the others
+  const int n_shares = min(n, a.n_splits);
+  auto at = [&](int i) { return share_of<D>(a, item * a.n_splits + (n < a.n_splits ? ((i + 1) * a.n_splits - 1) / n : i), unit); };
   float m = -INFINITY;
 #pragma unroll 8
   for (int i = 0; i < n_shares; ++i) m = fmaxf(m, __ldg(at(i) + r));
@@ -417,7 +373,7 @@ __device__ __forceinline__ float2 unpack_pair(uint32_t x) {
   else return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x));
 }
 
-template <typename T, int D, bool kMask, bool kSplit>
+template <typename T, int D, bool kMask, bool kSplit, bool kCut>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
@@ -479,7 +435,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     it.nkv = nkv - it.j0;
     return it;
   };
-  // Whole items: place `item` of the CTAs' turns.  Under the causal rule the turns go forwards over the CTAs in even
+  // Whole items, then single tiles: place `item` of the CTAs' turns.  Under the causal rule the turns go forwards over the CTAs in even
   // rounds and backwards in odd ones, so that every CTA's items add up to about the same number of K/V blocks.
   auto decode_item = [&](int item) {
     int order = item;
@@ -489,33 +445,38 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       if (round & 1) pos = (int)gridDim.x - 1 - pos;
       order = round * (int)gridDim.x + pos;
     }
+    int tile = -1;
+    if constexpr (C::kTiles == 2) {
+      if (order >= a.n_slots) {  // single tiles (under the causal rule in a round that goes forwards)
+        tile = (order - a.n_slots) & 1;
+        order = a.n_slots + ((order - a.n_slots) >> 1);
+      }
+    }
     if (order >= a.n_items) {  // a slot of the last, incomplete round without an item
       return Item{};
     }
-    return item_at(order, -1);
+    return item_at(order, tile);
   };
-  // This CTA's work in turn: its whole items and then a single tile, or (a cut call has neither) its run of blocks, one
-  // item or share of one at a time.  One word of state, because the softmax warps carry it through their loops, where two
-  // more registers cost the 256-wide variant 2 %: the next whole item, n_slots + the next single tile, or the next block.
-  auto first_work = [&]() { return (int)blockIdx.x < a.n_cuts ? cut_at(a, blockIdx.x) : (int)blockIdx.x; };
+  // This CTA's work in turn: its whole items and then a single tile, or (cut) one run of an item's blocks.  A kernel of its own
+  // for cut calls, because what they need costs the others up to 1 us at the start and 2 % in the loops of the 256-wide variant.
   auto next_work = [&](int& next, Item& w) -> bool {
-    if (a.n_cuts == 0) {
-      while (next < a.n_slots + a.n_single) {
-        w = next < a.n_slots ? decode_item(next) : item_at(a.n_slots + ((next - a.n_slots) >> 1), (next - a.n_slots) & 1);
+    if constexpr (kCut) {
+      if (next != (int)blockIdx.x) return false;
+      next += gridDim.x;
+      const int order = blockIdx.x / a.n_splits, c = blockIdx.x - order * a.n_splits;
+      w = item_at(order, -1);
+      const int n = w.nkv;
+      w.j0 = cut_at(a, n, c);
+      w.nkv = cut_at(a, n, c + 1) - w.j0;
+      return w.nkv > 0;
+    } else {
+      while (next < a.n_places) {
+        w = decode_item(next);
         next += gridDim.x;
         if (w.nkv > 0) return true;
       }
       return false;
     }
-    const int end = cut_at(a, blockIdx.x + 1);
-    if (next >= end) return false;
-    int order = 0, start = 0;
-    const int n = find_cut_item(a, next, order, start);
-    w = item_at(order, -1);
-    w.j0 = next - start;
-    w.nkv = min(n, end - start) - w.j0;
-    next += w.nkv;
-    return true;
   };
 
   if (threadIdx.x == 0) {
@@ -576,7 +537,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           ++ring_it;
           return true;
         };
-        int walk = first_work();
+        int walk = blockIdx.x;
         Item w, nx;
         bool more_work = next_work(walk, nx);
         for (; more_work && ok; ++n_item) {
@@ -650,7 +611,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         auto advance = [&]() {
           if (++slot == C::kSlots) { slot = 0; par ^= 1; }
         };
-        int walk = first_work();
+        int walk = blockIdx.x;
         Item w;
         for (; ok && next_work(walk, w); ++n_item) {
           const int ntile = w.two ? 2 : 1;
@@ -804,7 +765,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     uint32_t n_blocks = 0;  // K/V blocks this warpgroup has handed over so far, over all items (one tile per item)
     const bool probe = (warp == 4 && lane == 0);
 
-    int walk = first_work();
+    int walk = blockIdx.x;
     Item w;
     while (ok && next_work(walk, w)) {
       if (t == 1 && !w.two) continue;  // this item has no second tile: neither side touches tile 1's barriers
@@ -1096,10 +1057,8 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       oph ^= 1;
       if (probe) stamp(a, 16 * n_item + 10);
       ptx::tc_fence_after();
-      // a share of an item: leave (maximum, sum, O) and go on
-      int item_begin = 0, item_order = 0;
-      if (a.n_cuts > 0 && w.nkv < find_cut_item(a, walk - w.nkv, item_order, item_begin)) {
-        float* mine = share_of<D>(a, C::kTiles * 4, blockIdx.x, item_begin, t * 4 + (warp & 3));
+      if constexpr (kCut) {  // the run's share: (maximum, sum, O)
+        float* mine = share_of<D>(a, blockIdx.x, warp & 3);
         __stcg(mine + lane, m_used);
         __stcg(mine + 32 + lane, l);
 #pragma unroll 1
@@ -1114,8 +1073,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                                __uint_as_float(ov[4 * i + 3])));
         }
         ptx::tc_fence_before();
-        ++n_item;
-        continue;
+        break;
       }
       if (a.sinks && row < w.sq) {
         // attention sink: one more score without a value row joins the denominator (l and O are relative to m_used)
@@ -1220,8 +1178,8 @@ size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 struct Plan {
   int item_rows, n_q, n_items;
   int n_whole;           // items taken whole, in full rounds
-  int n_single, n_cuts;  // the items behind them as single tiles, or cut into this many runs (0, 0: they are whole too)
-  int cut_blocks;
+  int n_single;          // the items behind them as single tiles (0: they are whole too)
+  int n_splits;          // CTAs per item of a cut call (0: not cut)
 };
 
 long long blocks_of_item(const dt_sdpa_params& p, int item_rows, int qt) {
@@ -1259,26 +1217,24 @@ Plan make_plan(const dt_sdpa_params& p, int tiles) {
     r.n_single = 2 * rest;
     return r;
   }
-  // A call that leaves half of the SMs without any item (a short chunk of queries behind a long prefix): its K/V blocks cut
-  // into equal runs over all SMs, when that saves at least kCutGain blocks' time on the longest item.  A cut costs
-  // about two: the shares' way through L2 and one more launch.
-  constexpr int kCutGain = 4, kMinRun = 4;
+  // A call that leaves half of the SMs without any item (a short chunk of queries behind a long prefix): every item's K/V blocks
+  // cut into as many equal runs as there are SMs per item, when that saves at least kCutGain blocks' time.  A run lies in one
+  // item: with runs of equal length over all SMs, whatever items they fell into, there were up to twice as many shares to write
+  // and read (400 x 1536, 16 / 4 heads of 256: 24.3 us uncut, 32.2 us so, 22.4 us by items).  Measured against the uncut call (Sq x
+  // Sk, time uncut / cut, saving 4 blocks): 24 heads of 64, 128 x 1024 causal: 18.2 / 14.7 us; 6 heads of 256, 128 x 1024: 18.5 /
+  // 17.6 us, but 16 heads (64 items, two runs each) 400 x 1024: 19.4 / 19.6, causal 19.9 / 20.6 us.  Runs of at least 4 blocks: of
+  // 2 the shares of a long item take longer to add (2 heads of 64, 8192 keys: 23.6 against 19.1 us; 1280 keys 11.7 against 14.9 us).
+  const int kCutGain = tiles == 1 && 3 * r.n_items > sms ? 5 : 4;
+  constexpr int kMinRun = 4;
   if (2 * r.n_items > sms || p.sliding_window > 0) return r;
-  long long blocks = 0, longest = 0;
-  for (int qt = 0; qt < r.n_q; ++qt) {
-    const long long n = blocks_of_item(p, r.item_rows, qt);
-    blocks += n * bh;
-    if (n > longest) longest = n;
-  }
-  const long long runs = blocks / kMinRun < sms ? blocks / kMinRun : sms;
-  if (runs <= r.n_items || blocks * runs >= (1LL << 31) || longest - (blocks + runs - 1) / runs < kCutGain) return r;
-  r.n_whole = 0;
-  r.n_cuts = (int)runs;
-  r.cut_blocks = (int)blocks;
+  const long long longest = blocks_of_item(p, r.item_rows, r.n_q - 1);  // (the last rows see the most)
+  const long long by_blocks = longest / kMinRun, splits = by_blocks < sms / r.n_items ? by_blocks : sms / r.n_items;
+  if (splits < 2 || longest * splits >= (1LL << 31) || longest - (longest + splits - 1) / splits < kCutGain) return r;
+  r.n_splits = (int)splits;
   return r;
 }
-size_t split_bytes(const Plan& plan, int tiles, int D) {  // two shares per run
-  return (size_t)2 * plan.n_cuts * tiles * 4 * (D + 2) * 32 * sizeof(float);
+size_t split_bytes(const Plan& plan, int D) {  // (a cut call's items are single tiles)
+  return (size_t)plan.n_items * plan.n_splits * (kBM / 32) * (D + 2) * 32 * sizeof(float);
 }
 
 bool mask_rows_aligned(const dt_sdpa_params& p) {
@@ -1298,7 +1254,7 @@ size_t prefill_repack_bytes_needed(const dt_sdpa_params& p) {  // the flags and 
 }
 size_t cut_bytes(const dt_sdpa_params& p) {
   const int D = p.D > 128 ? 256 : p.D > 64 ? 128 : 64, tiles = D == 256 ? 1 : 2;
-  return split_bytes(make_plan(p, tiles), tiles, D);
+  return split_bytes(make_plan(p, tiles), D);
 }
 
 template <typename T, int D, bool kMask, bool kSplit = false>
@@ -1362,30 +1318,27 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
   a.item_rows = plan.item_rows;
   a.n_qpairs = plan.n_q;
   a.n_items = plan.n_items;
-  auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit>;
-  DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
   const int n_sm = device_sm_count();
   const size_t split_at = kMask ? (kSplit ? prefill_repack_bytes_needed(p) : mask_flag_bytes(p)) : kTicketBytes;
-  const bool cut = plan.n_cuts > 0 && workspace && reinterpret_cast<uintptr_t>(workspace) % 16 == 0 &&
-                   workspace_bytes >= align256(split_at) + split_bytes(plan, C::kTiles, D);
-  dim3 grid(cut ? plan.n_cuts : a.n_items < n_sm ? a.n_items : n_sm);  // one persistent CTA per SM
-  if (plan.n_single > 0) {
-    a.n_slots = plan.n_whole;
-    a.n_single = plan.n_single;
-  } else if (cut) {
-    a.n_slots = 0;
-    a.n_cuts = plan.n_cuts;
-    a.cut_blocks = plan.cut_blocks;
+  if (plan.n_splits > 0 && n_extra == 0 && workspace && reinterpret_cast<uintptr_t>(workspace) % 16 == 0 &&
+      workspace_bytes >= align256(split_at) + split_bytes(plan, D)) {
+    a.n_splits = plan.n_splits;
     a.part = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + align256(split_at));
-  } else {
-    a.n_slots = (a.n_items + (int)grid.x - 1) / (int)grid.x * (int)grid.x;
-  }
-  kern<<<grid, kThreads, C::kSmemBytes, stream>>>(mq, mk, mv, mo, a);
-  DT_CUDA_TRY(cudaGetLastError());
-  if (cut) {
-    cut_combine_kernel<T, D><<<dim3((a.n_items - a.n_slots) * C::kTiles * 4, (p.D + 63) / 64), 256, 0, stream>>>(a, C::kTiles * 4);
+    auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, true>;
+    DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
+    kern<<<plan.n_items * plan.n_splits, kThreads, C::kSmemBytes, stream>>>(mq, mk, mv, mo, a);
     DT_CUDA_TRY(cudaGetLastError());
+    cut_combine_kernel<T, D><<<dim3(plan.n_items * (kBM / 32), (p.D + 63) / 64), 256, 0, stream>>>(a);
+    DT_CUDA_TRY(cudaGetLastError());
+    return DT_OK;
   }
+  auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, false>;
+  DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
+  const int ctas = a.n_items < n_sm ? a.n_items : n_sm;  // one persistent CTA per SM
+  a.n_slots = plan.n_single > 0 ? plan.n_whole : (a.n_items + ctas - 1) / ctas * ctas;
+  a.n_places = a.n_slots + plan.n_single;
+  kern<<<ctas, kThreads, C::kSmemBytes, stream>>>(mq, mk, mv, mo, a);
+  DT_CUDA_TRY(cudaGetLastError());
   return DT_OK;
 }
 

@@ -23,12 +23,13 @@ def forward(dtattn, p, scratch):
 
 @pytest.mark.parametrize("case", [
     # B, Sq, Sk, Hq, Hkv, D, causal, extra, dtype
-    (1, 130, 2000, 4, 2, 64, False, "", torch.float16),        # fewer items than SMs: every item in several runs
+    (1, 130, 2000, 4, 2, 64, False, "", torch.float16),        # every item in several runs
     (1, 128, 16384, 1, 1, 128, False, "", torch.bfloat16),     # one item over 32 runs
     (1, 600, 1500, 12, 4, 128, False, "sinks", torch.bfloat16),
     (2, 300, 1700, 8, 4, 256, True, "", torch.bfloat16),       # causal levels of different lengths, head dim 256
     (1, 513, 2900, 4, 1, 256, True, "", torch.float16),        # a last tile of one row
     (1, 1200, 1200, 7, 1, 80, True, "sinks", torch.float16),   # as many keys as queries: the first levels are short
+    (1, 2000, 2000, 1, 1, 64, True, "", torch.bfloat16),       # items with fewer key blocks than runs
     (1, 200, 1600, 4, 2, 128, True, "mask", torch.bfloat16),   # masked, aligned rows
     (1, 200, 1601, 4, 2, 64, False, "mask", torch.float16)])   # masked, copied rows
 def test_against_the_oracle_and_the_uncut_call(dtattn, case):
