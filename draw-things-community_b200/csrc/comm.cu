@@ -273,10 +273,20 @@ int dt_comm_register_output(void* comm, void* o_full, size_t bytes) {
 
 static size_t al256(size_t x) { return (x + 255) / 256 * 256; }
 
+// Scratch of the local attention call.  None for the tensor-core kernel, whose scratch is optional (no masks here): a call cut
+// over the SMs adds in another order, and the fused mode, which cannot be cut, must give the same bits as the gathered one.
+static int inner_scratch(const dt_sdpa_params* local, size_t* inner) {
+  const char* name = nullptr;
+  const int st = dt_sdpa_kernel_name(local, &name);
+  if (st != DT_OK) return st;
+  *inner = 0;
+  return strcmp(name, "prefill_tcgen05") == 0 ? DT_OK : dt_sdpa_workspace_size(local, inner);
+}
+
 int dt_sdpa_headsharded_workspace_size(const dt_sdpa_params* local, int world, int chunks, size_t* bytes) {
   if (!local || !bytes || world <= 0 || chunks <= 0 || chunks > kMaxChunks) return DT_BAD_ARG;
   size_t inner = 0;
-  int st = dt_sdpa_workspace_size(local, &inner);
+  int st = inner_scratch(local, &inner);
   if (st != DT_OK) return st;
   const size_t slice = (size_t)local->B * local->Sq * local->Hq * local->D * dtype_size(local->dtype);
   // every chunk gets its own staging and gather region, so no region is reused while in flight
@@ -338,7 +348,7 @@ int dt_sdpa_forward_headsharded(void* comm, const dt_sdpa_params* local, dt_tens
   int st = dt_sdpa_headsharded_workspace_size(local, c->world, chunks, &need);
   if (st != DT_OK) return st;
   if (!workspace || workspace_bytes < need) return DT_WORKSPACE;
-  dt_sdpa_workspace_size(local, &inner);
+  inner_scratch(local, &inner);
   cudaStream_t s = (cudaStream_t)cuda_stream;
   const size_t es = dtype_size(local->dtype);
   const int B = local->B, Hl = local->Hq, D = local->D;
@@ -373,7 +383,7 @@ int dt_sdpa_forward_headsharded(void* comm, const dt_sdpa_params* local, dt_tens
     p.o.stride_h = D;
     p.o.stride_s = (int64_t)Hl * D;
     p.o.stride_b = (int64_t)rows * Hl * D;
-    st = dt_sdpa_forward(&p, inner_ws, inner, s);
+    st = dt_sdpa_forward(&p, inner ? inner_ws : nullptr, inner, s);
     if (st != DT_OK) return st;
     DT_CUDA_TRY(cudaEventRecord(c->chunk_done[ci], s));
     DT_CUDA_TRY(cudaStreamWaitEvent(c->side, c->chunk_done[ci], 0));

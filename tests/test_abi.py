@@ -218,3 +218,27 @@ def test_projected_headsharded_sizes(dtattn):
     assert lib.dt_sdpa_projected_headsharded_sizes(ctypes.byref(p), 8, 3070, None, None, None) == dtattn.DT_UNSUPPORTED
     from dtattn import sharding
     assert sharding.projection_rows(4608, 8)[0] == 640
+
+
+@pytest.mark.parametrize("case", [
+    # Sq, Sk, heads per rank, D, chunks: calls that the single-GPU entry point cuts over the SMs (it asks for scratch)
+    (1000, 1000, 4, 128, 3), (256, 8192, 4, 64, 1), (300, 4096, 2, 256, 1)])
+def test_gathered_head_sharded_calls_are_laid_out_like_the_fused_ones(dtattn, case):
+    """The fused mode runs the attention kernel without scratch, so nothing is cut there; the gathered mode, which must give
+    the same bits, may have none either: its workspace is the staging and gather regions alone."""
+    Sq, Sk, H, D, chunks = case
+    world, al = 2, lambda x: (x + 255) // 256 * 256
+    q, k = torch.zeros(1, Sq, H, D, dtype=torch.bfloat16), torch.zeros(1, Sk, H, D, dtype=torch.bfloat16)
+    p = dtattn.make_params(q, k, k, q, D ** -0.5)
+    assert dtattn.kernel_name(p) == "prefill_tcgen05" and dtattn.workspace_size(p) > 0
+    n = ctypes.c_size_t()
+    assert dtattn.lib().dt_sdpa_headsharded_workspace_size(ctypes.byref(p), world, chunks, ctypes.byref(n)) == dtattn.DT_OK
+    slice_bytes = q.numel() * 2
+    assert n.value == al(slice_bytes) + al(slice_bytes * world) + 256 * chunks * 2
+    # kernels that cannot do without scratch, or whose other way is a slower one with the same rule for every rank, keep theirs
+    q = torch.zeros(1, 1, H, 128, dtype=torch.bfloat16)
+    k = torch.zeros(1, 8192, H, 128, dtype=torch.bfloat16)
+    p = dtattn.make_params(q, k, k, q, D ** -0.5)
+    assert dtattn.kernel_name(p) == "decode_splitkv"
+    assert dtattn.lib().dt_sdpa_headsharded_workspace_size(ctypes.byref(p), world, 1, ctypes.byref(n)) == dtattn.DT_OK
+    assert n.value == al(dtattn.workspace_size(p)) + al(q.numel() * 2) + al(q.numel() * 2 * world) + 512
