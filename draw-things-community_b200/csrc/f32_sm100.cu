@@ -1,11 +1,13 @@
 // Attention of fp32 tensors on the tensor cores (the reference's upcastAttention,
 // Libraries/SwiftDiffusion/Sources/Models/UNet.swift:217-265: fp32 scores, softmax over the keys, P*V).
 //
-// An fp32 number is the exact sum of three bf16 numbers: its top 8 significant bits, the next 8 and the last 8 (each cut
-// off, not rounded, so the parts share its sign and nothing is left over).  A product x*y is then formed from the six
-// partial products x_a*y_b with a + b <= 2; the dropped ones are below 2^-22 of it at worst and 2^-25 on average, the
-// size of one fp32 rounding.  Q, K and V are split once per call by split_planes_kernel into a workspace; the weights P
-// are split in registers on their way into TMEM, so no operand ever carries fewer than 24 bits.
+// An fp32 number is the exact sum of three bf16 numbers: itself rounded to bf16, the rest rounded to bf16, and what that
+// leaves.  A product x*y is then formed from the six partial products x_a*y_b with a + b <= 2; the dropped ones are below
+// 2^-23 of it at worst, with either sign, and about 2^-26 on average: less than one fp32 rounding.  Q, K and V are split once per
+// call by split_planes_kernel into a workspace.  The weights P are split in registers on their way into TMEM, their parts cut
+// off instead of rounded, which takes an instruction less per part: there the dropped products are below 2^-22 at worst, of V's
+// parts' signs.  (With the inputs' parts cut off as well all dropped products had the sign of the product and were up to 2^-21
+// of it: scores of numbers like 1 + 2^-7 - 2^-23 came out short by that much.)
 //
 // The tensor core adds into fp32 accumulators without rounding to nearest, so long sums are kept off it: a block's scores
 // take the small partial products first, and O is accumulated over ONE block of keys in TMEM and added to fp32 registers
@@ -121,12 +123,13 @@ __global__ void __launch_bounds__(kSplitThreads) split_planes_kernel(const Split
       const float x0 = x[2 * i], x1 = x[2 * i + 1];
       // the bits of 2^58: larger finite numbers, infinities and NaNs all compare above it
       bad |= (__float_as_uint(x0) & 0x7fffffffu) >= 0x5c800000u || (__float_as_uint(x1) & 0x7fffffffu) >= 0x5c800000u;
-      const float r0 = x0 - __uint_as_float(__float_as_uint(x0) & 0xffff0000u);
-      const float r1 = x1 - __uint_as_float(__float_as_uint(x1) & 0xffff0000u);
-      const float t0 = r0 - __uint_as_float(__float_as_uint(r0) & 0xffff0000u);
-      const float t1 = r1 - __uint_as_float(__float_as_uint(r1) & 0xffff0000u);
-      w[0][i] = __byte_perm(__float_as_uint(x0), __float_as_uint(x1), 0x7632);
-      w[1][i] = __byte_perm(__float_as_uint(r0), __float_as_uint(r1), 0x7632);
+      // x = a + r, r = b + t: a and b to the nearest bf16 (both differences are exact)
+      const uint32_t a0 = (__float_as_uint(x0) + 0x8000u) & 0xffff0000u, a1 = (__float_as_uint(x1) + 0x8000u) & 0xffff0000u;
+      const float r0 = x0 - __uint_as_float(a0), r1 = x1 - __uint_as_float(a1);
+      const uint32_t b0 = (__float_as_uint(r0) + 0x8000u) & 0xffff0000u, b1 = (__float_as_uint(r1) + 0x8000u) & 0xffff0000u;
+      const float t0 = r0 - __uint_as_float(b0), t1 = r1 - __uint_as_float(b1);
+      w[0][i] = __byte_perm(a0, a1, 0x7632);
+      w[1][i] = __byte_perm(b0, b1, 0x7632);
       w[2][i] = __byte_perm(__float_as_uint(t0), __float_as_uint(t1), 0x7632);
     }
     uint4* dst = t.dst + (size_t)row * 3 * a.per_row + ch;
@@ -393,7 +396,7 @@ f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             ptx::unpack_f32x2(x2, x0, x1);
             const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
             lsum[i & 1] = ptx::add_f32x2(lsum[i & 1], ptx::pack_f32x2(p0, p1));
-            // three planes, cut off and not rounded: the same exact split as the inputs'
+            // three planes, cut off and not rounded
             const float r0 = p0 - __uint_as_float(__float_as_uint(p0) & 0xffff0000u);
             const float r1 = p1 - __uint_as_float(__float_as_uint(p1) & 0xffff0000u);
             const float t0 = r0 - __uint_as_float(__float_as_uint(r0) & 0xffff0000u);

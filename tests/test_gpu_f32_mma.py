@@ -101,3 +101,29 @@ def test_without_scratch_the_cuda_cores_serve_the_call(dtattn):
         assert torch.equal(out, want) == same
         assert float((out - want).abs().max()) < 4e-5
     assert bool((scratch[:4096] == 0xff).all())  # the split-KV ticket counters' area
+
+
+# low 16 bits of the mantissa: all parts of one sign and as large as they get when cut off; the same when rounded
+@pytest.mark.parametrize("low", [0xffff, 0x7f3f])
+@pytest.mark.parametrize("which", ["q and k", "v", "q, k and v"])
+def test_mantissas_with_the_largest_dropped_products(dtattn, which, low):
+    """Numbers whose parts are as large as they can be: the partial products left out must not show beside the CUDA-core
+    kernel's own roundings."""
+    B, S, H, D = 1, 300, 2, 64
+    g = torch.Generator().manual_seed(1351)
+
+    def worst(*shape, signs):
+        exponent = torch.randint(-2, 2, shape, generator=g, dtype=torch.int32)
+        bits = ((exponent + 127) << 23) | low
+        x = bits.view(torch.float32)
+        return torch.where(torch.rand(shape, generator=g) < 0.5, -x, x) if signs else x
+
+    q, k, v = inputs(B, S, S, H, H, D, torch.float32, 1352)
+    if "q" in which:
+        q, k = worst(B, S, H, D, signs=True), worst(B, S, H, D, signs=True)
+    if "v" in which:
+        v = worst(B, S, H, D, signs=False)
+    ref = so.sdpa_explicit(q, k, v, D ** -0.5, False, compute_dtype=torch.float64)
+    (out, _), (out_cc, _) = both(dtattn, q.to(DEV), k.to(DEV), v.to(DEV), D ** -0.5)
+    err, err_cc = rms(out.cpu() - ref.double()), rms(out_cc.cpu() - ref.double())
+    assert err <= 1.25 * err_cc + 1e-8 * rms(ref), (which, err, err_cc)
