@@ -31,8 +31,8 @@
 // Per 128 x 128 scores at D = 40 the tensor pipe has 18 N=128 MMAs for Q K^T and 48 N=48 MMAs for P V.
 // Every mbarrier wait is bounded, as in the half-precision kernel.
 //
-// Inputs that hold an infinity, a NaN or a magnitude of 2^58 and above (a score of 128 such products may leave the fp32
-// range) are not for this kernel: split_planes_kernel reports them, f32_tcgen05_kernel then does nothing and the CUDA-core
+// Inputs that hold an infinity, a NaN, a magnitude of 2^58 and above (a score of 128 such products may leave the fp32
+// range) or one below 2^-110 other than zero (its parts leave the bf16 range) are not for this kernel: split_planes_kernel reports them, f32_tcgen05_kernel then does nothing and the CUDA-core
 // kernel behind it in the stream, which otherwise returns at once, computes the call.
 #include "sm100_ptx.cuh"
 
@@ -104,6 +104,13 @@ struct SplitArgs {
   uint32_t* flags;
 };
 
+// The bits of 2^58 (larger numbers, infinities and NaN all compare above them) and of 2^-110 (the last of a smaller number's
+// 24 bits is below the smallest bf16, 2^-133; zero is fine).
+__device__ __forceinline__ uint32_t out_of_range(float x) {
+  const uint32_t u = __float_as_uint(x) & 0x7fffffffu;
+  return u != 0u && u - 0x08800000u >= 0x5c800000u - 0x08800000u ? 1u : 0u;
+}
+
 // Bound: HBM / L2 writes (10 bytes moved per element in, 4 read and 6 written).  One 8-element piece per thread and step:
 // two 16-byte loads, three 16-byte stores.
 __global__ void __launch_bounds__(kSplitThreads) split_planes_kernel(const SplitArgs a) {
@@ -121,8 +128,7 @@ __global__ void __launch_bounds__(kSplitThreads) split_planes_kernel(const Split
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const float x0 = x[2 * i], x1 = x[2 * i + 1];
-      // the bits of 2^58: larger finite numbers, infinities and NaNs all compare above it
-      bad |= (__float_as_uint(x0) & 0x7fffffffu) >= 0x5c800000u || (__float_as_uint(x1) & 0x7fffffffu) >= 0x5c800000u;
+      bad |= out_of_range(x0) | out_of_range(x1);
       // x = a + r, r = b + t: a and b to the nearest bf16 (both differences are exact)
       const uint32_t a0 = (__float_as_uint(x0) + 0x8000u) & 0xffff0000u, a1 = (__float_as_uint(x1) + 0x8000u) & 0xffff0000u;
       const float r0 = x0 - __uint_as_float(a0), r1 = x1 - __uint_as_float(a1);

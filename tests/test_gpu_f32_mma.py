@@ -60,7 +60,7 @@ def test_strided_views_and_outputs(dtattn):
     assert bool((wide[:, :, H] == 7.0).all()) and bool((wide[..., D:] == 7.0).all())
 
 
-@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 2.0 ** 58, -3e38])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 2.0 ** 58, -3e38, 2.0 ** -111, -1e-38, 1e-44])
 @pytest.mark.parametrize("where", ["q", "k", "v"])
 def test_values_outside_the_split_range_take_the_cuda_cores(dtattn, value, where):
     B, S, H, D = 1, 300, 2, 64
@@ -127,3 +127,15 @@ def test_mantissas_with_the_largest_dropped_products(dtattn, which, low):
     (out, _), (out_cc, _) = both(dtattn, q.to(DEV), k.to(DEV), v.to(DEV), D ** -0.5)
     err, err_cc = rms(out.cpu() - ref.double()), rms(out_cc.cpu() - ref.double())
     assert err <= 1.25 * err_cc + 1e-8 * rms(ref), (which, err, err_cc)
+
+
+@pytest.mark.parametrize("exponent", [-80, -100, -112, -120, -135])
+def test_tiny_values(dtattn, exponent):
+    """Values down to the smallest fp32 numbers: relative to the output's size as exact as on the CUDA cores."""
+    q, k, v = (x.to(DEV) for x in inputs(1, 200, 300, 2, 2, 64, torch.float32, 1361))
+    v = (v.double() * 2.0 ** exponent).float()
+    ref = so.sdpa_explicit(q.cpu(), k.cpu(), v.cpu(), 0.125, False, compute_dtype=torch.float64)
+    (out, _), (out_cc, _) = both(dtattn, q, k, v, 0.125)
+    err, err_cc = rms(out.cpu().double() - ref.double()), rms(out_cc.cpu().double() - ref.double())
+    assert err <= 1.25 * err_cc + 1e-8 * rms(ref), (exponent, err, err_cc)
+    assert torch.equal(out, out_cc) == (exponent < -80)  # one number below 2^-110 (the smallest of these is 2^-16 of the usual) and it is the CUDA cores' call
