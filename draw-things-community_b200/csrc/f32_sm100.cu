@@ -563,7 +563,8 @@ int launch_t(const dt_sdpa_params& p, void* workspace, cudaStream_t stream) {
 bool f32_mma_supported(const dt_sdpa_params& p) {
   if (p.dtype != DT_F32 || p.D % 8 || p.D > 128) return false;
   if (p.mask || p.is_causal || p.sliding_window > 0 || p.sinks || p.seq_offsets_q) return false;
-  if ((p.flags & DT_FLAG_FORCE_GENERIC) || !(p.scale > 0.f) || !(p.scale * kLog2e < INFINITY)) return false;
+  // (a score is below 2^123: times 2^4 it stays finite, and so does every difference from a maximum)
+  if ((p.flags & DT_FLAG_FORCE_GENERIC) || !(p.scale > 0.f) || p.scale * kLog2e > 16.f) return false;
   if (p.Sq < kBM || p.Sk < kBM) return false;
   if (p.Hq > 65535 || p.B > 65535) return false;
   auto ok = [](const dt_tensor4& t) {

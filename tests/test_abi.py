@@ -242,3 +242,11 @@ def test_gathered_head_sharded_calls_are_laid_out_like_the_fused_ones(dtattn, ca
     assert dtattn.kernel_name(p) == "decode_splitkv"
     assert dtattn.lib().dt_sdpa_headsharded_workspace_size(ctypes.byref(p), world, 1, ctypes.byref(n)) == dtattn.DT_OK
     assert n.value == al(dtattn.workspace_size(p)) + al(q.numel() * 2) + al(q.numel() * 2 * world) + 512
+
+
+def test_fp32_calls_whose_scores_may_overflow_stay_on_the_cuda_cores(dtattn):
+    """The fp32 tensor-core kernel takes scores below 2^123 (numbers below 2^58, 128 of them); a scale that could carry them
+    out of the fp32 range leaves the call where a row of such scores has always been answered."""
+    q = torch.zeros(1, 256, 2, 64)
+    for scale, there in ((0.125, True), (1.0, True), (11.0, True), (11.2, False), (1e4, False), (1e38, False)):
+        assert (dtattn.workspace_size(dtattn.make_params(q, q, q, q, scale)) > 0) == there, scale

@@ -139,3 +139,14 @@ def test_tiny_values(dtattn, exponent):
     err, err_cc = rms(out.cpu().double() - ref.double()), rms(out_cc.cpu().double() - ref.double())
     assert err <= 1.25 * err_cc + 1e-8 * rms(ref), (exponent, err, err_cc)
     assert torch.equal(out, out_cc) == (exponent < -80)  # one number below 2^-110 (the smallest of these is 2^-16 of the usual) and it is the CUDA cores' call
+
+
+def test_scores_beyond_the_fp32_range(dtattn):
+    """Scores that overflow once scaled, to either side: the same rows as on the CUDA cores."""
+    B, S, H, D = 1, 200, 2, 64
+    q, k, v = (x.to(DEV) for x in inputs(B, S, S, H, H, D, torch.float32, 1371))
+    q[:, ::3] = 2.0 ** 57
+    k[:] = -(2.0 ** 57)
+    q[:, 1::3] = -(2.0 ** 57)
+    (out, lse), (out_cc, lse_cc) = both(dtattn, q, k, v, 2.0 ** 8)
+    assert torch.equal(out.view(torch.int32), out_cc.view(torch.int32)) and torch.equal(lse.view(torch.int32), lse_cc.view(torch.int32))
