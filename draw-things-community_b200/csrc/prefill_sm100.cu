@@ -842,11 +842,16 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         if (probe && j == 0) stamp(a, 16 * n_item + 8);
         ptx::tc_fence_after();
         uint32_t s[4][32];
+        const float sl2 = a.scale_log2;
+        float half_scale[2] = {sl2, sl2};  // from a half's scores to log2 units
         if constexpr (kMask) {
           // scores in two halves of 64 keys; each half gets mask / scale added once its mask values have landed (the
           // scores stay in the unscaled domain of the unmasked kernel).  A half whose mask values are all zero for the
           // whole warp -- most of a padding mask -- is left as it is.
-          const uint64_t inv2 = ptx::pack_f32x2(1.f / a.scale, 1.f / a.scale);
+          // kSplit: the half goes to log2 units and gets mask * log2(e), as in the CUDA-core kernel that these calls come from:
+          // mask / scale overflows for entries that do not overflow there (-1e38 in a fully masked row), or scales below 2^-128.
+          const uint64_t inv2 = ptx::pack_f32x2(kSplit ? kLog2e : 1.f / a.scale, kSplit ? kLog2e : 1.f / a.scale);
+          const uint64_t to_log2 = ptx::pack_f32x2(sl2, sl2);
           auto add_mask_half = [&](int half) {
             if (!((flags_cur >> half) & 1u)) return;  // the same answer for the whole warp
             const uint32_t buf = (half ? mask_smem : stage_smem) + (uint32_t)(warp - 4) * (32 * 128) + (uint32_t)lane * 128;
@@ -864,14 +869,16 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 for (int u = 0; u < 4; ++u) {
                   const float2 mf = unpack_pair<T>(mw[u]);
                   const int c = half * 2 + (q >> 2), i = (q & 3) * 8 + u * 2;
-                  const uint64_t r2 = ptx::fma_f32x2(ptx::pack_f32x2(mf.x, mf.y), inv2,
-                                                     ptx::pack_f32x2(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])));
+                  uint64_t s2 = ptx::pack_f32x2(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
+                  if constexpr (kSplit) s2 = ptx::mul_f32x2(s2, to_log2);
+                  const uint64_t r2 = ptx::fma_f32x2(ptx::pack_f32x2(mf.x, mf.y), inv2, s2);
                   float r0, r1;
                   ptx::unpack_f32x2(r2, r0, r1);
                   s[c][i] = __float_as_uint(r0);
                   s[c][i + 1] = __float_as_uint(r1);
                 }
               }
+              if constexpr (kSplit) half_scale[half] = 1.f;
             }
             __syncwarp();  // every lane has read its row: the buffer may be refilled
           };
@@ -897,7 +904,6 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           ptx::tmem_ld32(t_s + 96, s[3]);
           ptx::tc_wait_ld();
         }
-        const float sl2 = a.scale_log2;
         if (probe && j == 0) stamp(a, 16 * n_item + 4);
 
 #ifdef DT_BRINGUP
@@ -953,9 +959,10 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           for (int i = 3; i < 31; i += 2) mxc[c] = ptx::max3(mxc[c], __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
           mxc[c] = fmaxf(mxc[c], __uint_as_float(s[c][31]));
         }
-        float mx = fmaxf(fmaxf(mxc[0], mxc[1]), fmaxf(mxc[2], mxc[3]));
-        if (DT_OPT(32)) mx = __uint_as_float(s[0][0]);  // bring-up: no row maximum
-        mx *= sl2;  // scale > 0 is a precondition of this kernel
+        // (scale > 0 is a precondition of this kernel)
+        float mx = kSplit ? fmaxf(fmaxf(mxc[0], mxc[1]) * half_scale[0], fmaxf(mxc[2], mxc[3]) * half_scale[1])
+                          : fmaxf(fmaxf(mxc[0], mxc[1]), fmaxf(mxc[2], mxc[3])) * sl2;
+        if (DT_OPT(32)) mx = __uint_as_float(s[0][0]) * sl2;  // bring-up: no row maximum
         const float m_cand = fmaxf(m_used, mx);
         // Lazy rescale: keep the old reference max unless the new one is larger by more than the threshold.
         const bool grow = (m_cand - m_used > kRescaleThreshold) || (m_used == -INFINITY && m_cand != -INFINITY);
@@ -993,10 +1000,10 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         if (probe && j == 0) stamp(a, 16 * n_item + 13);
         const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
         const uint64_t neg_m2 = ptx::pack_f32x2(neg_m, neg_m);
-        const uint64_t scale2 = ptx::pack_f32x2(sl2, sl2);
         uint64_t lsum[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
+          const uint64_t scale2 = ptx::pack_f32x2(half_scale[c >> 1], half_scale[c >> 1]);
           lsum[c] = 0ull;
           if (c < nch) {
           uint32_t rest[16];

@@ -94,3 +94,31 @@ def test_expanded_views_stay_on_the_cuda_cores(dtattn, what):
     assert dtattn.device_status() == 0
     check(out, ref.float(), dtype, what)
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("fill", [-1e38, -3e37, -1e4, -float("inf"), "lowest"])
+@pytest.mark.parametrize("scale", [0.125, 1.0, 2.0 ** -133])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_fully_masked_rows_and_small_scales(dtattn, dtype, scale, fill):
+    """Rows whose every key is masked: an average where the fill stays finite times log2(e), zeros where it does not, as on
+    the CUDA cores, whatever the scale is."""
+    if dtype == torch.float16 and isinstance(fill, float) and -float("inf") < fill < -65504:
+        pytest.skip("not a half-precision number")
+    B, S, H, D = 1, 151, 2, 64
+    q, k, v = (x.to(DEV) for x in inputs(B, S, S, H, H, D, dtype, 1441))
+    mask = make_mask(1, 1, S, S, dtype, 1442).to(DEV)
+    mask[..., ::7, :] = -torch.finfo(dtype).max if fill == "lowest" else fill
+    mask[..., 3::7, 70:] = -torch.finfo(dtype).max if fill == "lowest" else fill
+    got = []
+    for flags in (0, dtattn.DT_FLAG_FORCE_GENERIC):
+        lse = torch.full((B, H, S), float("nan"), device=DEV)
+        got.append((dtattn.sdpa_forward(q, k, v, scale, mask=mask, lse=lse, flags=flags), lse))
+    torch.cuda.synchronize()
+    assert dtattn.device_status() == 0
+    (out, lse), (want, lse_want) = got
+    assert torch.equal(out == 0, want == 0)
+    # (the same number before it is rounded, to fp32's precision: at most the neighbouring 16-bit value, one unit in the last place)
+    assert float((out.float() - want.float()).abs().max()) <= 2.0 ** (-7 if dtype == torch.bfloat16 else -10) * float(want.abs().max())
+    assert torch.equal(lse.isinf(), lse_want.isinf())
+    fin = ~lse_want.isinf()
+    assert torch.allclose(lse[fin], lse_want[fin], atol=2e-3, rtol=1e-4)
