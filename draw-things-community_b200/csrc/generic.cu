@@ -17,16 +17,14 @@ constexpr int kRows = 8;    // query rows (= warps) per CTA
 constexpr int kKeys = 32;   // keys per tile
 
 template <typename T>
-__global__ void __launch_bounds__(kRows * 32)
-generic_sdpa_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ o,
+__device__ __forceinline__ void generic_sdpa_block(const dim3 block, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ o,
                     const T* __restrict__ mask, float* __restrict__ lse,
                     int64_t q_sb, int64_t q_ss, int64_t q_sh, int64_t k_sb, int64_t k_ss, int64_t k_sh,
                     int64_t v_sb, int64_t v_ss, int64_t v_sh, int64_t o_sb, int64_t o_ss, int64_t o_sh,
                     int64_t m_sb, int64_t m_sh, int64_t m_sq,
                     int Sq, int Sk, int Hq, int Hkv, int D, float scale_log2, int is_causal,
                     const T* __restrict__ sinks, int window, const int32_t* __restrict__ off_q,
-                    const int32_t* __restrict__ off_k, const uint32_t* __restrict__ only_if) {
-  if (only_if && *only_if == 0u) return;  // another kernel has computed this call
+                    const int32_t* __restrict__ off_k) {
   extern __shared__ float smem[];
   const int Dp = D | 1;
   float* Qs = smem;                    // [kRows][D]
@@ -34,14 +32,14 @@ generic_sdpa_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* _
   float* Vs = Ks + kKeys * Dp;         // [kKeys][D]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int b = blockIdx.z;
-  const int h = blockIdx.y;
+  int b = block.z;
+  const int h = block.y;
   const int kvh = h / (Hq / Hkv);
-  const int row0 = blockIdx.x * kRows;
+  const int row0 = block.x * kRows;
   const int lse_rows = Sq;  // rows per head of the lse output (packed rows for variable-length batches)
   int lse_row0 = 0;
   if (off_q) {
-    // variable-length batch: blockIdx.z is the sequence; its rows are a slice of the packed tensors
+    // variable-length batch: block.z is the sequence; its rows are a slice of the packed tensors
     const int q0 = off_q[b], k0 = off_k[b];
     Sq = off_q[b + 1] - q0;
     Sk = off_k[b + 1] - k0;
@@ -175,16 +173,14 @@ __host__ __device__ inline int tiled_pitch(int D) {  // multiple of 4, >= D + 4,
 }
 
 template <typename T, int R>  // R = 4-wide output column groups per thread (D <= 64 R)
-__global__ void __launch_bounds__(kTThreads)
-generic_tiled_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ o,
+__device__ __forceinline__ void generic_tiled_block(const dim3 block, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ o,
                      const T* __restrict__ mask, float* __restrict__ lse,
                      int64_t q_sb, int64_t q_ss, int64_t q_sh, int64_t k_sb, int64_t k_ss, int64_t k_sh,
                      int64_t v_sb, int64_t v_ss, int64_t v_sh, int64_t o_sb, int64_t o_ss, int64_t o_sh,
                      int64_t m_sb, int64_t m_sh, int64_t m_sq,
                      int Sq, int Sk, int Hq, int Hkv, int D, float scale_log2, int is_causal,
                      const T* __restrict__ sinks, int window, const int32_t* __restrict__ off_q,
-                     const int32_t* __restrict__ off_k, const uint32_t* __restrict__ only_if) {
-  if (only_if && *only_if == 0u) return;  // another kernel has computed this call
+                     const int32_t* __restrict__ off_k) {
   extern __shared__ __align__(16) float smem[];
   const int P1 = tiled_pitch(D);
   float* Qs = smem;              // [64][P1]
@@ -194,10 +190,10 @@ generic_tiled_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tx = tid & 15, ty = tid >> 4;
-  int b = blockIdx.z;
-  const int h = blockIdx.y;
+  int b = block.z;
+  const int h = block.y;
   const int kvh = h / (Hq / Hkv);
-  const int row0 = blockIdx.x * kTM;
+  const int row0 = block.x * kTM;
   const int lse_rows = Sq;
   int lse_row0 = 0;
   if (off_q) {
@@ -380,20 +376,66 @@ generic_tiled_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
   }
 }
 
+// The kernels: one block of the work per CTA, or, where another kernel may have computed the call already, as many CTAs as the
+// SMs hold at a time, which look into only_if first and then take all the blocks in turn: a CTA per block that only returns cost
+// 4 us for 1024 of them.
+template <bool kIf, typename Body>
+__device__ __forceinline__ void run_blocks(const uint32_t* __restrict__ only_if, const dim3 grid, Body body) {
+  if constexpr (kIf) {
+    if (*only_if == 0u) return;
+    const uint64_t total = (uint64_t)grid.x * grid.y * grid.z;
+    for (uint64_t i = blockIdx.x; i < total; i += gridDim.x) {
+      const uint64_t yz = i / grid.x;
+      body(dim3((unsigned)(i - yz * grid.x), (unsigned)(yz % grid.y), (unsigned)(yz / grid.y)));
+      __syncthreads();  // shared memory is used again
+    }
+  } else {
+    body(dim3(blockIdx.x, blockIdx.y, blockIdx.z));
+  }
+}
+dim3 launch_grid(dim3 grid, int threads, size_t smem, const uint32_t* only_if) {
+  if (!only_if) return grid;
+  const uint64_t total = (uint64_t)grid.x * grid.y * grid.z;
+  const uint64_t by_smem = 227 * 1024 / (smem + 1024), by_threads = 2048 / threads, per_sm = by_smem < by_threads ? by_smem : by_threads;
+  const uint64_t ctas = device_sm_count() * (per_sm ? per_sm : 1);
+  return dim3((unsigned)(total < ctas ? total : ctas));
+}
+
+#define DT_GENERIC_PARAMS                                                                                                      \
+  const T *__restrict__ q, const T *__restrict__ k, const T *__restrict__ v, T *__restrict__ o, const T *__restrict__ mask,    \
+      float *__restrict__ lse, int64_t q_sb, int64_t q_ss, int64_t q_sh, int64_t k_sb, int64_t k_ss, int64_t k_sh,              \
+      int64_t v_sb, int64_t v_ss, int64_t v_sh, int64_t o_sb, int64_t o_ss, int64_t o_sh, int64_t m_sb, int64_t m_sh,           \
+      int64_t m_sq, int Sq, int Sk, int Hq, int Hkv, int D, float scale_log2, int is_causal, const T *__restrict__ sinks,       \
+      int window, const int32_t *__restrict__ off_q, const int32_t *__restrict__ off_k, const uint32_t *__restrict__ only_if,   \
+      const dim3 grid
+#define DT_GENERIC_ARGS                                                                                                        \
+  q, k, v, o, mask, lse, q_sb, q_ss, q_sh, k_sb, k_ss, k_sh, v_sb, v_ss, v_sh, o_sb, o_ss, o_sh, m_sb, m_sh, m_sq, Sq, Sk, Hq,  \
+      Hkv, D, scale_log2, is_causal, sinks, window, off_q, off_k
+template <typename T, bool kIf>
+__global__ void __launch_bounds__(kRows * 32) generic_sdpa_kernel(DT_GENERIC_PARAMS) {
+  run_blocks<kIf>(only_if, grid, [&](const dim3 block) { generic_sdpa_block<T>(block, DT_GENERIC_ARGS); });
+}
+template <typename T, int R, bool kIf>
+__global__ void __launch_bounds__(kTThreads) generic_tiled_kernel(DT_GENERIC_PARAMS) {
+  run_blocks<kIf>(only_if, grid, [&](const dim3 block) { generic_tiled_block<T, R>(block, DT_GENERIC_ARGS); });
+}
+#undef DT_GENERIC_PARAMS
+#undef DT_GENERIC_ARGS
+
 template <typename T, int R>
 int launch_tiled(const dt_sdpa_params& p, cudaStream_t stream, const uint32_t* only_if) {
   const int D = p.D;
   const size_t smem = sizeof(float) * ((size_t)(kTM + kTN) * tiled_pitch(D) + (size_t)kTN * D + (size_t)kTM * kPPitch);
-  auto kern = generic_tiled_kernel<T, R>;
+  auto kern = only_if ? generic_tiled_kernel<T, R, true> : generic_tiled_kernel<T, R, false>;
   if (smem > 48 * 1024) DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const bool varlen = p.seq_offsets_q != nullptr;
   dim3 grid(((varlen ? p.max_seq_q : p.Sq) + kTM - 1) / kTM, p.Hq, varlen ? p.n_seq : p.B);
-  kern<<<grid, kTThreads, smem, stream>>>(
+  kern<<<launch_grid(grid, kTThreads, smem, only_if), kTThreads, smem, stream>>>(
       (const T*)p.q.ptr, (const T*)p.k.ptr, (const T*)p.v.ptr, (T*)p.o.ptr, (const T*)p.mask, p.lse,
       p.q.stride_b, p.q.stride_s, p.q.stride_h, p.k.stride_b, p.k.stride_s, p.k.stride_h,
       p.v.stride_b, p.v.stride_s, p.v.stride_h, p.o.stride_b, p.o.stride_s, p.o.stride_h,
       p.mask_stride_b, p.mask_stride_h, p.mask_stride_q, p.Sq, p.Sk, p.Hq, p.Hkv, D, p.scale * kLog2e,
-      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if);
+      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if, grid);
   DT_CUDA_TRY(cudaGetLastError());
   return DT_OK;
 }
@@ -409,16 +451,16 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, const uint32_t* only_
     return launch_tiled<T, 4>(p, stream, only_if);
   }
   const size_t smem = sizeof(float) * ((size_t)kRows * D + (size_t)kKeys * (D | 1) + (size_t)kKeys * D);
-  auto kern = generic_sdpa_kernel<T>;
+  auto kern = only_if ? generic_sdpa_kernel<T, true> : generic_sdpa_kernel<T, false>;
   if (smem > 48 * 1024) DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const bool varlen = p.seq_offsets_q != nullptr;
   dim3 grid(((varlen ? p.max_seq_q : p.Sq) + kRows - 1) / kRows, p.Hq, varlen ? p.n_seq : p.B);
-  kern<<<grid, kRows * 32, smem, stream>>>(
+  kern<<<launch_grid(grid, kRows * 32, smem, only_if), kRows * 32, smem, stream>>>(
       (const T*)p.q.ptr, (const T*)p.k.ptr, (const T*)p.v.ptr, (T*)p.o.ptr, (const T*)p.mask, p.lse,
       p.q.stride_b, p.q.stride_s, p.q.stride_h, p.k.stride_b, p.k.stride_s, p.k.stride_h,
       p.v.stride_b, p.v.stride_s, p.v.stride_h, p.o.stride_b, p.o.stride_s, p.o.stride_h,
       p.mask_stride_b, p.mask_stride_h, p.mask_stride_q, p.Sq, p.Sk, p.Hq, p.Hkv, D, p.scale * kLog2e,
-      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if);
+      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if, grid);
   DT_CUDA_TRY(cudaGetLastError());
   return DT_OK;
 }

@@ -94,6 +94,7 @@ struct PrefillArgs {
   // [mask batches][mask heads][n_rg row groups][n_kh key halves, padded to an even count]
   const unsigned char* mask_flags;
   int n_rg, n_kh;
+  uint32_t* not_finite;  // kSplit: set when some O is an infinity or NaN, for the kernel behind
   float scale;  // the plain scale (scale_log2 = scale * log2(e)); the masked variant adds the mask in this domain
   int item_rows;          // query rows of a work item: a pair of tiles, or one tile where pairs would leave SMs idle
   int n_qpairs, n_items;  // work items = (batch, head, item_rows query rows)
@@ -333,9 +334,11 @@ __global__ void __launch_bounds__(256) mask_flags_kernel(const unsigned short* _
 __global__ void __launch_bounds__(256) mask_repack_kernel(const unsigned short* __restrict__ mask, int64_t m_sb, int64_t m_sh,
                                                           int64_t m_sq, int Hm, int Sq, int Sk, int n_rg, int n_kh,
                                                           int is_causal, unsigned char* __restrict__ flags,
-                                                          unsigned short* __restrict__ copy, int ld) {
+                                                          unsigned short* __restrict__ copy, int ld,
+                                                          uint32_t* __restrict__ not_finite) {
   const int lane = threadIdx.x & 31;
   const int kh = blockIdx.x * 8 + (threadIdx.x >> 5), rg = blockIdx.y, bh = blockIdx.z;
+  if (threadIdx.x == 0 && blockIdx.x == 0 && rg == 0 && bh == 0) *not_finite = 0u;
   if (kh >= n_kh) return;
   const int mb = bh / Hm, mh = bh - mb * Hm;
   const unsigned short* base = mask + mb * m_sb + mh * m_sh;
@@ -1073,6 +1076,11 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           uint32_t ov[16];
           ptx::tmem_ld16(t_o + c * 16, ov);
           ptx::tc_wait_ld();
+          if constexpr (kSplit) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (!(__uint_as_float(ov[i]) * 0.f == 0.f)) *a.not_finite = 1u;
+          }
 #pragma unroll
           for (int i = 0; i < 4; ++i)  // [D / 4][32 rows][4]: a warp writes 512 consecutive bytes
             __stcg(reinterpret_cast<float4*>(mine + 64) + (c * 4 + i) * 32 + lane,
@@ -1092,6 +1100,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           l += fast_exp2(sl - m_used);
         }
       }
+      uint64_t probe = 0ull;  // kSplit: O * 0 added up, NaN where an O is not finite
       // a row that never saw a visible key (m_used still -inf) yields zeros, whatever the masked entries summed to
       const float inv = (l > 0.f && m_used != -INFINITY) ? 1.f / l : 0.f;
       // O goes out through shared memory and a TMA store per warp (32 rows x 64 columns): whole 128-byte
@@ -1114,6 +1123,11 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             uint32_t ov[32];
             ptx::tmem_ld32(t_o + hf * 64 + c * 32, ov);
             ptx::tc_wait_ld();
+            if constexpr (kSplit) {
+#pragma unroll
+              for (int i = 0; i < 16; ++i)
+                probe = ptx::fma_f32x2(ptx::pack_f32x2(__uint_as_float(ov[2 * i]), __uint_as_float(ov[2 * i + 1])), 0ull, probe);
+            }
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
               uint4 pk;
@@ -1153,6 +1167,11 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           }
           __syncwarp();
         }
+      }
+      if constexpr (kSplit) {
+        float p0, p1;
+        ptx::unpack_f32x2(probe, p0, p1);
+        if (!(p0 + p1 == 0.f)) *a.not_finite = 1u;
       }
       if (a.lse && row < w.sq)
         a.lse[((int64_t)w.b * a.Hq + w.h) * a.Sq + w.qrow + row] =
@@ -1255,9 +1274,9 @@ size_t mask_flag_bytes(const dt_sdpa_params& p) {
   return kTicketBytes + (Bm * Hm * n_rg * n_kh + 255) / 256 * 256;
 }
 int repacked_row(const dt_sdpa_params& p) { return (p.Sk + 7) / 8 * 8; }
-size_t prefill_repack_bytes_needed(const dt_sdpa_params& p) {  // the flags and the copy
+size_t prefill_repack_bytes_needed(const dt_sdpa_params& p) {  // the flags, the word that says "not finite" and the copy
   const size_t Bm = p.mask_stride_b ? p.B : 1, Hm = p.mask_stride_h ? p.Hq : 1;
-  return mask_flag_bytes(p) + Bm * Hm * p.Sq * (size_t)repacked_row(p) * 2;
+  return mask_flag_bytes(p) + 256 + Bm * Hm * p.Sq * (size_t)repacked_row(p) * 2;
 }
 size_t cut_bytes(const dt_sdpa_params& p) {
   const int D = p.D > 128 ? 256 : p.D > 64 ? 128 : 64, tiles = D == 256 ? 1 : 2;
@@ -1299,10 +1318,11 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
     if (fgrid.y > 65535 || fgrid.z > 65535) return DT_UNSUPPORTED;
     if (kSplit) {
       const int ld = repacked_row(p);
-      unsigned short* copy = reinterpret_cast<unsigned short*>(static_cast<uint8_t*>(workspace) + mask_flag_bytes(p));
+      a.not_finite = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(workspace) + mask_flag_bytes(p));
+      unsigned short* copy = reinterpret_cast<unsigned short*>(reinterpret_cast<uint8_t*>(a.not_finite) + 256);
       mask_repack_kernel<<<fgrid, 256, 0, stream>>>(static_cast<const unsigned short*>(p.mask), p.mask_stride_b, p.mask_stride_h,
                                                    p.mask_stride_q, Hm, p.Sq, p.Sk, a.n_rg, a.n_kh, p.is_causal,
-                                                   flags, copy, ld);
+                                                   flags, copy, ld, a.not_finite);
       a.mask = copy;
       a.m_sq = ld;
       a.m_sh = Hm > 1 ? (int64_t)p.Sq * ld : 0;
@@ -1397,12 +1417,18 @@ size_t prefill_repack_workspace_bytes(const dt_sdpa_params& p) {
   return cut ? align256(prefill_repack_bytes_needed(p)) + cut : prefill_repack_bytes_needed(p);
 }
 
+// An infinity in V is 0 * inf = NaN to the second part of a weight that has none, and a NaN in V reaches the rows of other tiles
+// than on the CUDA cores.  Either makes every O of the tiles that see its key an infinity or NaN, as NaN scores do: where one came
+// out, the CUDA-core kernel behind, which otherwise returns at once, computes the call (encoder of 333 tokens 24 -> 27 us; looking V
+// over in the first pass, a few dozen blocks, took 15 us).
 int launch_prefill_repack(const dt_sdpa_params& p, cudaStream_t stream, void* workspace, size_t workspace_bytes) {
 #define DT_REPACK_GO(T, DD) launch_t<T, DD, true, true>(p, stream, nullptr, 0, workspace, workspace_bytes)
 #define DT_REPACK_BY_D(T) (p.D > 128 ? DT_REPACK_GO(T, 256) : p.D > 64 ? DT_REPACK_GO(T, 128) : DT_REPACK_GO(T, 64))
-  return p.dtype == DT_F16 ? DT_REPACK_BY_D(__half) : DT_REPACK_BY_D(__nv_bfloat16);
+  const int st = p.dtype == DT_F16 ? DT_REPACK_BY_D(__half) : DT_REPACK_BY_D(__nv_bfloat16);
 #undef DT_REPACK_BY_D
 #undef DT_REPACK_GO
+  if (st != DT_OK) return st;
+  return launch_generic(p, stream, reinterpret_cast<const uint32_t*>(static_cast<uint8_t*>(workspace) + mask_flag_bytes(p)));
 }
 
 int launch_prefill(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra_outputs, int n_extra, void* workspace,

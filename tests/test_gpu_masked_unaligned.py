@@ -122,3 +122,32 @@ def test_fully_masked_rows_and_small_scales(dtattn, dtype, scale, fill):
     assert torch.equal(lse.isinf(), lse_want.isinf())
     fin = ~lse_want.isinf()
     assert torch.allclose(lse[fin], lse_want[fin], atol=2e-3, rtol=1e-4)
+
+
+@pytest.mark.parametrize("where", ["v", "k", "q"])
+@pytest.mark.parametrize("value", [float("inf"), -float("inf"), float("nan")])
+@pytest.mark.parametrize("key", [3, 100, 1500])
+@pytest.mark.parametrize("case", [(201, 201, True, torch.bfloat16, 64), (130, 2101, False, torch.float16, 128), (77, 2101, True, torch.bfloat16, 256)])
+def test_infinities_and_nan(dtattn, case, key, value, where):
+    """They reach the rows and columns that they reach on the CUDA cores, bit for bit; the next call is itself again."""
+    Sq, Sk, causal, dtype, D = case
+    q, k, v = (x.to(DEV) for x in inputs(1, Sq, Sk, 4, 2, D, dtype, 1451))
+    x = dict(q=q, k=k, v=v)[where]
+    key = min(key, x.shape[1] - 1)
+    mask = make_mask(1, 1, Sq, Sk, dtype, 1452).to(DEV)
+    clean = dtattn.sdpa_forward(q, k, v, D ** -0.5, causal, mask)
+    keep = x[0, key, 1, 5].item()
+    x[0, key, 1, 5] = value
+    got = []
+    for flags in (0, dtattn.DT_FLAG_FORCE_GENERIC):
+        lse = torch.full((1, 4, Sq), float("nan"), device=DEV)
+        got.append((dtattn.sdpa_forward(q, k, v, D ** -0.5, causal, mask, lse=lse, flags=flags), lse))
+    x[0, key, 1, 5] = keep
+    again = dtattn.sdpa_forward(q, k, v, D ** -0.5, causal, mask)
+    torch.cuda.synchronize()
+    assert dtattn.device_status() == 0
+    if where == "v":
+        assert not bool(got[0][0].isfinite().all())
+    for a, b in zip(*got):
+        assert torch.equal(a.view(torch.int16 if a.dtype == dtype else torch.int32), b.view(torch.int16 if b.dtype == dtype else torch.int32))
+    assert torch.equal(again, clean)
