@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import ctypes
 import enum
+import operator
 import os
 import struct
 
@@ -324,7 +325,7 @@ def make_step_params(q, k_cache, v_cache, k_new, v_new, rotary, o, scale, total_
                      sliding_window=0) -> DecodeStepParams:
     """k_cache / v_cache: [B, capacity, Hkv, D]; the step attends over their first `total_len` rows, of which
     the last k_new.shape[1] are written by the call."""
-    total_len = int(total_len)
+    total_len = operator.index(total_len)  # (a fractional length is refused, as a slice refuses it)
     if not 0 < total_len <= min(k_cache.shape[1], v_cache.shape[1]):  # the slices' own rules for anything else
         k_cache, v_cache = k_cache[:, :total_len], v_cache[:, :total_len]
         total_len = None

@@ -250,3 +250,15 @@ def test_fp32_calls_whose_scores_may_overflow_stay_on_the_cuda_cores(dtattn):
     q = torch.zeros(1, 256, 2, 64)
     for scale, there in ((0.125, True), (1.0, True), (11.0, True), (11.2, False), (1e4, False), (1e38, False)):
         assert (dtattn.workspace_size(dtattn.make_params(q, q, q, q, scale)) > 0) == there, scale
+
+
+def test_decode_step_lengths_are_whole_numbers(dtattn):
+    """The cached length may be anything a slice takes, and nothing else."""
+    import numpy as np
+    q, kc = torch.zeros(1, 1, 8, 64, dtype=torch.float16), torch.zeros(1, 32, 2, 64, dtype=torch.float16)
+    kn = kc[:, :1]
+    for n in (5, np.int64(5), torch.tensor(5)):
+        assert dtattn.make_step_params(q, kc, kc, kn, kn, None, q, 0.125, n).attn.Sk == 5
+    for n in (5.0, 5.5, "5", None):
+        with pytest.raises(TypeError):
+            dtattn.make_step_params(q, kc, kc, kn, kn, None, q, 0.125, n)
