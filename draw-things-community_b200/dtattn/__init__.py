@@ -103,6 +103,11 @@ def _f32(x):
     return ctypes.c_float(x).value
 
 
+def _i32(x):
+    """x as a 32-bit int, wrapped as in a C assignment."""
+    return ((int(x) + 0x80000000) & 0xffffffff) - 0x80000000
+
+
 def _quad(t):
     """(pointer, batch, token and head stride) of a [B,S,H,D] view."""
     st = t.stride()
@@ -221,8 +226,8 @@ def _pack_params(q, k, v, o, scale, is_causal, mask, lse, flags, sinks, sliding_
     else:
         max_seq_q = max_seq_k = 0
     return _PACK_SDPA.pack(B, Sq, Sk, Hq, Hkv, D, _DTYPES[q.dtype], _f32(scale), 1 if is_causal else 0, int(flags) & 0xffffffff,
-                           *_quad(q), *_quad(k), *_quad(v), *_quad(o), *mask_fields, lse_ptr, sinks_ptr, int(sliding_window),
-                           n_seq, max_seq_q, max_seq_k, offs_q, offs_k)
+                           *_quad(q), *_quad(k), *_quad(v), *_quad(o), *mask_fields, lse_ptr, sinks_ptr, _i32(sliding_window),
+                           n_seq, _i32(max_seq_q), _i32(max_seq_k), offs_q, offs_k)
 
 
 def make_params(q, k, v, o, scale, is_causal=False, mask=None, lse=None, flags=0, sinks=None, sliding_window=0,
@@ -464,7 +469,7 @@ def sparse_indexed_attention(q, k_raw, v_raw, k_comp, v_comp, selected, scale, s
         lse_ptr = lse.data_ptr()
     p = SparseIndexedParams.from_buffer_copy(_PACK_SPARSE.pack(
         B, Sq, Hq, k_raw.shape[2], D, k_raw.shape[1], Sc, n_selected, _DTYPES[q.dtype], _f32(scale), 1 if is_causal else 0,
-        int(sliding_window), *_quad(q), *_quad(out), *_quad(k_raw), *_quad(v_raw), *comp[0], *comp[1], *sel, sinks_ptr, lse_ptr,
+        _i32(sliding_window), *_quad(q), *_quad(out), *_quad(k_raw), *_quad(v_raw), *comp[0], *comp[1], *sel, sinks_ptr, lse_ptr,
         int(flags) & 0xffffffff))
     s = _stream_of(q.device, stream)
     _check(lib().dt_sparse_indexed_attention(ctypes.byref(p), ctypes.c_void_p(s)), "dt_sparse_indexed_attention")

@@ -262,3 +262,13 @@ def test_decode_step_lengths_are_whole_numbers(dtattn):
     for n in (5.0, 5.5, "5", None):
         with pytest.raises(TypeError):
             dtattn.make_step_params(q, kc, kc, kn, kn, None, q, 0.125, n)
+
+
+def test_integers_wrap_as_in_a_c_assignment(dtattn):
+    """Numbers beyond 32 bits are no Python error: they reach the library as C would pass them, and it judges them."""
+    q = torch.zeros(1, 8, 2, 64, dtype=torch.float16)
+    for x, want in ((7, 7), (2 ** 31, -2 ** 31), (2 ** 32 + 3, 3), (-1, -1)):
+        assert dtattn.make_params(q, q, q, q, 0.125, sliding_window=x).sliding_window == want
+    n = ctypes.c_size_t()
+    p = dtattn.make_params(q, q, q, q, 0.125, sliding_window=2 ** 31)
+    assert dtattn.lib().dt_sdpa_workspace_size(ctypes.byref(p), ctypes.byref(n)) == dtattn.DT_BAD_ARG
