@@ -476,27 +476,33 @@ PrologueTensor to_arg(const dt_qk_prologue_params* p) {
   return t;
 }
 
-// Normalised and rotated with nothing behind, a token's heads share their rotary row, and there are enough of them to fill
-// the rows a warp takes at a time (the reference's joint attention: 12 heads, 20000 tokens 64.5 -> 55.3 us; 5 heads, 256
-// tokens 2.6 against 2.9 us); everything else, a table per head or a few KV heads among it, stays with the row kernel.
-bool by_token(const PrologueArgs& a, int rows_per_warp) {
+// Which calls the per-token kernel serves.  Normalised and rotated with nothing behind, and a token's heads share their rotary
+// row; a warp's chunks of heads at least two thirds full (queries and keys of 4608 tokens, heads of 128: 9 heads 13.0 us in the row
+// kernel, 14.8 here; 10 heads 14.1 and 14.6; 12 heads 16.1 and 14.8; 24 heads 31.7 and 22.6; of 64: 17 heads 12.7 and 14.5, 24
+// heads 16.3 and 14.4); and enough tasks that what each warp prepares first is hidden: with full chunks from 1024 on (8 heads
+// of 128, 384 tokens 3.04 and 3.23 us, 512 tokens 3.50 and 3.19), else from 2048 (12 heads, 384 tokens 3.47 and 3.60, 512: 4.22, 3.67).
+// Everything else, a table per head or a few KV heads among it, stays with the row kernel.
+bool by_token(const PrologueArgs& a, int chunk, int64_t* most_tasks) {
+  int64_t all = 0;
+  bool full = true;
+  *most_tasks = 0;
   for (int i = 0; i < a.n; ++i) {
     const PrologueTensor& t = a.t[i];
-    if (!t.weight || !t.rot || t.post_scale != 1.f || (t.r_sh != 0 && t.H > 1) || t.H < rows_per_warp * kHeadRows) return false;
+    const int n_chunks = (t.H + chunk - 1) / chunk;
+    if (!t.weight || !t.rot || t.post_scale != 1.f || (t.r_sh != 0 && t.H > 1) || 3 * t.H < 2 * n_chunks * chunk) return false;
+    const int64_t n = (int64_t)t.B * t.S * n_chunks;
+    all += n;
+    full = full && 8 * t.H >= 7 * n_chunks * chunk;
+    if (n > *most_tasks) *most_tasks = n;
   }
-  return true;
+  return all >= (full ? 1024 : 2048);
 }
 
 template <typename T>
 int launch_rows(const PrologueArgs& a, int D, int64_t max_rows, cudaStream_t stream) {
   const int lanes = D <= 64 ? 8 : (D <= 128 ? 16 : 32);
-  if (by_token(a, 32 / lanes)) {
-    int64_t tasks = 0;
-    for (int i = 0; i < a.n; ++i) {
-      const int chunk = 32 / lanes * kHeadRows;
-      const int64_t n = (int64_t)a.t[i].B * a.t[i].S * ((a.t[i].H + chunk - 1) / chunk);
-      tasks = n > tasks ? n : tasks;
-    }
+  int64_t tasks = 0;
+  if (by_token(a, 32 / lanes * kHeadRows, &tasks)) {
     const int64_t need = (tasks + 7) / 8, cap = (int64_t)sm_count_prologue() * 3 / a.n;  // persistent: three CTAs per SM
     dim3 grid((unsigned)(need < cap ? need : cap), a.n);
     if (lanes == 8) qk_prologue_heads_kernel<T, 8><<<grid, 256, 0, stream>>>(a);
