@@ -129,3 +129,40 @@ def test_prologue_argument_checks(dtattn):
     k = dtattn.make_prologue_params(x, x, norm_per_token=True)
     assert lib.dt_qk_prologue(ctypes.byref(q), ctypes.byref(k), None) == dtattn.DT_BAD_ARG
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("case", [
+    # B, S, Hq, Hk, D, dtype: calls for the kernel that takes a token's heads several at a time (chunks of 16 / 8 / 4 at D up to
+    # 64 / 128 / 256), each warp several of them: one chunk, one and a half, two; a chunk with a hole; fewer lanes than a row has
+    (2, 3000, 16, 16, 64, torch.float16), (2, 1600, 24, 32, 64, torch.bfloat16), (1, 3300, 27, 16, 40, torch.float16),
+    (2, 3000, 8, 8, 128, torch.bfloat16), (2, 1600, 12, 16, 128, torch.float16), (1, 3300, 24, 8, 128, torch.bfloat16),
+    (2, 1700, 15, 13, 96, torch.bfloat16), (2, 3000, 4, 4, 256, torch.float16), (2, 1600, 6, 8, 256, torch.bfloat16),
+    (1, 4100, 16, 4, 256, torch.bfloat16), (3, 700, 8, 8, 160, torch.float16)])
+@pytest.mark.parametrize("per_batch", [False, True])
+def test_heads_of_a_token_at_a_time(dtattn, case, per_batch):
+    """Bit for bit the row kernel's results, which serves the same call with the rotary table written out per head; also in
+    place, and into rows of wider buffers."""
+    B, S, Hq, Hk, D, dtype = case
+    g = torch.Generator(device=DEV).manual_seed(860)
+    rnd = lambda *shape: torch.randn(*shape, generator=g, device=DEV).to(dtype)  # noqa: E731
+    q, k, wq, wk = rnd(B, S, Hq, D) * 3, rnd(B, S, Hk, D), 1 + 0.3 * rnd(D), 1 + 0.3 * rnd(D)
+    angle = torch.rand(B if per_batch else 1, S, 1, D // 2, generator=g, device=DEV) * 6.3
+    rot = torch.stack([angle.cos(), angle.sin()], dim=-1).reshape(-1, S, 1, D).to(dtype)
+    want = dtattn.qk_prologue(q, k, q_weight=wq, k_weight=wk, rotary=rot.expand(-1, -1, Hq, -1).contiguous(),
+                              rotary_k=rot.expand(-1, -1, Hk, -1).contiguous())
+    got = dtattn.qk_prologue(q, k, q_weight=wq, k_weight=wk, rotary=rot)
+    wide = torch.full((B, S + 2, Hq + Hk, D), 7.0, dtype=dtype, device=DEV)
+    dtattn.qk_prologue(q, k, q_out=wide[:, 1:-1, :Hq], k_out=wide[:, 1:-1, Hq:], q_weight=wq, k_weight=wk, rotary=rot)
+    q_in, k_in = q.clone(), k.clone()
+    dtattn.qk_prologue(q_in, k_in, q_out=q_in, k_out=k_in, q_weight=wq, k_weight=wk, rotary=rot)
+    alone, _ = dtattn.qk_prologue(q, q_weight=wq, rotary=rot)
+    torch.cuda.synchronize()
+    bits = lambda t: t.contiguous().view(torch.int16)  # noqa: E731
+    for a, b in zip(want, got):
+        assert torch.equal(bits(a), bits(b))
+    assert torch.equal(bits(wide[:, 1:-1, :Hq]), bits(want[0])) and torch.equal(bits(wide[:, 1:-1, Hq:]), bits(want[1]))
+    assert bool((wide[:, 0] == 7).all()) and bool((wide[:, -1] == 7).all())
+    assert torch.equal(bits(q_in), bits(want[0])) and torch.equal(bits(k_in), bits(want[1])) and torch.equal(bits(alone), bits(want[0]))
+    rows = slice(S - 40, S)  # the oracle, on the last tokens
+    ref = so.qk_prologue_explicit(q[:, rows].cpu(), wq.cpu(), rot[:, rows].expand(B, -1, -1, -1).cpu(), 1e-6, dtype)
+    close_1ulp(got[0][:, rows], ref, dtype, str(case))
