@@ -540,9 +540,12 @@ bool sparse_tcgen05_supported(const dt_sparse_indexed_params& p, bool same_kv) {
   if (p.D % 256 || p.D > kMaxD || !same_kv || !(p.scale > 0.f) || (p.Hq / p.Hkv) % kHeads) return false;
   const bool raw = p.Sr > 0, comp = p.Sc > 0 && p.n_selected > 0;
   if ((!raw && !comp) || (raw && !key_map_fits(p.k_raw, p.Sr, p)) || (comp && !key_map_fits(p.k_comp, p.Sc, p))) return false;
-  // below 16 the keys of a token are better spread over a cluster of CTAs (8 tokens of 640 keys: 21 us there, 24 us here;
-  // 16: 30 and 24 us; 64: 76 and 24 us)
-  return (long long)p.B * p.Sq * p.Hq / kHeads >= 16 && (long long)p.B * p.Sq * p.Hq / kHeads < (1LL << 30);
+  // Few tokens leave SMs idle here, and the warp-level kernel spreads a token's keys over a cluster of CTAs, up to about 300 of
+  // them (four per token and 64 heads for 16 tokens, two for 19).  Tokens x 64 heads, 640 keys each, there and here: head dim
+  // 512: 8: 21 us (24 here with one part per weight), 16: 30.6 and 28.6, 18: 55 and 28.6, 64: 76 and 28; 4096 keys: 16: 134 and 140 us,
+  // 18: 248 and 140.  Head dim 256: 16: 19.8 and 23.7, 18: 21.6 and 24.0, 20: 34.6 and 24.1; 2176 keys: 18: 57 and 65, 20: 98 and 65.
+  const long long items = (long long)p.B * p.Sq * p.Hq / kHeads;
+  return items >= (p.D == 256 ? 19 : 16) && items < (1LL << 30);
 }
 
 int launch_sparse_tcgen05(const dt_sparse_indexed_params& p, cudaStream_t stream) {

@@ -19,6 +19,8 @@ pytestmark = pytest.mark.gpu
     (2, 70, 100, 40, 33, 128, 1, 512, torch.bfloat16, 0, True, True),   # two head groups, batch, no window
     (1, 40, 90, 25, 60, 128, 2, 256, torch.float16, 20, True, True),    # two KV heads, head dim 256
     (1, 80, 100, 16, 16, 64, 1, 256, torch.bfloat16, 0, True, False),   # every token sees every raw row
+    (1, 18, 700, 50, 60, 64, 1, 256, torch.float16, 128, True, True),   # either side of the dispatch at head dim 256
+    (1, 19, 700, 50, 60, 64, 1, 256, torch.float16, 128, True, True),
 ])
 def test_against_the_oracle(dtattn, case):
     B, Sq, Sr, Sc, n_sel, Hq, Hkv, D, dtype, window, with_sinks, causal = case
