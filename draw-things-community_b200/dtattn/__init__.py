@@ -261,7 +261,7 @@ def device_status(stream=None) -> int:
 def _alloc(nbytes, device, stream):
     """Device memory in the order of `stream` (a raw handle): a block that torch hands out on another stream may still be in
     use by that stream's queued kernels."""
-    if stream == torch.cuda.current_stream(device).cuda_stream:
+    if stream == _stream_of(device, None):
         return torch.empty(nbytes, dtype=torch.uint8, device=device)
     with torch.cuda.stream(torch.cuda.ExternalStream(stream, device=device)):
         return torch.empty(nbytes, dtype=torch.uint8, device=device)
