@@ -582,10 +582,9 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       }
     } else if (warp == 1) {
       // =========================== MMA issuer ===========================
-      // The whole warp walks the loop and one lane issues, which keeps the operands in uniform registers (Flux joint
-      // attention 227 -> 216 us, 2047 tokens with an unaligned mask 97 -> 86 us); the 64- and 256-wide variants, whose MMAs
-      // are fewer or longer, are 1 % faster with one lane walking it (SD1.5 self-attention 125 against 126 us, 1777 x 5873
-      // prompt chunk of dim 256 125 against 126 us).
+      // The whole warp walks the loop and one lane issues, which keeps the operands in uniform registers (joint attention of
+      // 4608 tokens 221 -> 217 us); the 64- and 256-wide variants, whose MMAs are fewer or longer, are 1 to 2 % faster with one
+      // lane walking it (2 x 4096 tokens, heads of 40: 123.2 against 125.1 us; 1777 x 5873, heads of 256: 126.3 against 127.2 us).
       constexpr bool kWarpIssue = D == 128;
       if (kWarpIssue || lane == 0) {
         const bool on = kWarpIssue ? ptx::elect_one() : true;
@@ -1399,15 +1398,17 @@ size_t prefill_workspace_bytes(const dt_sdpa_params& p) {
 
 // Masks whose rows are not 16-byte aligned: copied to aligned rows first.  The calls come from the CUDA-core kernel, whose
 // weights are fp32, so this variant multiplies V with two 16-bit parts of every weight: 333 tokens, 32 / 8 heads of 128,
-// causal and padding mask, bf16: 117 us there, 30 us here, error against 64 bits 1.6e-3 (the rounding of the result) in both.  A mask per head of a long
+// causal and padding mask, bf16: 117 us there, 27 us here, error against 64 bits 1.6e-3 (the rounding of the result) in both.  A mask per head of a long
 // sequence would need a copy as large as itself: up to 256 MB.
 bool prefill_repack_supported(const dt_sdpa_params& p) {
   if (!p.mask || mask_rows_aligned(p) || (p.flags & DT_FLAG_FORCE_GENERIC)) return false;
   dt_sdpa_params plain = p;
   plain.mask = nullptr;
-  // up to one 64-key tile the CUDA-core kernel takes a single step (41 tokens, 32 heads: 18.2 us there, 19.2 us here; 77
-  // tokens, 12 heads: 23.1 and 17.3 us)
+  // Up to one 64-key tile the CUDA-core kernel takes a single step (41 tokens, 32 heads: 18.2 us there, 19.2 us here), and with
+  // heads up to 64 and a block of its own for every CTA two steps cost less than three launches and scratch: 77 tokens, 12 heads of
+  // 64: 23.2 us on the device there and 19.6 here, but one call after another 23 and 33 (129 tokens: 33 and 21 on the device).
   if (p.Sk <= 64 || !prefill_supported(plain) || (p.Sq + 31) / 32 > 65535) return false;
+  if (p.Sk <= 128 && p.D <= 64 && (double)((p.Sq + 63) / 64) * p.Hq * p.B <= device_sm_count()) return false;
   const size_t Bm = p.mask_stride_b ? p.B : 1, Hm = p.mask_stride_h ? p.Hq : 1;
   return Bm * Hm <= 65535 && Bm * Hm * p.Sq * (size_t)repacked_row(p) * 2 <= ((size_t)256 << 20);
 }

@@ -69,7 +69,7 @@ def test_scratch_limits(dtattn):
 @pytest.mark.parametrize("what", ["k and v over the heads", "k and v over the batch", "v over the tokens", "q over the batch"])
 def test_expanded_views_stay_on_the_cuda_cores(dtattn, what):
     """A view with a zero stride (torch.expand) is not for tensor maps: served as before, whatever scratch there is."""
-    B, S, H, D, dtype = 2, 101, 4, 64, torch.bfloat16
+    B, S, H, D, dtype = 2, 151, 4, 64, torch.bfloat16
     q, k, v = inputs(B, S, S, H, H, D, dtype, 1431)
     if what == "k and v over the heads":
         k, v = k[:, :, :1].expand(B, S, H, D), v[:, :, :1].expand(B, S, H, D)
@@ -151,3 +151,31 @@ def test_infinities_and_nan(dtattn, case, key, value, where):
     for a, b in zip(*got):
         assert torch.equal(a.view(torch.int16 if a.dtype == dtype else torch.int32), b.view(torch.int16 if b.dtype == dtype else torch.int32))
     assert torch.equal(again, clean)
+
+
+@pytest.mark.parametrize("case", [
+    # Sq, Sk, H, D, scratch asked for: either side of the sizes that the CUDA cores keep
+    (77, 64, 12, 64, False), (77, 77, 12, 64, False), (100, 127, 4, 40, False), (100, 129, 4, 40, True), (77, 77, 12, 80, True),
+    (77, 65, 4, 128, True), (641, 127, 14, 64, True), (640, 127, 14, 64, False)])
+def test_which_calls_take_the_tensor_cores(dtattn, case):
+    """With the scratch that they ask for, or none, they answer as the CUDA cores do; with less than it bit for bit."""
+    import ctypes
+    Sq, Sk, H, D, asked = case
+    dtype = torch.float16
+    q, k, v = (x.to(DEV) for x in inputs(1, Sq, Sk, H, H, D, dtype, 1461))
+    store = torch.zeros(Sq * Sk + 1, dtype=dtype, device=DEV)
+    mask = store[1:].view(1, 1, Sq, Sk).copy_(make_mask(1, 1, Sq, Sk, dtype, 1462).to(DEV))
+    want = dtattn.sdpa_forward(q, k, v, D ** -0.5, mask=mask, flags=dtattn.DT_FLAG_FORCE_GENERIC)
+    out = torch.zeros_like(q)
+    p = dtattn.make_params(q, k, v, out, D ** -0.5, mask=mask)
+    need = dtattn.workspace_size(p)
+    assert (need > 0) == asked
+    scratch = torch.full((need + 256,), 0xff, dtype=torch.uint8, device=DEV)
+    s = torch.cuda.current_stream().cuda_stream
+    for ptr, nbytes in ((None, 0), (scratch.data_ptr(), max(need - 1, 0)), (scratch.data_ptr(), need)):
+        out.zero_()
+        assert dtattn.lib().dt_sdpa_forward(ctypes.byref(p), ctypes.c_void_p(ptr), nbytes, ctypes.c_void_p(s)) == dtattn.DT_OK
+        torch.cuda.synchronize()
+        assert torch.equal(out, want) or nbytes == need > 0
+        assert float((out.float() - want.float()).abs().max()) < 2e-3
+    assert bool((scratch[:4096] == 0xff).all()) and bool((scratch[need:] == 0xff).all())
