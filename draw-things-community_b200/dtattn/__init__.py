@@ -226,8 +226,9 @@ def _pack_params(q, k, v, o, scale, is_causal, mask, lse, flags, sinks, sliding_
     else:
         max_seq_q = max_seq_k = 0
     return _PACK_SDPA.pack(B, Sq, Sk, Hq, Hkv, D, _DTYPES[q.dtype], _f32(scale), 1 if is_causal else 0, int(flags) & 0xffffffff,
-                           *_quad(q), *_quad(k), *_quad(v), *_quad(o), *mask_fields, lse_ptr, sinks_ptr, _i32(sliding_window),
-                           n_seq, _i32(max_seq_q), _i32(max_seq_k), offs_q, offs_k)
+                           *_quad(q), *_quad(k), *_quad(v), *_quad(o), *mask_fields, lse_ptr, sinks_ptr,
+                           0 if sliding_window == 0 else _i32(sliding_window), n_seq, 0 if max_seq_q == 0 else _i32(max_seq_q),
+                           0 if max_seq_k == 0 else _i32(max_seq_k), offs_q, offs_k)
 
 
 def make_params(q, k, v, o, scale, is_causal=False, mask=None, lse=None, flags=0, sinks=None, sliding_window=0,
@@ -469,8 +470,8 @@ def sparse_indexed_attention(q, k_raw, v_raw, k_comp, v_comp, selected, scale, s
         lse_ptr = lse.data_ptr()
     p = SparseIndexedParams.from_buffer_copy(_PACK_SPARSE.pack(
         B, Sq, Hq, k_raw.shape[2], D, k_raw.shape[1], Sc, n_selected, _DTYPES[q.dtype], _f32(scale), 1 if is_causal else 0,
-        _i32(sliding_window), *_quad(q), *_quad(out), *_quad(k_raw), *_quad(v_raw), *comp[0], *comp[1], *sel, sinks_ptr, lse_ptr,
-        int(flags) & 0xffffffff))
+        0 if sliding_window == 0 else _i32(sliding_window), *_quad(q), *_quad(out), *_quad(k_raw), *_quad(v_raw), *comp[0], *comp[1],
+        *sel, sinks_ptr, lse_ptr, int(flags) & 0xffffffff))
     s = _stream_of(q.device, stream)
     _check(lib().dt_sparse_indexed_attention(ctypes.byref(p), ctypes.c_void_p(s)), "dt_sparse_indexed_attention")
     return out
