@@ -444,7 +444,8 @@ int dt_sdpa_forward_host(const dt_sdpa_params* ph) {
       return t.stride_h == p.D && t.stride_s >= (int64_t)H * p.D && (p.B == 1 || t.stride_b == (int64_t)S * t.stride_s);
     };
     const bool big = nq + nk + nv >= (size_t)(16u << 20);
-    // (a call whose work is cut over the SMs has few query rows to send back: it goes in one piece, cut the same way)
+    // (a call whose work is cut over the SMs goes in one piece, cut the same way: 256 x 16384, 32 / 8 heads of 128, pinned: 1440 us,
+    // in pieces of heads, uncut, 2255 us)
     const bool pipelined = big && !p.lse && choose(p) == kPrefill && wsb == 0 && regular(p.q, p.Sq, p.Hq) &&
                            regular(p.k, p.Sk, p.Hkv) && regular(p.v, p.Sk, p.Hkv) && regular(p.o, p.Sq, p.Hq);
     if (pipelined && !g_hs.s_in) {

@@ -50,13 +50,14 @@ bool decode_supported(const dt_sdpa_params& p);
 size_t decode_workspace_bytes(const dt_sdpa_params& p);
 int launch_decode(const dt_sdpa_params& p, void* workspace, size_t bytes, cudaStream_t stream);
 
-// TMA + tcgen05 flash attention: fp16/bf16, D <= 128 (a multiple of 8), optional 16-byte aligned additive mask.
+// TMA + tcgen05 flash attention: fp16/bf16, D <= 256 (a multiple of 8), optional 16-byte aligned additive mask.
 bool prefill_supported(const dt_sdpa_params& p);
 // extra_outputs: up to 7 more [B,Sq,Hq,D] views with the same strides as p.o (other GPUs' buffers in the
 // head-sharded mode) that receive a copy of every O tile.
 int launch_prefill(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra_outputs = nullptr, int n_extra = 0,
                    void* workspace = nullptr, size_t workspace_bytes = 0);
-// Scratch of the masked variant: one byte per (32 query rows x 64 keys) patch of the mask, "has a non-zero entry".
+// Scratch of the masked variant (needed): one byte per (32 query rows x 64 keys) patch of the mask, "has a non-zero entry";
+// and of a call that is cut over the SMs (optional): its shares.
 size_t prefill_workspace_bytes(const dt_sdpa_params& p);
 
 // The masked operator with mask rows that are not 16-byte aligned: the same kernel behind a pass that copies the mask to

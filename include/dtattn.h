@@ -120,17 +120,22 @@ int dt_abi_version(void);
  * SwiftLLM/Sources/Models/Qwen3_5.swift:193-196 (GQA decode over the KV cache).
  */
 
-/* Bytes of scratch dt_sdpa_forward needs for these params (0 is a valid answer).  Where dt_sdpa_kernel_name says
-   "generic" the scratch is optional (any contents): with it the plain fp32 operator and masks of
-   unaligned rows run on the tensor cores, without it, or with less, on the CUDA cores. */
+/* Bytes of scratch dt_sdpa_forward has a use for with these params (0 is a valid answer).
+   Needed (DT_WORKSPACE without it): "decode_splitkv" (zeroed once, see dt_sdpa_workspace_init) and, of
+   "prefill_tcgen05", calls with a mask.
+   Optional (any contents; without it, or with less, the call takes the other way): "generic" calls that ask for
+   some, which are the plain fp32 operator and masks of unaligned rows, run on the tensor cores with it and on the
+   CUDA cores without; "prefill_tcgen05" calls without a mask that ask for some, few query rows behind many keys,
+   are cut over the SMs with it, which adds in another order (last-bit differences). */
 int dt_sdpa_workspace_size(const dt_sdpa_params* p, size_t* bytes);
 /* Zero the workspace's ticket counters.  Call once after allocating a workspace (and again after any
    call that returned an error); dt_sdpa_forward leaves them zero on success. */
 int dt_sdpa_workspace_init(void* workspace, size_t bytes, void* cuda_stream);
 /* O = softmax(scale * Q K^T [+ mask] [causal]) V on `cuda_stream` of the current device. */
 int dt_sdpa_forward(const dt_sdpa_params* p, void* workspace, size_t workspace_bytes, void* cuda_stream);
-/* Which kernel dt_sdpa_forward would pick: writes a short static name ("prefill_tcgen05",
-   "decode_splitkv", "generic") to *name. */
+/* Which kernel dt_sdpa_forward would pick without optional scratch: writes a short static name ("prefill_tcgen05",
+   "crossattn_short", "decode_splitkv", "generic") to *name.  "generic" together with a dt_sdpa_workspace_size
+   above 0: the tensor cores, where that scratch is given. */
 int dt_sdpa_kernel_name(const dt_sdpa_params* p, const char** name);
 
 /* Same operator with HOST tensors: copies q, k, v (and sinks) to device scratch it owns, runs
