@@ -18,11 +18,11 @@
 //   warp 9      TMEM allocation, TMA of the next token's queries
 // Why two parts: a weight of 16 bits relative to a maximum that is older than the tile makes the result's error against 64 bits
 // 4 % larger than relative to the running maximum (2.07e-3 -> 2.15e-3 in bf16 for N(0,1) scores; 20 % where few keys carry the
-// weight), and rescaling O^T for every growth costs as much as the second part's products (659 and 660 us where one part and the
+// weight), and rescaling O^T for every growth costs more than the second part's products (659 and 608 us where one part and the
 // older maximum take 514).  With two parts the error is the rounding of the result, 1.66e-3.
-// Measured (prompt of 4096 tokens, 64 heads of 512, 128 + up to 512 keys each): 2110 us with warp-level MMAs, 660 us here
-// (415 TFLOP/s of visible work).  Bound: shared-memory reads of the products' operands (a second part's M = 128, N = 64 MMA takes 52
-// cycles where its share of the tensor pipe is 32) and the softmax warps' chain.
+// Measured (prompt of 4096 tokens, 64 heads of 512, 128 + up to 512 keys each): 2110 us with warp-level MMAs, 608 us here
+// (451 TFLOP/s of visible work).  Bound: the tensor pipe's operand reads from shared memory and the softmax warps' chain.  The
+// products of one accumulator follow one another: with the accumulators in turn the call took 660 us.
 // What set the time on the way: the gather.  With asynchronous 16-byte copies of four warps it moved 11 bytes per cycle
 // (1775 us), with all the TMA loads issued by one warp, 68 cycles each, 7 (1446 us).
 // Every mbarrier wait is bounded.  The softmax warps also meet at a named barrier once per tile; a wait that ran out is part
@@ -282,11 +282,11 @@ sparse_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         ptx::tc_fence_after();
         const uint64_t vd = vt_desc + (uint64_t)(vbuf * (kTileBytes >> 4));
 #pragma unroll
-        for (int part = 0; part < 2; ++part)  // the weights' high parts, then what those leave over
+        for (int mt = 0; mt < kMaxD / 128; ++mt)
 #pragma unroll
           for (int ks = 0; ks < kTK / 16; ++ks)
 #pragma unroll
-            for (int mt = 0; mt < kMaxD / 128; ++mt)
+            for (int part = 0; part < 2; ++part)  // the weights' high parts and what those leave over
               if (2 * mt < subs)
                 ptx::mma_ss_on(on, tmem + mt * kHeads, vd + (uint64_t)((mt * 2 * kSub + ks * 2048) >> 4),
                                p_desc + (uint64_t)((part * kPBytes + ks * 32) >> 4), idesc_pv, (t > 0 || part > 0 || ks > 0) ? 1u : 0u);
