@@ -542,8 +542,8 @@ bool sparse_tcgen05_supported(const dt_sparse_indexed_params& p, bool same_kv) {
   if ((!raw && !comp) || (raw && !key_map_fits(p.k_raw, p.Sr, p)) || (comp && !key_map_fits(p.k_comp, p.Sc, p))) return false;
   // Few tokens leave SMs idle here, and the warp-level kernel spreads a token's keys over a cluster of CTAs, up to about 300 of
   // them (four per token and 64 heads for 16 tokens, two for 19).  Tokens x 64 heads, 640 keys each, there and here: head dim
-  // 512: 8: 21 us (24 here with one part per weight), 16: 30.6 and 28.6, 18: 55 and 28.6, 64: 76 and 28; 4096 keys: 16: 134 and 140 us,
-  // 18: 248 and 140.  Head dim 256: 16: 19.8 and 23.7, 18: 21.6 and 24.0, 20: 34.6 and 24.1; 2176 keys: 18: 57 and 65, 20: 98 and 65.
+  // 512: 8: 21.5 us and (like 16) 27, 16: 30.8 and 27.2, 18: 55 and 27.1, 64: 76 and 27; 4096 keys: 16: 134 and 135 us, 18: 248 and
+  // 135.  Head dim 256: 16: 19.9 and 20.5, 18: 21.5 and 20.5, 20: 34.1 and 20.5; 4096 keys: 16: 82 and 95, 18: 91 and 95, 20: 156 and 95.
   const long long items = (long long)p.B * p.Sq * p.Hq / kHeads;
   return items >= (p.D == 256 ? 19 : 16) && items < (1LL << 30);
 }
