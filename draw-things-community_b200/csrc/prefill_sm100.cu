@@ -102,7 +102,7 @@ struct PrefillArgs {
   // n_slots on (fewer than one round) are pairs of tiles taken tile by tile; n_places counts those tiles too.
   int n_slots;
   int n_places;
-  // The cut kernel: an item's K/V blocks are the work of n_splits CTAs in turn, whose shares of the result go to `part`;
+  // The cut kernel: an item's K/V blocks are cut into n_splits runs, whose shares of the result go to `part`;
   // cut_combine_kernel puts them together.
   int n_splits;           // (times an item's K/V blocks below 2^31)
   float* part;            // [n_items * n_splits][kBM / 32][D + 2][32]: weights' maximum, their sum, O
@@ -460,18 +460,20 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
     return item_at(order, tile);
   };
-  // This CTA's work in turn: its whole items and then a single tile, or (cut) one run of an item's blocks.  A kernel of its own
+  // This CTA's work in turn: its whole items and then a single tile, or (cut) runs of items' blocks.  A kernel of its own
   // for cut calls, because what they need costs the others up to 1 us at the start and 2 % in the loops of the 256-wide variant.
   auto next_work = [&](int& next, Item& w) -> bool {
     if constexpr (kCut) {
-      if (next != (int)blockIdx.x) return false;
-      next += gridDim.x;
-      const int order = blockIdx.x / a.n_splits, c = blockIdx.x - order * a.n_splits;
-      w = item_at(order, -1);
-      const int n = w.nkv;
-      w.j0 = cut_at(a, n, c);
-      w.nkv = cut_at(a, n, c + 1) - w.j0;
-      return w.nkv > 0;
+      while (next < a.n_items * a.n_splits) {
+        const int order = next / a.n_splits, c = next - order * a.n_splits;
+        next += gridDim.x;
+        w = item_at(order, -1);
+        const int n = w.nkv;
+        w.j0 = cut_at(a, n, c);
+        w.nkv = cut_at(a, n, c + 1) - w.j0;
+        if (w.nkv > 0) return true;  // (empty: an item with fewer blocks than runs)
+      }
+      return false;
     } else {
       while (next < a.n_places) {
         w = decode_item(next);
@@ -1067,7 +1069,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       if (probe) stamp(a, 16 * n_item + 10);
       ptx::tc_fence_after();
       if constexpr (kCut) {  // the run's share: (maximum, sum, O)
-        float* mine = share_of<D>(a, blockIdx.x, warp & 3);
+        float* mine = share_of<D>(a, walk - (int)gridDim.x, warp & 3);
         __stcg(mine + lane, m_used);
         __stcg(mine + 32 + lane, l);
 #pragma unroll 1
@@ -1087,7 +1089,8 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                                __uint_as_float(ov[4 * i + 3])));
         }
         ptx::tc_fence_before();
-        break;
+        ++n_item;
+        continue;
       }
       if (a.sinks && row < w.sq) {
         // attention sink: one more score without a value row joins the denominator (l and O are relative to m_used)
@@ -1204,7 +1207,7 @@ struct Plan {
   int item_rows, n_q, n_items;
   int n_whole;           // items taken whole, in full rounds
   int n_single;          // the items behind them as single tiles (0: they are whole too)
-  int n_splits;          // CTAs per item of a cut call (0: not cut)
+  int n_splits;          // runs per item of a cut call (0: not cut)
 };
 
 long long blocks_of_item(const dt_sdpa_params& p, int item_rows, int qt) {
@@ -1243,7 +1246,7 @@ Plan make_plan(const dt_sdpa_params& p, int tiles) {
     return r;
   }
   // A call that leaves half of the SMs without any item (a short chunk of queries behind a long prefix): every item's K/V blocks
-  // cut into as many equal runs as there are SMs per item, when that saves at least kCutGain blocks' time.  A run lies in one
+  // cut into equal runs, when that saves at least kCutGain blocks' time.  A run lies in one
   // item: with runs of equal length over all SMs, whatever items they fell into, there were up to twice as many shares to write
   // and read (400 x 1536, 16 / 4 heads of 256: 24.3 us uncut, 32.2 us so, 22.4 us by items).  Measured against the uncut call (Sq x
   // Sk, time uncut / cut, saving 4 blocks): 24 heads of 64, 128 x 1024 causal: 18.2 / 14.7 us; 6 heads of 256, 128 x 1024: 18.5 /
@@ -1253,8 +1256,21 @@ Plan make_plan(const dt_sdpa_params& p, int tiles) {
   constexpr int kMinRun = 4;
   if (2 * r.n_items > sms || p.sliding_window > 0) return r;
   const long long longest = blocks_of_item(p, r.item_rows, r.n_q - 1);  // (the last rows see the most)
-  const long long by_blocks = longest / kMinRun, splits = by_blocks < sms / r.n_items ? by_blocks : sms / r.n_items;
-  if (splits < 2 || longest * splits >= (1LL << 31) || longest - (longest + splits - 1) / splits < kCutGain) return r;
+  // How many: one run per SM, or, where the items divide the SMs badly, up to four shorter ones (52 heads of 128, 128 x 16000: 2
+  // runs each, one per CTA, 111 us; 5 each, up to two per CTA, 102; 50 heads of 64: 108 and 95).  In quarters of a block's time a
+  // run's own start and end are about kRunCost, a share to add kShareCost (6 or 20 and 2 in their place: within 1 %).
+  constexpr int kRunCost = 12, kShareCost = 1;
+  long long splits = 0, saved = 0, best = 0;
+  for (long long n = 2; n <= longest / kMinRun && r.n_items * n <= 4 * sms && longest * n < (1LL << 31); ++n) {
+    const long long rounds = (r.n_items * n + sms - 1) / sms, per = (longest + n - 1) / n;
+    const long long cost = rounds * (4 * per + kRunCost) + n * kShareCost;
+    if (splits == 0 || cost < best) {
+      splits = n;
+      best = cost;
+      saved = longest - rounds * per;
+    }
+  }
+  if (splits == 0 || saved < kCutGain) return r;
   r.n_splits = (int)splits;
   return r;
 }
@@ -1352,7 +1368,8 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
     a.part = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + align256(split_at));
     auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, true>;
     DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
-    kern<<<plan.n_items * plan.n_splits, kThreads, C::kSmemBytes, stream>>>(mq, mk, mv, mo, a);
+    const int runs = plan.n_items * plan.n_splits;
+    kern<<<runs < n_sm ? runs : n_sm, kThreads, C::kSmemBytes, stream>>>(mq, mk, mv, mo, a);
     DT_CUDA_TRY(cudaGetLastError());
     cut_combine_kernel<T, D><<<dim3(plan.n_items * (kBM / 32), (p.D + 63) / 64), 256, 0, stream>>>(a);
     DT_CUDA_TRY(cudaGetLastError());

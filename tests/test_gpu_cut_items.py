@@ -30,6 +30,9 @@ def forward(dtattn, p, scratch):
     (1, 513, 2900, 4, 1, 256, True, "", torch.float16),        # a last tile of one row
     (1, 1200, 1200, 7, 1, 80, True, "sinks", torch.float16),   # as many keys as queries: the first levels are short
     (1, 2000, 2000, 1, 1, 64, True, "", torch.bfloat16),       # items with fewer key blocks than runs
+    (1, 100, 8192, 50, 2, 64, False, "sinks", torch.float16),  # several runs per CTA, the CTAs not all as many
+    (1, 100, 8200, 50, 1, 256, True, "", torch.bfloat16),
+    (1, 128, 8192, 50, 2, 128, True, "mask", torch.bfloat16),
     (1, 200, 1600, 4, 2, 128, True, "mask", torch.bfloat16),   # masked, aligned rows
     (1, 200, 1601, 4, 2, 64, False, "mask", torch.float16)])   # masked, copied rows
 def test_against_the_oracle_and_the_uncut_call(dtattn, case):
