@@ -550,6 +550,245 @@ sparse_mma_kernel(const SparseArgs a, const SparseMmaExtra x) {
   ptx::cluster_sync();  // nobody leaves while its shared memory is still being read
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// Few tokens with at most 640 keys each (the decode step: a window of 128 and 512 selected rows).  What costs there is the
+// chain of one token's steps, so every step is taken once: a cluster of eight CTAs shares a token's keys, each CTA (one head
+// group of 16, eight warps) gathers its up to 80 keys in one go and works on all of them together:
+//   S: warp w multiplies head dims [w D / 8, (w + 1) D / 8) for all keys (independent accumulators, Q fragments read once), the
+//      eight partial scores meet in shared memory, where half a warp per query row adds them and takes the softmax;
+//   O: warp w takes the same head dims of P V and stores its accumulators straight into the shared memory of CTA w of the
+//      cluster, which owns these columns: one cluster barrier later the eight shares are added from local memory.
+// Bound: latency (launch, index, row, two products, exchange).  64 heads of 512, 128 + 512 keys, one token, in a graph: 17.8 us in
+// sparse_mma_kernel (three tiles of 32 keys in turn per CTA, four warps, shares read from the other CTAs), 8.5 us here.
+constexpr int kOnceSplit = 8;    // CTAs of a cluster, and warps of a CTA
+constexpr int kOnceKeys = 80;    // keys per CTA
+constexpr int kOncePitch = 88;   // of the partial scores (words) and of P (16-bit): rows on distinct banks
+
+template <int D>
+constexpr size_t once_smem(bool same_kv) {
+  return 2 * ((size_t)16 * (D + 8) + (size_t)(same_kv ? 1 : 2) * kOnceKeys * (D + 8) + 16 * kOncePitch) +
+         4 * ((size_t)kOnceSplit * 16 * kOncePitch + (size_t)16 * D + 2 * kOnceSplit * 16 + kOnceKeys);
+}
+static_assert(once_smem<512>(true) <= 227 * 1024 && once_smem<256>(false) <= 227 * 1024, "shared memory");
+
+template <typename T, int D>
+__global__ void __launch_bounds__(32 * kOnceSplit) sparse_once_kernel(const SparseArgs a, const int per, const int same_kv) {
+  constexpr bool kBf16 = !std::is_same<T, __half>::value;
+  constexpr int P = D + 8, DW = D / kOnceSplit, KS = DW / 16, NT = kOnceKeys / 8;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float* Sp = reinterpret_cast<float*>(smem_raw);                        // [8 warps][16][kOncePitch] partial scores
+  float* Or = Sp + kOnceSplit * 16 * kOncePitch;                         // [8 CTAs][16][DW] this CTA's columns, from every CTA
+  float* mr = Or + 16 * D;                                               // [8 CTAs][16] row maxima
+  float* lr = mr + kOnceSplit * 16;                                      // [8 CTAs][16] row sums
+  int* codes = reinterpret_cast<int*>(lr + kOnceSplit * 16);             // [kOnceKeys] non-zero: a key
+  uint16_t* Qs = reinterpret_cast<uint16_t*>(codes + kOnceKeys);         // [16][P]
+  uint16_t* Pex = Qs + 16 * P;                                           // [16][kOncePitch]
+  uint16_t* Ks = Pex + 16 * kOncePitch;                                  // [kOnceKeys][P]
+  uint16_t* Vs = same_kv ? Ks : Ks + kOnceKeys * P;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tg = lane & 3;
+  const int i = blockIdx.x / kOnceSplit, rank = blockIdx.x % kOnceSplit, b = blockIdx.z;
+  const int G = a.Hq / a.Hkv, ng = (G + 15) / 16;
+  const int kvh = blockIdx.y / ng, hg = blockIdx.y - kvh * ng, h0 = kvh * G + hg * 16, nh = min(16, G - hg * 16);
+  constexpr int chunks = D / 8;  // 16-byte pieces of a row
+
+  ptx::cluster_arrive();  // (waited for before anything is stored into another CTA)
+  {
+    const T* q = reinterpret_cast<const T*>(a.q) + b * a.q_sb + (int64_t)i * a.q_ss + (int64_t)h0 * a.q_sh;
+#pragma unroll
+    for (int c = tid; c < 16 * chunks; c += 32 * kOnceSplit) {
+      const int r = c / chunks, ch = c - r * chunks;
+      ptx::cp_async_16(ptx::smem_u32(Qs + r * P + ch * 8), r < nh ? (const void*)(q + (int64_t)r * a.q_sh + ch * 8) : (const void*)q,
+                       r < nh ? 16 : 0);
+    }
+  }
+  const long long last = a.is_causal ? (long long)i + (a.Sr - a.Sq) : (long long)a.Sr - 1;
+  long long first = a.window > 0 ? (long long)i + (a.Sr - a.Sq) - a.window + 1 : 0;
+  if (first < 0) first = 0;
+  const long long last_c = last < (long long)a.Sr - 1 ? last : (long long)a.Sr - 1;
+  const int n_raw = last_c >= first ? (int)(last_c - first + 1) : 0;
+  const int n_keys = n_raw + (a.Sc > 0 ? a.n_sel : 0);
+  const int32_t* sel = a.selected ? a.selected + b * a.sel_sb + (int64_t)i * a.sel_sq : nullptr;
+  {
+    // Warp w gathers keys w, w + 8, ... of this CTA's share: lane l looks up key w + 8 l, all lanes copy every row.
+    const T* kr = reinterpret_cast<const T*>(a.k_raw) + b * a.kr_sb + kvh * a.kr_sh;
+    const T* vr = reinterpret_cast<const T*>(a.v_raw) + b * a.vr_sb + kvh * a.vr_sh;
+    const T* kc = reinterpret_cast<const T*>(a.k_comp) + b * a.kc_sb + kvh * a.kc_sh;
+    const T* vc = reinterpret_cast<const T*>(a.v_comp) + b * a.vc_sb + kvh * a.vc_sh;
+    const int n_mine = per / kOnceSplit;
+    int code = -1;  // -1 no key, >= 0 raw row, <= -2 compressed row -(code + 2)
+    if (lane < n_mine) {
+      const int key = rank * per + warp + kOnceSplit * lane;
+      if (key < n_raw) {
+        code = (int)(first + key);
+      } else if (key < n_keys) {
+        const int idx = __ldg(sel + (key - n_raw));
+        if (idx >= 0 && idx < a.Sc) code = -(idx + 2);
+      }
+      codes[warp + kOnceSplit * lane] = code != -1;
+    }
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      if (n >= n_mine) break;
+      const int c = __shfl_sync(0xffffffffu, code, n);
+      const T* ksrc = reinterpret_cast<const T*>(a.q);  // any valid address when nothing is copied (the raw tensors may be absent)
+      const T* vsrc = ksrc;
+      if (c >= 0) {
+        ksrc = kr + (int64_t)c * a.kr_ss;
+        vsrc = vr + (int64_t)c * a.vr_ss;
+      } else if (c <= -2) {
+        ksrc = kc + (int64_t)(-(c + 2)) * a.kc_ss;
+        vsrc = vc + (int64_t)(-(c + 2)) * a.vc_ss;
+      }
+      const int row = warp + kOnceSplit * n;
+#pragma unroll
+      for (int ch = lane; ch < chunks; ch += 32) {
+        const int e = c != -1 ? ch * 8 : 0;
+        ptx::cp_async_16(ptx::smem_u32(Ks + row * P + ch * 8), ksrc + e, c != -1 ? 16 : 0);
+        if (!same_kv) ptx::cp_async_16(ptx::smem_u32(Vs + row * P + ch * 8), vsrc + e, c != -1 ? 16 : 0);
+      }
+    }
+  }
+  ptx::cp_async_commit();
+  ptx::cp_async_wait<0>();
+  __syncthreads();
+
+  const int nt_on = per / 8;  // n-tiles of 8 keys (even)
+  {
+    float sc[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) sc[n][e] = 0.f;
+    const uint32_t q_addr = ptx::smem_u32(Qs) + (uint32_t)(((lane & 15) * P + (lane >> 4) * 8 + warp * DW) * 2);
+    const uint32_t k_addr = ptx::smem_u32(Ks) + (uint32_t)(((lane & 7) * P + (lane >> 3) * 8 + warp * DW) * 2);
+    uint32_t qa[KS][4];
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) ptx::ldmatrix_x4(qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], q_addr + (uint32_t)(ks * 32));
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      if (n >= nt_on) break;
+#pragma unroll
+      for (int ks = 0; ks < KS; ks += 2) {
+        uint32_t b0, b1, b2, b3;
+        ptx::ldmatrix_x4(b0, b1, b2, b3, k_addr + (uint32_t)(n * 8 * P * 2 + ks * 32));
+        ptx::mma_m16n8k16<kBf16>(sc[n], qa[ks], b0, b1);
+        ptx::mma_m16n8k16<kBf16>(sc[n], qa[ks + 1], b2, b3);
+      }
+    }
+    float* sp = Sp + (warp * 16 + g) * kOncePitch + 2 * tg;
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      if (n >= nt_on) break;
+      *reinterpret_cast<float2*>(sp + n * 8) = make_float2(sc[n][0], sc[n][1]);
+      *reinterpret_cast<float2*>(sp + 8 * kOncePitch + n * 8) = make_float2(sc[n][2], sc[n][3]);
+    }
+  }
+  __syncthreads();
+  ptx::cluster_wait();
+  {
+    // softmax over this CTA's keys: half a warp per query row, every 16th key per lane
+    const int row = warp * 2 + (lane >> 4), l16 = lane & 15;
+    float s[NT / 2], m = -INFINITY;
+#pragma unroll
+    for (int n = 0; n < NT / 2; ++n) {
+      s[n] = -INFINITY;
+      if (n * 16 >= per) continue;
+      const int key = n * 16 + l16;
+      float x[kOnceSplit];
+#pragma unroll
+      for (int w = 0; w < kOnceSplit; ++w) x[w] = Sp[(w * 16 + row) * kOncePitch + key];
+      const float sum = ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
+      if (codes[key]) s[n] = sum * a.scale_log2;
+      m = fmaxf(m, s[n]);
+    }
+#pragma unroll
+    for (int off = 8; off; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+    const float ref = m == -INFINITY ? 0.f : m;  // (no key, or nothing but NaN)
+    float l = 0.f;
+#pragma unroll
+    for (int n = 0; n < NT / 2; ++n) {
+      if (n * 16 >= per) continue;
+      const float p = exp2f(s[n] - ref);
+      l += p;
+      const T pt = from_float<T>(p);
+      Pex[row * kOncePitch + n * 16 + l16] = *reinterpret_cast<const uint16_t*>(&pt);
+    }
+#pragma unroll
+    for (int off = 8; off; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+    if (l16 < kOnceSplit) {
+      const uint32_t at = (uint32_t)(rank * 16 + row) * 4u;
+      ptx::st_cluster_f32(ptx::map_to_cta(ptx::smem_u32(mr) + at, (uint32_t)l16), m);
+      ptx::st_cluster_f32(ptx::map_to_cta(ptx::smem_u32(lr) + at, (uint32_t)l16), l);
+    }
+  }
+  __syncthreads();
+  {
+    float acc[DW / 8][4];
+#pragma unroll
+    for (int n = 0; n < DW / 8; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
+    const uint32_t p_addr = ptx::smem_u32(Pex) + (uint32_t)(((lane & 15) * kOncePitch + (lane >> 4) * 8) * 2);
+    const uint32_t v_addr = ptx::smem_u32(Vs) + (uint32_t)((((lane & 7) + ((lane >> 3) & 1) * 8) * P + warp * DW + (lane >> 4) * 8) * 2);
+#pragma unroll
+    for (int k2 = 0; k2 < NT / 2; ++k2) {
+      if (k2 * 16 >= per) break;
+      uint32_t pa[4];
+      ptx::ldmatrix_x4(pa[0], pa[1], pa[2], pa[3], p_addr + (uint32_t)(k2 * 32));
+#pragma unroll
+      for (int n = 0; n < DW / 8; n += 2) {
+        uint32_t b0, b1, b2, b3;
+        ptx::ldmatrix_x4_trans(b0, b1, b2, b3, v_addr + (uint32_t)(n * 16 + k2 * 16 * P * 2));
+        ptx::mma_m16n8k16<kBf16>(acc[n], pa, b0, b1);
+        ptx::mma_m16n8k16<kBf16>(acc[n + 1], pa, b2, b3);
+      }
+    }
+    // these columns are CTA `warp`'s
+    const uint32_t dst = ptx::map_to_cta(ptx::smem_u32(Or), (uint32_t)warp) + (uint32_t)((rank * 16 + g) * DW + 2 * tg) * 4u;
+#pragma unroll
+    for (int n = 0; n < DW / 8; ++n) {
+      ptx::st_cluster_f32x2(dst + (uint32_t)(n * 32), acc[n][0], acc[n][1]);
+      ptx::st_cluster_f32x2(dst + (uint32_t)(8 * DW * 4 + n * 32), acc[n][2], acc[n][3]);
+    }
+  }
+  ptx::cluster_sync();  // every share of this CTA's columns has arrived, and nobody is stored into any more
+  const int row = tid / (DW / 4), c4 = tid - row * (DW / 4);
+  if (row < nh) {
+    const T* sinks = reinterpret_cast<const T*>(a.sinks);
+    float ms[kOnceSplit], m = -INFINITY;
+#pragma unroll
+    for (int r = 0; r < kOnceSplit; ++r) {
+      ms[r] = mr[r * 16 + row];
+      m = fmaxf(m, ms[r]);
+    }
+    const float sl = sinks ? to_float(sinks[h0 + row]) * kLog2e : -INFINITY;
+    const float m_f = fmaxf(m, sl);
+    float l = sl == -INFINITY ? 0.f : exp2f(sl - m_f);  // the sink: a score without a value row
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < kOnceSplit; ++r) {
+      const float wgt = ms[r] == -INFINITY ? 0.f : exp2f(ms[r] - m_f);  // (0 * NaN keeps a share's NaN)
+      const float4 x = *reinterpret_cast<const float4*>(Or + (r * 16 + row) * DW + c4 * 4);
+      l += wgt * lr[r * 16 + row];
+      o.x += wgt * x.x; o.y += wgt * x.y; o.z += wgt * x.z; o.w += wgt * x.w;
+    }
+    const float inv = l > 0.f ? 1.f / l : 0.f;
+    const int col = rank * DW + c4 * 4;
+    T* dst = reinterpret_cast<T*>(a.o) + b * a.o_sb + (int64_t)i * a.o_ss + (int64_t)(h0 + row) * a.o_sh + col;
+    uint2 pk;
+    if constexpr (kBf16) {
+      pk.x = ptx::cvt_pack_bf16(o.x * inv, o.y * inv);
+      pk.y = ptx::cvt_pack_bf16(o.z * inv, o.w * inv);
+    } else {
+      pk.x = ptx::cvt_pack_f16(o.x * inv, o.y * inv);
+      pk.y = ptx::cvt_pack_f16(o.z * inv, o.w * inv);
+    }
+    *reinterpret_cast<uint2*>(dst) = pk;
+    if (a.lse && col == 0) a.lse[((int64_t)b * a.Hq + h0 + row) * a.Sq + i] = l > 0.f ? m_f * kLn2 + logf(l) : -INFINITY;
+  }
+}
+
 // What the tensor-core variant needs: 16-bit tensors, head dim a multiple of 64, every row it gathers 16-byte aligned.
 bool sparse_mma_supported(const dt_sparse_indexed_params& p) {
   if (p.dtype != DT_F16 && p.dtype != DT_BF16) return false;
@@ -559,6 +798,33 @@ bool sparse_mma_supported(const dt_sparse_indexed_params& p) {
                                 t.stride_h % 8 == 0);
   };
   return ok(p.q) && ok(p.o) && ok(p.k_raw) && ok(p.v_raw) && ok(p.k_comp) && ok(p.v_comp);
+}
+
+// The keys that a token may have
+int most_keys(const dt_sparse_indexed_params& p) {
+  return (p.sliding_window > 0 ? (p.sliding_window < p.Sr ? p.sliding_window : p.Sr) : p.Sr) + (p.Sc > 0 ? p.n_selected : 0);
+}
+
+template <typename T, int D>
+int launch_sparse_once(const dt_sparse_indexed_params& p, const SparseArgs& a, bool same_kv, cudaStream_t stream) {
+  const int per = (most_keys(p) + kOnceSplit * 16 - 1) / (kOnceSplit * 16) * 16, ng = (p.Hq / p.Hkv + 15) / 16;
+  const size_t smem = once_smem<D>(same_kv);
+  auto kern = sparse_once_kernel<T, D>;
+  DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(p.Sq * kOnceSplit), (unsigned)(p.Hkv * ng), (unsigned)p.B);
+  cfg.blockDim = dim3(32 * kOnceSplit);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kOnceSplit;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  DT_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a, per, same_kv ? 1 : 0));
+  return DT_OK;
 }
 
 template <typename T, int TK>
@@ -572,7 +838,7 @@ int launch_sparse_mma_tk(const dt_sparse_indexed_params& p, const SparseArgs& a,
   const long long ctas = (long long)p.Sq * ng * p.Hkv * p.B;
   // few tokens (the decode step): a token's keys are shared out over a cluster of CTAs, as long as every CTA still gets
   // a few tiles and the grid stays within about two rounds over the SMs
-  const int keys = (p.sliding_window > 0 ? (p.sliding_window < p.Sr ? p.sliding_window : p.Sr) : p.Sr) + (p.Sc > 0 ? p.n_selected : 0);
+  const int keys = most_keys(p);
   const int tiles = (keys + TK - 1) / TK;
   int split = 1;
   const int sms = device_sm_count();
@@ -614,7 +880,12 @@ int launch_sparse_mma_t(const dt_sparse_indexed_params& p, const SparseArgs& a, 
     const int st = launch_sparse_tcgen05(p, stream);
     if (st != DT_UNSUPPORTED) return st;  // (views that no tensor map describes, expanded queries for one: nothing was launched)
   }
-  const int keys = (p.sliding_window > 0 ? (p.sliding_window < p.Sr ? p.sliding_window : p.Sr) : p.Sr) + (p.Sc > 0 ? p.n_selected : 0);
+  // Clusters that fit the SMs in one wave (a CTA's 180 KB leave room for one per SM).
+  const int keys = most_keys(p);
+  const long long groups = (long long)p.Hkv * ((p.Hq / p.Hkv + 15) / 16);
+  if ((p.D == 256 || (p.D == 512 && same_kv)) && keys > 0 && keys <= kOnceSplit * kOnceKeys && groups <= 65535 &&
+      kOnceSplit * groups * p.Sq * p.B <= device_sm_count())
+    return p.D == 512 ? launch_sparse_once<T, 512>(p, a, same_kv, stream) : launch_sparse_once<T, 256>(p, a, same_kv, stream);
   if (same_kv && keys >= 256 && (long long)p.Sq * p.B >= 64) return launch_sparse_mma_tk<T, 64>(p, a, stream);
   return launch_sparse_mma_tk<T, 32>(p, a, stream);
 }
