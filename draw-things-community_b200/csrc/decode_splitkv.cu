@@ -66,7 +66,13 @@ struct Cfg {
   // (A deeper ring for grids that leave every CTA an SM of its own was measured on B200 and changed nothing.)
   static constexpr int kStages = D == 64 ? 4 : 3;
   static constexpr int kRingBytes = kStages * kStageBytes;
-  static constexpr int kSmemBytes = kRingBytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
+  static constexpr int kNewBytes = kDimSplit * kWarpTileBytes;  // the decode step's unit of new rows
+  // A step of up to kStageRows new tokens has its norm weights, rotary rows and new rows brought to shared memory together: read
+  // where they are needed, one behind the other, they were four round trips to memory in a row (one token, 32/8 heads of 128, 4096
+  // rows: 13.9 us so, 11.7 now, the attention alone 10.6).
+  static constexpr int kStageRows = 4;
+  static constexpr int kStepBytes = (2 + 3 * kStageRows) * D * 2;
+  static constexpr int kSmemBytes = kRingBytes + kNewBytes + kStepBytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
 };
 
 struct DecodeArgs {
@@ -189,7 +195,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
   const uint32_t ring = (raw + 1023u) & ~1023u;
   uint8_t* ring_ptr = smem_raw + (ring - raw);
   constexpr int nst = C::kStages;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(ring_ptr + C::kRingBytes);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(ring_ptr + C::kRingBytes + C::kNewBytes + C::kStepBytes);
   uint64_t* empty_bar = full_bar + nst;
   __shared__ int s_abort;
   __shared__ int s_is_last;
@@ -238,12 +244,32 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
   const int cq = (lane & 3) * 2;
   // Q fragments (A operand, rows = (query token, group head), k = head dim)
   uint32_t qa[D / 16][4];
+  const bool staged = a.Tn > 0 && a.Tn <= C::kStageRows;
+  T* step_rows = reinterpret_cast<T*>(ring_ptr + C::kRingBytes + C::kNewBytes);  // [q weight][k weight][rotary x 4][new keys x 4][new values x 4]
+  constexpr int kRotAt = 2, kKnAt = 2 + C::kStageRows, kVnAt = 2 + 2 * C::kStageRows;
   if (warp < kConsumerWarps) {
     // Programmatic dependent launch (DT_FLAG_KV_PREFIX_STABLE): this grid may have started while the kernel before
     // it in the stream was still running.  The producer warp streams the K/V prefix at once (the caller guarantees
     // that kernel does not write it); everything else -- Q, the new rows, the workspace, the outputs -- is
     // touched only after the preceding grid has completed.  Without the launch attribute this returns at once.
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (staged) {
+      constexpr int kPieces = D / 8;  // 16 bytes each
+      const int n_rows = 2 + (split == a.nsplit - 1 ? 3 : 1) * a.Tn;
+      for (int c = threadIdx.x; c < n_rows * kPieces; c += kConsumerWarps * 32) {
+        const int r = c / kPieces, col = (c - r * kPieces) * 8;
+        const int kind = r < 2 ? r : 2 + (r - 2) / a.Tn, t = r < 2 ? 0 : (r - 2) % a.Tn;
+        const T* src = nullptr;
+        if (kind == 0) src = reinterpret_cast<const T*>(a.q_norm_w);
+        else if (kind == 1) src = reinterpret_cast<const T*>(a.k_norm_w);
+        else if (kind == 2) src = a.rotary ? reinterpret_cast<const T*>(a.rotary) + b * a.rot_sb + (int64_t)t * a.rot_ss : nullptr;
+        else if (kind == 3) src = reinterpret_cast<const T*>(a.k_new) + b * a.kn_sb + (int64_t)t * a.kn_ss + (int64_t)kvh * a.kn_sh;
+        else src = reinterpret_cast<const T*>(a.v_new) + b * a.vn_sb + (int64_t)t * a.vn_ss + (int64_t)kvh * a.vn_sh;
+        const int at = kind < 2 ? kind : kind == 2 ? kRotAt + t : kind == 3 ? kKnAt + t : kVnAt + t;
+        if (src) ptx::cp_async_16(ptx::smem_u32(step_rows + at * D + col), src + col, 16);
+      }
+      ptx::cp_async_commit();
+    }
     const T* q = reinterpret_cast<const T*>(a.q);
     const T* rot = reinterpret_cast<const T*>(a.rotary);
     const T* p_lo = nullptr;
@@ -252,11 +278,13 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     const T* t_hi = nullptr;
     if (r_lo < a.M) {
       p_lo = q + b * a.q_sb + (int64_t)(r_lo / a.G) * a.q_ss + (int64_t)(kvh * a.G + r_lo % a.G) * a.q_sh;
-      if (rot) t_lo = rot + b * a.rot_sb + (int64_t)(a.Tn - a.Sq + r_lo / a.G) * a.rot_ss;
+      const int t = a.Tn - a.Sq + r_lo / a.G;
+      if (rot) t_lo = staged ? step_rows + (kRotAt + t) * D : rot + b * a.rot_sb + (int64_t)t * a.rot_ss;
     }
     if (r_hi < a.M) {
       p_hi = q + b * a.q_sb + (int64_t)(r_hi / a.G) * a.q_ss + (int64_t)(kvh * a.G + r_hi % a.G) * a.q_sh;
-      if (rot) t_hi = rot + b * a.rot_sb + (int64_t)(a.Tn - a.Sq + r_hi / a.G) * a.rot_ss;
+      const int t = a.Tn - a.Sq + r_hi / a.G;
+      if (rot) t_hi = staged ? step_rows + (kRotAt + t) * D : rot + b * a.rot_sb + (int64_t)t * a.rot_ss;
     }
 #pragma unroll
     for (int ks = 0; ks < D / 16; ++ks) {
@@ -265,9 +293,13 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
       qa[ks][2] = p_lo ? *reinterpret_cast<const uint32_t*>(p_lo + ks * 16 + cq + 8) : 0u;
       qa[ks][3] = p_hi ? *reinterpret_cast<const uint32_t*>(p_hi + ks * 16 + cq + 8) : 0u;
     }
+    if (staged) {  // (the loads of Q above are on their way meanwhile)
+      ptx::cp_async_wait<0>();
+      asm volatile("bar.sync 1, %0;" ::"n"(kConsumerWarps * 32) : "memory");
+    }
     if (a.q_norm_w) {
       // per-row RMSNorm: a row's D elements sit in the four lanes that share lane >> 2
-      const T* gw = reinterpret_cast<const T*>(a.q_norm_w);
+      const T* gw = staged ? step_rows : reinterpret_cast<const T*>(a.q_norm_w);
       float ss_lo = 0.f, ss_hi = 0.f;
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) {
@@ -400,6 +432,79 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     }
   };
 
+  // ---------------- decode step fusion: rotate, append and attend the new K/V rows ----------------
+  // The cache rows that are streamed end at Sk - Tn; the Tn new rows come from k_new / v_new.  The last split of
+  // each (batch, KV head) rotates the new keys, stores new keys and values into the cache for later steps and
+  // attends to them as one more unit built in shared memory of its own, while the first streamed rows are on their way.
+  if (a.k_new != nullptr) {
+    if (split == a.nsplit - 1 && warp < kConsumerWarps && uslot == 0) {
+      const uint32_t tile = ring + C::kRingBytes + dhalf * C::kWarpTileBytes;  // with D = 256 the two warps of the pair build one copy each
+      auto kn = [&](int row) -> const T* {
+        return staged ? step_rows + (kKnAt + row) * D : reinterpret_cast<const T*>(a.k_new) + b * a.kn_sb + (int64_t)row * a.kn_ss + (int64_t)kvh * a.kn_sh;
+      };
+      auto vn = [&](int row) -> const T* {
+        return staged ? step_rows + (kVnAt + row) * D : reinterpret_cast<const T*>(a.v_new) + b * a.vn_sb + (int64_t)row * a.vn_ss + (int64_t)kvh * a.vn_sh;
+      };
+      auto rot = [&](int row) -> const T* {
+        return staged ? step_rows + (kRotAt + row) * D : reinterpret_cast<const T*>(a.rotary) + b * a.rot_sb + (int64_t)row * a.rot_ss;
+      };
+      T* kc = reinterpret_cast<T*>(a.k_cache);
+      T* vc = reinterpret_cast<T*>(a.v_cache);
+      const int t_old = a.stream_keys;
+      constexpr int kChunks = D / 8;  // 16-byte chunks per row
+      // RMSNorm of the new keys: lanes l and l + 16 each sum half of row l's squares; lane l then holds 1 / rms
+      const T* kw = staged && a.k_norm_w ? step_rows + D : reinterpret_cast<const T*>(a.k_norm_w);
+      float inv_row = 1.f;
+      if (kw) {
+        const int row = lane & 15, half = lane >> 4;
+        float ss = 0.f;
+        if (row < a.Tn) {
+          const T* src = kn(row) + half * (D / 2);
+#pragma unroll
+          for (int c = 0; c < D / 16; ++c) {
+            const uint4 x = *reinterpret_cast<const uint4*>(src + c * 8);
+            ss += sumsq_pair<T>(x.x) + sumsq_pair<T>(x.y) + sumsq_pair<T>(x.z) + sumsq_pair<T>(x.w);
+          }
+        }
+        ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+        inv_row = rsqrt_approx(fmaf(ss, 1.f / (float)D, a.norm_eps));
+      }
+      for (int it = lane; it < kUnitKeys * kChunks; it += 32) {
+        const int row = it / kChunks, ch = it - row * kChunks;
+        const float inv_k = __shfl_sync(0xffffffffu, inv_row, row);  // uniform trip count: every lane takes part
+        uint4 kq = make_uint4(0u, 0u, 0u, 0u), vq = make_uint4(0u, 0u, 0u, 0u);
+        if (row < a.Tn) {
+          kq = *reinterpret_cast<const uint4*>(kn(row) + ch * 8);
+          vq = *reinterpret_cast<const uint4*>(vn(row) + ch * 8);
+          if (kw) {
+            const uint4 g = *reinterpret_cast<const uint4*>(kw + ch * 8);
+            kq.x = norm_pair<T>(kq.x, inv_k, g.x);
+            kq.y = norm_pair<T>(kq.y, inv_k, g.y);
+            kq.z = norm_pair<T>(kq.z, inv_k, g.z);
+            kq.w = norm_pair<T>(kq.w, inv_k, g.w);
+          }
+          if (a.rotary) {
+            const uint4 rq = *reinterpret_cast<const uint4*>(rot(row) + ch * 8);
+            kq.x = cmul_pair<T>(kq.x, rq.x);
+            kq.y = cmul_pair<T>(kq.y, rq.y);
+            kq.z = cmul_pair<T>(kq.z, rq.z);
+            kq.w = cmul_pair<T>(kq.w, rq.w);
+          }
+          if (dhalf == 0) {
+            *reinterpret_cast<uint4*>(kc + b * a.kc_sb + (int64_t)(t_old + row) * a.kc_ss + (int64_t)kvh * a.kc_sh + ch * 8) = kq;
+            *reinterpret_cast<uint4*>(vc + b * a.vc_sb + (int64_t)(t_old + row) * a.vc_ss + (int64_t)kvh * a.vc_sh + ch * 8) = vq;
+          }
+        }
+        const uint32_t o = (uint32_t)(ch >> 3) * kBoxBytes + (uint32_t)row * 128 + ((((uint32_t)ch & 7u) ^ ((uint32_t)row & 7u)) << 4);
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile + o), "r"(kq.x), "r"(kq.y), "r"(kq.z), "r"(kq.w) : "memory");
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile + C::kHalves * kBoxBytes + o), "r"(vq.x), "r"(vq.y),
+                     "r"(vq.z), "r"(vq.w)
+                     : "memory");
+      }
+      __syncwarp();
+      process_unit(tile, tile + C::kHalves * kBoxBytes, t_old, a.Sk - 1, (uint32_t)kBoxBytes);
+    }
+  }
   if (warp == kConsumerWarps) {
     // ---------------- producer ----------------
 #ifdef DT_BRINGUP
@@ -463,74 +568,6 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     }
   }
 
-  // ---------------- decode step fusion: rotate, append and attend the new K/V rows ----------------
-  // The cache rows streamed above end at Sk - Tn; the Tn new rows come from k_new / v_new.  The last split of
-  // each (batch, KV head) rotates the new keys, stores new keys and values into the cache for later steps and
-  // attends to them as one more unit built in shared memory (the ring is idle after the barrier).
-  if (a.k_new != nullptr) {
-    __syncthreads();
-    if (split == a.nsplit - 1 && warp < kConsumerWarps && uslot == 0) {
-      const uint32_t tile = ring + dhalf * C::kWarpTileBytes;  // with D = 256 the two warps of the pair build one copy each
-      const T* kn = reinterpret_cast<const T*>(a.k_new);
-      const T* vn = reinterpret_cast<const T*>(a.v_new);
-      const T* rot = reinterpret_cast<const T*>(a.rotary);
-      T* kc = reinterpret_cast<T*>(a.k_cache);
-      T* vc = reinterpret_cast<T*>(a.v_cache);
-      const int t_old = a.stream_keys;
-      constexpr int kChunks = D / 8;  // 16-byte chunks per row
-      // RMSNorm of the new keys: lanes l and l + 16 each sum half of row l's squares; lane l then holds 1 / rms
-      const T* kw = reinterpret_cast<const T*>(a.k_norm_w);
-      float inv_row = 1.f;
-      if (kw) {
-        const int row = lane & 15, half = lane >> 4;
-        float ss = 0.f;
-        if (row < a.Tn) {
-          const T* src = kn + b * a.kn_sb + (int64_t)row * a.kn_ss + (int64_t)kvh * a.kn_sh + half * (D / 2);
-#pragma unroll
-          for (int c = 0; c < D / 16; ++c) {
-            const uint4 x = *reinterpret_cast<const uint4*>(src + c * 8);
-            ss += sumsq_pair<T>(x.x) + sumsq_pair<T>(x.y) + sumsq_pair<T>(x.z) + sumsq_pair<T>(x.w);
-          }
-        }
-        ss += __shfl_xor_sync(0xffffffffu, ss, 16);
-        inv_row = rsqrt_approx(fmaf(ss, 1.f / (float)D, a.norm_eps));
-      }
-      for (int it = lane; it < kUnitKeys * kChunks; it += 32) {
-        const int row = it / kChunks, ch = it - row * kChunks;
-        const float inv_k = __shfl_sync(0xffffffffu, inv_row, row);  // uniform trip count: every lane takes part
-        uint4 kq = make_uint4(0u, 0u, 0u, 0u), vq = make_uint4(0u, 0u, 0u, 0u);
-        if (row < a.Tn) {
-          kq = *reinterpret_cast<const uint4*>(kn + b * a.kn_sb + (int64_t)row * a.kn_ss + (int64_t)kvh * a.kn_sh + ch * 8);
-          vq = *reinterpret_cast<const uint4*>(vn + b * a.vn_sb + (int64_t)row * a.vn_ss + (int64_t)kvh * a.vn_sh + ch * 8);
-          if (kw) {
-            const uint4 g = *reinterpret_cast<const uint4*>(kw + ch * 8);
-            kq.x = norm_pair<T>(kq.x, inv_k, g.x);
-            kq.y = norm_pair<T>(kq.y, inv_k, g.y);
-            kq.z = norm_pair<T>(kq.z, inv_k, g.z);
-            kq.w = norm_pair<T>(kq.w, inv_k, g.w);
-          }
-          if (rot) {
-            const uint4 rq = *reinterpret_cast<const uint4*>(rot + b * a.rot_sb + (int64_t)row * a.rot_ss + ch * 8);
-            kq.x = cmul_pair<T>(kq.x, rq.x);
-            kq.y = cmul_pair<T>(kq.y, rq.y);
-            kq.z = cmul_pair<T>(kq.z, rq.z);
-            kq.w = cmul_pair<T>(kq.w, rq.w);
-          }
-          if (dhalf == 0) {
-            *reinterpret_cast<uint4*>(kc + b * a.kc_sb + (int64_t)(t_old + row) * a.kc_ss + (int64_t)kvh * a.kc_sh + ch * 8) = kq;
-            *reinterpret_cast<uint4*>(vc + b * a.vc_sb + (int64_t)(t_old + row) * a.vc_ss + (int64_t)kvh * a.vc_sh + ch * 8) = vq;
-          }
-        }
-        const uint32_t o = (uint32_t)(ch >> 3) * kBoxBytes + (uint32_t)row * 128 + ((((uint32_t)ch & 7u) ^ ((uint32_t)row & 7u)) << 4);
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile + o), "r"(kq.x), "r"(kq.y), "r"(kq.z), "r"(kq.w) : "memory");
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile + C::kHalves * kBoxBytes + o), "r"(vq.x), "r"(vq.y),
-                     "r"(vq.z), "r"(vq.w)
-                     : "memory");
-      }
-      __syncwarp();
-      process_unit(tile, tile + C::kHalves * kBoxBytes, t_old, a.Sk - 1, (uint32_t)kBoxBytes);
-    }
-  }
   if (warp < kConsumerWarps) {
     l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
     l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
@@ -868,6 +905,7 @@ int first_unit(const dt_sdpa_params& p) {
 // use as few CTAs as keep every SM streaming: the largest power of two with pairs * splits <= the CTAs that are
 // resident at once (one wave), and at least four 16-key units per split.  (Measured on B200: B=16 runs at 99% of
 // the copy peak with 2 splits and at 57% with 37.)  The caller may fix the count with DT_FLAG_DECODE_SPLITS.
+constexpr int kClusterSplits = 8, kClusterUnits = 16;
 Plan make_plan(const dt_sdpa_params& p, int stream_keys) {
   Plan pl;
   pl.cluster = 1;
@@ -882,6 +920,10 @@ Plan make_plan(const dt_sdpa_params& p, int stream_keys) {
   const int slots = (p.D > 128 ? 1 : 2) * sm_count();
   int ns = 1;
   while (pairs * ns * 2 <= slots && pl.total_units / (ns * 2) >= 4) ns *= 2;
+  // Up to kClusterUnits units per split the eight splits of one cluster, which combine through distributed shared memory, are
+  // faster than more splits that meet in global memory (one token, us with 8 splits and with 32: 16/4 heads of 256, 1024 rows 7.97 and
+  // 9.97, 2048 rows 10.45 and 10.98, 3072 rows 12.81 and 11.72; 32/8 heads of 128, 2048 rows 8.61 and 9.39, 3072 rows 10.53 and 10.25).
+  if (ns > kClusterSplits && pl.total_units <= kClusterSplits * kClusterUnits) ns = kClusterSplits;
   int forced = (int)((p.flags >> 16) & 0xFFFu);
 #ifdef DT_BRINGUP
   if (const char* env = getenv("DTATTN_DECODE_SPLITS")) forced = atoi(env);
