@@ -74,8 +74,32 @@ WAIT_TEST_LIB = os.path.join(LIB_DIR, "libdtattn_waittest.so")
 WAIT_TEST_DEFINES = ("DT_BRINGUP", "DT_WAIT_LIMIT_NS=5000000ull")
 
 
+# The Python surface's calls in native code (an extension module on torch's own headers and libraries).
+CALLS = os.path.join(LIB_DIR, "dtattn_calls.so")
+
+
+def build_calls(force=False):
+    import sysconfig
+    import torch
+    src, header = os.path.join(CSRC, "py_calls.cpp"), os.path.join(HERE, "..", "include", "dtattn.h")
+    if force or not os.path.exists(CALLS) or os.path.getmtime(CALLS) < _newest([src, header]):
+        os.makedirs(LIB_DIR, exist_ok=True)
+        t = os.path.dirname(torch.__file__)
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               *["-I" + d for d in (os.path.join(HERE, "..", "include"), os.path.join(t, "include"),
+                                    os.path.join(t, "include", "torch", "csrc", "api", "include"),
+                                    sysconfig.get_paths()["include"], "/usr/local/cuda/include")],
+               src, "-o", CALLS, "-L" + os.path.join(t, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode:
+            sys.stderr.write(r.stdout + r.stderr)
+            raise RuntimeError("g++ failed: " + src)
+    return CALLS
+
+
 def build_all(force=False):
     path = build(force=force)
+    build_calls(force=force)
     build(force=force, defines=WAIT_TEST_DEFINES, out=WAIT_TEST_LIB)
     return path
 
@@ -87,4 +111,6 @@ if __name__ == "__main__":
         sys.exit(0)
     defs = [argv[i + 1] for i, a in enumerate(argv[:-1]) if a == "--define"]
     outs = [argv[i + 1] for i, a in enumerate(argv[:-1]) if a == "--out"]
+    if not outs:
+        build_calls(force="--force" in argv)
     print(build(force="--force" in argv, verbose="--verbose" in argv, defines=defs, out=outs[0] if outs else None))

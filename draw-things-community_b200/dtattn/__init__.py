@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import ctypes
 import enum
+import importlib.util
 import operator
 import os
 import struct
@@ -179,7 +180,39 @@ def lib():
             fn = getattr(_lib, name)
             fn.restype = res
             fn.argtypes = args
+        _calls.bind(*[ctypes.cast(getattr(_lib, name), ctypes.c_void_p).value for name in _CALLS])
     return _lib
+
+
+# What the native module calls, in the order of its bind
+_CALLS = ["dt_sdpa_workspace_size", "dt_sdpa_kernel_name", "dt_sdpa_forward", "dt_sdpa_decode_step_workspace_size",
+          "dt_sdpa_decode_step", "dt_qk_prologue", "dt_sparse_indexed_attention"]
+
+
+def _load_calls():
+    """The usual calls in native code (csrc/py_calls.cpp).  Raises (never falls back) when it has not been built."""
+    path = os.path.abspath(os.path.join(_HERE, "..", "lib", "dtattn_calls.so"))
+    if not os.path.exists(path):
+        raise ImportError(f"{path} not found: build it with `python draw-things-community_b200/build.py`")
+    spec = importlib.util.spec_from_file_location("dtattn_calls", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
+_calls = _load_calls()
+
+
+def _raw_stream(index):
+    return torch._C._cuda_getCurrentRawStream(index)
+
+
+def _place(q):
+    """(stream, workspace, its bytes) of a call on q's device: the current stream and the device's own workspace as it is."""
+    index = q.get_device()
+    ws = _workspaces.get(("cuda", index))
+    buf = None if ws is None else ws.buf
+    return (_raw_stream(index), 0, 0) if buf is None else (_raw_stream(index), buf.data_ptr(), buf.numel())
 
 
 def status_string(status):
@@ -303,6 +336,17 @@ def sdpa_forward(q, k, v, scale, is_causal=False, mask=None, out=None, lse=None,
     CUDA tensors -> dt_sdpa_forward on the current (or given) stream; CPU tensors -> dt_sdpa_forward_host,
     which stages through device memory (the end-to-end path).
     """
+    if workspace is None and stream is None and seq_offsets_q is None and q.is_cuda:  # the usual call, in native code
+        lib()
+        s, ptr, nbytes = _place(q)
+        got = _calls.sdpa(q, k, v, out, scale, is_causal, mask, lse, flags, sinks, sliding_window, s, ptr, nbytes)
+        if type(got) is tuple:
+            got, params, need, optional = got
+            scratch = _call_scratch(need, q.device, s, optional)
+            ptr, nbytes = (0, 0) if scratch is None else (scratch.data_ptr(), scratch.numel())
+            got = _calls.run(params, got, ptr, nbytes, s)
+        if got is not None:
+            return got if type(got) is not int else _check(got, "dt_sdpa_forward")
     if out is None:
         out = _new_output(q)
     p = make_params(q, k, v, out, scale, is_causal, mask, lse, flags, sinks, sliding_window, seq_offsets_q,
@@ -359,6 +403,12 @@ def decode_step(q, k_cache, v_cache, k_new, v_new, rotary, scale, cached_len, ou
     [cached_len, cached_len + T_new) and return causal attention of the rotated queries over rows
     [0, cached_len + T_new).  q holds the last Sq <= T_new tokens' queries."""
     assert q.is_cuda, "the fused decode step takes device tensors"
+    if workspace is None and stream is None and type(cached_len) is int:  # the usual call, in native code
+        lib()
+        got = _calls.step(q, k_cache, v_cache, k_new, v_new, rotary, out, scale, cached_len + k_new.shape[1], lse, flags,
+                          q_norm_weight, k_norm_weight, norm_eps, sinks, sliding_window, *_place(q))
+        if got is not None:
+            return got if type(got) is not int else _check(got, "dt_sdpa_decode_step")
     if out is None:
         out = _new_output(q)
     sp = make_step_params(q, k_cache, v_cache, k_new, v_new, rotary, out, scale, cached_len + k_new.shape[1], True, lse,
@@ -398,6 +448,12 @@ def qk_prologue(q, k=None, *, q_out=None, k_out=None, q_weight=None, k_weight=No
     node at Flux1.swift:164-188, Wan.swift:86-98, Qwen3_5.swift:164-182).  Outputs default to new tensors; pass
     q_out / k_out views (e.g. row-offset views of a joint buffer) to write in place or to fuse a concat."""
     assert q.is_cuda
+    if stream is None:  # the usual call, in native code
+        lib()
+        got = _calls.prologue(q, k, q_out, k_out, q_weight, k_weight, rotary, rotary_k, eps, norm_per_token, post_scale,
+                              _raw_stream(q.get_device()))
+        if got is not None:
+            return got if type(got) is not int else _check(got, "dt_qk_prologue")
     q_out = torch.empty_like(q) if q_out is None else q_out
     pq = make_prologue_params(q, q_out, q_weight, rotary, eps, norm_per_token, post_scale)
     pk = None
@@ -451,6 +507,12 @@ def sparse_indexed_attention(q, k_raw, v_raw, k_comp, v_comp, selected, scale, s
     `selected` (int32 [B or 1, Sq, n_selected]; entries outside [0, Sc) mean "no row") names, in one softmax with the
     sinks [Hq].  Device tensors."""
     assert q.is_cuda
+    if stream is None:  # the usual call, in native code
+        lib()
+        got = _calls.sparse(q, k_raw, v_raw, k_comp, v_comp, selected, scale, sinks, sliding_window, is_causal, out, lse, flags,
+                            _raw_stream(q.get_device()))
+        if got is not None:
+            return got if type(got) is not int else _check(got, "dt_sparse_indexed_attention")
     B, Sq, Hq, D = q.shape
     if out is None:
         out = torch.empty_like(q)

@@ -1,0 +1,82 @@
+"""The Python surface's calls in native code: what they serve, what they leave to the Python path, and that both answer alike."""
+import pytest
+import torch
+
+from test_gpu_masked_prefill import make_mask
+from test_gpu_parity import DEV, inputs
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def python_only(dtattn, monkeypatch):
+    """Switches the native calls off."""
+    def off():
+        class Declines:
+            def __getattr__(self, name):
+                return lambda *a: None
+        monkeypatch.setattr(dtattn, "_calls", Declines())
+    return off
+
+
+def bits(t):
+    return [x.clone().view(torch.int16 if x.element_size() == 2 else torch.int32) for x in (t if isinstance(t, (tuple, list)) else [t])]
+
+
+def test_both_paths_answer_alike(dtattn, python_only):
+    H = torch.float16
+    q, k, v = (x.to(DEV) for x in inputs(2, 200, 300, 8, 4, 64, H, 2001))
+    mask, sinks = make_mask(1, 1, 200, 300, H, 2002).to(DEV), torch.randn(8, device=DEV).to(H)
+    odd = torch.zeros(200 * 301, device=DEV, dtype=H).view(1, 1, 200, 301)[..., 1:].copy_(mask)
+    qd = q[:, :1]
+    f = [x.float() for x in (q, k, v)]
+    kc, vc = torch.zeros(1, 400, 2, 128, device=DEV, dtype=H), torch.zeros(1, 400, 2, 128, device=DEV, dtype=H)
+    qs, kn, vn = (x.to(DEV) for x in inputs(1, 1, 1, 8, 2, 128, H, 2003))
+    w, rot = torch.randn(128, device=DEV).to(H), torch.randn(1, 1, 128, device=DEV).to(H)
+    px, pr = torch.randn(1, 70, 4, 64, device=DEV).to(H), torch.randn(1, 70, 1, 64, device=DEV).to(H)
+    sq, kr = torch.randn(1, 2, 64, 512, device=DEV).to(H), torch.randn(1, 90, 1, 512, device=DEV).to(H)
+    sel = torch.randint(-1, 90, (1, 2, 33), device=DEV, dtype=torch.int32)
+    si = torch.randn(64, device=DEV).to(H)
+    lse = torch.zeros(2, 8, 200, device=DEV)
+    cases = [
+        lambda: dtattn.sdpa_forward(q, k, v, 0.125), lambda: dtattn.sdpa_forward(q, k, v, 0.125, True, lse=lse),
+        lambda: dtattn.sdpa_forward(q, k, v, 0.125, mask=mask), lambda: dtattn.sdpa_forward(q, k, v, 0.125, mask=odd),
+        lambda: dtattn.sdpa_forward(q, k, v, 0.125, True, sinks=sinks, sliding_window=70), lambda: dtattn.sdpa_forward(qd, k, v, 0.125),
+        lambda: dtattn.sdpa_forward(q[..., :40], k[..., :40], v[..., :40], 0.2), lambda: dtattn.sdpa_forward(*f, 0.125),
+        lambda: dtattn.sdpa_forward(q.transpose(1, 2).contiguous().transpose(1, 2), k, v, 0.125),
+        lambda: dtattn.decode_step(qs, kc, vc, kn, vn, rot, 0.1, 399, q_norm_weight=w, k_norm_weight=w),
+        lambda: dtattn.qk_prologue(px, px, q_weight=w[:64], k_weight=w[64:], rotary=pr, post_scale=0.5),
+        lambda: dtattn.sparse_indexed_attention(sq, kr, kr, kr, kr, sel, 0.05, si, 16)]
+    cases[5]()  # (the device's own workspace is there from now on)
+    native = [bits(fn()) for fn in cases]
+    kept = [kc.clone(), vc.clone(), lse.clone()]
+    python_only()
+    for a, fn in zip(native, cases):
+        b = bits(fn())
+        assert len(a) == len(b) and all(torch.equal(x, y) for x, y in zip(a, b))
+    assert all(torch.equal(x, y) for x, y in zip(kept, (kc, vc, lse)))
+    torch.cuda.synchronize()
+    assert dtattn.device_status() == 0
+
+
+def test_what_is_left_to_the_python_path(dtattn):
+    q, k, v = (x.to(DEV) for x in inputs(1, 64, 64, 2, 2, 64, torch.float16, 2011))
+    sdpa = lambda *a: dtattn._calls.sdpa(*a, None, 0.125, False, None, None, 0, None, 0, 0, 0, 0)  # noqa: E731
+    assert isinstance(sdpa(q, k, v), torch.Tensor)
+
+    class Sub(torch.Tensor):
+        pass
+
+    for t in (q.as_subclass(Sub), q.cpu(), q[0], q.double(), q.transpose(2, 3), q.float(), None, 3):
+        assert sdpa(t, k, v) is None and sdpa(q, t, v) is None
+    seen = []
+    torch.vmap(lambda x: (seen.append(sdpa(x, k, v)), x)[1])(q[None])
+    assert seen == [None]
+    for bad in (dict(scale="x"), dict(mask=q), dict(lse=torch.zeros(3, device=DEV)), dict(sinks=k[0, 0, :, 0].float())):
+        with pytest.raises((AssertionError, TypeError, dtattn.DtError)):
+            dtattn.sdpa_forward(q, k, v, **dict(dict(scale=0.125), **bad))
+    with pytest.raises(TypeError):
+        dtattn._calls.sdpa(q, k, v)
+    out = torch.zeros_like(q)
+    assert dtattn.sdpa_forward(q, k, v, 0.125, out=out) is out
+    assert dtattn.sdpa_forward(q, k, v, 1).shape == q.shape  # (a whole number as the scale)
