@@ -246,6 +246,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
   uint32_t qa[D / 16][4];
   const bool staged = a.Tn > 0 && a.Tn <= C::kStageRows;
   T* step_rows = reinterpret_cast<T*>(ring_ptr + C::kRingBytes + C::kNewBytes);  // [q weight][k weight][rotary x 4][new keys x 4][new values x 4]
+  auto consumer_barrier = []() { asm volatile("bar.sync 1, %0;" ::"n"(kConsumerWarps * 32) : "memory"); };
   constexpr int kRotAt = 2, kKnAt = 2 + C::kStageRows, kVnAt = 2 + 2 * C::kStageRows;
   if (warp < kConsumerWarps) {
     // Programmatic dependent launch (DT_FLAG_KV_PREFIX_STABLE): this grid may have started while the kernel before
@@ -271,71 +272,73 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
       ptx::cp_async_commit();
     }
     const T* q = reinterpret_cast<const T*>(a.q);
-    const T* rot = reinterpret_cast<const T*>(a.rotary);
-    const T* p_lo = nullptr;
-    const T* p_hi = nullptr;
-    const T* t_lo = nullptr;
-    const T* t_hi = nullptr;
-    if (r_lo < a.M) {
-      p_lo = q + b * a.q_sb + (int64_t)(r_lo / a.G) * a.q_ss + (int64_t)(kvh * a.G + r_lo % a.G) * a.q_sh;
-      const int t = a.Tn - a.Sq + r_lo / a.G;
-      if (rot) t_lo = staged ? step_rows + (kRotAt + t) * D : rot + b * a.rot_sb + (int64_t)t * a.rot_ss;
-    }
-    if (r_hi < a.M) {
-      p_hi = q + b * a.q_sb + (int64_t)(r_hi / a.G) * a.q_ss + (int64_t)(kvh * a.G + r_hi % a.G) * a.q_sh;
-      const int t = a.Tn - a.Sq + r_hi / a.G;
-      if (rot) t_hi = staged ? step_rows + (kRotAt + t) * D : rot + b * a.rot_sb + (int64_t)t * a.rot_ss;
-    }
-#pragma unroll
-    for (int ks = 0; ks < D / 16; ++ks) {
-      qa[ks][0] = p_lo ? *reinterpret_cast<const uint32_t*>(p_lo + ks * 16 + cq) : 0u;
-      qa[ks][1] = p_hi ? *reinterpret_cast<const uint32_t*>(p_hi + ks * 16 + cq) : 0u;
-      qa[ks][2] = p_lo ? *reinterpret_cast<const uint32_t*>(p_lo + ks * 16 + cq + 8) : 0u;
-      qa[ks][3] = p_hi ? *reinterpret_cast<const uint32_t*>(p_hi + ks * 16 + cq + 8) : 0u;
-    }
-    if (staged) {  // (the loads of Q above are on their way meanwhile)
-      ptx::cp_async_wait<0>();
-      asm volatile("bar.sync 1, %0;" ::"n"(kConsumerWarps * 32) : "memory");
-    }
-    if (a.q_norm_w) {
-      // per-row RMSNorm: a row's D elements sit in the four lanes that share lane >> 2
-      const T* gw = staged ? step_rows : reinterpret_cast<const T*>(a.q_norm_w);
-      float ss_lo = 0.f, ss_hi = 0.f;
+    if (a.k_new == nullptr) {
+      const T* p_lo = nullptr;
+      const T* p_hi = nullptr;
+      if (r_lo < a.M) p_lo = q + b * a.q_sb + (int64_t)(r_lo / a.G) * a.q_ss + (int64_t)(kvh * a.G + r_lo % a.G) * a.q_sh;
+      if (r_hi < a.M) p_hi = q + b * a.q_sb + (int64_t)(r_hi / a.G) * a.q_ss + (int64_t)(kvh * a.G + r_hi % a.G) * a.q_sh;
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) {
-        ss_lo += sumsq_pair<T>(qa[ks][0]) + sumsq_pair<T>(qa[ks][2]);
-        ss_hi += sumsq_pair<T>(qa[ks][1]) + sumsq_pair<T>(qa[ks][3]);
+        qa[ks][0] = p_lo ? *reinterpret_cast<const uint32_t*>(p_lo + ks * 16 + cq) : 0u;
+        qa[ks][1] = p_hi ? *reinterpret_cast<const uint32_t*>(p_hi + ks * 16 + cq) : 0u;
+        qa[ks][2] = p_lo ? *reinterpret_cast<const uint32_t*>(p_lo + ks * 16 + cq + 8) : 0u;
+        qa[ks][3] = p_hi ? *reinterpret_cast<const uint32_t*>(p_hi + ks * 16 + cq + 8) : 0u;
       }
-      ss_lo += __shfl_xor_sync(0xffffffffu, ss_lo, 1);
-      ss_lo += __shfl_xor_sync(0xffffffffu, ss_lo, 2);
-      ss_hi += __shfl_xor_sync(0xffffffffu, ss_hi, 1);
-      ss_hi += __shfl_xor_sync(0xffffffffu, ss_hi, 2);
-      const float inv_lo = rsqrt_approx(fmaf(ss_lo, 1.f / (float)D, a.norm_eps));
-      const float inv_hi = rsqrt_approx(fmaf(ss_hi, 1.f / (float)D, a.norm_eps));
+    } else {
+      // A step's queries are normalised and rotated once per CTA, a warp per row, and read back as fragments: with every warp
+      // doing it for its own fragments, a lone warp per scheduler spent 3 us on it at head dim 256.  They lie where the last split
+      // builds its unit of new rows afterwards.
+      constexpr int kPairs = D / 64, kQPitch = D + 8;  // 32-bit pairs of a row per lane
+      T* qs = reinterpret_cast<T*>(ring_ptr + C::kRingBytes);
+      static_assert(kMaxRows * kQPitch * 2 <= C::kNewBytes, "queries in the new rows' place");
+      uint32_t x[kMaxRows / kConsumerWarps][kPairs];
+#pragma unroll
+      for (int u = 0; u < kMaxRows / kConsumerWarps; ++u) {
+        const int r = warp + u * kConsumerWarps;
+        if (r >= a.M) break;
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(q + b * a.q_sb + (int64_t)(r / a.G) * a.q_ss + (int64_t)(kvh * a.G + r % a.G) * a.q_sh);
+#pragma unroll
+        for (int e = 0; e < kPairs; ++e) x[u][e] = src[lane * kPairs + e];
+      }
+      if (staged) {  // (the loads of Q above are on their way meanwhile)
+        ptx::cp_async_wait<0>();
+        consumer_barrier();
+      }
+      const uint32_t* gw = reinterpret_cast<const uint32_t*>(staged ? step_rows : reinterpret_cast<const T*>(a.q_norm_w));
+#pragma unroll
+      for (int u = 0; u < kMaxRows / kConsumerWarps; ++u) {
+        const int r = warp + u * kConsumerWarps;
+        if (r >= a.M) break;
+        if (a.q_norm_w) {
+          float ss = 0.f;
+#pragma unroll
+          for (int e = 0; e < kPairs; ++e) ss += sumsq_pair<T>(x[u][e]);
+#pragma unroll
+          for (int o2 = 16; o2; o2 >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o2);
+          const float inv = rsqrt_approx(fmaf(ss, 1.f / (float)D, a.norm_eps));
+#pragma unroll
+          for (int e = 0; e < kPairs; ++e) x[u][e] = norm_pair<T>(x[u][e], inv, gw[lane * kPairs + e]);
+        }
+        if (a.rotary) {  // a pair is exactly one (cos, sin) pair of the rotary table
+          const int t = a.Tn - a.Sq + r / a.G;
+          const uint32_t* tr = reinterpret_cast<const uint32_t*>(staged ? step_rows + (kRotAt + t) * D
+                                                                        : reinterpret_cast<const T*>(a.rotary) + b * a.rot_sb + (int64_t)t * a.rot_ss);
+#pragma unroll
+          for (int e = 0; e < kPairs; ++e) x[u][e] = cmul_pair<T>(x[u][e], tr[lane * kPairs + e]);
+        }
+        uint32_t* dst = reinterpret_cast<uint32_t*>(qs + r * kQPitch);
+#pragma unroll
+        for (int e = 0; e < kPairs; ++e) dst[lane * kPairs + e] = x[u][e];
+      }
+      consumer_barrier();
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) {
-        const uint32_t g0 = *reinterpret_cast<const uint32_t*>(gw + ks * 16 + cq);
-        const uint32_t g1 = *reinterpret_cast<const uint32_t*>(gw + ks * 16 + cq + 8);
-        qa[ks][0] = norm_pair<T>(qa[ks][0], inv_lo, g0);
-        qa[ks][1] = norm_pair<T>(qa[ks][1], inv_hi, g0);
-        qa[ks][2] = norm_pair<T>(qa[ks][2], inv_lo, g1);
-        qa[ks][3] = norm_pair<T>(qa[ks][3], inv_hi, g1);
+        qa[ks][0] = r_lo < a.M ? *reinterpret_cast<const uint32_t*>(qs + r_lo * kQPitch + ks * 16 + cq) : 0u;
+        qa[ks][1] = r_hi < a.M ? *reinterpret_cast<const uint32_t*>(qs + r_hi * kQPitch + ks * 16 + cq) : 0u;
+        qa[ks][2] = r_lo < a.M ? *reinterpret_cast<const uint32_t*>(qs + r_lo * kQPitch + ks * 16 + cq + 8) : 0u;
+        qa[ks][3] = r_hi < a.M ? *reinterpret_cast<const uint32_t*>(qs + r_hi * kQPitch + ks * 16 + cq + 8) : 0u;
       }
-    }
-    // rotation as a second pass, so that the loads above stay back to back when there is no table: a fragment
-    // register holds head dims (d, d+1) with d even, exactly one (cos, sin) pair of the rotary table
-    if (rot) {
-#pragma unroll
-      for (int ks = 0; ks < D / 16; ++ks) {
-        const uint32_t c0 = t_lo ? *reinterpret_cast<const uint32_t*>(t_lo + ks * 16 + cq) : 0u;
-        const uint32_t c1 = t_hi ? *reinterpret_cast<const uint32_t*>(t_hi + ks * 16 + cq) : 0u;
-        const uint32_t c2 = t_lo ? *reinterpret_cast<const uint32_t*>(t_lo + ks * 16 + cq + 8) : 0u;
-        const uint32_t c3 = t_hi ? *reinterpret_cast<const uint32_t*>(t_hi + ks * 16 + cq + 8) : 0u;
-        qa[ks][0] = cmul_pair<T>(qa[ks][0], c0);
-        qa[ks][1] = cmul_pair<T>(qa[ks][1], c1);
-        qa[ks][2] = cmul_pair<T>(qa[ks][2], c2);
-        qa[ks][3] = cmul_pair<T>(qa[ks][3], c3);
-      }
+      if (split == a.nsplit - 1) consumer_barrier();  // everybody has its fragments: the unit of new rows may be built there
     }
   }
   // last visible key per row (inclusive)
