@@ -148,6 +148,7 @@ crossattn_short_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     ptx::fence_mbar_init();
     // first loads of the pipeline (K/V of its first head, its first two Q tiles): they need only the barriers
     // above and run while TMEM is being allocated
+    ptx::wait_for_previous();
     const int tb = run_begin(g), te = run_end(g);
     if (tb < te) {
       const ShortTile w0 = decode_short_tile(a, tb);
@@ -165,6 +166,8 @@ crossattn_short_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_all = tmem_base_s;
+  ptx::wait_for_previous();
+  ptx::let_next_start();
 
   if (warp < 4) {
     ptx::setmaxnreg_dec<kRegsIssuer>();
@@ -402,8 +405,7 @@ int launch_short_t(const dt_sdpa_params& p, cudaStream_t stream) {
   const int n_sm = device_sm_count();
   const int want = (a.n_tiles + kGroups - 1) / kGroups;  // at least one tile per warpgroup
   dim3 grid(want < n_sm ? want : n_sm);                   // one persistent CTA per SM
-  kern<<<grid, kThreadsShort, C::kSmemBytes, stream>>>(mq, mk, mv, mo, a);
-  DT_CUDA_TRY(cudaGetLastError());
+  DT_CUDA_TRY(launch_behind(kern, grid, dim3(kThreadsShort), C::kSmemBytes, stream, 1, mq, mk, mv, mo, a));
   return DT_OK;
 }
 

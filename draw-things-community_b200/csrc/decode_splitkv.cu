@@ -100,6 +100,7 @@ struct DecodeArgs {
   const void* q_norm_w;  // [D] RMSNorm weights applied to the queries / new keys before the rotation, or null
   const void* k_norm_w;
   float norm_eps;
+  int prefix_stable;  // the streamed rows may be read while the kernel before this one runs
   int Tn;           // new rows appended by the step fusion (<= 16), 0 otherwise
   int nsplit, units_per_split, total_units;
   int cluster;  // nsplit when the splits of a (batch, KV head) form one thread-block cluster, else 1
@@ -211,10 +212,6 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
   const int n_units = max(0, unit_end - unit_begin);
   const int n_stages = (n_units + C::kUnitsPerStage - 1) / C::kUnitsPerStage;
 
-  // A kernel launched behind this one with programmatic stream serialization (the next decode call, see
-  // DT_FLAG_KV_PREFIX_STABLE) may be scheduled as soon as every CTA of this grid has got here; it takes the SM slots
-  // that this grid's CTAs free when they exit, while the last CTAs still combine.
-  if (threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == kConsumerWarps * 32) {  // the producer lane: the descriptor fetch (about 1 us when cold) starts at once
     ptx::prefetch_tensormap(&map_k);
     ptx::prefetch_tensormap(&map_v);
@@ -249,11 +246,11 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
   auto consumer_barrier = []() { asm volatile("bar.sync 1, %0;" ::"n"(kConsumerWarps * 32) : "memory"); };
   constexpr int kRotAt = 2, kKnAt = 2 + C::kStageRows, kVnAt = 2 + 2 * C::kStageRows;
   if (warp < kConsumerWarps) {
-    // Programmatic dependent launch (DT_FLAG_KV_PREFIX_STABLE): this grid may have started while the kernel before
-    // it in the stream was still running.  The producer warp streams the K/V prefix at once (the caller guarantees
-    // that kernel does not write it); everything else -- Q, the new rows, the workspace, the outputs -- is
-    // touched only after the preceding grid has completed.  Without the launch attribute this returns at once.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // This grid may have started while the kernel before it in the stream was still running: Q, the new rows, the workspace and
+    // the outputs are touched only after that one has completed.  The next kernel may be brought in as soon as every CTA of this
+    // grid has got here; it takes the SM slots that this grid's CTAs free when they exit, while the last CTAs still combine.
+    ptx::wait_for_previous();
+    ptx::let_next_start();
     if (staged) {
       constexpr int kPieces = D / 8;  // 16 bytes each
       const int n_rows = 2 + (split == a.nsplit - 1 ? 3 : 1) * a.Tn;
@@ -515,6 +512,9 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
 #else
     if (lane == 0) {
 #endif
+      // with DT_FLAG_KV_PREFIX_STABLE the K/V prefix is streamed at once: the caller guarantees that the kernel before this one
+      // does not write it
+      if (!a.prefix_stable) ptx::wait_for_previous();
       for (int st = 0; st < n_stages; ++st) {
         const int slot = st % nst;
         if (st >= nst) {
@@ -1084,28 +1084,8 @@ int launch_t(const dt_sdpa_params& p, const dt_decode_step_params* step, const S
   a.sinks = p.sinks;
   a.scale_log2 = p.scale * kLog2e;
   a.is_causal = p.is_causal;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(pl.nsplit, p.Hkv, p.B);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = C::kSmemBytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  int n_attr = 0;
-  if (a.cluster > 1) {
-    attr[n_attr].id = cudaLaunchAttributeClusterDimension;
-    attr[n_attr].val.clusterDim.x = a.cluster;
-    attr[n_attr].val.clusterDim.y = 1;
-    attr[n_attr].val.clusterDim.z = 1;
-    ++n_attr;
-  }
-  if (p.flags & DT_FLAG_KV_PREFIX_STABLE) {
-    attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
-    ++n_attr;
-  }
-  cfg.attrs = attr;
-  cfg.numAttrs = n_attr;
-  DT_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, mk, mv, a));
+  a.prefix_stable = (p.flags & DT_FLAG_KV_PREFIX_STABLE) != 0;
+  DT_CUDA_TRY(launch_behind(kern, dim3(pl.nsplit, p.Hkv, p.B), dim3(kThreads), C::kSmemBytes, stream, a.cluster, mk, mv, a));
   return DT_OK;
 }
 

@@ -115,6 +115,8 @@ __device__ __forceinline__ uint32_t out_of_range(float x) {
 // Bound: HBM / L2 writes (10 bytes moved per element in, 4 read and 6 written).  One 8-element piece per thread and step:
 // two 16-byte loads, three 16-byte stores.
 __global__ void __launch_bounds__(kSplitThreads) split_planes_kernel(const SplitArgs a) {
+  ptx::wait_for_previous();
+  ptx::let_next_start();
   uint32_t bad = 0;
   for (unsigned g = blockIdx.x * kSplitThreads + threadIdx.x; g < a.n_pieces; g += gridDim.x * kSplitThreads) {
     const SplitTensor& t = g < a.t[0].end ? a.t[0] : g < a.t[1].end ? a.t[1] : a.t[2];
@@ -185,6 +187,7 @@ f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     bars->abort_flag = 0;
     ptx::fence_mbar_init();
   }
+  ptx::wait_for_previous();
   uint32_t bad = 0;
   for (int i = threadIdx.x; i < a.n_flags; i += kThreads) bad |= a.flags[i];
   const int skip = __syncthreads_or((int)bad);
@@ -199,6 +202,7 @@ f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   ptx::tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
   volatile int* abort_flag = &bars->abort_flag;
+  if (a.n_items <= (int)gridDim.x) ptx::let_next_start();  // (as in the half-precision kernel)
   const int nkv = (a.Sk + kBN - 1) / kBN, G = a.Hq / a.Hkv;
   const int dsteps = (a.D + 15) >> 4;  // k-steps of Q K^T (columns beyond D are zeros in both operands)
 
@@ -549,10 +553,9 @@ int launch_t(const dt_sdpa_params& p, void* workspace, cudaStream_t stream) {
   auto kern = f32_tcgen05_kernel<NPV>;
   DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
   const int n_sm = device_sm_count();
-  split_planes_kernel<<<ctas, kSplitThreads, 0, stream>>>(sp);
-  DT_CUDA_TRY(cudaGetLastError());
-  kern<<<a.n_items < n_sm ? a.n_items : n_sm, kThreads, C::kSmemBytes, stream>>>(maps[0], maps[1], maps[2], a);
-  DT_CUDA_TRY(cudaGetLastError());
+  DT_CUDA_TRY(launch_behind(split_planes_kernel, dim3(ctas), dim3(kSplitThreads), 0, stream, 1, sp));
+  DT_CUDA_TRY(launch_behind(kern, dim3(a.n_items < n_sm ? a.n_items : n_sm), dim3(kThreads), C::kSmemBytes, stream, 1, maps[0], maps[1],
+                            maps[2], a));
   return launch_generic(p, stream, a.any_flag);  // returns at once unless the inputs could not be split
 }
 

@@ -8,7 +8,7 @@
 // One warp per query row (everything else): one CTA = 8 query rows of one (batch, head); keys are visited 32 at
 // a time from a shared-memory tile (fp32, odd row pitch so that lane j reading key row j is conflict
 // free); lane j owns key j of the tile for Q.K^T, then owns head dims {lane, lane+32, ...} for P.V.
-#include "common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace dt {
 namespace {
@@ -381,6 +381,8 @@ __device__ __forceinline__ void generic_tiled_block(const dim3 block, const T* _
 // 4 us for 1024 of them.
 template <bool kIf, typename Body>
 __device__ __forceinline__ void run_blocks(const uint32_t* __restrict__ only_if, const dim3 grid, Body body) {
+  ptx::wait_for_previous();
+  ptx::let_next_start();
   if constexpr (kIf) {
     if (*only_if == 0u) return;
     const uint64_t total = (uint64_t)grid.x * grid.y * grid.z;
@@ -430,13 +432,13 @@ int launch_tiled(const dt_sdpa_params& p, cudaStream_t stream, const uint32_t* o
   if (smem > 48 * 1024) DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const bool varlen = p.seq_offsets_q != nullptr;
   dim3 grid(((varlen ? p.max_seq_q : p.Sq) + kTM - 1) / kTM, p.Hq, varlen ? p.n_seq : p.B);
-  kern<<<launch_grid(grid, kTThreads, smem, only_if), kTThreads, smem, stream>>>(
+  DT_CUDA_TRY(launch_behind(
+      kern, launch_grid(grid, kTThreads, smem, only_if), dim3(kTThreads), smem, stream, 1,
       (const T*)p.q.ptr, (const T*)p.k.ptr, (const T*)p.v.ptr, (T*)p.o.ptr, (const T*)p.mask, p.lse,
       p.q.stride_b, p.q.stride_s, p.q.stride_h, p.k.stride_b, p.k.stride_s, p.k.stride_h,
       p.v.stride_b, p.v.stride_s, p.v.stride_h, p.o.stride_b, p.o.stride_s, p.o.stride_h,
       p.mask_stride_b, p.mask_stride_h, p.mask_stride_q, p.Sq, p.Sk, p.Hq, p.Hkv, D, p.scale * kLog2e,
-      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if, grid);
-  DT_CUDA_TRY(cudaGetLastError());
+      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if, grid));
   return DT_OK;
 }
 
@@ -455,13 +457,13 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, const uint32_t* only_
   if (smem > 48 * 1024) DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const bool varlen = p.seq_offsets_q != nullptr;
   dim3 grid(((varlen ? p.max_seq_q : p.Sq) + kRows - 1) / kRows, p.Hq, varlen ? p.n_seq : p.B);
-  kern<<<launch_grid(grid, kRows * 32, smem, only_if), kRows * 32, smem, stream>>>(
+  DT_CUDA_TRY(launch_behind(
+      kern, launch_grid(grid, kRows * 32, smem, only_if), dim3(kRows * 32), smem, stream, 1,
       (const T*)p.q.ptr, (const T*)p.k.ptr, (const T*)p.v.ptr, (T*)p.o.ptr, (const T*)p.mask, p.lse,
       p.q.stride_b, p.q.stride_s, p.q.stride_h, p.k.stride_b, p.k.stride_s, p.k.stride_h,
       p.v.stride_b, p.v.stride_s, p.v.stride_h, p.o.stride_b, p.o.stride_s, p.o.stride_h,
       p.mask_stride_b, p.mask_stride_h, p.mask_stride_q, p.Sq, p.Sk, p.Hq, p.Hkv, D, p.scale * kLog2e,
-      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if, grid);
-  DT_CUDA_TRY(cudaGetLastError());
+      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if, grid));
   return DT_OK;
 }
 

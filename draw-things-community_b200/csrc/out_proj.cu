@@ -120,6 +120,8 @@ out_proj_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  ptx::wait_for_previous();
+  ptx::let_next_start();
 
   if (warp == 0) {
     // =========================== TMA producer ===========================
@@ -330,8 +332,7 @@ int launch_proj_t(const dt_tensor4& a_view, int B, int S, int K, const void* wei
   mb_tail = mb;
   if (a.tail_split > 1 && !make_bshd_tensor_map(&mb_tail, w_view, 1, N, 1, K, dtype, kTileN / a.tail_split)) return DT_UNSUPPORTED;
   dim3 grid((unsigned)(a.full_rounds > 0 ? sms : a.tail_units));  // one persistent CTA per SM
-  kern<<<grid, kProjThreads, kProjSmem, stream>>>(ma, mb, mb_tail, mc, a);
-  DT_CUDA_TRY(cudaGetLastError());
+  DT_CUDA_TRY(launch_behind(kern, grid, dim3(kProjThreads), kProjSmem, stream, 1, ma, mb, mb_tail, mc, a));
   return DT_OK;
 }
 

@@ -12,7 +12,7 @@
 // The output may be a strided view, e.g. a row-offset view of the joint text+image buffer, which fuses the concat.
 #include <stdlib.h>
 
-#include "common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace dt {
 namespace {
@@ -165,6 +165,8 @@ __device__ __forceinline__ uint4 norm_rotate8(const uint64_t (&v)[4], float inv,
 constexpr int kHeadRows = 4;
 template <typename T, int LANES>
 __global__ void __launch_bounds__(256, 3) qk_prologue_heads_kernel(const PrologueArgs a) {
+  ptx::wait_for_previous();
+  ptx::let_next_start();
   const PrologueTensor& t = a.t[blockIdx.y];
   const int lane = threadIdx.x & 31;
   constexpr int kRowsPerWarp = 32 / LANES;
@@ -261,6 +263,8 @@ __global__ void __launch_bounds__(256, 3) qk_prologue_heads_kernel(const Prologu
 // every thread keeps one row piece and its table piece in flight while it computes.
 template <typename T, int LANES>
 __global__ void __launch_bounds__(256, 4) qk_prologue_rows_kernel(const PrologueArgs a) {
+  ptx::wait_for_previous();
+  ptx::let_next_start();
   const PrologueTensor& t = a.t[blockIdx.y];
   const int lane = threadIdx.x & 31, warp_in_cta = threadIdx.x >> 5;
   constexpr int kRowsPerWarp = 32 / LANES;
@@ -332,6 +336,8 @@ constexpr int kTokVecs = 8;  // 16-byte pieces held per thread at most: H*D <= 2
 
 template <typename T, int VECS>
 __global__ void __launch_bounds__(kTokThreads) qk_prologue_tokens_kernel(const PrologueArgs a, const int G) {
+  ptx::wait_for_previous();
+  ptx::let_next_start();
   const PrologueTensor& t = a.t[blockIdx.y];
   __shared__ float red[kTokThreads / 32];
   const int vecs_per_head = t.D / 8, n_vec = t.H * vecs_per_head;
@@ -505,10 +511,8 @@ int launch_rows(const PrologueArgs& a, int D, int64_t max_rows, cudaStream_t str
   if (by_token(a, 32 / lanes * kHeadRows, &tasks)) {
     const int64_t need = (tasks + 7) / 8, cap = (int64_t)sm_count_prologue() * 3 / a.n;  // persistent: three CTAs per SM
     dim3 grid((unsigned)(need < cap ? need : cap), a.n);
-    if (lanes == 8) qk_prologue_heads_kernel<T, 8><<<grid, 256, 0, stream>>>(a);
-    else if (lanes == 16) qk_prologue_heads_kernel<T, 16><<<grid, 256, 0, stream>>>(a);
-    else qk_prologue_heads_kernel<T, 32><<<grid, 256, 0, stream>>>(a);
-    DT_CUDA_TRY(cudaGetLastError());
+    auto kern = lanes == 8 ? qk_prologue_heads_kernel<T, 8> : lanes == 16 ? qk_prologue_heads_kernel<T, 16> : qk_prologue_heads_kernel<T, 32>;
+    DT_CUDA_TRY(launch_behind(kern, grid, dim3(256), 0, stream, 1, a));
     return DT_OK;
   }
   const int rows_per_cta = 8 * (32 / lanes);
@@ -516,10 +520,8 @@ int launch_rows(const PrologueArgs& a, int D, int64_t max_rows, cudaStream_t str
   const int64_t cap = (int64_t)sm_count_prologue() * 4;  // persistent: four CTAs per SM sweep the rows
   if (ctas > cap) ctas = cap;
   dim3 grid((unsigned)ctas, a.n);
-  if (lanes == 8) qk_prologue_rows_kernel<T, 8><<<grid, 256, 0, stream>>>(a);
-  else if (lanes == 16) qk_prologue_rows_kernel<T, 16><<<grid, 256, 0, stream>>>(a);
-  else qk_prologue_rows_kernel<T, 32><<<grid, 256, 0, stream>>>(a);
-  DT_CUDA_TRY(cudaGetLastError());
+  auto kern = lanes == 8 ? qk_prologue_rows_kernel<T, 8> : lanes == 16 ? qk_prologue_rows_kernel<T, 16> : qk_prologue_rows_kernel<T, 32>;
+  DT_CUDA_TRY(launch_behind(kern, grid, dim3(256), 0, stream, 1, a));
   return DT_OK;
 }
 
@@ -568,7 +570,7 @@ extern "C" int dt_qk_prologue(const dt_qk_prologue_params* q, const dt_qk_prolog
       per_sm = 1;                                                                                                 \
     const int64_t cap = (int64_t)sms * per_sm; /* persistent: resident CTAs sweep the tokens */                   \
     dim3 grid((unsigned)(ctas < cap ? ctas : cap), a.n);                                                          \
-    kern<<<grid, kTokThreads, 0, stream>>>(a, G);                                                     \
+    DT_CUDA_TRY(launch_behind(kern, grid, dim3(kTokThreads), 0, stream, 1, a, G));                                \
   } while (0)
     if (vecs <= 1) DT_TOK_LAUNCH(1);
     else if (vecs <= 2) DT_TOK_LAUNCH(2);

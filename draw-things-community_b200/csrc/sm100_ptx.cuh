@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 #include "common.cuh"
 
 namespace dt {
@@ -461,7 +463,40 @@ __device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.
 template <int N>
 __device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
+// ---- launches that overlap the end of the kernel before them (launch_behind) ----
+// The kernel before this one has finished and what it wrote is visible.  Before any access to global memory.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The kernel behind this one may be brought onto the SMs.  Said behind wait_for_previous(), so that a kernel runs beside its
+// predecessor at most, never beside the one before that (which a decode call with DT_FLAG_KV_PREFIX_STABLE relies on), and behind
+// the TMEM allocation, since CTAs of the next kernel that came first on an SM would keep the columns while they wait for this one.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 }  // namespace ptx
+
+// ---- host: a launch whose CTAs may start while the kernel before it in the stream runs out: launch overhead, barrier set-up, TMEM
+// allocation and the fetch of the tensor maps are then off the path.  Every thread that touches global memory calls
+// wait_for_previous() first or is behind a barrier with one that has, in every CTA (so that a kernel's end still means that all
+// before it have ended); the order of results is that of an ordinary launch.
+template <typename... P, typename... A>
+cudaError_t launch_behind(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2] = {};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  if (cluster > 1) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
 
 // ---- host: tensor-map encoding through the driver entry point (no link-time libcuda dependency) ----
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

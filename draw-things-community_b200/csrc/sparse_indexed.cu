@@ -593,6 +593,8 @@ __global__ void __launch_bounds__(32 * kOnceSplit) sparse_once_kernel(const Spar
   constexpr int chunks = D / 8;  // 16-byte pieces of a row
 
   ptx::cluster_arrive();  // (waited for before anything is stored into another CTA)
+  ptx::wait_for_previous();
+  ptx::let_next_start();
   {
     const T* q = reinterpret_cast<const T*>(a.q) + b * a.q_sb + (int64_t)i * a.q_ss + (int64_t)h0 * a.q_sh;
 #pragma unroll
@@ -811,19 +813,8 @@ int launch_sparse_once(const dt_sparse_indexed_params& p, const SparseArgs& a, b
   const size_t smem = once_smem<D>(same_kv);
   auto kern = sparse_once_kernel<T, D>;
   DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(p.Sq * kOnceSplit), (unsigned)(p.Hkv * ng), (unsigned)p.B);
-  cfg.blockDim = dim3(32 * kOnceSplit);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = kOnceSplit;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  DT_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a, per, same_kv ? 1 : 0));
+  const dim3 grid((unsigned)(p.Sq * kOnceSplit), (unsigned)(p.Hkv * ng), (unsigned)p.B);
+  DT_CUDA_TRY(launch_behind(kern, grid, dim3(32 * kOnceSplit), smem, stream, kOnceSplit, a, per, same_kv ? 1 : 0));
   return DT_OK;
 }
 
