@@ -57,10 +57,10 @@ typedef struct {
 #define DT_FLAG_FORCE_GENERIC 2u   /* route to the CUDA-core kernel (second GPU opinion in tests)        */
 #define DT_FLAG_KV_PREFIX_STABLE 4u /* decode over a KV cache: the kernel that precedes this call in the stream does
                                       not write the K/V rows this call streams (rows [0, Sk), or the cached prefix
-                                      [0, Sk - T_new) of dt_sdpa_decode_step).  The decode kernel is then launched with
-                                      programmatic stream serialization: its producer warp starts filling shared
-                                      memory from the cache while the preceding kernel drains, and everything else
-                                      (Q, new rows, workspace, outputs) waits for that kernel to complete.  Ignored by
+                                      [0, Sk - T_new) of dt_sdpa_decode_step).  The decode kernel's producer warp then
+                                      starts filling shared memory from the cache while the preceding kernel drains;
+                                      everything else (Q, new rows, workspace, outputs), and without the flag the
+                                      cache too, waits for that kernel to complete.  Ignored by
                                       the other kernels. */
 /* Split-KV decode tuning: fix the number of splits of every (batch, KV head) to n (1..256; 0 = the library's own
    choice, which fills the SMs once).  The value is part of what dt_sdpa_workspace_size depends on: pass the same
