@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(32 * kOnceSplit) sparse_once_kernel(const Spar
   if (first < 0) first = 0;
   const long long last_c = last < (long long)a.Sr - 1 ? last : (long long)a.Sr - 1;
   const int n_raw = last_c >= first ? (int)(last_c - first + 1) : 0;
-  const int n_keys = n_raw + (a.Sc > 0 ? a.n_sel : 0);
+  const int n_keys = n_raw + (a.Sc > 0 ? a.n_sel : 0);  // at most kOnceSplit * per: see most_keys
   const int32_t* sel = a.selected ? a.selected + b * a.sel_sb + (int64_t)i * a.sel_sq : nullptr;
   {
     // Warp w gathers keys w, w + 8, ... of this CTA's share: lane l looks up key w + 8 l, all lanes copy every row.
@@ -802,14 +802,16 @@ bool sparse_mma_supported(const dt_sparse_indexed_params& p) {
   return ok(p.q) && ok(p.o) && ok(p.k_raw) && ok(p.v_raw) && ok(p.k_comp) && ok(p.v_comp);
 }
 
-// The keys that a token may have
-int most_keys(const dt_sparse_indexed_params& p) {
-  return (p.sliding_window > 0 ? (p.sliding_window < p.Sr ? p.sliding_window : p.Sr) : p.Sr) + (p.Sc > 0 ? p.n_selected : 0);
+// The most keys that a token has: its raw rows and its list.  A window counts back from the token's own position; without causality the
+// rows behind that position are seen too, and the first token has one of them for every token behind it.
+long long most_keys(const dt_sparse_indexed_params& p) {
+  const long long seen = p.sliding_window > 0 ? (long long)p.sliding_window + (p.is_causal ? 0 : p.Sq - 1) : (long long)p.Sr;
+  return (seen < p.Sr ? seen : p.Sr) + (p.Sc > 0 ? p.n_selected : 0);
 }
 
 template <typename T, int D>
 int launch_sparse_once(const dt_sparse_indexed_params& p, const SparseArgs& a, bool same_kv, cudaStream_t stream) {
-  const int per = (most_keys(p) + kOnceSplit * 16 - 1) / (kOnceSplit * 16) * 16, ng = (p.Hq / p.Hkv + 15) / 16;
+  const int per = (int)((most_keys(p) + kOnceSplit * 16 - 1) / (kOnceSplit * 16) * 16), ng = (p.Hq / p.Hkv + 15) / 16;
   const size_t smem = once_smem<D>(same_kv);
   auto kern = sparse_once_kernel<T, D>;
   DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -829,8 +831,7 @@ int launch_sparse_mma_tk(const dt_sparse_indexed_params& p, const SparseArgs& a,
   const long long ctas = (long long)p.Sq * ng * p.Hkv * p.B;
   // few tokens (the decode step): a token's keys are shared out over a cluster of CTAs, as long as every CTA still gets
   // a few tiles and the grid stays within about two rounds over the SMs
-  const int keys = most_keys(p);
-  const int tiles = (keys + TK - 1) / TK;
+  const long long tiles = (most_keys(p) + TK - 1) / TK;
   int split = 1;
   const int sms = device_sm_count();
   while (split < kMmaMaxSplit && ctas * (split * 2) <= 2LL * sms && tiles >= 2 * (split * 2)) split *= 2;
@@ -872,7 +873,7 @@ int launch_sparse_mma_t(const dt_sparse_indexed_params& p, const SparseArgs& a, 
     if (st != DT_UNSUPPORTED) return st;  // (views that no tensor map describes, expanded queries for one: nothing was launched)
   }
   // Clusters that fit the SMs in one wave (a CTA's 180 KB leave room for one per SM).
-  const int keys = most_keys(p);
+  const long long keys = most_keys(p);
   const long long groups = (long long)p.Hkv * ((p.Hq / p.Hkv + 15) / 16);
   if ((p.D == 256 || (p.D == 512 && same_kv)) && keys > 0 && keys <= kOnceSplit * kOnceKeys && groups <= 65535 &&
       kOnceSplit * groups * p.Sq * p.B <= device_sm_count())
