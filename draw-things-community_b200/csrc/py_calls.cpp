@@ -1,8 +1,10 @@
 // The Python surface's usual calls in native code: exact torch.Tensor arguments on the GPU, the library's own scratch, the
 // current stream.  A call that looks like anything else (a subclass, a wrapped or traced tensor, another type, a shape that an
 // assertion refuses, a workspace that has to grow) is answered with None, and the Python path, which says what is wrong with
-// it, serves it.  Bound: the host.  A call's Python attribute look-ups, struct packing and ctypes conversions took 5 to 10 us,
-// where the kernels of the smallest calls take 8 to 15.
+// it, serves it.  Arguments are read with the interpreter lock; the output is allocated and the library called without it
+// (Unlocked): an allocation and a launch into a full queue may wait, and other threads go on meanwhile.
+// Bound: the host.  A call's Python attribute look-ups, struct packing and ctypes conversions took 5 to 10 us, where the kernels of
+// the smallest calls take 8 to 15.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -29,6 +31,15 @@ decltype(&dt_sparse_indexed_attention) f_sparse;
 struct NotMine {};
 
 [[noreturn]] void decline() { throw NotMine(); }
+
+// Without the interpreter lock as long as it lives: no Python object is touched then.
+struct Unlocked {
+  PyThreadState* const state = PyEval_SaveThread();
+  Unlocked() = default;
+  Unlocked(const Unlocked&) = delete;
+  Unlocked& operator=(const Unlocked&) = delete;
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
 
 const at::Tensor& tensor(PyObject* o) {
   if (!THPVariable_CheckExact(o)) decline();
@@ -83,23 +94,22 @@ const void* vector(PyObject* o, const at::Tensor& like, int64_t n) {
 void same_kind(const at::Tensor& t, const at::Tensor& q) {
   if (t.scalar_type() != q.scalar_type() || t.device() != q.device()) decline();
 }
-// the output tensor: the caller's, or a new one
-at::Tensor output(PyObject* o, const at::Tensor& q) {
-  if (!none(o)) return tensor(o);
+// the caller's output tensor, or an undefined one where it is for the call to allocate
+at::Tensor given(PyObject* o) { return none(o) ? at::Tensor() : tensor(o); }
+at::Tensor new_output(const at::Tensor& q) {
   return q.is_contiguous() ? at::empty_like(q) : at::empty(q.sizes(), q.options().requires_grad(false));
 }
 
-dt_sdpa_params attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& o, double scale, bool causal,
-                         PyObject* mask, PyObject* lse, uint32_t flags, PyObject* sinks, int32_t window, int32_t Sk) {
+// All but the output (place)
+dt_sdpa_params attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, double scale, bool causal, PyObject* mask,
+                         PyObject* lse, uint32_t flags, PyObject* sinks, int32_t window, int32_t Sk) {
   dt_sdpa_params p;
   memset(&p, 0, sizeof(p));
   p.q = quad(q);
   p.k = quad(k);
   p.v = quad(v);
-  p.o = quad(o);
   same_kind(k, q);
   same_kind(v, q);
-  same_kind(o, q);
   p.B = dim(q, 0);
   p.Sq = dim(q, 1);
   p.Hq = dim(q, 2);
@@ -128,6 +138,13 @@ dt_sdpa_params attention(const at::Tensor& q, const at::Tensor& k, const at::Ten
   p.sinks = vector(sinks, q, p.Hq);
   p.sliding_window = window;
   return p;
+}
+
+// The output of a call, allocated where there is none yet
+void place(dt_sdpa_params& p, at::Tensor& out, const at::Tensor& q) {
+  if (!out.defined()) out = new_output(q);
+  p.o = quad(out);
+  same_kind(out, q);
 }
 
 // The status of a failed call as a number, its output otherwise.
@@ -160,19 +177,29 @@ PyObject* py_sdpa(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const uint32_t flags = (uint32_t)whole(a[8], 0, 0xffffffffll);
     const int32_t window = (int32_t)whole(a[10], -0x7fffffffll, 0x7fffffffll);
     void* const stream = PyLong_AsVoidPtr(a[11]);
-    const at::Tensor out = output(a[3], q);
-    const dt_sdpa_params p = attention(q, k, v, out, number(a[4]), truth(a[5]), a[6], a[7], flags, a[9], window, -1);
+    void* const ws = PyLong_AsVoidPtr(a[12]);
+    const size_t bytes = (size_t)whole(a[13], 0, 1ll << 62);
+    at::Tensor out = given(a[3]);
+    dt_sdpa_params p = attention(q, k, v, number(a[4]), truth(a[5]), a[6], a[7], flags, a[9], window, -1);
     size_t need = 0;
-    if (f_workspace_size(&p, &need) != DT_OK) decline();
-    if (need == 0) return answer(f_forward(&p, nullptr, 0, stream), out, a[3]);
-    const char* name = nullptr;
-    if (f_kernel_name(&p, &name) != DT_OK) decline();
-    if (strcmp(name, "decode_splitkv") == 0) {  // (its tickets have to start at zero: the device's own workspace, if it is large enough)
-      void* const ws = PyLong_AsVoidPtr(a[12]);
-      const size_t bytes = (size_t)whole(a[13], 0, 1ll << 62);
-      if (!ws || bytes < need) decline();
-      return answer(f_forward(&p, ws, bytes, stream), out, a[3]);
+    const char* name = "";
+    int status = DT_OK;
+    bool done = true;
+    {
+      Unlocked here;
+      place(p, out, q);
+      if (f_workspace_size(&p, &need) != DT_OK) decline();
+      if (need != 0 && f_kernel_name(&p, &name) != DT_OK) decline();
+      if (need == 0) {
+        status = f_forward(&p, nullptr, 0, stream);
+      } else if (strcmp(name, "decode_splitkv") == 0) {  // (its tickets have to start at zero: the device's own workspace, if it is large enough)
+        if (!ws || bytes < need) decline();
+        status = f_forward(&p, ws, bytes, stream);
+      } else {
+        done = false;
+      }
     }
+    if (done) return answer(status, out, a[3]);
     PyObject* o = none(a[3]) ? THPVariable_Wrap(out) : Py_NewRef(a[3]);
     return Py_BuildValue("(Ny#nO)", o, reinterpret_cast<const char*>(&p), (Py_ssize_t)sizeof(p), (Py_ssize_t)need,
                          none(a[6]) || strcmp(name, "generic") == 0 ? Py_True : Py_False);
@@ -185,8 +212,15 @@ PyObject* py_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
     dt_sdpa_params p;
     if (!PyBytes_CheckExact(a[0]) || PyBytes_GET_SIZE(a[0]) != (Py_ssize_t)sizeof(p)) decline();
     memcpy(&p, PyBytes_AS_STRING(a[0]), sizeof(p));
-    const int st = f_forward(&p, PyLong_AsVoidPtr(a[2]), (size_t)whole(a[3], 0, 1ll << 62), PyLong_AsVoidPtr(a[4]));
-    return st == DT_OK ? Py_NewRef(a[1]) : PyLong_FromLong(st);
+    void* const scratch = PyLong_AsVoidPtr(a[2]);
+    const size_t bytes = (size_t)whole(a[3], 0, 1ll << 62);
+    void* const stream = PyLong_AsVoidPtr(a[4]);
+    int status;
+    {
+      Unlocked here;
+      status = f_forward(&p, scratch, bytes, stream);
+    }
+    return status == DT_OK ? Py_NewRef(a[1]) : PyLong_FromLong(status);
   });
 }
 
@@ -200,10 +234,12 @@ PyObject* py_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const uint32_t flags = (uint32_t)whole(a[10], 0, 0xffffffffll);
     const int32_t window = (int32_t)whole(a[15], -0x7fffffffll, 0x7fffffffll);
     void* const stream = PyLong_AsVoidPtr(a[16]);
-    const at::Tensor out = output(a[6], q);
+    void* const ws = PyLong_AsVoidPtr(a[17]);
+    const size_t bytes = (size_t)whole(a[18], 0, 1ll << 62);
+    at::Tensor out = given(a[6]);
     dt_decode_step_params s;
     memset(&s, 0, sizeof(s));
-    s.attn = attention(q, k, v, out, number(a[7]), true, Py_None, a[9], flags, a[14], window, total);
+    s.attn = attention(q, k, v, number(a[7]), true, Py_None, a[9], flags, a[14], window, total);
     s.k_new = quad(kn);
     s.v_new = quad(vn);
     same_kind(kn, q);
@@ -220,21 +256,24 @@ PyObject* py_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     s.q_norm_weight = vector(a[11], q, q.size(3));
     s.k_norm_weight = vector(a[12], q, q.size(3));
     s.norm_eps = (float)number(a[13]);
-    size_t need = 0;
-    if (f_step_workspace_size(&s, &need) != DT_OK) decline();
-    void* const ws = need ? PyLong_AsVoidPtr(a[17]) : nullptr;
-    const size_t bytes = need ? (size_t)whole(a[18], 0, 1ll << 62) : 0;
-    if (need && (!ws || bytes < need)) decline();
-    return answer(f_step(&s, ws, bytes, stream), out, a[6]);
+    int status;
+    {
+      Unlocked here;
+      place(s.attn, out, q);
+      size_t need = 0;
+      if (f_step_workspace_size(&s, &need) != DT_OK) decline();
+      if (need && (!ws || bytes < need)) decline();
+      status = f_step(&s, need ? ws : nullptr, need ? bytes : 0, stream);
+    }
+    return answer(status, out, a[6]);
   });
 }
 
-dt_qk_prologue_params prologue(const at::Tensor& x, const at::Tensor& y, PyObject* weight, PyObject* rotary, double eps, bool per_token,
-                               double post_scale) {
+// All but the output
+dt_qk_prologue_params prologue(const at::Tensor& x, PyObject* weight, PyObject* rotary, double eps, bool per_token, double post_scale) {
   dt_qk_prologue_params p;
   memset(&p, 0, sizeof(p));
   p.x = quad(x);
-  p.y = quad(y);
   p.B = dim(x, 0);
   p.S = dim(x, 1);
   p.H = dim(x, 2);
@@ -262,12 +301,20 @@ PyObject* py_prologue(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (q.dim() != 4 || k.dim() != 4) decline();
     const double eps = number(a[8]), post_scale = number(a[10]);
     const bool per_token = truth(a[9]);
-    const at::Tensor q_out = none(a[2]) ? at::empty_like(q) : tensor(a[2]);
-    const at::Tensor k_out = none(a[3]) ? at::empty_like(k) : tensor(a[3]);
-    const dt_qk_prologue_params pq = prologue(q, q_out, a[4], a[6], eps, per_token, post_scale);
-    const dt_qk_prologue_params pk = prologue(k, k_out, a[5], none(a[7]) ? a[6] : a[7], eps, per_token, post_scale);
-    const int st = f_prologue(&pq, &pk, PyLong_AsVoidPtr(a[11]));
-    if (st != DT_OK) return PyLong_FromLong(st);
+    void* const stream = PyLong_AsVoidPtr(a[11]);
+    at::Tensor q_out = given(a[2]), k_out = given(a[3]);
+    dt_qk_prologue_params pq = prologue(q, a[4], a[6], eps, per_token, post_scale);
+    dt_qk_prologue_params pk = prologue(k, a[5], none(a[7]) ? a[6] : a[7], eps, per_token, post_scale);
+    int status;
+    {
+      Unlocked here;
+      if (!q_out.defined()) q_out = at::empty_like(q);
+      if (!k_out.defined()) k_out = at::empty_like(k);
+      pq.y = quad(q_out);
+      pk.y = quad(k_out);
+      status = f_prologue(&pq, &pk, stream);
+    }
+    if (status != DT_OK) return PyLong_FromLong(status);
     PyObject* first = none(a[2]) ? THPVariable_Wrap(q_out) : Py_NewRef(a[2]);
     PyObject* second = none(a[3]) ? THPVariable_Wrap(k_out) : Py_NewRef(a[3]);
     PyObject* both = first && second ? PyTuple_Pack(2, first, second) : nullptr;
@@ -284,9 +331,9 @@ PyObject* py_sparse(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (q.dim() != 4 || kr.dim() != 4) decline();
     dt_sparse_indexed_params p;
     memset(&p, 0, sizeof(p));
-    const at::Tensor out = none(a[10]) ? at::empty_like(q) : tensor(a[10]);
+    at::Tensor out = given(a[10]);
+    void* const stream = PyLong_AsVoidPtr(a[13]);
     p.q = quad(q);
-    p.o = quad(out);
     p.k_raw = quad(kr);
     p.v_raw = quad(vr);
     p.B = dim(q, 0);
@@ -324,7 +371,14 @@ PyObject* py_sparse(PyObject*, PyObject* const* a, Py_ssize_t n) {
       p.lse = t.data_ptr<float>();
     }
     p.flags = (uint32_t)whole(a[12], 0, 0xffffffffll);
-    return answer(f_sparse(&p, PyLong_AsVoidPtr(a[13])), out, a[10]);
+    int status;
+    {
+      Unlocked here;
+      if (!out.defined()) out = at::empty_like(q);
+      p.o = quad(out);
+      status = f_sparse(&p, stream);
+    }
+    return answer(status, out, a[10]);
   });
 }
 
