@@ -165,6 +165,7 @@ PyObject* guarded(Py_ssize_t n, Py_ssize_t want, F body) {
   } catch (const NotMine&) {
   } catch (const std::exception&) {  // (no room for the output, a tensor without data: the Python path raises the same)
   }
+  PyErr_Clear();  // what a dispatch mode raised while the output was allocated comes with the error indicator set
   Py_RETURN_NONE;
 }
 

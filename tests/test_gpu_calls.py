@@ -80,3 +80,20 @@ def test_what_is_left_to_the_python_path(dtattn):
     out = torch.zeros_like(q)
     assert dtattn.sdpa_forward(q, k, v, 0.125, out=out) is out
     assert dtattn.sdpa_forward(q, k, v, 1).shape == q.shape  # (a whole number as the scale)
+
+
+def test_what_a_dispatch_mode_raises(dtattn):
+    """An exception from Python code that torch runs inside a native call arrives as it was raised."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Refuses(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            raise ValueError("refused")
+
+    x, row = (torch.zeros(1, n, 2, 64, dtype=torch.float16, device=DEV) for n in (4, 1))
+    for call in (lambda: dtattn.sdpa_forward(x, x, x, 0.125), lambda: dtattn.qk_prologue(x, x),
+                 lambda: dtattn.decode_step(row, x, x, row, row, None, 0.125, 3),
+                 lambda: dtattn.sparse_indexed_attention(x, x, x, None, None, None, 0.125)):
+        call()
+        with pytest.raises(ValueError, match="refused"), Refuses():
+            call()
