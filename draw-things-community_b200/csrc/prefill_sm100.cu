@@ -385,18 +385,15 @@ __device__ __forceinline__ float2 unpack_pair(uint32_t x) {
   else return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x));
 }
 
-template <typename T, int D, bool kMask, bool kSplit, bool kCut>
+// kAhead: see launch_t
+template <typename T, int D, bool kMask, bool kSplit, bool kCut, bool kAhead>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
                        const PrefillArgs a) {
   using C = Cfg<D, kMask>;
   constexpr int kBf16 = std::is_same<T, __half>::value ? 0 : 1;
-  // Two tiles of head dim 64 leave 128 TMEM columns, so P does not have to overwrite S: the next block's Q K^T is issued as soon as
-  // the first half of P says that S has been read, and runs under the second half of the softmax, which used to wait for it (a
-  // quarter of a block's 3600 cycles).  2 images, 4096 tokens, heads of 64: 20 heads 290.2 -> 275.7 us, 10 heads 175.3 -> 163.1; 8 heads
-  // of 40: 124.3 -> 119.5; 300 tokens, 10 heads: 8.8 -> 8.3.
-  constexpr bool kAhead = D == 64 && !kMask;
+  static_assert(!kAhead || (D == 64 && !kMask), "columns for P beside S and O");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -1362,6 +1359,16 @@ template <typename T, int D, bool kMask, bool kSplit = false>
 int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, int n_extra, void* workspace,
              size_t workspace_bytes) {
   using C = Cfg<D, kMask>;
+  // Head dim 64: P beside S and O, and each block's Q K^T ahead of the end of the one before.  Two tiles of head dim 64 leave 128 TMEM
+  // columns, so P does not have to overwrite S: the next block's Q K^T is issued as soon as the first half of P says that S has been
+  // read, and runs under the second half of the softmax, which used to wait for it (a quarter of a block's 3600 cycles).  2 images, 4096
+  // tokens, heads of 64: 20 heads 290.2 -> 275.7 us, 10 heads 175.3 -> 163.1; 8 heads of 40: 124.3 -> 119.5; 300 tokens, 10 heads: 8.8 -> 8.3.
+  // Not where the second block is the last and holds 32 keys at most (two text prompts): its products are short, and every item has a
+  // hand-over more.  Over 48 calls of 777 to 9216 rows, 8 to 20 heads, 2 and 4 images, time without / with it, mean and worst: 154 keys
+  // 0.996 and 0.950 (4 images, 4641 rows, 10 heads: 37.5 / 39.5 us), 160 keys 0.995 and 0.946; 176 keys 1.019 and 0.989, 231 keys
+  // 1.019 and 0.976, 260 keys 1.015 and 1.003, 520 keys 1.033 and 1.017.  (The masked variant has not been built with it.)
+  constexpr bool kMayAhead = D == 64 && !kMask;
+  constexpr int kAheadKeys = kBN + 32;
   CUtensorMap mq, mk, mv, mo;
   if (!make_bshd_tensor_map(&mq, p.q, p.B, p.Sq, p.Hq, p.D, p.dtype, kBM)) return DT_UNSUPPORTED;
   if (!make_bshd_tensor_map(&mk, p.k, p.B, p.Sk, p.Hkv, p.D, p.dtype, kBN)) return DT_UNSUPPORTED;
@@ -1425,14 +1432,17 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
       workspace_bytes >= align256(split_at) + split_bytes(plan, D)) {
     a.n_splits = plan.n_splits;
     a.part = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + align256(split_at));
-    auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, true>;
+    auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, true, kMayAhead>;  // (its runs have at least four blocks)
     DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
     const int runs = plan.n_items * plan.n_splits;
     DT_CUDA_TRY(launch_behind(kern, dim3(runs < n_sm ? runs : n_sm), dim3(kThreads), C::kSmemBytes, stream, 1, mq, mk, mv, mo, a));
     DT_CUDA_TRY(launch_behind(cut_combine_kernel<T, D>, dim3(plan.n_items * (kBM / 32), (p.D + 63) / 64), dim3(256), 0, stream, 1, a));
     return DT_OK;
   }
-  auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, false>;
+  auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, false, false>;
+  if constexpr (kMayAhead) {
+    if ((p.seq_offsets_q != nullptr ? p.max_seq_k : p.Sk) > kAheadKeys) kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, false, true>;
+  }
   DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
   const int ctas = a.n_items < n_sm ? a.n_items : n_sm;  // one persistent CTA per SM
   a.n_slots = plan.n_single > 0 ? plan.n_whole : (a.n_items + ctas - 1) / ctas * ctas;

@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("causal,window", [(False, 0), (True, 0), (True, 200)])
 @pytest.mark.parametrize("D", [40, 64, 128, 256])
-@pytest.mark.parametrize("Sq,Sk", [(130, 640), (300, 1000)])  # whole blocks; a last block of 104 keys
+@pytest.mark.parametrize("Sq,Sk", [(130, 640), (300, 1000),  # whole blocks; a last block of 104 keys
+                                   (300, 160), (300, 161)])  # either side of where the order of the products changes at head dim 64
 def test_growing_maxima(dtattn, Sq, Sk, D, causal, window, dtype):
     q, k, v = inputs(1, Sq, Sk, 2, 1, D, dtype, 1701)
     # The queries' first dimension against a ramp in the keys' first dimension, one step per 64 keys: row i's scores rise by 2^17 from
