@@ -153,7 +153,7 @@ PyObject* answer(int status, const at::Tensor& out, PyObject* given) {
   return none(given) ? THPVariable_Wrap(out) : Py_NewRef(given);
 }
 
-// Runs `body`, with what it throws turned into None.
+// Runs `body`, with what it throws turned into None.  (Nothing is called before bind, whose last assignment is f_sparse.)
 template <typename F>
 PyObject* guarded(Py_ssize_t n, Py_ssize_t want, F body) {
   if (n != want) {
@@ -161,6 +161,7 @@ PyObject* guarded(Py_ssize_t n, Py_ssize_t want, F body) {
     return nullptr;
   }
   try {
+    if (!f_sparse) decline();
     return body();
   } catch (const NotMine&) {
   } catch (const std::exception&) {  // (no room for the output, a tensor without data: the Python path raises the same)

@@ -20,6 +20,7 @@ import importlib.util
 import operator
 import os
 import struct
+import threading
 
 import torch
 
@@ -169,19 +170,29 @@ SYMBOLS = [
 ]
 
 
+_lib_lock = threading.Lock()
+
+
 def lib():
     """The loaded library.  Raises (never falls back) when it has not been built."""
+    return _lib if _lib is not None else _load_lib()
+
+
+def _load_lib():
+    """First use.  The library is published when everything is bound: other threads wait for that, and a failure leaves nothing behind."""
     global _lib
-    if _lib is None:
-        if not os.path.exists(LIB_PATH):
-            raise ImportError(f"{LIB_PATH} not found: build it with `python draw-things-community_b200/build.py`")
-        _lib = ctypes.CDLL(os.path.abspath(LIB_PATH))
-        for name, res, args in SYMBOLS:
-            fn = getattr(_lib, name)
-            fn.restype = res
-            fn.argtypes = args
-        _calls.bind(*[ctypes.cast(getattr(_lib, name), ctypes.c_void_p).value for name in _CALLS])
-    return _lib
+    with _lib_lock:
+        if _lib is None:
+            if not os.path.exists(LIB_PATH):
+                raise ImportError(f"{LIB_PATH} not found: build it with `python draw-things-community_b200/build.py`")
+            loaded = ctypes.CDLL(os.path.abspath(LIB_PATH))
+            for name, res, args in SYMBOLS:
+                fn = getattr(loaded, name)
+                fn.restype = res
+                fn.argtypes = args
+            _calls.bind(*[ctypes.cast(getattr(loaded, name), ctypes.c_void_p).value for name in _CALLS])
+            _lib = loaded
+        return _lib
 
 
 # What the native module calls, in the order of its bind

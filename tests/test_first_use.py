@@ -1,0 +1,74 @@
+"""The library on first use: published when it is ready, whoever asks for it."""
+import ctypes
+import os
+import subprocess
+import sys
+import threading
+import time
+
+import pytest
+
+
+class Calls:
+    """Stands in for the native module."""
+
+    def __init__(self, on_bind):
+        self.on_bind = on_bind
+
+    def bind(self, *addresses):
+        self.on_bind()
+
+
+@pytest.fixture
+def unloaded(dtattn, monkeypatch):
+    """As before the first use, with a native module whose bind does what the test says."""
+    def prepare(on_bind):
+        monkeypatch.setattr(dtattn, "_lib", None)
+        monkeypatch.setattr(dtattn, "_calls", Calls(on_bind))
+        monkeypatch.setattr(dtattn, "_load_calls", lambda: Calls(on_bind), raising=False)
+    return prepare
+
+
+def test_a_second_thread_waits_for_the_first(dtattn, unloaded):
+    bound, early = [], []
+
+    def slowly():
+        time.sleep(0.3)
+        bound.append(True)
+
+    def use():
+        dtattn.lib().dt_abi_version()
+        early.append(not bound)
+
+    unloaded(slowly)
+    threads = [threading.Thread(target=use) for _ in range(4)]
+    for t in threads:
+        t.start()
+        time.sleep(0.03)
+    for t in threads:
+        t.join()
+    assert early == [False] * 4 and bound == [True]
+
+
+def test_a_failure_is_not_taken_for_a_library(dtattn, unloaded):
+    def fails():
+        raise OSError("no such symbol")
+
+    unloaded(fails)
+    for _ in range(2):
+        with pytest.raises(OSError):
+            dtattn.lib()
+    assert dtattn._lib is None
+
+
+def test_the_native_module_calls_nothing_before_it_is_bound(dtattn):
+    child = """
+import importlib.util, sys, torch
+spec = importlib.util.spec_from_file_location("dtattn_calls", sys.argv[1])
+module = importlib.util.module_from_spec(spec)
+spec.loader.exec_module(module)
+print("RESULT", module.run(bytes(int(sys.argv[2])), None, 0, 0, 0))
+"""
+    r = subprocess.run([sys.executable, "-c", child, dtattn._calls.__file__, str(ctypes.sizeof(dtattn.SdpaParams))],
+                       capture_output=True, text=True, cwd=os.path.dirname(os.path.abspath(__file__)))
+    assert r.returncode == 0 and "RESULT None" in r.stdout, r.stderr
