@@ -180,7 +180,7 @@ def lib():
 
 def _load_lib():
     """First use.  The library is published when everything is bound: other threads wait for that, and a failure leaves nothing behind."""
-    global _lib
+    global _lib, _calls
     with _lib_lock:
         if _lib is None:
             if not os.path.exists(LIB_PATH):
@@ -190,6 +190,7 @@ def _load_lib():
                 fn = getattr(loaded, name)
                 fn.restype = res
                 fn.argtypes = args
+            _calls = _load_calls()
             _calls.bind(*[ctypes.cast(getattr(loaded, name), ctypes.c_void_p).value for name in _CALLS])
             _lib = loaded
         return _lib
@@ -211,7 +212,7 @@ def _load_calls():
     return module
 
 
-_calls = _load_calls()
+_calls = None  # with _lib
 
 
 def _raw_stream(index):

@@ -1,6 +1,7 @@
 """The library on first use: published when it is ready, whoever asks for it."""
 import ctypes
 import os
+import shutil
 import subprocess
 import sys
 import threading
@@ -72,3 +73,27 @@ print("RESULT", module.run(bytes(int(sys.argv[2])), None, 0, 0, 0))
     r = subprocess.run([sys.executable, "-c", child, dtattn._calls.__file__, str(ctypes.sizeof(dtattn.SdpaParams))],
                        capture_output=True, text=True, cwd=os.path.dirname(os.path.abspath(__file__)))
     assert r.returncode == 0 and "RESULT None" in r.stdout, r.stderr
+
+
+def test_importing_needs_no_build(dtattn, tmp_path):
+    """What calls no kernel works from the sources alone; the first use of the library says what is missing."""
+    shutil.copytree(os.path.dirname(dtattn.__file__), tmp_path / "pkg" / "dtattn", ignore=shutil.ignore_patterns("__pycache__"))
+    child = """
+import os, sys
+sys.path.insert(0, sys.argv[1])
+import dtattn
+from dtattn import selection, sharding
+assert os.path.dirname(dtattn.__file__).startswith(sys.argv[1])
+dtattn.SdpaParams()
+for library in (dtattn.LIB_PATH, sys.argv[2]):  # neither is there; only the native module is missing
+    dtattn.LIB_PATH = library
+    for _ in range(2):
+        try:
+            dtattn.lib()
+        except ImportError as e:
+            print("RESULT", str(e).split()[0])
+"""
+    r = subprocess.run([sys.executable, "-c", child, str(tmp_path / "pkg"), dtattn.LIB_PATH], capture_output=True, text=True)
+    said = [os.path.basename(line.split()[1]) for line in r.stdout.splitlines() if line.startswith("RESULT")]
+    assert r.returncode == 0 and [x.startswith("libdtattn") for x in said] == [True, True, False, False], (said, r.stderr)
+    assert all("dtattn_calls" in x for x in said[2:])
