@@ -75,26 +75,31 @@ WAIT_TEST_DEFINES = ("DT_BRINGUP", "DT_WAIT_LIMIT_NS=5000000ull")
 
 
 # The Python surface's calls in native code (an extension module on torch's own headers and libraries).
-CALLS = os.path.join(LIB_DIR, "dtattn_calls.so")
+def calls_path():
+    if HERE not in sys.path:
+        sys.path.insert(0, HERE)
+    import dtattn
+    return os.path.join(LIB_DIR, dtattn.calls_name())
 
 
 def build_calls(force=False):
     import sysconfig
     import torch
+    out = calls_path()
     src, header = os.path.join(CSRC, "py_calls.cpp"), os.path.join(HERE, "..", "include", "dtattn.h")
-    if force or not os.path.exists(CALLS) or os.path.getmtime(CALLS) < _newest([src, header]):
+    if force or not os.path.exists(out) or os.path.getmtime(out) < _newest([src, header]):
         os.makedirs(LIB_DIR, exist_ok=True)
         t = os.path.dirname(torch.__file__)
         cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
                *["-I" + d for d in (os.path.join(HERE, "..", "include"), os.path.join(t, "include"),
                                     os.path.join(t, "include", "torch", "csrc", "api", "include"),
                                     sysconfig.get_paths()["include"], "/usr/local/cuda/include")],
-               src, "-o", CALLS, "-L" + os.path.join(t, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10"]
+               src, "-o", out, "-L" + os.path.join(t, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10"]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("g++ failed: " + src)
-    return CALLS
+    return out
 
 
 def build_all(force=False):

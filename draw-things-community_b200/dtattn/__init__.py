@@ -20,6 +20,7 @@ import importlib.util
 import operator
 import os
 import struct
+import sysconfig
 import threading
 
 import torch
@@ -201,9 +202,15 @@ _CALLS = ["dt_sdpa_workspace_size", "dt_sdpa_kernel_name", "dt_sdpa_forward", "d
           "dt_sdpa_decode_step", "dt_qk_prologue", "dt_sparse_indexed_attention"]
 
 
+def calls_name():
+    """The native module's file name: it is compiled against one torch's and one Python's headers, and carries both in its name, so that a
+    file built for others is neither loaded nor taken for up to date."""
+    return f"dtattn_calls.torch{torch.__version__}.abi{int(torch._C._GLIBCXX_USE_CXX11_ABI)}.{sysconfig.get_config_var('SOABI')}.so"
+
+
 def _load_calls():
     """The usual calls in native code (csrc/py_calls.cpp).  Raises (never falls back) when it has not been built."""
-    path = os.path.abspath(os.path.join(_HERE, "..", "lib", "dtattn_calls.so"))
+    path = os.path.abspath(os.path.join(_HERE, "..", "lib", calls_name()))
     if not os.path.exists(path):
         raise ImportError(f"{path} not found: build it with `python draw-things-community_b200/build.py`")
     spec = importlib.util.spec_from_file_location("dtattn_calls", path)

@@ -1,13 +1,16 @@
 """The library on first use: published when it is ready, whoever asks for it."""
 import ctypes
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import threading
 import time
 
 import pytest
+import torch
 
 
 class Calls:
@@ -97,3 +100,20 @@ for library in (dtattn.LIB_PATH, sys.argv[2]):  # neither is there; only the nat
     said = [os.path.basename(line.split()[1]) for line in r.stdout.splitlines() if line.startswith("RESULT")]
     assert r.returncode == 0 and [x.startswith("libdtattn") for x in said] == [True, True, False, False], (said, r.stderr)
     assert all("dtattn_calls" in x for x in said[2:])
+
+
+def test_a_module_built_for_another_torch_is_not_loaded(dtattn, monkeypatch):
+    """Neither loaded nor taken for up to date: the torch and the Python that it is compiled against are in its name."""
+    spec = importlib.util.spec_from_file_location("dt_build", os.path.join(os.path.dirname(dtattn.__file__), "..", "build.py"))
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    here = build.build_calls()
+    assert os.path.samefile(here, dtattn._calls.__file__)
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    assert not os.path.exists(build.calls_path())
+    with pytest.raises(ImportError, match="torch0.0.1"):
+        dtattn._load_calls()
+    monkeypatch.undo()
+    monkeypatch.setattr(sysconfig, "get_config_var", lambda name: "cpython-000")
+    with pytest.raises(ImportError, match="cpython-000"):
+        dtattn._load_calls()
