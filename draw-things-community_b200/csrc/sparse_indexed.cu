@@ -558,8 +558,8 @@ sparse_mma_kernel(const SparseArgs a, const SparseMmaExtra x) {
 //      eight partial scores meet in shared memory, where half a warp per query row adds them and takes the softmax;
 //   O: warp w takes the same head dims of P V and stores its accumulators straight into the shared memory of CTA w of the
 //      cluster, which owns these columns: one cluster barrier later the eight shares are added from local memory.
-// Bound: latency (launch, index, row, two products, exchange).  64 heads of 512, 128 + 512 keys, one token, in a graph: 17.8 us in
-// sparse_mma_kernel (three tiles of 32 keys in turn per CTA, four warps, shares read from the other CTAs), 8.5 us here.
+// Bound: latency (launch, index, row, two products, exchange).  64 heads of 512, 128 + 512 keys, one token, in a graph: 17.7 us in
+// sparse_mma_kernel (three tiles of 32 keys in turn per CTA, four warps, shares read from the other CTAs), 7.7 us here.
 constexpr int kOnceSplit = 8;    // CTAs of a cluster, and warps of a CTA
 constexpr int kOnceKeys = 80;    // keys per CTA
 constexpr int kOncePitch = 88;   // of the partial scores (words) and of P (16-bit): rows on distinct banks
@@ -872,7 +872,12 @@ int launch_sparse_mma_t(const dt_sparse_indexed_params& p, const SparseArgs& a, 
     const int st = launch_sparse_tcgen05(p, stream);
     if (st != DT_UNSUPPORTED) return st;  // (views that no tensor map describes, expanded queries for one: nothing was launched)
   }
-  // Clusters that fit the SMs in one wave (a CTA's 180 KB leave room for one per SM).
+  // Up to 640 keys (a CTA's share of 80 rows: 180 of 227 KB at head dim 512) and clusters that fit the SMs in one wave (one CTA per SM).
+  // One token of 64 heads, in a graph, us here / in sparse_mma_kernel, head dim 512 and (256): 128 keys 5.1 / 15.2 (4.0 / 9.9), 512
+  // keys 7.1 / 13.8 (5.5 / 9.3), 640 keys 7.7 / 17.7 (6.0 / 11.5).  640 is what the shares were laid out for and not where it stops
+  // paying: with shares of 96 rows (207 KB) 641 to 768 keys took 8.3 / 17.7 (6.4 / 11.7).  One wave: 4 tokens (128 CTAs) of 256 keys 11.7 /
+  // 14.4 (9.4 / 9.7), of 640 keys 15.1 / 20.3 (11.9 / 13.7); 5 tokens (160 CTAs) of 640 keys 15.5 / 20.4 (12.0 / 13.8), 8 tokens (256)
+  // of 256 keys 17.6 / 14.9 (13.8 / 9.9), of 640 keys 23.1 / 21.1 (17.9 / 14.0): the line lies between 5 and 8 tokens, not tried closer.
   const long long keys = most_keys(p);
   const long long groups = (long long)p.Hkv * ((p.Hq / p.Hkv + 15) / 16);
   if ((p.D == 256 || (p.D == 512 && same_kv)) && keys > 0 && keys <= kOnceSplit * kOnceKeys && groups <= 65535 &&

@@ -97,3 +97,49 @@ def test_what_a_dispatch_mode_raises(dtattn):
         call()
         with pytest.raises(ValueError, match="refused"), Refuses():
             call()
+
+
+def test_both_paths_refuse_alike(dtattn, python_only):
+    """The same exception with the same text, whichever path a call takes first.  (Every call here is refused on the host.)"""
+    H = torch.float16
+    q, k, v = (x.to(DEV) for x in inputs(1, 64, 64, 4, 2, 64, H, 2021))
+    mask, lse, sinks = torch.zeros(1, 1, 64, 64, device=DEV, dtype=H), torch.zeros(1, 4, 64, device=DEV), torch.zeros(4, device=DEV, dtype=H)
+    row, kn, rot, w = q[:, :1], k[:, :1].clone(), torch.zeros(1, 1, 64, device=DEV, dtype=H), torch.zeros(64, device=DEV, dtype=H)
+    table, sel = torch.zeros(1, 64, 1, 64, device=DEV, dtype=H), torch.zeros(1, 64, 8, device=DEV, dtype=torch.int32)
+    wide = torch.zeros(1, 4, 4, 1024, device=DEV, dtype=H)
+    nan = float("nan")
+    sdpa = lambda **kw: dtattn.sdpa_forward(**dict(dict(q=q, k=k, v=v, scale=0.125), **kw))  # noqa: E731
+    step = lambda **kw: dtattn.decode_step(**dict(dict(q=row, k_cache=k, v_cache=v, k_new=kn, v_new=kn, rotary=rot, scale=0.125,  # noqa: E731
+                                                       cached_len=63), **kw))
+    prologue = lambda **kw: dtattn.qk_prologue(**dict(dict(q=q, k=k, q_weight=w, k_weight=w, rotary=table), **kw))  # noqa: E731
+    sparse = lambda **kw: dtattn.sparse_indexed_attention(**dict(dict(q=q, k_raw=k, v_raw=v, k_comp=k, v_comp=v, selected=sel,  # noqa: E731
+                                                                      scale=0.125), **kw))
+    refused = [
+        (sdpa, kw) for kw in (dict(q=q[0]), dict(q=q.transpose(2, 3)), dict(q=q.double(), k=k.double(), v=v.double()), dict(scale="x"), dict(scale=nan),
+                              dict(sliding_window=-1), dict(mask=mask[0]), dict(mask=mask[..., :63]), dict(mask=mask.float()),
+                              dict(mask=mask.transpose(2, 3)), dict(lse=lse[..., :63]), dict(lse=lse.to(H)), dict(sinks=sinks[:3]), dict(sinks=sinks.float()),
+                              dict(q=q[:, :, :3]), dict(q=wide, k=wide, v=wide), dict(flags="x"), dict(sliding_window="x"))] + [
+        (step, kw) for kw in (dict(cached_len=63.0), dict(cached_len="x"), dict(rotary=rot[0]), dict(rotary=rot.float()), dict(rotary=rot[:, :0]),
+                              dict(q_norm_weight=w[:63]), dict(k_norm_weight=w.float()), dict(scale=nan), dict(sliding_window=-1),
+                              dict(lse=lse), dict(sinks=sinks[:3]), dict(norm_eps="x"), dict(q=q))] + [
+        (prologue, kw) for kw in (dict(q=q[0]), dict(q_weight=w[:63]), dict(k_weight=w.float()), dict(rotary=table[0]), dict(rotary=table[:, :63]),
+                                  dict(rotary=table.float()), dict(rotary_k=table[..., :32]), dict(eps="x"), dict(norm_per_token=True),
+                                  dict(q=q.double(), q_weight=None, rotary=None))] + [
+        (sparse, kw) for kw in (dict(q=q[0]), dict(selected=sel.long()), dict(selected=sel[0]), dict(selected=sel[:, :63]), dict(scale=nan),
+                                dict(sliding_window=-1), dict(sinks=sinks[:3]), dict(sinks=sinks.float()), dict(lse=lse[..., :63]), dict(lse=lse.to(H)),
+                                dict(q=q[:, :, :3]), dict(q=wide, k_raw=wide, v_raw=wide, k_comp=None, v_comp=None, selected=None), dict(scale="x"))]
+
+    def answers():
+        out = []
+        for call, kw in refused:
+            with pytest.raises(Exception) as e:
+                call(**kw)
+            out.append((call, list(kw), e.type, str(e.value)))
+        return out
+
+    native = answers()
+    python_only()
+    for a, b in zip(native, answers()):
+        assert a == b
+    torch.cuda.synchronize()
+    assert dtattn.device_status() == 0

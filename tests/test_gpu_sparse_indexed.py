@@ -19,9 +19,9 @@ def make_case(B, Sq, Sr, Sc, n_sel, Hq, Hkv, D, dtype, seed, per_batch_lists=Fal
     kc = so.seeded_normal((B, max(Sc, 1), Hkv, D), seed + 3).to(dtype)[:, :Sc]
     vc = so.seeded_normal((B, max(Sc, 1), Hkv, D), seed + 4).to(dtype)[:, :Sc]
     g = torch.Generator().manual_seed(seed)
-    # lists with duplicates, "no row" entries (-1 and beyond the end) and, for some queries, nothing valid at all
+    # lists with duplicates, "no row" entries (-1 and beyond the end) and, for some queries (never the only one), nothing valid at all
     sel = torch.randint(-2, Sc + 2, (B if per_batch_lists else 1, Sq, n_sel), generator=g, dtype=torch.int32)
-    sel[:, ::5] = -1
+    sel[:, 1::5] = -1
     sinks = (so.seeded_normal((Hq,), seed + 5) * 2).to(dtype)
     return q, kr, vr, kc, vc, sel, sinks
 
