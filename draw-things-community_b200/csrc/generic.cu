@@ -380,9 +380,9 @@ __device__ __forceinline__ void generic_tiled_block(const dim3 block, const T* _
 // SMs hold at a time, which look into only_if first and then take all the blocks in turn: a CTA per block that only returns cost
 // 4 us for 1024 of them.
 template <bool kIf, typename Body>
-__device__ __forceinline__ void run_blocks(const uint32_t* __restrict__ only_if, const dim3 grid, Body body) {
+__device__ __forceinline__ void run_blocks(const uint32_t* __restrict__ only_if, const dim3 grid, const int let_next, Body body) {
   ptx::wait_for_previous();
-  ptx::let_next_start();
+  if (let_next) ptx::let_next_start();
   if constexpr (kIf) {
     if (*only_if == 0u) return;
     const uint64_t total = (uint64_t)grid.x * grid.y * grid.z;
@@ -394,6 +394,13 @@ __device__ __forceinline__ void run_blocks(const uint32_t* __restrict__ only_if,
   } else {
     body(dim3(blockIdx.x, blockIdx.y, blockIdx.z));
   }
+}
+// Whether the next kernel may be brought in while this one runs: only where it finds SMs without a CTA.  Its CTAs are placed where there
+// is room at that moment, so a call of a full round had the next one's crowd onto the SMs that were done first (300 tokens under a
+// mask, 8 heads of 37, fp32: 304 CTAs, 69.8 us alone, 86.5 behind another that way; 1200 tokens, 2 heads: 264 and 315; 8 heads of 64, 152
+// CTAs: 291 and 303).  With a CTA on half of the SMs at most it gains up to 1 us (600 tokens, 2 heads of 64: 125.2 and 124.0).
+int lets_next_start(dim3 ctas, const uint32_t* only_if) {
+  return only_if != nullptr || 2ull * ctas.x * ctas.y * ctas.z <= (uint64_t)device_sm_count();
 }
 dim3 launch_grid(dim3 grid, int threads, size_t smem, const uint32_t* only_if) {
   if (!only_if) return grid;
@@ -409,17 +416,17 @@ dim3 launch_grid(dim3 grid, int threads, size_t smem, const uint32_t* only_if) {
       int64_t v_sb, int64_t v_ss, int64_t v_sh, int64_t o_sb, int64_t o_ss, int64_t o_sh, int64_t m_sb, int64_t m_sh,           \
       int64_t m_sq, int Sq, int Sk, int Hq, int Hkv, int D, float scale_log2, int is_causal, const T *__restrict__ sinks,       \
       int window, const int32_t *__restrict__ off_q, const int32_t *__restrict__ off_k, const uint32_t *__restrict__ only_if,   \
-      const dim3 grid
+      const dim3 grid, const int let_next
 #define DT_GENERIC_ARGS                                                                                                        \
   q, k, v, o, mask, lse, q_sb, q_ss, q_sh, k_sb, k_ss, k_sh, v_sb, v_ss, v_sh, o_sb, o_ss, o_sh, m_sb, m_sh, m_sq, Sq, Sk, Hq,  \
       Hkv, D, scale_log2, is_causal, sinks, window, off_q, off_k
 template <typename T, bool kIf>
 __global__ void __launch_bounds__(kRows * 32) generic_sdpa_kernel(DT_GENERIC_PARAMS) {
-  run_blocks<kIf>(only_if, grid, [&](const dim3 block) { generic_sdpa_block<T>(block, DT_GENERIC_ARGS); });
+  run_blocks<kIf>(only_if, grid, let_next, [&](const dim3 block) { generic_sdpa_block<T>(block, DT_GENERIC_ARGS); });
 }
 template <typename T, int R, bool kIf>
 __global__ void __launch_bounds__(kTThreads) generic_tiled_kernel(DT_GENERIC_PARAMS) {
-  run_blocks<kIf>(only_if, grid, [&](const dim3 block) { generic_tiled_block<T, R>(block, DT_GENERIC_ARGS); });
+  run_blocks<kIf>(only_if, grid, let_next, [&](const dim3 block) { generic_tiled_block<T, R>(block, DT_GENERIC_ARGS); });
 }
 #undef DT_GENERIC_PARAMS
 #undef DT_GENERIC_ARGS
@@ -438,7 +445,7 @@ int launch_tiled(const dt_sdpa_params& p, cudaStream_t stream, const uint32_t* o
       p.q.stride_b, p.q.stride_s, p.q.stride_h, p.k.stride_b, p.k.stride_s, p.k.stride_h,
       p.v.stride_b, p.v.stride_s, p.v.stride_h, p.o.stride_b, p.o.stride_s, p.o.stride_h,
       p.mask_stride_b, p.mask_stride_h, p.mask_stride_q, p.Sq, p.Sk, p.Hq, p.Hkv, D, p.scale * kLog2e,
-      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if, grid));
+      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if, grid, lets_next_start(grid, only_if)));
   return DT_OK;
 }
 
@@ -463,7 +470,7 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, const uint32_t* only_
       p.q.stride_b, p.q.stride_s, p.q.stride_h, p.k.stride_b, p.k.stride_s, p.k.stride_h,
       p.v.stride_b, p.v.stride_s, p.v.stride_h, p.o.stride_b, p.o.stride_s, p.o.stride_h,
       p.mask_stride_b, p.mask_stride_h, p.mask_stride_q, p.Sq, p.Sk, p.Hq, p.Hkv, D, p.scale * kLog2e,
-      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if, grid));
+      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if, grid, lets_next_start(grid, only_if)));
   return DT_OK;
 }
 
