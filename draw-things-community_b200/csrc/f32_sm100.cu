@@ -539,10 +539,10 @@ int launch_t(const dt_sdpa_params& p, void* workspace, cudaStream_t stream) {
     planes += plane_bytes(p, S, H);
   }
   const unsigned need = (sp.n_pieces + kSplitThreads - 1) / kSplitThreads;
-  const unsigned ctas = need < (unsigned)kSplitCtas ? need : (unsigned)kSplitCtas;
+  const unsigned split_ctas = need < (unsigned)kSplitCtas ? need : (unsigned)kSplitCtas;
   a.flags = flags;
   a.any_flag = flags + kSplitCtas;
-  a.n_flags = (int)ctas;
+  a.n_flags = (int)split_ctas;
   a.o = static_cast<float*>(p.o.ptr);
   a.lse = p.lse;
   a.o_sb = p.o.stride_b; a.o_ss = p.o.stride_s; a.o_sh = p.o.stride_h;
@@ -553,9 +553,22 @@ int launch_t(const dt_sdpa_params& p, void* workspace, cudaStream_t stream) {
   auto kern = f32_tcgen05_kernel<NPV>;
   DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
   const int n_sm = device_sm_count();
-  DT_CUDA_TRY(launch_behind(split_planes_kernel, dim3(ctas), dim3(kSplitThreads), 0, stream, 1, sp));
-  DT_CUDA_TRY(launch_behind(kern, dim3(a.n_items < n_sm ? a.n_items : n_sm), dim3(kThreads), C::kSmemBytes, stream, 1, maps[0], maps[1],
-                            maps[2], a));
+  DT_CUDA_TRY(launch_behind(split_planes_kernel, dim3(split_ctas), dim3(kSplitThreads), 0, stream, 1, sp));
+  // CTAs that come in while the splitting pass runs out land where there is room, not spread over the SM pairs and dies as those of an ordinary
+  // launch are.  Long calls lose more by that than the hidden launch gives: those of several rounds, and those of one round that leaves
+  // a tenth to half of the SMs empty.  Us in a graph, ordinary launches before and after / overlapped / this rule: 2 x 6144 tokens, 10 heads of
+  // 40 894 / 933 / 874, 10 heads of 64 856 / 900 / 860 (cool GPU); one image, 5200 tokens, 8 heads of 64 318 / 327 / 319; 2500 tokens, 5 heads of
+  // 64 (100 items) 59.5 / 62.2 / 58.8, of 40 54.7 / 56.4 / 53.6.  Shorter calls gain (2 x 1800 tokens, 8 heads of 40, called from Python:
+  // ordinary 86.7, overlapped 84.1), and so do all of head dims 65 to 80 (2 x 4100 tokens, 10 heads of 80: 740 / 706, ordinary 727).
+  const bool uneven = a.n_items <= n_sm && 2 * a.n_items > n_sm && 10 * a.n_items <= 9 * n_sm && p.Sk > 1536;
+  const bool rounds = a.n_items > n_sm && p.Sk > 2048;
+  const int ctas = a.n_items < n_sm ? a.n_items : n_sm;
+  if (NPV == 80 || !(uneven || rounds)) {
+    DT_CUDA_TRY(launch_behind(kern, dim3(ctas), dim3(kThreads), C::kSmemBytes, stream, 1, maps[0], maps[1], maps[2], a));
+  } else {
+    kern<<<ctas, kThreads, C::kSmemBytes, stream>>>(maps[0], maps[1], maps[2], a);
+    DT_CUDA_TRY(cudaGetLastError());
+  }
   return launch_generic(p, stream, a.any_flag);  // returns at once unless the inputs could not be split
 }
 
