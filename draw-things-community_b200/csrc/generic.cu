@@ -395,12 +395,23 @@ __device__ __forceinline__ void run_blocks(const uint32_t* __restrict__ only_if,
     body(dim3(blockIdx.x, blockIdx.y, blockIdx.z));
   }
 }
-// Whether the next kernel may be brought in while this one runs: only where it finds SMs without a CTA.  Its CTAs are placed where there
-// is room at that moment, so a call of a full round had the next one's crowd onto the SMs that were done first (300 tokens under a
-// mask, 8 heads of 37, fp32: 304 CTAs, 69.8 us alone, 86.5 behind another that way; 1200 tokens, 2 heads: 264 and 315; 8 heads of 64, 152
-// CTAs: 291 and 303).  With a CTA on half of the SMs at most it gains up to 1 us (600 tokens, 2 heads of 64: 125.2 and 124.0).
-int lets_next_start(dim3 ctas, const uint32_t* only_if) {
-  return only_if != nullptr || 2ull * ctas.x * ctas.y * ctas.z <= (uint64_t)device_sm_count();
+// How a launch goes behind the kernel before it, and the next one behind it.  CTAs that are placed while the kernel before them runs out
+// crowd together, several to an SM, and these compute for long.  Behind a prologue of 64 tokens, both kernels, us, ordinary / early: 300
+// tokens under a mask, 8 heads of 37, fp32 72.1 / 91.3; 100 tokens, 4 heads of 64 30.5 / 37.1; behind themselves 69.8 / 86.5 (304 CTAs of 300
+// tokens), 264 / 315 (1200 tokens, 2 heads of 37), 291 / 303 (152 CTAs of 1200 tokens, 8 heads of 64).  So a launch comes in early only as
+// the one that usually returns at once, or with at most a CTA per SM, and then asks for more than half of an SM's shared memory, which keeps
+// them one to an SM.  It lets the next kernel in early where that finds SMs without a CTA (600 tokens, 2 heads of 64: 125.2 / 124.0).
+struct Neighbours {
+  bool early;
+  int let_next;
+  size_t smem;
+};
+Neighbours neighbours(dim3 ctas, size_t smem, const uint32_t* only_if) {
+  if (only_if) return {true, 1, smem};
+  const uint64_t n = (uint64_t)ctas.x * ctas.y * ctas.z, sms = (uint64_t)device_sm_count();
+  if (n > sms) return {false, 0, smem};
+  constexpr size_t kLone = 116 * 1024;
+  return {true, 2 * n <= sms, smem < kLone ? kLone : smem};
 }
 dim3 launch_grid(dim3 grid, int threads, size_t smem, const uint32_t* only_if) {
   if (!only_if) return grid;
@@ -436,16 +447,17 @@ int launch_tiled(const dt_sdpa_params& p, cudaStream_t stream, const uint32_t* o
   const int D = p.D;
   const size_t smem = sizeof(float) * ((size_t)(kTM + kTN) * tiled_pitch(D) + (size_t)kTN * D + (size_t)kTM * kPPitch);
   auto kern = only_if ? generic_tiled_kernel<T, R, true> : generic_tiled_kernel<T, R, false>;
-  if (smem > 48 * 1024) DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const bool varlen = p.seq_offsets_q != nullptr;
   dim3 grid(((varlen ? p.max_seq_q : p.Sq) + kTM - 1) / kTM, p.Hq, varlen ? p.n_seq : p.B);
-  DT_CUDA_TRY(launch_behind(
-      kern, launch_grid(grid, kTThreads, smem, only_if), dim3(kTThreads), smem, stream, 1,
+  const Neighbours nb = neighbours(grid, smem, only_if);
+  if (nb.smem > 48 * 1024) DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nb.smem));
+  DT_CUDA_TRY(launch(
+      nb.early, kern, launch_grid(grid, kTThreads, smem, only_if), dim3(kTThreads), nb.smem, stream, 1,
       (const T*)p.q.ptr, (const T*)p.k.ptr, (const T*)p.v.ptr, (T*)p.o.ptr, (const T*)p.mask, p.lse,
       p.q.stride_b, p.q.stride_s, p.q.stride_h, p.k.stride_b, p.k.stride_s, p.k.stride_h,
       p.v.stride_b, p.v.stride_s, p.v.stride_h, p.o.stride_b, p.o.stride_s, p.o.stride_h,
       p.mask_stride_b, p.mask_stride_h, p.mask_stride_q, p.Sq, p.Sk, p.Hq, p.Hkv, D, p.scale * kLog2e,
-      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if, grid, lets_next_start(grid, only_if)));
+      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if, grid, nb.let_next));
   return DT_OK;
 }
 
@@ -461,16 +473,17 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, const uint32_t* only_
   }
   const size_t smem = sizeof(float) * ((size_t)kRows * D + (size_t)kKeys * (D | 1) + (size_t)kKeys * D);
   auto kern = only_if ? generic_sdpa_kernel<T, true> : generic_sdpa_kernel<T, false>;
-  if (smem > 48 * 1024) DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const bool varlen = p.seq_offsets_q != nullptr;
   dim3 grid(((varlen ? p.max_seq_q : p.Sq) + kRows - 1) / kRows, p.Hq, varlen ? p.n_seq : p.B);
-  DT_CUDA_TRY(launch_behind(
-      kern, launch_grid(grid, kRows * 32, smem, only_if), dim3(kRows * 32), smem, stream, 1,
+  const Neighbours nb = neighbours(grid, smem, only_if);
+  if (nb.smem > 48 * 1024) DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nb.smem));
+  DT_CUDA_TRY(launch(
+      nb.early, kern, launch_grid(grid, kRows * 32, smem, only_if), dim3(kRows * 32), nb.smem, stream, 1,
       (const T*)p.q.ptr, (const T*)p.k.ptr, (const T*)p.v.ptr, (T*)p.o.ptr, (const T*)p.mask, p.lse,
       p.q.stride_b, p.q.stride_s, p.q.stride_h, p.k.stride_b, p.k.stride_s, p.k.stride_h,
       p.v.stride_b, p.v.stride_s, p.v.stride_h, p.o.stride_b, p.o.stride_s, p.o.stride_h,
       p.mask_stride_b, p.mask_stride_h, p.mask_stride_q, p.Sq, p.Sk, p.Hq, p.Hkv, D, p.scale * kLog2e,
-      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if, grid, lets_next_start(grid, only_if)));
+      p.is_causal, (const T*)p.sinks, p.sliding_window, p.seq_offsets_q, p.seq_offsets_k, only_if, grid, nb.let_next));
   return DT_OK;
 }
 

@@ -476,26 +476,33 @@ __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.
 // ---- host: a launch whose CTAs may start while the kernel before it in the stream runs out: launch overhead, barrier set-up, TMEM
 // allocation and the fetch of the tensor maps are then off the path.  Every thread that touches global memory calls
 // wait_for_previous() first or is behind a barrier with one that has, in every CTA (so that a kernel's end still means that all
-// before it have ended); the order of results is that of an ordinary launch.
+// before it have ended); the order of results is that of an ordinary launch, which launch(false, ...) is.
 template <typename... P, typename... A>
-cudaError_t launch_behind(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, A&&... args) {
+cudaError_t launch(bool behind, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2] = {};
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  unsigned n = 0;
+  if (behind) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
   if (cluster > 1) {
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = (unsigned)cluster;
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = (unsigned)cluster;
+    attr[n].val.clusterDim.y = 1;
+    attr[n++].val.clusterDim.z = 1;
   }
   cfg.attrs = attr;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
+template <typename... P, typename... A>
+cudaError_t launch_behind(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, A&&... args) {
+  return launch(true, kern, grid, block, smem, stream, cluster, std::forward<A>(args)...);
 }
 
 // ---- host: tensor-map encoding through the driver entry point (no link-time libcuda dependency) ----
