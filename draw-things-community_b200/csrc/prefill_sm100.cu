@@ -99,7 +99,6 @@ struct PrefillArgs {
   float scale;  // the plain scale (scale_log2 = scale * log2(e)); the masked variant adds the mask in this domain
   int item_rows;          // query rows of a work item: a pair of tiles, or one tile where pairs would leave SMs idle
   int n_qpairs, n_items;  // work items = (batch, head, item_rows query rows)
-  int let_next;           // the next kernel may be brought in while this one runs
   // Items in whole rounds over the grid: n_slots of them, of which the causal order may leave some empty.  The items from
   // n_slots on (fewer than one round) are pairs of tiles taken tile by tile; n_places counts those tiles too.
   int n_slots;
@@ -117,6 +116,7 @@ struct PrefillArgs {
   void* extra_o[kMaxExtraOutputs];
   int n_extra;
   int d_real;  // the tensors' head dim (<= the kernel's D): TMA zero-fills the columns beyond it on load and clips them on store
+  int cut_lets_next;  // the cut kernel: cut_combine_kernel may be brought in while it runs
 };
 
 struct Barriers {
@@ -525,7 +525,9 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const uint32_t tmem = bars->tmem_base;
   volatile int* abort_flag = &bars->abort_flag;
   ptx::wait_for_previous();
-  if (a.let_next) ptx::let_next_start();
+  // (Calls of several rounds do not overlap their neighbours: 32 / 8 heads of 128 under an unaligned mask, 1001 tokens 47.4 -> 45.7 us
+  // with it, but 1501 tokens 62.1 -> 65.0 and 2047 tokens 76.5 -> 82.4.)
+  if (kCut ? a.cut_lets_next != 0 : a.n_items <= (int)gridDim.x) ptx::let_next_start();
 
   // Register budget: the data-movement warpgroup gives registers back, the softmax warpgroups take them.
   // (Each setmaxnreg must dominate the code it governs, hence the nesting.)
@@ -1438,7 +1440,7 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
     // are free.  Launched behind the runs / early / by this rule, us: 8 heads of 256, 128 x 16000 (144 runs) 32.0 / 34.1 / 30.4, 256 x 5000
     // (128) 22.1 / 23.5 / 21.9; 4 heads of 256, 256 x 12000 (128) 27.6 / 29.7 / 26.6; not early / early: 400 x 3000 (96) 20.3 / 19.1; 16 heads
     // of 256, 128 x 2000 (64) 19.2 / 17.6.  (The first figure has ordinary launches on both sides.)
-    a.let_next = 3 * runs <= 2 * n_sm;
+    a.cut_lets_next = 3 * runs <= 2 * n_sm;
     DT_CUDA_TRY(launch_behind(kern, dim3(runs < n_sm ? runs : n_sm), dim3(kThreads), C::kSmemBytes, stream, 1, mq, mk, mv, mo, a));
     DT_CUDA_TRY(launch_behind(cut_combine_kernel<T, D>, dim3(plan.n_items * (kBM / 32), (p.D + 63) / 64), dim3(256), 0, stream, 1, a));
     return DT_OK;
@@ -1451,10 +1453,7 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
   const int ctas = a.n_items < n_sm ? a.n_items : n_sm;  // one persistent CTA per SM
   a.n_slots = plan.n_single > 0 ? plan.n_whole : (a.n_items + ctas - 1) / ctas * ctas;
   a.n_places = a.n_slots + plan.n_single;
-  // Calls of several rounds do not overlap their neighbours: 32 / 8 heads of 128 under an unaligned mask, 1001 tokens 47.4 -> 45.7 us
-  // with it, but 1501 tokens 62.1 -> 65.0 and 2047 tokens 76.5 -> 82.4.
-  a.let_next = a.n_items <= n_sm;
-  if (a.let_next) {
+  if (a.n_items <= n_sm) {
     DT_CUDA_TRY(launch_behind(kern, dim3(ctas), dim3(kThreads), C::kSmemBytes, stream, 1, mq, mk, mv, mo, a));
   } else {
     kern<<<ctas, kThreads, C::kSmemBytes, stream>>>(mq, mk, mv, mo, a);
