@@ -1364,10 +1364,12 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
   // columns, so P does not have to overwrite S: the next block's Q K^T is issued as soon as the first half of P says that S has been
   // read, and runs under the second half of the softmax, which used to wait for it (a quarter of a block's 3600 cycles).  2 images, 4096
   // tokens, heads of 64: 20 heads 290.2 -> 275.7 us, 10 heads 175.3 -> 163.1; 8 heads of 40: 124.3 -> 119.5; 300 tokens, 10 heads: 8.8 -> 8.3.
-  // Not where the second block is the last and holds 32 keys at most (two text prompts): its products are short, and every item has a
-  // hand-over more.  Over 48 calls of 777 to 9216 rows, 8 to 20 heads, 2 and 4 images, time without / with it, mean and worst: 154 keys
-  // 0.996 and 0.950 (4 images, 4641 rows, 10 heads: 37.5 / 39.5 us), 160 keys 0.995 and 0.946; 176 keys 1.019 and 0.989, 231 keys
-  // 1.019 and 0.976, 260 keys 1.015 and 1.003, 520 keys 1.033 and 1.017.  (The masked variant has not been built with it.)
+  // Not where the second block is the last and holds 32 keys at most (two text prompts), the call has several rounds and every head ends in a
+  // lone tile: nothing stands beside that tile's softmax, its products are short, and it has a hand-over more.  Time without / with
+  // it, mean and worst over 12 such calls (777 to 4641 rows, 8 to 20 heads, 2 and 4 images): 129 keys 0.985 and 0.955, 154 keys 0.982 and
+  // 0.950 (4 images, 4641 rows, 10 heads: 37.5 / 39.5 us), 160 keys 0.985 and 0.946; 176 keys 1.012 and 0.989, 260 keys 1.011 and 1.003, 520
+  // keys 1.037 and 1.026.  Pairs of tiles only (28 calls): 154 keys 0.999 and 0.991, 176 keys 1.023 and 1.010.  Nor for a single block, where
+  // nothing is ahead of anything: 100 keys, 48 calls, 0.993 and 0.975.  (The masked variant has not been built with it.)
   constexpr bool kMayAhead = D == 64 && !kMask;
   constexpr int kAheadKeys = kBN + 32;
   CUtensorMap mq, mk, mv, mo;
@@ -1447,7 +1449,9 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
   }
   auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, false, false>;
   if constexpr (kMayAhead) {
-    if ((p.seq_offsets_q != nullptr ? p.max_seq_k : p.Sk) > kAheadKeys) kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, false, true>;
+    const bool lone_ends = p.seq_offsets_q == nullptr && plan.item_rows > kBM && plan.n_items > n_sm && (p.Sq + kBM - 1) / kBM % 2 == 1;
+    const int keys = p.seq_offsets_q ? p.max_seq_k : p.Sk;
+    if (keys > (lone_ends ? kAheadKeys : kBN)) kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, false, true>;
   }
   DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
   const int ctas = a.n_items < n_sm ? a.n_items : n_sm;  // one persistent CTA per SM
