@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("causal,window", [(False, 0), (True, 0), (True, 200)])
 @pytest.mark.parametrize("D", [40, 64, 128, 256])
 @pytest.mark.parametrize("Sq,Sk", [(130, 640), (300, 1000),  # whole blocks; a last block of 104 keys
-                                   (300, 160), (300, 161)])  # either side of where the order of the products changes at head dim 64
+                                   (300, 160), (300, 161)])  # a second block of 32 and 33 keys
 def test_growing_maxima(dtattn, Sq, Sk, D, causal, window, dtype):
     q, k, v = inputs(1, Sq, Sk, 2, 1, D, dtype, 1701)
     # The queries' first dimension against a ramp in the keys' first dimension, one step per 64 keys: row i's scores rise by 2^17 from
@@ -47,3 +47,19 @@ def test_one_late_key_outweighs_all_others(dtattn, peak, D, dtype):
     torch.cuda.synchronize()
     assert dtattn.device_status() == 0
     check(out, ref.float(), dtype, f"peak {peak} D{D}")
+
+
+@pytest.mark.parametrize("D", [40, 64])
+@pytest.mark.parametrize("Sq,H", [(300, 80), (300, 60), (500, 80)])  # several rounds, every head ends in a lone tile; one round; pairs only
+@pytest.mark.parametrize("Sk", [97, 128, 129, 154, 160, 161])
+def test_where_the_order_of_the_products_changes(dtattn, Sk, Sq, H, D):
+    """Head dim 64: at one block, and in several rounds with lone last tiles at 160 keys.  Every third row's maximum lies in the second
+    block, or in the second half of the only one."""
+    q, k, v = inputs(1, Sq, Sk, H, H, D, torch.float16, 1721)
+    k[0, :, :, 0] = (torch.arange(Sk) >= min(128, Sk - 20)).half()[:, None]
+    q[0, :, :, 0] = (12.0 * D ** 0.5 * torch.tensor([1.0, -1.0, 0.0])[torch.arange(Sq) % 3]).half()[:, None]
+    ref = so.sdpa_explicit(q, k, v, D ** -0.5, False, compute_dtype=torch.float64)
+    out = dtattn.sdpa_forward(q.to(DEV), k.to(DEV), v.to(DEV), D ** -0.5)
+    torch.cuda.synchronize()
+    assert dtattn.device_status() == 0
+    check(out, ref.float(), torch.float16, f"{Sq}x{Sk} H{H} D{D}")
