@@ -154,7 +154,7 @@ out_proj_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
   } else if (warp == 1) {
     // =========================== MMA issuer ===========================
-    if (lane == 0) {
+    if (ptx::elect_one()) {  // (operands in uniform registers; 2 x 1024 tokens, 8 heads of 80 with attention: 29.3 -> 28.7 us)
       const uint64_t desc = ptx::make_smem_desc_sw128(0, 16, 1024);
       bool ok = true;
       int it = 0, n_tile = 0;

@@ -600,11 +600,14 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       }
     } else if (warp == 1) {
       // =========================== MMA issuer ===========================
-      // The whole warp walks the loop and one lane issues, which keeps the operands in uniform registers (joint attention of
-      // 4608 tokens 221 -> 217 us); the 64- and 256-wide variants, whose MMAs are fewer or longer, are 1 to 2 % faster with one
-      // lane walking it (2 x 4096 tokens, heads of 40: 123.2 against 125.1 us; 1777 x 5873, heads of 256: 126.3 against 127.2 us).
-      constexpr bool kWarpIssue = D == 128;
-      if (kWarpIssue || lane == 0) {
+      // The lane that issues is the elected one, which keeps the operands in uniform registers: behind "lane == 0" each MMA took at
+      // least 45 cycles to issue, where one of N = 64 with its rows in TMEM runs for 32 (one elected lane or the whole warp in step:
+      // 10).  Two text prompts of 77 tokens, 4 images of 9216 tokens, 20 heads of 64: 118.0 -> 108.5 us; 300 tokens, 10 heads 8.8 -> 8.6;
+      // window of 300, 5000 tokens, 16 / 4 heads 47.0 -> 44.4.  The whole warp walks the loop at head dims 64 and 128 (a window of 300,
+      // 2100 tokens, heads of 64: 19.7 us, one lane 20.2; 4096 tokens, 20 heads of 64: 273.6 and 277.3), one lane in cut calls of 64
+      // (8 heads, 128 x 16000: 25.6, the warp 26.4) and at 256, where the two are alike.
+      constexpr bool kWarpIssue = D == 128 || (D == 64 && !kCut);
+      if (kWarpIssue || ptx::elect_one()) {
         const bool on = kWarpIssue ? ptx::elect_one() : true;
         constexpr uint32_t idesc_qk = ptx::make_idesc_f16(kBf16, kBM, kBN, 0, 0);
         constexpr uint32_t idesc_pv = ptx::make_idesc_f16(kBf16, kBM, D, 0, 1);
