@@ -386,15 +386,15 @@ __device__ __forceinline__ float2 unpack_pair(uint32_t x) {
   else return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x));
 }
 
-// kAhead: see launch_t
-template <typename T, int D, bool kMask, bool kSplit, bool kCut, bool kAhead>
+// kLong: see launch_t
+template <typename T, int D, bool kMask, bool kSplit, bool kCut, bool kLong>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
                        const PrefillArgs a) {
   using C = Cfg<D, kMask>;
   constexpr int kBf16 = std::is_same<T, __half>::value ? 0 : 1;
-  static_assert(!kAhead || (D == 64 && !kMask), "columns for P beside S and O");
+  constexpr bool kAhead = kLong && D == 64 && !kMask;  // columns for P beside S and O: see launch_t
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -834,6 +834,10 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const int row = w.q0 + t * kBM + row_in_tile;
       const long long vis = a.is_causal ? (long long)row + w.off : (long long)w.sk;  // last visible key
       const long long lo = a.window > 0 ? (long long)row + w.off - a.window + 1 : 0;  // first visible key
+      // Blocks below j_seen lie wholly at or before this row's last key, those from j_near on wholly at or behind its first one: worked out
+      // once, and a block's test is two comparisons (kLong at head dim 64: 2 images, 4096 tokens, 20 heads 254.8 -> 251.0 us; 128 loses 1 % by it).
+      const int j_seen = (int)max(0LL, (min((long long)w.sk - 1, vis) + 1) / kBN - w.j0);
+      const int j_near = (int)max(0LL, (lo + kBN - 1) / kBN - w.j0);
       float m_used = -INFINITY, l = 0.f;
       // masked variant: this warp's row of patch flags (null when its 32 rows lie beyond Sq: nothing to add there)
       const unsigned char* patch_flags = nullptr;
@@ -980,9 +984,10 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 #endif
 
         const int key0 = (w.j0 + j) * kBN;
-        const bool need_mask = (key0 + kBN > w.sk) || (a.is_causal && (long long)(key0 + kBN - 1) > vis) || (long long)key0 < lo;
+        const bool need_mask = kLong && D == 64 ? j >= j_seen || j < j_near
+                                     : (key0 + kBN > w.sk) || (a.is_causal && (long long)(key0 + kBN - 1) > vis) || (long long)key0 < lo;
         // chunks of 32 keys that lie entirely beyond Sk are skipped (short K/V such as 77 text tokens)
-        const int nch = max(1, (min(kBN, w.sk - key0) + 31) >> 5);  // at least the chunk the MMA warp always reads
+        const int nch = kLong && j + 1 < w.nkv ? 4 : max(1, (min(kBN, w.sk - key0) + 31) >> 5);  // at least the chunk the MMA warp always reads
         if (need_mask) {
           // bounds relative to this block as 32-bit values, so that each element costs one compare against a
           // constant: columns hi_rel+1 .. 127 and 0 .. lo_rel-1 are hidden
@@ -1008,8 +1013,22 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           }
         }
         if (probe && j == 0) stamp(a, 16 * n_item + 12);
+        // kLong: whole blocks take a path without a branch per chunk of 32 keys, so that the chunks' instructions interleave; with the branches
+        // a chunk's chain of maxima ended before the next began (630 cycles of a warp's 2650 for a block, now 400).
+        auto block = [&](auto whole_block) -> bool {
+        constexpr bool kWhole = decltype(whole_block)::value;
         // row max: four independent chains of 3-input max (one per 32-column chunk)
         float mxc[4];
+        if constexpr (kWhole) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) mxc[c] = ptx::max3(__uint_as_float(s[c][0]), __uint_as_float(s[c][1]), __uint_as_float(s[c][2]));
+#pragma unroll
+          for (int i = 3; i < 31; i += 2)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) mxc[c] = ptx::max3(mxc[c], __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
+#pragma unroll
+          for (int c = 0; c < 4; ++c) mxc[c] = fmaxf(mxc[c], __uint_as_float(s[c][31]));
+        } else {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           if (c >= nch) {
@@ -1020,6 +1039,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 #pragma unroll
           for (int i = 3; i < 31; i += 2) mxc[c] = ptx::max3(mxc[c], __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
           mxc[c] = fmaxf(mxc[c], __uint_as_float(s[c][31]));
+        }
         }
         // (scale > 0 is a precondition of this kernel)
         float mx = kSplit ? fmaxf(fmaxf(mxc[0], mxc[1]) * half_scale[0], fmaxf(mxc[2], mxc[3]) * half_scale[1])
@@ -1038,10 +1058,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
               // With S double-buffered, or P not in its place, this block's scores arrive before the previous block's P V has run: O may only
               // be touched once that one has retired.  (It cannot be more than one phase behind: the P V of this block
               // waits for the P written below.)
-              if (!wait_pv(n_blocks)) {
-                ok = false;
-                break;
-              }
+              if (!wait_pv(n_blocks)) return false;
             }
 #pragma unroll
             for (int c = 0; c < D / 32; ++c) {
@@ -1064,7 +1081,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         for (int c = 0; c < 4; ++c) {
           const uint64_t scale2 = ptx::pack_f32x2(half_scale[c >> 1], half_scale[c >> 1]);
           lsum[c] = 0ull;
-          if (c < nch) {
+          if (kWhole || c < nch) {
           uint32_t rest[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
@@ -1094,7 +1111,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           if constexpr (kAhead) {
             // the previous block's last MMAs read these columns (the first half's are free: the commit that announced S stood behind
             // the MMAs that read them)
-            if (c == 2 && n_blocks > 0 && !wait_pv(n_blocks)) ok = false;
+            if (c == 2 && n_blocks > 0 && !wait_pv(n_blocks)) return false;
           }
           ptx::tmem_st16((kAhead ? t_p : t_s) + c * 16, s[c]);
           if constexpr (kSplit) ptx::tmem_st16(t_s + 64 + c * 16, rest);
@@ -1113,8 +1130,12 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           ptx::unpack_f32x2(ptx::add_f32x2(lsum[2], lsum[3]), b0, b1);
           l += (a0 + a1) + (b0 + b1);
         }
+        return true;
+        };
+        if constexpr (kLong) ok = nch == 4 ? block(std::true_type{}) : block(std::false_type{});
+        else ok = block(std::false_type{});
+        if (!ok) break;
         ++n_blocks;
-        if (kAhead && !ok) break;
       }
       if (!ok) break;
       if (probe) stamp(a, 16 * n_item + 9);
@@ -1373,7 +1394,12 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
   // 0.950 (4 images, 4641 rows, 10 heads: 37.5 / 39.5 us), 160 keys 0.985 and 0.946; 176 keys 1.012 and 0.989, 260 keys 1.011 and 1.003, 520
   // keys 1.037 and 1.026.  Pairs of tiles only (28 calls): 154 keys 0.999 and 0.991, 176 keys 1.023 and 1.010.  Nor for a single block, where
   // nothing is ahead of anything: 100 keys, 48 calls, 0.993 and 0.975.  (The masked variant has not been built with it.)
-  constexpr bool kMayAhead = D == 64 && !kMask;
+  // And for all widths: a softmax without branches inside whole blocks (kLong), where items have more than three blocks or end in more than 32
+  // keys.  us in a graph before / with it: joint attention, 4608 tokens, 24 heads of 128 229 / 216; 2 images, 4096 tokens, 20 heads of 64 275 /
+  // 255; 16384 x 512, 40 heads of 128 210 / 201; causal, 5000 tokens, 16 / 4 heads of 128 103.6 / 98.6, of 256 165.9 / 164.9; 4096 tokens
+  // under a padding mask 332 / 319.  Two paths in turn cost shorter items more: 4096 x 257, 40 heads of 128 44.9 / 45.6; 160 keys, 4 images
+  // of 4641 rows, 10 heads of 64 36.3 / 37.4; and masks with two parts per weight (kSplit), whose registers are full: 1501 tokens 107.8 / 110.3.
+  constexpr bool kMayLong = !kSplit;
   constexpr int kAheadKeys = kBN + 32;
   CUtensorMap mq, mk, mv, mo;
   if (!make_bshd_tensor_map(&mq, p.q, p.B, p.Sq, p.Hq, p.D, p.dtype, kBM)) return DT_UNSUPPORTED;
@@ -1438,7 +1464,7 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
       workspace_bytes >= align256(split_at) + split_bytes(plan, D)) {
     a.n_splits = plan.n_splits;
     a.part = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + align256(split_at));
-    auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, true, kMayAhead>;  // (its runs have at least four blocks)
+    auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, true, kMayLong>;  // (its runs have at least four blocks)
     DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
     const int runs = plan.n_items * plan.n_splits;
     // The kernel that adds the shares comes in early only where a third of the SMs has no run: otherwise its CTAs crowd onto the few that
@@ -1451,10 +1477,11 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
     return DT_OK;
   }
   auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, false, false>;
-  if constexpr (kMayAhead) {
+  if constexpr (kMayLong) {
     const bool lone_ends = p.seq_offsets_q == nullptr && plan.item_rows > kBM && plan.n_items > n_sm && (p.Sq + kBM - 1) / kBM % 2 == 1;
     const int keys = p.seq_offsets_q ? p.max_seq_k : p.Sk;
-    if (keys > (lone_ends ? kAheadKeys : kBN)) kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, false, true>;
+    const bool is_long = D == 64 && !kMask ? keys > (lone_ends ? kAheadKeys : kBN) : keys > 3 * kBN || (keys > kBN && (keys - 1) % kBN >= 32);
+    if (is_long) kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, false, true>;
   }
   DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
   const int ctas = a.n_items < n_sm ? a.n_items : n_sm;  // one persistent CTA per SM
