@@ -44,7 +44,9 @@ constexpr int kMaxExtraOutputs = 7;
 #endif
 constexpr int kPolyPeriod = DT_POLY_PERIOD;
 // 128 * kRegsLow + 256 * kRegsHigh must not exceed what the CTA was launched with (384 threads * 168)
-constexpr int kRegsLow = 80, kRegsHigh = 208;
+// (with 208 the softmax loop spilt up to 37 registers; joint attention 218.3 -> 216.1 us, 2 x 4096 tokens, 20 heads of 64 260.8 -> 254.6, chunk of
+// 1777 x 5873, heads of 256 133.4 -> 129.8)
+constexpr int kRegsLow = 56, kRegsHigh = 224;
 
 template <int D, bool kMask = false>
 struct Cfg {
@@ -835,7 +837,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const long long vis = a.is_causal ? (long long)row + w.off : (long long)w.sk;  // last visible key
       const long long lo = a.window > 0 ? (long long)row + w.off - a.window + 1 : 0;  // first visible key
       // Blocks below j_seen lie wholly at or before this row's last key, those from j_near on wholly at or behind its first one: worked out
-      // once, and a block's test is two comparisons (kLong at head dim 64: 2 images, 4096 tokens, 20 heads 254.8 -> 251.0 us; 128 loses 1 % by it).
+      // once, and a block's test is two comparisons (kLong; 2 images, 4096 tokens, 20 heads of 64 254.8 -> 251.0 us).
       const int j_seen = (int)max(0LL, (min((long long)w.sk - 1, vis) + 1) / kBN - w.j0);
       const int j_near = (int)max(0LL, (lo + kBN - 1) / kBN - w.j0);
       float m_used = -INFINITY, l = 0.f;
@@ -984,7 +986,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 #endif
 
         const int key0 = (w.j0 + j) * kBN;
-        const bool need_mask = kLong && D == 64 ? j >= j_seen || j < j_near
+        const bool need_mask = kLong ? j >= j_seen || j < j_near
                                      : (key0 + kBN > w.sk) || (a.is_causal && (long long)(key0 + kBN - 1) > vis) || (long long)key0 < lo;
         // chunks of 32 keys that lie entirely beyond Sk are skipped (short K/V such as 77 text tokens)
         const int nch = kLong && j + 1 < w.nkv ? 4 : max(1, (min(kBN, w.sk - key0) + 31) >> 5);  // at least the chunk the MMA warp always reads
@@ -1076,11 +1078,11 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         if (probe && j == 0) stamp(a, 16 * n_item + 13);
         const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
         const uint64_t neg_m2 = ptx::pack_f32x2(neg_m, neg_m);
-        uint64_t lsum[4];
+        uint64_t lsum[4][2];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const uint64_t scale2 = ptx::pack_f32x2(half_scale[c >> 1], half_scale[c >> 1]);
-          lsum[c] = 0ull;
+          lsum[c][0] = lsum[c][1] = 0ull;
           if (kWhole || c < nch) {
           uint32_t rest[16];
 #pragma unroll
@@ -1098,7 +1100,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
               p0 = fast_exp2(x0);
               p1 = fast_exp2(x1);
             }
-            lsum[c] = ptx::add_f32x2(lsum[c], ptx::pack_f32x2(p0, p1));
+            lsum[c][i & 1] = ptx::add_f32x2(lsum[c][i & 1], ptx::pack_f32x2(p0, p1));
             // the packed pair goes into the register score i of this chunk came in (scores 2i and 2i+1 are used up)
             if constexpr (kSplit) {  // weights of 16 bits and more: the rounded one and the rest of it
               const uint32_t hi = pack_pair<T>(p0, p1);
@@ -1126,8 +1128,10 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         }
         {
           float a0, a1, b0, b1;
-          ptx::unpack_f32x2(ptx::add_f32x2(lsum[0], lsum[1]), a0, a1);
-          ptx::unpack_f32x2(ptx::add_f32x2(lsum[2], lsum[3]), b0, b1);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) lsum[c][0] = ptx::add_f32x2(lsum[c][0], lsum[c][1]);
+          ptx::unpack_f32x2(ptx::add_f32x2(lsum[0][0], lsum[1][0]), a0, a1);
+          ptx::unpack_f32x2(ptx::add_f32x2(lsum[2][0], lsum[3][0]), b0, b1);
           l += (a0 + a1) + (b0 + b1);
         }
         return true;
