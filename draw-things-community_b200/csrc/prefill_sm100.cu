@@ -388,14 +388,15 @@ __device__ __forceinline__ float2 unpack_pair(uint32_t x) {
   else return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x));
 }
 
-// kLong: see launch_t
-template <typename T, int D, bool kMask, bool kSplit, bool kCut, bool kLong>
+// kForm: see launch_t
+template <typename T, int D, bool kMask, bool kSplit, bool kCut, int kForm>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
                        const PrefillArgs a) {
   using C = Cfg<D, kMask>;
   constexpr int kBf16 = std::is_same<T, __half>::value ? 0 : 1;
+  constexpr bool kLong = kForm > 0, kMayEarly = kForm > 1;
   constexpr bool kAhead = kLong && D == 64 && !kMask;  // columns for P beside S and O: see launch_t
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
@@ -990,16 +991,16 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                                      : (key0 + kBN > w.sk) || (a.is_causal && (long long)(key0 + kBN - 1) > vis) || (long long)key0 < lo;
         // chunks of 32 keys that lie entirely beyond Sk are skipped (short K/V such as 77 text tokens)
         const int nch = kLong && j + 1 < w.nkv ? 4 : max(1, (min(kBN, w.sk - key0) + 31) >> 5);  // at least the chunk the MMA warp always reads
-        if (need_mask) {
-          // bounds relative to this block as 32-bit values, so that each element costs one compare against a
-          // constant: columns hi_rel+1 .. 127 and 0 .. lo_rel-1 are hidden
+        // bounds relative to this block as 32-bit values, so that each element costs one compare against a
+        // constant: columns hi_rel+1 .. 127 and 0 .. lo_rel-1 are hidden
+        auto hide = [&](int c_begin, int c_end) {
           const long long lim = min((long long)w.sk - 1, vis);  // keys <= lim visible
           const int hi_rel = (int)max(-1LL, min(lim - key0, (long long)(kBN - 1)));
           const int lo_rel = (int)max(0LL, min(lo - key0, (long long)kBN));
           if (lo_rel == 0) {
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-              if (c >= nch || (c + 1) * 32 - 1 <= hi_rel) continue;  // chunk never read, or entirely visible
+              if (c < c_begin || c >= c_end || c >= nch || (c + 1) * 32 - 1 <= hi_rel) continue;  // chunk never read, or entirely visible
 #pragma unroll
               for (int i = 0; i < 32; ++i)
                 if (c * 32 + i > hi_rel) s[c][i] = 0xff800000u;  // -inf
@@ -1007,21 +1008,70 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           } else {
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-              if (c >= nch) continue;
+              if (c < c_begin || c >= c_end || c >= nch) continue;
 #pragma unroll
               for (int i = 0; i < 32; ++i)
                 if (c * 32 + i > hi_rel || c * 32 + i < lo_rel) s[c][i] = 0xff800000u;  // -inf
             }
           }
-        }
+        };
+        if (need_mask) hide(0, 4);
         if (probe && j == 0) stamp(a, 16 * n_item + 12);
         // kLong: whole blocks take a path without a branch per chunk of 32 keys, so that the chunks' instructions interleave; with the branches
         // a chunk's chain of maxima ended before the next began (630 cycles of a warp's 2650 for a block, now 400).
-        auto block = [&](auto whole_block) -> bool {
-        constexpr bool kWhole = decltype(whole_block)::value;
+        auto block = [&](auto path) -> bool {
+        constexpr bool kWhole = decltype(path)::value > 0, kEarly = decltype(path)::value > 1;
+        uint64_t lsum[4][2];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) lsum[c][0] = lsum[c][1] = 0ull;
+        uint32_t rest[16];  // (kSplit)
+        // p = exp2(s * scale_log2 - m) of scores 2i and 2i+1 of chunk c: packed fp32x2 multiply-add, packed row sums in two
+        // accumulators per chunk, packed conversion to the 16-bit P the second MMA reads from TMEM
+        auto weigh = [&](int c, int i, uint64_t scale2, uint64_t neg_m2) {
+          const uint64_t x2 = ptx::fma_f32x2(ptx::pack_f32x2(__uint_as_float(s[c][2 * i]), __uint_as_float(s[c][2 * i + 1])),
+                                             scale2, neg_m2);
+          float p0, p1;
+          if (DT_OPT(8)) {  // bring-up: no exponentials
+            ptx::unpack_f32x2(x2, p0, p1);
+          } else if ((i % kPolyPeriod) == kPolyPeriod - 1) {  // a share of the exponentials runs on the FMA pipes
+            ptx::exp2_poly_x2(x2, p0, p1);
+          } else {
+            float x0, x1;
+            ptx::unpack_f32x2(x2, x0, x1);
+            p0 = fast_exp2(x0);
+            p1 = fast_exp2(x1);
+          }
+          lsum[c][i & 1] = ptx::add_f32x2(lsum[c][i & 1], ptx::pack_f32x2(p0, p1));
+          // the packed pair goes into the register score i of this chunk came in (scores 2i and 2i+1 are used up)
+          if constexpr (kSplit) {  // weights of 16 bits and more: the rounded one and the rest of it
+            const uint32_t hi = pack_pair<T>(p0, p1);
+            const float2 f = unpack_pair<T>(hi);
+            s[c][i] = hi;
+            rest[i] = pack_pair<T>(p0 - f.x, p1 - f.y);
+          } else if constexpr (kBf16 != 0) ptx::cvt_pack_bf16_into(s[c][i], p0, p1);
+          else ptx::cvt_pack_f16_into(s[c][i], p0, p1);
+        };
         // row max: four independent chains of 3-input max (one per 32-column chunk)
         float mxc[4];
-        if constexpr (kWhole) {
+        if constexpr (kEarly) {
+          // Between blocks the reference maximum hardly ever moves, so the first half's exponentials (bound by the special-function unit) do
+          // not wait for the block's maximum, which is found beside them; where it does move they are taken again.  (2 x 4096 tokens, 20
+          // heads of 64 246.6 -> 236.4 us, 2304 tokens, 10 heads 57.4 -> 55.4.  At 128, where the products take twice as long, the two tiles' warps
+          // get in each other's way: joint attention 233 -> 237 us; at 256 119.5 -> 125.2 for a chunk of 1777 x 5873.)  Not for an item's first
+          // block, which has no maximum yet.
+          const uint64_t scale2 = ptx::pack_f32x2(sl2, sl2);
+          const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
+          const uint64_t neg_m2 = ptx::pack_f32x2(neg_m, neg_m);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) mxc[c] = -INFINITY;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) mxc[c] = ptx::max3(mxc[c], __uint_as_float(s[c][2 * i]), __uint_as_float(s[c][2 * i + 1]));
+            weigh(0, i, scale2, neg_m2);
+            weigh(1, i, scale2, neg_m2);
+          }
+        } else if constexpr (kWhole) {
 #pragma unroll
           for (int c = 0; c < 4; ++c) mxc[c] = ptx::max3(__uint_as_float(s[c][0]), __uint_as_float(s[c][1]), __uint_as_float(s[c][2]));
 #pragma unroll
@@ -1072,43 +1122,32 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
               ptx::tmem_st32(t_o + c * 32, ov);
             }
           }
+          if constexpr (kEarly) {
+            ptx::tmem_ld32(t_s + 0, s[0]);
+            ptx::tmem_ld32(t_s + 32, s[1]);
+            ptx::tc_wait_ld();
+            if (need_mask) hide(0, 2);
+            const uint64_t scale2 = ptx::pack_f32x2(sl2, sl2);
+            const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
+            const uint64_t neg_m2 = ptx::pack_f32x2(neg_m, neg_m);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+              lsum[c][0] = lsum[c][1] = 0ull;
+#pragma unroll
+              for (int i = 0; i < 16; ++i) weigh(c, i, scale2, neg_m2);
+            }
+          }
         }
-        // p = exp2(s * scale_log2 - m): packed fp32x2 multiply-add, packed row sums in four independent
-        // accumulators, packed conversion to the 16-bit P the second MMA reads from TMEM
         if (probe && j == 0) stamp(a, 16 * n_item + 13);
         const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
         const uint64_t neg_m2 = ptx::pack_f32x2(neg_m, neg_m);
-        uint64_t lsum[4][2];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const uint64_t scale2 = ptx::pack_f32x2(half_scale[c >> 1], half_scale[c >> 1]);
-          lsum[c][0] = lsum[c][1] = 0ull;
           if (kWhole || c < nch) {
-          uint32_t rest[16];
+          if (!kEarly || c > 1) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const uint64_t x2 = ptx::fma_f32x2(ptx::pack_f32x2(__uint_as_float(s[c][2 * i]), __uint_as_float(s[c][2 * i + 1])),
-                                               scale2, neg_m2);
-            float p0, p1;
-            if (DT_OPT(8)) {  // bring-up: no exponentials
-              ptx::unpack_f32x2(x2, p0, p1);
-            } else if ((i % kPolyPeriod) == kPolyPeriod - 1) {  // a share of the exponentials runs on the FMA pipes
-              ptx::exp2_poly_x2(x2, p0, p1);
-            } else {
-              float x0, x1;
-              ptx::unpack_f32x2(x2, x0, x1);
-              p0 = fast_exp2(x0);
-              p1 = fast_exp2(x1);
-            }
-            lsum[c][i & 1] = ptx::add_f32x2(lsum[c][i & 1], ptx::pack_f32x2(p0, p1));
-            // the packed pair goes into the register score i of this chunk came in (scores 2i and 2i+1 are used up)
-            if constexpr (kSplit) {  // weights of 16 bits and more: the rounded one and the rest of it
-              const uint32_t hi = pack_pair<T>(p0, p1);
-              const float2 f = unpack_pair<T>(hi);
-              s[c][i] = hi;
-              rest[i] = pack_pair<T>(p0 - f.x, p1 - f.y);
-            } else if constexpr (kBf16 != 0) ptx::cvt_pack_bf16_into(s[c][i], p0, p1);
-            else ptx::cvt_pack_f16_into(s[c][i], p0, p1);
+            for (int i = 0; i < 16; ++i) weigh(c, i, scale2, neg_m2);
           }
           if constexpr (kAhead) {
             // the previous block's last MMAs read these columns (the first half's are free: the commit that announced S stood behind
@@ -1136,8 +1175,9 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         }
         return true;
         };
-        if constexpr (kLong) ok = nch == 4 ? block(std::true_type{}) : block(std::false_type{});
-        else ok = block(std::false_type{});
+        if (kMayEarly && nch == 4 && j > 0) ok = block(std::integral_constant<int, kMayEarly ? 2 : 0>{});
+        else if (kLong && nch == 4) ok = block(std::integral_constant<int, kLong ? 1 : 0>{});
+        else ok = block(std::integral_constant<int, 0>{});
         if (!ok) break;
         ++n_blocks;
       }
@@ -1404,6 +1444,10 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
   // under a padding mask 332 / 319.  Two paths in turn cost shorter items more: 4096 x 257, 40 heads of 128 44.9 / 45.6; 160 keys, 4 images
   // of 4641 rows, 10 heads of 64 36.3 / 37.4; and masks with two parts per weight (kSplit), whose registers are full: 1501 tokens 107.8 / 110.3.
   constexpr bool kMayLong = !kSplit;
+  // At head dim 64 a third path (kMayEarly) for calls of eight blocks and more without a window; as code in the way of shorter ones and of
+  // windows, whose edges move the maximum, it costs (300 keys, 4 images of 9216 rows 74.7 / 76.5 us, 700 tokens causal 10.9 / 11.2, window of 300,
+  // 5000 tokens 42.6 / 47.6).
+  constexpr int kEarlyKeys = 1024;
   constexpr int kAheadKeys = kBN + 32;
   CUtensorMap mq, mk, mv, mo;
   if (!make_bshd_tensor_map(&mq, p.q, p.B, p.Sq, p.Hq, p.D, p.dtype, kBM)) return DT_UNSUPPORTED;
@@ -1468,7 +1512,7 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
       workspace_bytes >= align256(split_at) + split_bytes(plan, D)) {
     a.n_splits = plan.n_splits;
     a.part = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + align256(split_at));
-    auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, true, kMayLong>;  // (its runs have at least four blocks)
+    auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, true, kMayLong ? 1 : 0>;  // (its runs have at least four blocks)
     DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
     const int runs = plan.n_items * plan.n_splits;
     // The kernel that adds the shares comes in early only where a third of the SMs has no run: otherwise its CTAs crowd onto the few that
@@ -1480,12 +1524,15 @@ int launch_t(const dt_sdpa_params& p, cudaStream_t stream, void* const* extra, i
     DT_CUDA_TRY(launch_behind(cut_combine_kernel<T, D>, dim3(plan.n_items * (kBM / 32), (p.D + 63) / 64), dim3(256), 0, stream, 1, a));
     return DT_OK;
   }
-  auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, false, false>;
+  auto kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, false, 0>;
   if constexpr (kMayLong) {
     const bool lone_ends = p.seq_offsets_q == nullptr && plan.item_rows > kBM && plan.n_items > n_sm && (p.Sq + kBM - 1) / kBM % 2 == 1;
     const int keys = p.seq_offsets_q ? p.max_seq_k : p.Sk;
     const bool is_long = D == 64 && !kMask ? keys > (lone_ends ? kAheadKeys : kBN) : keys > 3 * kBN || (keys > kBN && (keys - 1) % kBN >= 32);
-    if (is_long) kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, false, true>;
+    if (is_long) kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, false, 1>;
+    if constexpr (D == 64 && !kMask) {
+      if (is_long && keys >= kEarlyKeys && p.sliding_window == 0) kern = prefill_tcgen05_kernel<T, D, kMask, kSplit, false, 2>;
+    }
   }
   DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
   const int ctas = a.n_items < n_sm ? a.n_items : n_sm;  // one persistent CTA per SM
