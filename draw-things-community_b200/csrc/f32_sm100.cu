@@ -28,7 +28,8 @@
 // of weights, the latency of the chain, and the call took 700 us).
 // Measured (SD1.5 upcast self-attention: 2 images, 4096 tokens, 8 heads of 40): 3309 us on the CUDA cores (fp32 multiply-
 // adds, 13 TFLOP/s), 299 us here in short bursts, 343 to 355 us one call after another for a second, when the power cap holds
-// the clock at 1.8 instead of 1.97 GHz; error against 64 bits 1.2e-6 there, 2.6e-7 here (2-norm, relative).
+// the clock at 1.8 instead of 1.97 GHz; error against 64 bits 1.2e-6 there, 2.6e-7 here (2-norm, relative).  Calls of that kind, more than one
+// round of tiles at head dims 33 to 64, now take two tiles to a CTA (f32_pair_sm100.cu: 241 us); the others stay here.
 // Per 128 x 128 scores at D = 40 the tensor pipe has 18 N=128 MMAs for Q K^T and 48 N=48 MMAs for P V.
 // Every mbarrier wait is bounded, as in the half-precision kernel.
 //

@@ -36,9 +36,10 @@ constexpr int kHalfBytes = 128 * 128;  // [128 rows][64 x 16-bit] = 16 KB, one T
 constexpr float kRescaleThreshold = 8.f;
 constexpr int kMaxExtraOutputs = 7;
 // every kPolyPeriod-th pair of exponentials is evaluated with the polynomial instead of MUFU.EX2 (1 of 16 pairs with
-// period 16).  The softmax warps are bound by the number of instructions they issue, not by the special-function unit
+// period 16), where fewer instructions have been worth more than relief of the special-function unit
 // (measured on B200, Flux shape, TFLOP/s: period 1 (all polynomial) 996, 2: 1066, 3: 1123, 4: 1140, 6: 1157, 8: 1149,
-// 16: 1160, none: 1147; with the softmax and the MMA warps free-running, never waiting for each other, the same order)
+// 16: 1160, none: 1147; with the softmax and the MMA warps free-running, never waiting for each other, the same order; since whole blocks
+// have a path without branches the joint attention takes 222.6 / 217.6 / 219.5 / 218.2 us with 4 / 8 / 16 / none)
 #ifndef DT_POLY_PERIOD
 #define DT_POLY_PERIOD 16
 #endif
