@@ -28,8 +28,7 @@
 // of weights, the latency of the chain, and the call took 700 us).
 // Measured (SD1.5 upcast self-attention: 2 images, 4096 tokens, 8 heads of 40): 3309 us on the CUDA cores (fp32 multiply-
 // adds, 13 TFLOP/s), 299 us here in short bursts, 343 to 355 us one call after another for a second, when the power cap holds
-// the clock at 1.8 instead of 1.97 GHz; error against 64 bits 1.2e-6 there, 2.6e-7 here (2-norm, relative).  Calls of that kind, more than one
-// round of tiles at head dims 33 to 64, now take two tiles to a CTA (f32_pair_sm100.cu: 241 us); the others stay here.
+// the clock at 1.8 instead of 1.97 GHz; error against 64 bits 1.2e-6 there, 2.6e-7 here (2-norm, relative).
 // Per 128 x 128 scores at D = 40 the tensor pipe has 18 N=128 MMAs for Q K^T and 48 N=48 MMAs for P V.
 // Every mbarrier wait is bounded, as in the half-precision kernel.
 //
@@ -37,7 +36,6 @@
 // range) or one below 2^-110 other than zero (its parts leave the bf16 range) are not for this kernel: split_planes_kernel reports them, f32_tcgen05_kernel then does nothing and the CUDA-core
 // kernel behind it in the stream, which otherwise returns at once, computes the call.
 #include "sm100_ptx.cuh"
-#include "f32_split.cuh"
 
 namespace dt {
 namespace {
@@ -85,7 +83,7 @@ struct F32Args {
   float* lse;
   int64_t o_sb, o_ss, o_sh;
   unsigned int* status;
-  const uint32_t* flags;  // [n_flags] non-zero: some input cannot be split, or f32_pair_kernel has computed the call
+  const uint32_t* flags;  // [kSplitCtas] non-zero: some input cannot be split
   uint32_t* any_flag;     // their union, written for the kernel behind this one
   int n_flags;
   int Sq, Sk, Hq, Hkv, D;
@@ -93,11 +91,61 @@ struct F32Args {
   float scale_log2;
 };
 
-// Bound: HBM / L2 writes (10 bytes moved per element in, 4 read and 6 written).  One 8-element piece per thread and step.
-__global__ void __launch_bounds__(kSplitThreads) split_planes_kernel(const F32SplitArgs a) {
+struct SplitTensor {
+  const float* src;
+  uint4* dst;  // [B, S, H, 3, D] bf16
+  int64_t sb, ss, sh;
+  int S, H;
+  unsigned begin, end;  // its 8-element pieces in the launch's numbering
+};
+struct SplitArgs {
+  SplitTensor t[3];
+  unsigned n_pieces;
+  int per_row;  // D / 8
+  uint32_t* flags;
+};
+
+// The bits of 2^58 (larger numbers, infinities and NaN all compare above them) and of 2^-110 (the last of a smaller number's
+// 24 bits is below the smallest bf16, 2^-133; zero is fine).
+__device__ __forceinline__ uint32_t out_of_range(float x) {
+  const uint32_t u = __float_as_uint(x) & 0x7fffffffu;
+  return u != 0u && u - 0x08800000u >= 0x5c800000u - 0x08800000u ? 1u : 0u;
+}
+
+// Bound: HBM / L2 writes (10 bytes moved per element in, 4 read and 6 written).  One 8-element piece per thread and step:
+// two 16-byte loads, three 16-byte stores.
+__global__ void __launch_bounds__(kSplitThreads) split_planes_kernel(const SplitArgs a) {
   ptx::wait_for_previous();
   ptx::let_next_start();
-  const int any = __syncthreads_or((int)f32_split_planes(a, blockIdx.x * kSplitThreads + threadIdx.x, gridDim.x * kSplitThreads));
+  uint32_t bad = 0;
+  for (unsigned g = blockIdx.x * kSplitThreads + threadIdx.x; g < a.n_pieces; g += gridDim.x * kSplitThreads) {
+    const SplitTensor& t = g < a.t[0].end ? a.t[0] : g < a.t[1].end ? a.t[1] : a.t[2];
+    const unsigned piece = g - t.begin;
+    const unsigned row = piece / a.per_row, ch = piece - row * a.per_row;
+    const unsigned tok = row / t.H, h = row - tok * t.H;
+    const unsigned b = tok / t.S, s = tok - b * t.S;
+    const float4* src = reinterpret_cast<const float4*>(t.src + b * t.sb + s * t.ss + h * t.sh + ch * 8);
+    const float4 lo = __ldg(src), hi = __ldg(src + 1);
+    const float x[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    uint32_t w[3][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float x0 = x[2 * i], x1 = x[2 * i + 1];
+      bad |= out_of_range(x0) | out_of_range(x1);
+      // x = a + r, r = b + t: a and b to the nearest bf16 (both differences are exact)
+      const uint32_t a0 = (__float_as_uint(x0) + 0x8000u) & 0xffff0000u, a1 = (__float_as_uint(x1) + 0x8000u) & 0xffff0000u;
+      const float r0 = x0 - __uint_as_float(a0), r1 = x1 - __uint_as_float(a1);
+      const uint32_t b0 = (__float_as_uint(r0) + 0x8000u) & 0xffff0000u, b1 = (__float_as_uint(r1) + 0x8000u) & 0xffff0000u;
+      const float t0 = r0 - __uint_as_float(b0), t1 = r1 - __uint_as_float(b1);
+      w[0][i] = __byte_perm(a0, a1, 0x7632);
+      w[1][i] = __byte_perm(b0, b1, 0x7632);
+      w[2][i] = __byte_perm(__float_as_uint(t0), __float_as_uint(t1), 0x7632);
+    }
+    uint4* dst = t.dst + (size_t)row * 3 * a.per_row + ch;
+#pragma unroll
+    for (int p = 0; p < 3; ++p) dst[p * a.per_row] = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+  }
+  const int any = __syncthreads_or((int)bad);
   if (threadIdx.x == 0) a.flags[blockIdx.x] = any ? 1u : 0u;
 }
 
@@ -470,15 +518,14 @@ int launch_t(const dt_sdpa_params& p, void* workspace, cudaStream_t stream) {
   a.status = device_status_word();
   if (!a.status) return DT_CUDA;
 
-  F32SplitArgs sp{};
+  SplitArgs sp{};
   sp.per_row = p.D / 8;
   sp.flags = flags;
   const dt_tensor4* src[3] = {&p.q, &p.k, &p.v};
   CUtensorMap maps[3];
-  F32PairScratch pair{};
   for (int i = 0; i < 3; ++i) {
     const int S = i ? p.Sk : p.Sq, H = i ? p.Hkv : p.Hq;
-    F32SplitTensor& t = sp.t[i];
+    SplitTensor& t = sp.t[i];
     t.src = static_cast<const float*>(src[i]->ptr);
     t.dst = reinterpret_cast<uint4*>(planes);
     t.sb = src[i]->stride_b; t.ss = src[i]->stride_s; t.sh = src[i]->stride_h;
@@ -489,7 +536,6 @@ int launch_t(const dt_sdpa_params& p, void* workspace, cudaStream_t stream) {
     // the planes as one more factor of the head axis: [B, S, 3 H, D]
     const dt_tensor4 view{planes, (int64_t)S * H * 3 * p.D, (int64_t)H * 3 * p.D, p.D};
     if (!make_bshd_tensor_map(&maps[i], view, p.B, S, 3 * H, p.D, DT_BF16, i ? C::kBN : kBM)) return DT_UNSUPPORTED;
-    pair.planes[i] = planes;
     planes += plane_bytes(p, S, H);
   }
   const unsigned need = (sp.n_pieces + kSplitThreads - 1) / kSplitThreads;
@@ -497,25 +543,6 @@ int launch_t(const dt_sdpa_params& p, void* workspace, cudaStream_t stream) {
   a.flags = flags;
   a.any_flag = flags + kSplitCtas;
   a.n_flags = (int)split_ctas;
-  const uint32_t* generic_if = a.any_flag;
-  const bool left_over = f32_pair_pays(p);  // this kernel then runs for what that one has left
-  if (left_over) {
-    const unsigned units = f32_pair_units(p);
-    pair.flags = flags;
-    pair.n_flags = (int)(units < (unsigned)kSplitCtas ? units : (unsigned)kSplitCtas);
-    pair.done = a.any_flag + 1;
-    pair.no_parts = a.any_flag + 2;
-    a.flags = pair.done;
-    a.n_flags = 1;
-    generic_if = pair.no_parts;
-    F32SplitArgs v = sp;  // V alone
-    v.t[0] = v.t[1] = v.t[2];
-    v.n_pieces -= v.t[2].begin;
-    for (F32SplitTensor& t : v.t) t.begin = 0, t.end = v.n_pieces;
-    pair.v_parts = &v;
-    const int st = launch_f32_pair(p, pair, stream);
-    if (st != DT_OK) return st;
-  }
   a.o = static_cast<float*>(p.o.ptr);
   a.lse = p.lse;
   a.o_sb = p.o.stride_b; a.o_ss = p.o.stride_s; a.o_sh = p.o.stride_h;
@@ -526,7 +553,7 @@ int launch_t(const dt_sdpa_params& p, void* workspace, cudaStream_t stream) {
   auto kern = f32_tcgen05_kernel<NPV>;
   DT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
   const int n_sm = device_sm_count();
-  if (!left_over) DT_CUDA_TRY(launch_behind(split_planes_kernel, dim3(split_ctas), dim3(kSplitThreads), 0, stream, 1, sp));
+  DT_CUDA_TRY(launch_behind(split_planes_kernel, dim3(split_ctas), dim3(kSplitThreads), 0, stream, 1, sp));
   // CTAs that come in while the splitting pass runs out land where there is room, not spread over the SM pairs and dies as those of an ordinary
   // launch are.  Long calls lose more by that than the hidden launch gives: those of several rounds, and those of one round that leaves
   // a tenth to half of the SMs empty.  Us in a graph, ordinary launches before and after / overlapped / this rule: 2 x 6144 tokens, 10 heads of
@@ -536,13 +563,13 @@ int launch_t(const dt_sdpa_params& p, void* workspace, cudaStream_t stream) {
   const bool uneven = a.n_items <= n_sm && 2 * a.n_items > n_sm && 10 * a.n_items <= 9 * n_sm && p.Sk > 1536;
   const bool rounds = a.n_items > n_sm && p.Sk > 2048;
   const int ctas = a.n_items < n_sm ? a.n_items : n_sm;
-  if (NPV == 80 || left_over || !(uneven || rounds)) {
+  if (NPV == 80 || !(uneven || rounds)) {
     DT_CUDA_TRY(launch_behind(kern, dim3(ctas), dim3(kThreads), C::kSmemBytes, stream, 1, maps[0], maps[1], maps[2], a));
   } else {
     kern<<<ctas, kThreads, C::kSmemBytes, stream>>>(maps[0], maps[1], maps[2], a);
     DT_CUDA_TRY(cudaGetLastError());
   }
-  return launch_generic(p, stream, generic_if);  // returns at once unless the inputs could not be split
+  return launch_generic(p, stream, a.any_flag);  // returns at once unless the inputs could not be split
 }
 
 }  // namespace

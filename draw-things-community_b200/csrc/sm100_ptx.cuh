@@ -425,10 +425,6 @@ __device__ __forceinline__ uint32_t cvt_pack_f16(float lo, float hi) {
   return d;
 }
 
-__device__ __forceinline__ void unpack_f16(uint32_t v, float& lo, float& hi) {
-  asm("{\n\t.reg .b16 a, b;\n\tmov.b32 {a, b}, %2;\n\tcvt.f32.f16 %0, a;\n\tcvt.f32.f16 %1, b;\n\t}" : "=f"(lo), "=f"(hi) : "r"(v));
-}
-
 // The same conversions writing INTO a register that already holds something else ("+r": input and output are one PTX
 // register).  The softmax uses it to put the packed P words into the registers the scores came in, a block of
 // consecutive registers that tcgen05.ld filled and tcgen05.st can read again without a register move per word.
