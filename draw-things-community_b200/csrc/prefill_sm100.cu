@@ -44,10 +44,6 @@ constexpr int kMaxExtraOutputs = 7;
 #define DT_POLY_PERIOD 16
 #endif
 constexpr int kPolyPeriod = DT_POLY_PERIOD;
-// 128 * kRegsLow + 256 * kRegsHigh must not exceed what the CTA was launched with (384 threads * 168)
-// (with 208 the softmax loop spilt up to 37 registers; joint attention 218.3 -> 216.1 us, 2 x 4096 tokens, 20 heads of 64 260.8 -> 254.6, chunk of
-// 1777 x 5873, heads of 256 133.4 -> 129.8)
-constexpr int kRegsLow = 56, kRegsHigh = 224;
 
 template <int D, bool kMask = false>
 struct Cfg {
@@ -58,6 +54,13 @@ struct Cfg {
   // work of a D = 128 tile under the same softmax, so one warpgroup keeps up).
   static constexpr int kTiles = D == 256 ? 1 : 2;
   static constexpr int kSoftmaxWarps = 4 * kTiles;
+  // Registers of a loading or issuing and of a softmax thread.  With 208 the softmax loop spilt up to 37 (80 / 208 -> 56 / 224: joint attention
+  // 218.3 -> 216.1 us, 2 x 4096 tokens, 20 heads of 64 260.8 -> 254.6).  With one tile warps 8 to 11 have nothing to do and need none of theirs: an
+  // issuer that walks its loop with one lane spills at 56 (96 to 192 bytes at head dim 256, 0 to 12 with 80; cut calls of 64 spill 64
+  // bytes, but with 72 / 216 they were 0.7 % slower), and the masked softmax still spilt at 224.  Before / now, us: chunk of 1777 x 5873
+  // 120.5 -> 117.6, 8192 tokens, 12 heads 631.6 -> 625.5, masks of 1501 and 2766 tokens, 16 / 8 heads 50.8 -> 49.1 and 117.9 -> 117.0.
+  static constexpr int kRegsLow = kTiles == 1 ? 80 : 56, kRegsHigh = kTiles == 1 ? 240 : 224, kRegsIdle = 24;
+  static_assert(128 * (kRegsLow + kTiles * kRegsHigh + (2 - kTiles) * kRegsIdle) <= kThreads * 168, "more registers than the CTA is launched with");
   static constexpr int kHalves = D / 64;
   static constexpr int kTileBytes = kHalves * kHalfBytes;  // one Q tile / one K block / one V block
   // the masked variant gives 32 KB of the K/V ring to the second mask staging buffers (D = 256: two 64 KB slots,
@@ -536,7 +539,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   // Register budget: the data-movement warpgroup gives registers back, the softmax warpgroups take them.
   // (Each setmaxnreg must dominate the code it governs, hence the nesting.)
   if (warp < 4) {
-    ptx::setmaxnreg_dec<kRegsLow>();
+    ptx::setmaxnreg_dec<C::kRegsLow>();
     if (warp == 0) {
       // =========================== TMA producer ===========================
       if (lane == 0) {
@@ -803,8 +806,10 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         }
       }
     }
+  } else if (C::kTiles == 1 && warp >= 8) {
+    ptx::setmaxnreg_dec<C::kRegsIdle>();  // (no second tile)
   } else {
-    ptx::setmaxnreg_inc<kRegsHigh>();
+    ptx::setmaxnreg_inc<C::kRegsHigh>();
     // =========================== softmax / correction / epilogue ===========================
     const int t = (warp - 4) >> 2;  // tile
     const int row_in_tile = ((warp & 3) << 5) + lane;
