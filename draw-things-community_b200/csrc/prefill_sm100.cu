@@ -8,7 +8,7 @@
 // One CTA = one (batch, head, pair of 128-row query tiles); at head dim 256 (AuraFlow.swift:358, Gemma3.swift:148,
 // Qwen3_5.swift:59-82) one tile, because TMEM holds S and O of only one.  12 warps:
 //   warp 0      TMA producer: Q tiles once, then K(j), V(j) blocks of 128 keys through a ring of slots
-//   warp 1      MMA issuer (one thread): S_t = Q_t K(j)^T  (operands in shared memory) and
+//   warp 1      MMA issuer (one elected lane): S_t = Q_t K(j)^T  (operands in shared memory) and
 //               O_t += P_t V(j) (P read from TMEM, V from shared memory), interleaved over the two tiles so
 //               that the tensor pipe works on one tile while the other tile's softmax runs
 //   warp 2      TMEM allocation / release
@@ -16,7 +16,7 @@
 //               max / sum, rescales O in TMEM only when the max grew by more than 2^8 (the final 1/l
 //               normalisation makes the result independent of that choice), writes P as 16-bit back to
 //               TMEM over the S columns, and at the end normalises O and stores it
-//   warps 8-11  the same for tile 1
+//   warps 8-11  the same for tile 1 (at head dim 256 nothing)
 // TMEM (512 columns x 128 lanes, fp32): S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [256+D,256+2D).
 // Every mbarrier wait is bounded; a wait that runs out stores a code into the device status word and the
 // CTA unwinds (TMEM is released on that path too).
